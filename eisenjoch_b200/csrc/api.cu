@@ -255,10 +255,12 @@ struct LegalSlot {
   DBuf<double> cost;
   DBuf<LegalOut> out;
   PinBuf<LegalOut> hout;
-  // round buffers of the parallel legaliser (legal_par.cu)
-  DBuf<uint64_t> fm;
-  DBuf<int32_t> list, len, info, hmark, dmark, pick;
-  DBuf<uint8_t> dist, fresh;
+  // working state of the parallel legaliser (legal_par.cu)
+  DBuf<int32_t> own, choice;
+  DBuf<uint2> seg;
+  DBuf<double> mcost;
+  DBuf<LpFreed> freed;
+  DBuf<unsigned long long> hint;
   DBuf<LpState> lst;
   LpGraph graph;        // the whole legalisation: rounds in a device-side loop
   uint64_t gen = ~0ull;  // problem load this slot is prepared for
@@ -1359,16 +1361,16 @@ void prepare_slot(eplace_ctx *c, LegalSlot &L) {
   L.loc.ensure((size_t)hp.N + hp.F + 1);
   L.cost.ensure(N1);
   const int WR = (hp.W + 63) / 64;
-  const size_t sites = (size_t)hp.W * hp.H;
-  L.fm.ensure((size_t)WR * hp.H);
-  L.list.ensure((size_t)kLpMaxWindow * kLpList);
-  L.len.ensure(kLpMaxWindow);
-  L.info.ensure(kLpMaxWindow);
-  L.pick.ensure(kLpMaxWindow);
-  L.dist.ensure(kLpMaxWindow);
-  L.fresh.ensure(kLpMaxWindow);
-  L.hmark.ensure(sites);
-  L.dmark.ensure(sites);
+  const int SW = (hp.W + 31) / 32;
+  uint32_t n_mac = 0;  // the order has the macros first
+  const std::vector<uint32_t> &order = c->lbase->order;
+  while (n_mac < order.size() && hp.cw[order[n_mac]] * hp.ch[order[n_mac]] > 1) ++n_mac;
+  L.own.ensure((size_t)32 * SW * hp.H);
+  L.seg.ensure((size_t)SW * hp.H);
+  L.choice.ensure(std::max<size_t>(n_mac, 1));
+  L.mcost.ensure(std::max<size_t>(n_mac, 1));
+  L.freed.ensure(2 * (size_t)kLpWindow);
+  L.hint.ensure(lp_hint_count(hp.W, hp.H));
   L.lst.ensure(1);
   std::vector<int2> floc(hp.F);
   for (uint32_t f = 0; f < hp.F; ++f) floc[f] = make_int2(hp.fx[f], hp.fy[f]);
@@ -1380,27 +1382,26 @@ void prepare_slot(eplace_ctx *c, LegalSlot &L) {
   a.pos = L.pos.p;
   a.order = c->lg_order.p;
   a.fsize = c->lg_macros ? c->lg_fsize.p : nullptr;
-  a.n = (uint32_t)c->lbase->order.size();
+  a.n = (uint32_t)order.size();
+  a.n_mac = n_mac;
   a.W = hp.W;
   a.H = hp.H;
   a.WR = WR;
+  a.SW = SW;
   a.free0 = c->lg_free0.p;
-  a.fm = L.fm.p;
-  a.list = L.list.p;
-  a.len = L.len.p;
-  a.info = L.info.p;
-  a.hmark = L.hmark.p;
-  a.dmark = L.dmark.p;
-  a.dist = L.dist.p;
-  a.fresh = L.fresh.p;
-  a.pick = L.pick.p;
+  a.own = L.own.p;
+  a.seg = L.seg.p;
+  a.choice = L.choice.p;
+  a.mcost = L.mcost.p;
+  a.freed = L.freed.p;
+  a.hint = L.hint.p;
   a.st = L.lst.p;
   a.sites = L.sites.p;
   a.loc = L.loc.p;
   a.cost = L.cost.p;
   a.disp = &L.out.p->disp;
   a.status = &L.out.p->status;
-  a.max_rounds = a.n + 64;
+  a.max_rounds = 2 * n_mac + 64;
   CK(lp_build_graph(a, L.graph, L.stream));
   L.gen = c->load_gen;
 }
@@ -2643,8 +2644,8 @@ uint64_t eplace_ctx::device_bytes() const {
   add(B3t_h); add(B3t_l); add(B5t_h); add(B5t_l); add(L4_h); add(L4_l); add(L6_h); add(L6_l);
   add(B3gt_h); add(B3gt_l); add(L6g_h); add(L6g_l); add(lg_order); add(lg_fsize); add(lg_free0);
   for (const auto &l : lslots) {
-    add(l->pos); add(l->sites); add(l->loc); add(l->cost); add(l->out); add(l->fm); add(l->list); add(l->len); add(l->info);
-    add(l->hmark); add(l->dmark); add(l->pick); add(l->dist); add(l->fresh); add(l->lst);
+    add(l->pos); add(l->sites); add(l->loc); add(l->cost); add(l->out); add(l->own); add(l->seg); add(l->choice);
+    add(l->mcost); add(l->freed); add(l->hint); add(l->lst);
   }
   return b;
 }

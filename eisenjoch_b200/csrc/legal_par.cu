@@ -4,32 +4,44 @@
 // the free anchor of minimum (bx - x)^2 + (by - y)^2 in FP64, ties to the
 // lowest tile.
 //
-// The greedy is sequential, but most of its work is not.  The cells are
-// placed in rounds; a round takes a window of the next cells in order and
-// the free map as it stands (every earlier cell committed):
-//  1. lists (one warp per cell): every free anchor whose cost is at most a
-//     threshold tau, sorted by (cost, tile), first kLpList kept.  Whatever
-//     the later cells of the window take, a cell's serial choice is the first
-//     entry of its list that no earlier window cell took -- the free set only
-//     shrinks and everything outside the list costs more.  If every entry is
-//     taken, the round ends before that cell.
-//  2. disturbance (a few parallel passes): a cell is disturbed when an
-//     earlier window cell's head (list entry 0) overlaps its head, or an
-//     earlier disturbed cell's list does.  An undisturbed cell's head can be
-//     taken by no earlier cell, so it is the serial choice.
-//  3. serial pass (one CTA, shared memory): undisturbed heads are entered as
-//     taken, then the disturbed cells, in order, take the first entry of
-//     their list not taken -- exactly the sequential algorithm restricted to
-//     the cells that need it.
-//  4. commit the window's prefix up to the first exhausted list; advance.
-// Rounds loop on the device (a CUDA-graph while node), no host round trip.
-// Each round commits at least one cell (the window's first cell has no
-// earlier cell to lose its head to) or stops on a cell with no free anchor,
-// and the loop also stops after max_rounds, so it always terminates.
+// The greedy is sequential as written, but its result does not need the
+// sequence.  own[s] holds the lowest order index that claims site s; a site
+// is open to cell q while own[s] > q (or own[s] == q, its own claim).
+//
+// Unit cells: the greedy is a serial dictatorship, which is the stable
+// matching in which every site prefers the lower order index, and a stable
+// matching with strict preferences is reached by deferred acceptance whatever
+// the order of the proposals.  A warp takes a cell q, finds the open site of
+// least (cost, tile) and claims it with atomicMin(own, q).  If the site was
+// held by a later cell, the warp goes on with the cell it displaced; if an
+// earlier cell got there first, it looks again.  own[s] only ever falls, so
+// a site once closed to q stays closed: no waiting, no rounds, and every
+// lost or won claim lowers some own[s], so it ends.
+//
+// Macros (several sites per claim, and a macro that moves opens sites again)
+// reach their fixed point in rounds over a window of the next kLpWindow
+// macros: each macro of the window takes the best anchor given the claims of
+// the earlier ones as they stand, if anything that could matter to it changed
+// in the last round (its block is under an earlier claim, or an earlier macro
+// gave up a block next to an anchor no worse than its own).  The macros
+// before the first one that changed in a round are final: each has the best
+// anchor given earlier ones that did not move.  The lowest macro of the window
+// does not change twice, so the window advances at least every second round.
+// 9,980 macros of a 200k-cell checkpoint take about 55 rounds.
+//
+// The displacement is the sequential FP64 sum of the costs, formed in
+// parallel: while the running total stays within one binade, adding a cost
+// adds a whole number of units in the last place that depends on the total
+// only through its lowest bit (round half to even), so the additions compose
+// as maps of that bit and are scanned.
+//
+// A 200k-cell checkpoint (5 % macros, half of the cells in six piles): 150 to
+// 200 ms as rounds of candidate lists, disturbance passes and one CTA's serial
+// pass over the cells whose lists interact (a hundred rounds and more of 20
+// launches), 11 ms in this form.
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <type_traits>
 
 #include "legal_par.cuh"
 
@@ -37,136 +49,704 @@ namespace eplace {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int32_t kNoMark = 0x7f7f7f7f;   // byte-fill value of the mark arrays
-constexpr int kListWarps = 8;             // warps per CTA of the list kernel
-constexpr int kCandBuf = 256;             // candidates a warp collects before sorting
-constexpr int kListMin = 24;              // threshold search aims at >= this many candidates
-constexpr int kSerialThreads = 1024;
-constexpr int kChunk = 64;                // disturbed cells staged per chunk
+constexpr int32_t kNone = 0x7fffffff;  // own[] of a site nobody claims
+constexpr int kInfHi = 0x7ff00000;     // high word of +infinity
+constexpr int kLpWarps = 8;            // warps per CTA of the macro kernels
 
 __device__ __forceinline__ double sq(double d) { return __dmul_rn(d, d); }
+
+// own[] and seg[] change under the readers: L2 loads, never kept in L1.
+__device__ __forceinline__ int32_t ld_own(const int32_t *p) {
+  int32_t v;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint2 ld_seg(const uint2 *p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return make_uint2((unsigned)v, (unsigned)(v >> 32));
+}
+// Bit b set: site b of the segment has a claim of q or later, or none; only
+// the groups of four sites with a bit in `ask` are looked at.
+__device__ __forceinline__ unsigned open_sites(const int32_t *own32, unsigned ask, int32_t q) {
+  unsigned m = 0;
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    if (!((ask >> (4 * u)) & 15u)) continue;
+    int4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.s32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(own32 + 4 * u)
+                 : "memory");
+    m |= ((v.x >= q ? 1u : 0u) | (v.y >= q ? 2u : 0u) | (v.z >= q ? 4u : 0u) | (v.w >= q ? 8u : 0u)) << (4 * u);
+  }
+  return m;
+}
+__device__ __forceinline__ int32_t *own_at(const LpArgs &a, int x, int y) {
+  return a.own + (size_t)y * (32 * a.SW) + x;
+}
+__device__ __forceinline__ uint2 *seg_at(const LpArgs &a, int x, int y) { return a.seg + (size_t)y * a.SW + (x >> 5); }
 
 struct Cell {
   double tx, ty;  // target (the continuous position)
   double ox, oy;  // anchor -> block centre offset, (w - 1) / 2
   int w, h;
   int AW, AH;     // anchor grid
+  int cx, cy;     // the anchor nearest to the target
+  int fx;         // the last anchor column at or left of the target, -1: none
+  bool inside;    // the target lies on the anchor grid
 };
 
-__device__ __forceinline__ Cell load_cell(const LpArgs &a, uint32_t cell) {
+__device__ __forceinline__ int nearest_in(double v, int n) {  // n >= 1
+  return (int)fmin(fmax(rint(v), 0.0), (double)(n - 1));
+}
+
+__device__ __forceinline__ Cell make_cell(const LpArgs &a, float2 p, uchar2 s) {
   Cell c;
-  const float2 p = a.pos[cell];
   c.tx = (double)p.x;
   c.ty = (double)p.y;
-  const uchar2 s = a.fsize ? a.fsize[cell] : make_uchar2(1, 1);
   c.w = s.x;
   c.h = s.y;
   c.ox = 0.5 * (double)(c.w - 1);
   c.oy = 0.5 * (double)(c.h - 1);
   c.AW = a.W - c.w + 1;
   c.AH = a.H - c.h + 1;
+  const double ux = __dsub_rn(c.tx, c.ox), uy = __dsub_rn(c.ty, c.oy);
+  c.cx = nearest_in(ux, c.AW);
+  c.cy = nearest_in(uy, c.AH);
+  c.fx = (int)fmin(fmax(floor(ux), -1.0), (double)(c.AW - 1));
+  c.inside = ux >= 0.0 && ux <= (double)(c.AW - 1) && uy >= 0.0 && uy <= (double)(c.AH - 1);
   return c;
+}
+__device__ __forceinline__ Cell load_cell(const LpArgs &a, uint32_t q, bool unit) {
+  const uint32_t cell = a.order[q];
+  return make_cell(a, a.pos[cell], unit ? make_uchar2(1, 1) : a.fsize[cell]);
+}
+
+// A cell with no finite target has no site of least cost.
+__device__ __forceinline__ bool placeable(const Cell &c) {
+  return isfinite(c.tx) && isfinite(c.ty) && c.AW > 0 && c.AH > 0;
 }
 
 // Cost of anchor (ax, ay), formed as the host legaliser forms it.
-__device__ __forceinline__ double anchor_cost(const Cell &c, int ax, double dy2) {
-  const double dx = __dsub_rn(__dadd_rn((double)ax, c.ox), c.tx);
-  return __dadd_rn(sq(dx), dy2);
+__device__ __forceinline__ double axis2(double at, double off, double target) {
+  return sq(__dsub_rn(__dadd_rn(at, off), target));
 }
-__device__ __forceinline__ double row_dy2(const Cell &c, int ay) {
-  return sq(__dsub_rn(__dadd_rn((double)ay, c.oy), c.ty));
-}
+__device__ __forceinline__ double col_dx2(const Cell &c, int ax) { return axis2((double)ax, c.ox, c.tx); }
+__device__ __forceinline__ double row_dy2(const Cell &c, int ay) { return axis2((double)ay, c.oy, c.ty); }
 
-// Word j of anchor row ay: bit b set when the w x h block at anchor
-// (64 j + b, ay) is free.  Anchors past AW - 1 are never valid.
-__device__ __forceinline__ uint64_t valid_word(const LpArgs &a, const Cell &c, int ay, int j) {
-  const int lastw = (c.AW - 1) >> 6;
-  if (j > lastw) return 0ull;
-  uint64_t m = ~0ull, mn = ~0ull;
-  for (int dy = 0; dy < c.h; ++dy) {
-    const uint64_t *r = a.fm + (size_t)(ay + dy) * a.WR;
-    m &= __ldg(reinterpret_cast<const unsigned long long *>(r + j));
-    if (c.w > 1) mn &= (j + 1 < a.WR) ? __ldg(reinterpret_cast<const unsigned long long *>(r + j + 1)) : 0ull;
-  }
-  uint64_t v = m;
-  for (int k = 1; k < c.w; ++k) v &= (m >> k) | (mn << (64 - k));
-  if (j == lastw && ((c.AW - 1) & 63) != 63) v &= (2ull << ((c.AW - 1) & 63)) - 1;
-  return v;
-}
-
-struct Cand {
-  unsigned long long key;  // cost bits (costs are >= 0, so the bits order like the values)
+// The least (cost, tile) seen; tile kNone: none.  Costs are >= 0, so the
+// words of a cost order like the cost.
+struct Best {
+  double cost;
   int tile;
-  int pad_;
+  __device__ __forceinline__ void take(double c, int t) {
+    if (c < cost || (c == cost && t < tile)) {
+      cost = c;
+      tile = t;
+    }
+  }
+  __device__ __forceinline__ Best warp_min() const {
+    const unsigned hi = (unsigned)__double2hiint(cost), lo = (unsigned)__double2loint(cost);
+    const unsigned mh = __reduce_min_sync(kFull, hi);
+    const unsigned ml = __reduce_min_sync(kFull, hi == mh ? lo : ~0u);
+    const int t = (int)__reduce_min_sync(kFull, (unsigned)(hi == mh && lo == ml ? tile : kNone));
+    return Best{__hiloint2double((int)mh, (int)ml), t};
+  }
 };
+// High word of a cost; a larger word means a larger cost.
+__device__ __forceinline__ unsigned hi(double cost) { return (unsigned)__double2hiint(cost); }
+__device__ __forceinline__ Best no_best() { return Best{__hiloint2double(kInfHi, 0), kNone}; }
 
-__device__ __forceinline__ bool cand_less(const Cand &x, const Cand &y) {
-  return x.key < y.key || (x.key == y.key && x.tile < y.tile);
+// Hints.  When cell k has its place, every anchor cheaper than its own was
+// closed to it, and what is closed to k is closed to every later cell of the
+// same or a larger footprint.  Entry (size class, 16 x 16 sites) keeps the
+// largest such radius seen from the middle of those sites, with its k: a
+// later cell with a target near by starts its search on that circle instead
+// of at its target.  A pile of some hundred sites is walked through once for
+// each 16 x 16 of targets instead of once for each cell.
+__device__ __forceinline__ float2 hint_middle(int cx, int cy) {
+  return make_float2((float)((cx & ~15) + 8), (float)((cy & ~15) + 8));
+}
+__device__ __forceinline__ float hint_dist(const Cell &c) {  // target to the middle, rounding allowed for
+  const float2 m = hint_middle(c.cx, c.cy);
+  const float dx = (float)(c.tx - c.ox) - m.x, dy = (float)(c.ty - c.oy) - m.y;
+  return sqrtf(dx * dx + dy * dy) + 0.01f;
+}
+__device__ __forceinline__ unsigned long long *hint_at(const LpArgs &a, const Cell &c, int size) {
+  const size_t tw = (a.W + 15) / 16, tiles = tw * ((a.H + 15) / 16);
+  return a.hint + (size - 1) * tiles + (c.cy >> 4) * tw + (c.cx >> 4);
+}
+__device__ __forceinline__ void put_hint(const LpArgs &a, int32_t q, const Cell &c, double cost) {
+  const int size = max(c.w, c.h);
+  if (!c.inside || size > kLpHintClasses || !(cost > 64.0)) return;
+  const float r = sqrtf((float)cost) * 0.9999f - hint_dist(c);
+  if (r > 4.0f) atomicMax(hint_at(a, c, size), ((unsigned long long)__float_as_uint(r) << 32) | (unsigned)q);
+}
+// A cost below which no anchor is open to q.
+__device__ __forceinline__ double get_hint(const LpArgs &a, int32_t q, const Cell &c) {
+  if (!c.inside) return 0.0;
+  float r = 0.0f;
+  for (int size = min(min(c.w, c.h), kLpHintClasses); size >= 1; --size) {
+    const unsigned long long e = __ldcg(hint_at(a, c, size));
+    if ((int32_t)(unsigned)e < q) r = fmaxf(r, __uint_as_float((unsigned)(e >> 32)));
+  }
+  r = (r - hint_dist(c)) * 0.9999f;
+  return r > 0.0f ? (double)r * (double)r : 0.0;
 }
 
-// Visits the valid anchors of cell c with cost <= tau.  Without buf it
-// returns their number (warp-uniform); with buf it appends them (at most
-// cap) and returns the number found.
-__device__ int scan_tau(const LpArgs &a, const Cell &c, double tau, int lane, Cand *buf, int cap, int *nbuf) {
-  const double r = sqrt(tau);
-  const double uy = __dsub_rn(c.ty, c.oy), ux = __dsub_rn(c.tx, c.ox);
-  const int ay0 = max(0, (int)floor(uy - r) - 1);
-  const int ay1 = min(c.AH - 1, (int)ceil(uy + r) + 1);
-  int found = 0;
-  for (int ay = ay0 + lane; ay <= ay1; ay += 32) {
-    const double dy2 = row_dy2(c, ay);
-    if (dy2 > tau) continue;
-    const double hx = sqrt(__dsub_rn(tau, dy2));
-    // approximate bounds, then exact ones: within a row the anchors with
-    // cost <= tau form an interval (the cost is convex in ax)
-    // (each loop moves one bound monotonically inside [0, AW - 1], so all
-    // four end; the estimate is off by at most a step or two)
-    int lo = max(0, (int)ceil(ux - hx)), hi = min(c.AW - 1, (int)floor(ux + hx));
-    while (lo > 0 && anchor_cost(c, lo - 1, dy2) <= tau) --lo;
-    while (lo <= hi && anchor_cost(c, lo, dy2) > tau) ++lo;
-    while (hi < c.AW - 1 && anchor_cost(c, hi + 1, dy2) <= tau) ++hi;
-    while (hi >= lo && anchor_cost(c, hi, dy2) > tau) --hi;
-    if (lo > hi) continue;
-    const int j0 = lo >> 6, j1 = hi >> 6;
-    for (int j = j0; j <= j1; ++j) {
-      uint64_t v = valid_word(a, c, ay, j);
-      if (j == j0) v &= ~0ull << (lo & 63);
-      if (j == j1 && (hi & 63) != 63) v &= (2ull << (hi & 63)) - 1;
-      if (!buf) {
-        found += __popcll(v);
-        continue;
+// ---------------------------------------------------------------------------
+// Macros
+// ---------------------------------------------------------------------------
+
+// seg[] while the macros are placed: x has a bit for each site without a
+// final claim (of a macro before the window, or a fixed cell), y for each site
+// with a claim of the window.  Sites with both bits are open to some macros of
+// the window only; their own[] tells.
+__device__ __forceinline__ unsigned open_word(const LpArgs &a, int32_t q, int y, int g, uint2 s) {
+  const unsigned ask = s.x & s.y;
+  return ask ? (s.x & (~s.y | open_sites(own_at(a, 32 * g, y), ask, q))) : s.x;
+}
+
+// The open anchor of least (cost, tile) for macro q of at most 32 x 16 sites,
+// none of cost below c0 being open: bands of 33 - h anchor rows outward from
+// the target, a lane per site row, in a band the segments outward from the
+// target (from the circle of cost c0), each tested as bit words (a run of w
+// open sites along the row, then h such rows), stopped by the least cost so
+// far, which the CTA's warps share through *least; the warps take the bands in
+// turn.  Latency bound (a word per lane and segment from L2, four segments in
+// flight).
+__device__ Best search_block(const LpArgs &a, int32_t q, const Cell &c, double c0, int warp, int lane,
+                             unsigned *least) {
+  Best b = no_best();
+  unsigned bhi = kInfHi;  // high word of the least cost so far
+  const int nb = 33 - c.h;
+  // anchors of segment g whose block is open: wc, wn the words of segments g, g + 1
+  auto eval = [&](int g, int a0, unsigned wc, unsigned wn) {
+    if (!__any_sync(kFull, wc != 0)) return;
+    uint64_t t = (uint64_t)wc | ((uint64_t)wn << 32);
+    for (int s = 1; s < c.w;) {
+      const int d = min(s, c.w - s);
+      t &= t >> d;
+      s += d;
+    }
+    unsigned v = (unsigned)t;
+    for (int s = 1; s < c.h;) {
+      const int d = min(s, c.h - s);
+      v &= __shfl_down_sync(kFull, v, d);
+      s += d;
+    }
+    if (lane >= nb) v = 0;  // its rows below the band are not here
+    if (v) {
+      const int ay = a0 + lane, f = c.fx - 32 * g;
+      // (split at the target, not at the nearest column: two columns half a
+      // site away on either side are a tie for the lower one)
+      const double dy2 = row_dy2(c, ay);
+      const unsigned left = f < 0 ? 0u : (f >= 31 ? ~0u : (2u << f) - 1u);
+      const unsigned vl = v & left, vr = v & ~left;
+      if (vl) {
+        const int ax = 32 * g + 31 - __clz(vl);
+        b.take(__dadd_rn(col_dx2(c, ax), dy2), ay * a.W + ax);
       }
-      while (v) {
-        const int ax = (j << 6) + __ffsll(v) - 1;
-        v &= v - 1;
-        const double cost = anchor_cost(c, ax, dy2);
-        if (cost > tau) continue;  // never: the interval is exact
-        const int slot = atomicAdd(nbuf, 1);
-        if (slot < cap) {
-          buf[slot].key = (unsigned long long)__double_as_longlong(cost);
-          buf[slot].tile = ay * a.W + ax;
+      if (vr) {
+        const int ax = 32 * g + __ffs(vr) - 1;
+        b.take(__dadd_rn(col_dx2(c, ax), dy2), ay * a.W + ax);
+      }
+    }
+    bhi = __reduce_min_sync(kFull, (unsigned)__double2hiint(b.cost));
+    if (lane == 0) bhi = min(atomicMin(least, bhi), bhi);
+    bhi = __shfl_sync(kFull, bhi, 0);
+  };
+  const int base0 = c.cy - nb / 2;
+  for (int k = 0;; ++k) {
+    bool any = false;
+    for (int side = 0; side < (k ? 2 : 1); ++side) {
+      const int a0 = base0 + (side ? -k * nb : k * nb);
+      const int r0 = max(a0, 0), r1 = min(a0 + nb, c.AH) - 1;
+      if (r0 > r1) continue;
+      const double dmin = row_dy2(c, min(max(c.cy, r0), r1));
+      if (hi(dmin) > bhi) continue;
+      any = true;
+      if ((2 * k + side) % kLpWarps != warp) continue;  // another warp's band
+      bhi = min(bhi, *(volatile unsigned *)least);
+      const int y = a0 + lane;
+      const bool row = y >= 0 && y < a.H;
+      auto raw = [&](int g) {
+        return row && g >= 0 && g < a.SW ? ld_seg(a.seg + (size_t)y * a.SW + g) : make_uint2(0u, 0u);
+      };
+      // Columns nearer than `skip` cost less than c0 in every row of the band.
+      const double far = fmax(row_dy2(c, r0), row_dy2(c, r1));
+      const int skip = c0 > far ? max((int)sqrtf((float)__dsub_rn(c0, far)) - 2, 0) : 0;
+      const int gr = min(max(c.fx + skip, 0), c.AW - 1) >> 5, gl = max(c.fx - skip, 0) >> 5;
+      uint2 p[5];
+#pragma unroll
+      for (int u = 0; u < 5; ++u) p[u] = raw(gr + u);
+      unsigned cur = open_word(a, q, y, gr, p[0]);
+      const unsigned w0 = cur;
+      for (int g = gr;; g += 4) {
+        bool done = false;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int at = g + u;
+          if (!done && (32 * at >= c.AW ||
+                        (at > gr && hi(__dadd_rn(col_dx2(c, 32 * at), dmin)) > bhi)))
+            done = true;
+          if (!done) {
+            const unsigned nxt = open_word(a, q, y, at + 1, p[u + 1]);
+            eval(at, a0, cur, nxt);
+            cur = nxt;
+          }
         }
-        ++found;
+        if (done) break;
+#pragma unroll
+        for (int u = 1; u < 5; ++u) p[u] = raw(g + 4 + u);
+      }
+      unsigned nxt = gl == gr ? w0 : open_word(a, q, y, gl + 1, raw(gl + 1));
+      for (int g = gl == gr ? gl - 1 : gl; g >= 0; g -= 4) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) p[u] = raw(g - u);
+        bool done = false;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int at = g - u;
+          if (!done && (at < 0 || (at < (c.cx >> 5) &&
+                                   hi(__dadd_rn(col_dx2(c, 32 * at + 31), dmin)) > bhi)))
+            done = true;
+          if (!done) {
+            cur = open_word(a, q, y, at, p[u]);
+            eval(at, a0, cur, nxt);
+            nxt = cur;
+          }
+        }
+        if (done) break;
+      }
+    }
+    if (!any) break;  // outside the chip or too far on both sides, and the next bands too
+  }
+  return b;  // this lane's
+}
+
+// The same for any footprint (wider or higher ones): a lane per anchor.
+__device__ Best search_any(const LpArgs &a, int32_t q, const Cell &c, int lane) {
+  Best b = no_best();
+  int bhi = kInfHi;
+  const int gc = c.cx >> 5;
+  for (int k = 0;; ++k) {
+    bool any = false;
+    for (int side = 0; side < (k ? 2 : 1); ++side) {
+      const int ay = c.cy + (side ? -k : k);
+      if (ay < 0 || ay >= c.AH) continue;
+      const double dy2 = row_dy2(c, ay);
+      if (__double2hiint(dy2) > bhi) continue;
+      any = true;
+      for (int dir = 0; dir < 2; ++dir)
+        for (int g = dir ? gc - 1 : gc; g >= 0 && 32 * g < c.AW; g += dir ? -1 : 1) {
+          if (g != gc && __double2hiint(__dadd_rn(col_dx2(c, dir ? 32 * g + 31 : 32 * g), dy2)) > bhi) break;
+          const int ax = 32 * g + lane;
+          if (ax < c.AW) {
+            bool open = true;
+            for (int s = 0; s < c.w * c.h && open; ++s)
+              open = ld_own(own_at(a, ax + s % c.w, ay + s / c.w)) >= q;
+            if (open) b.take(__dadd_rn(col_dx2(c, ax), dy2), ay * a.W + ax);
+          }
+          bhi = (int)__reduce_min_sync(kFull, (unsigned)__double2hiint(b.cost));
+        }
+    }
+    if (!any) break;
+  }
+  return b.warp_min();
+}
+
+__global__ void __launch_bounds__(256) k_lp_init(const LpArgs a) {
+  const int lane = threadIdx.x & 31;
+  const int nseg = a.SW * a.H;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nseg; i += (gridDim.x * blockDim.x) >> 5) {
+    const int y = i / a.SW, x = 32 * (i - y * a.SW) + lane;
+    const bool open = x < a.W && ((a.free0[(size_t)y * a.WR + (x >> 6)] >> (x & 63)) & 1u);
+    *own_at(a, x, y) = open ? kNone : -1;
+    const unsigned m = __ballot_sync(kFull, open);
+    if (lane == 0) a.seg[i] = make_uint2(m, 0u);
+  }
+  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < a.n_mac; q += gridDim.x * blockDim.x) a.choice[q] = -1;
+  const uint32_t hints = kLpHintClasses * (uint32_t)((a.W + 15) / 16) * (uint32_t)((a.H + 15) / 16);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < hints; i += gridDim.x * blockDim.x) a.hint[i] = 0ull;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.st = LpState{0u, 0u, (uint32_t)kNone, 0u, {0u, 0u}, 0, 0u};
+}
+
+// A round, first half: each macro of the window whose choice may have become
+// wrong chooses again; the blocks given up are entered in this round's list
+// and leave own[].  (A macro that reads own[] while another leaves it sees
+// some sites of the old block open and some not; the block is in the list, so
+// it is looked at again in the next round if that could matter to it.)
+// A CTA per macro: a round lasts as long as its longest search, and only some
+// of the window's macros search at all.
+__global__ void __launch_bounds__(kLpWarps * 32) k_lp_choose(const LpArgs a) {
+  __shared__ Best sbest[kLpWarps];
+  __shared__ unsigned least;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  LpState *st = a.st;
+  const uint32_t base = st->base, par = st->rounds & 1u;
+  const uint32_t qi = base + blockIdx.x;
+  if (qi >= a.n_mac) return;
+  const int32_t q = (int32_t)qi;
+  const Cell c = load_cell(a, qi, false);
+  const int32_t old = a.choice[q];
+  const int oldx = old % a.W, oldy = old / a.W;
+  double c0 = 0.0;  // no anchor of a lower cost is open
+  if (tid == 0) least = kInfHi;
+  if (old != -1) {
+    bool lost = false, freed = false;
+    if (old >= 0)
+      for (int s = tid; s < c.w * c.h; s += kLpWarps * 32)
+        lost |= ld_own(own_at(a, oldx + s % c.w, oldy + s / c.w)) < q;
+    const double mine = old >= 0 ? a.mcost[q] : __hiloint2double(kInfHi, 0);
+    const uint32_t nf = st->nfreed[par];
+    for (uint32_t e = tid; e < nf; e += kLpWarps * 32) {
+      const LpFreed f = a.freed[par * kLpWindow + e];
+      if (f.q >= q) continue;
+      // the least cost of an anchor whose block meets the freed one
+      const int fx = f.tile % a.W, fy = f.tile / a.W;
+      const int x0 = max(fx - c.w + 1, 0), x1 = min(fx + f.w - 1, c.AW - 1);
+      const int y0 = max(fy - c.h + 1, 0), y1 = min(fy + f.h - 1, c.AH - 1);
+      if (x0 > x1 || y0 > y1) continue;
+      freed |= __dadd_rn(col_dx2(c, min(max(c.cx, x0), x1)), row_dy2(c, min(max(c.cy, y0), y1))) <= mine;
+    }
+    lost = __syncthreads_or(lost);
+    freed = __syncthreads_or(freed);
+    if (!lost && !freed) return;
+    if (!freed && old >= 0 && c.inside) c0 = mine;
+  }
+  c0 = fmax(c0, get_hint(a, q, c));
+  __syncthreads();  // least
+  Best b = no_best();
+  if (placeable(c)) {
+    if (c.w <= 32 && c.h <= 16) b = search_block(a, q, c, c0, warp, lane, &least);
+    else if (warp == 0) b = search_any(a, q, c, lane);
+  }
+  b = b.warp_min();
+  if (lane == 0) sbest[warp] = b;
+  __syncthreads();
+  if (warp != 0) return;
+  b = (lane < kLpWarps ? sbest[lane] : no_best()).warp_min();
+  const int32_t now = b.tile == kNone ? -2 : b.tile;
+  if (now == old) return;
+  if (old >= 0) {
+    for (int s = lane; s < c.w * c.h; s += 32) {
+      const int x = oldx + s % c.w, y = oldy + s / c.w;
+      int32_t *o = own_at(a, x, y);
+      if (ld_own(o) == q) {  // nobody else writes a site that q holds
+        *o = kNone;
+        atomicAnd(&seg_at(a, x, y)->y, ~(1u << (x & 31)));
       }
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) found += __shfl_xor_sync(kFull, found, o);
-  return found;
+  if (lane == 0) {
+    atomicMin(&st->first, qi);
+    if (old >= 0) a.freed[(par ^ 1u) * kLpWindow + atomicAdd(&st->nfreed[par ^ 1u], 1u)] = LpFreed{q, old, c.w, c.h};
+    a.choice[q] = now;
+    a.mcost[q] = b.cost;
+  }
 }
 
-// Bitonic sort of buf[0..n2) (n2 a power of two, >= 32) by one warp.
-__device__ void warp_sort(Cand *buf, int n2, int lane) {
-  for (int k = 2; k <= n2; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = lane; i < n2; i += 32) {
-        const int p = i ^ j;
-        if (p > i) {
-          const bool up = (i & k) == 0;
-          Cand x = buf[i], y = buf[p];
-          if (cand_less(y, x) == up) {
-            buf[i] = y;
-            buf[p] = x;
+// Second half: every macro of the window enters its claim again (a macro that
+// left may have covered a later one's), and the last CTA moves the window to
+// the first macro that changed.
+__global__ void __launch_bounds__(kLpWarps * 32) k_lp_claim(const LpArgs a) {
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31;
+  LpState *st = a.st;
+  const uint32_t base = st->base, end = min(base + kLpWindow, a.n_mac);
+  const uint32_t stop = min(__ldcg(&st->first), end);
+  const uint32_t q = base + blockIdx.x * kLpWarps + (threadIdx.x >> 5);
+  if (q < end) {
+    const int32_t t = a.choice[q];
+    if (t >= 0) {
+      const uchar2 s = a.fsize[a.order[q]];
+      const int ax = t % a.W, ay = t / a.W;
+      for (int k = lane; k < s.x * s.y; k += 32) {
+        const int x = ax + k % s.x, y = ay + k / s.x;
+        int32_t *o = own_at(a, x, y);
+        if (ld_own(o) > (int32_t)q) {
+          atomicMin(o, (int32_t)q);
+          atomicOr(&seg_at(a, x, y)->y, 1u << (x & 31));
+        }
+        if (q < stop) atomicAnd(&seg_at(a, x, y)->x, ~(1u << (x & 31)));  // final
+      }
+      if (q < stop && lane == 0) put_hint(a, (int32_t)q, load_cell(a, q, false), a.mcost[q]);
+    } else if (q < stop && lane == 0) {
+      atomicMax(&st->status, 1);  // final, and no anchor was open
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&st->ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last || threadIdx.x != 0) return;
+  __threadfence();
+  st->base = stop;
+  st->first = (uint32_t)kNone;
+  st->nfreed[st->rounds & 1u] = 0;
+  st->rounds += 1;
+  st->ticket = 0;
+  if (stop < a.n_mac && st->rounds >= a.max_rounds) atomicMax(&st->status, 2);
+  if (stop >= a.n_mac || atomicAdd(&st->status, 0) != 0) cudaGraphSetConditional(a.handle, 0u);
+}
+
+// ---------------------------------------------------------------------------
+// Unit cells
+// ---------------------------------------------------------------------------
+
+// seg[] while the unit cells are placed: x has a bit for each site that
+// nobody has claimed yet (cleared after the claim, so a bit may be late), y
+// the largest order index that ever claimed a free site of the segment
+// (raised before the claim's bit goes).  A segment with x == 0 and y < q has
+// no site open to q; with y < q the bits of x are the open sites.
+__global__ void __launch_bounds__(256) k_lp_segments(const LpArgs a) {
+  const int lane = threadIdx.x & 31;
+  const int nseg = a.SW * a.H;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nseg; i += (gridDim.x * blockDim.x) >> 5) {
+    const unsigned m = __ballot_sync(kFull, a.own[(size_t)32 * i + lane] == kNone);
+    if (lane == 0) a.seg[i] = make_uint2(m, ~0u);
+  }
+}
+
+// Search of the sites around unit cell q's target by one warp: the 5 x 5 sites
+// around the nearest one, a lane each.  A site outside costs at least 2.5^2,
+// so a cheaper one inside is the answer.
+__device__ Best search_near(const LpArgs &a, int32_t q, const Cell &c, int lane) {
+  Best b = no_best();
+  if (lane < 25) {
+    const int x = c.cx - 2 + lane % 5, y = c.cy - 2 + lane / 5;
+    if (x >= 0 && x < a.W && y >= 0 && y < a.H && ld_own(own_at(a, x, y)) > q)
+      b.take(__dadd_rn(col_dx2(c, x), row_dy2(c, y)), y * a.W + x);
+  }
+  return b.warp_min();
+}
+
+// The search over the whole chip by the CTA, none of cost below c0 being
+// open: rows outward from the target, sixteen per warp and pass, two lanes a
+// row, one for each direction, from the circle of cost c0 on.  A lane first
+// walks the segments away from the target to the first site that nobody holds
+// (their bits alone); the least of these bounds the cost for the whole CTA
+// (*least).  Then it looks for a site held by a later cell that is cheaper
+// still, in the segments where there can be one, within the bound.  Bounds
+// are FP32 costs: coordinates are whole or FP32 numbers, so such a cost is
+// within 2^-21 of the exact one, and kOver covers twice that; the few sites
+// within the bound are costed in FP64.  Bound by the latency of a pass (a few
+// hundred instructions, two or three loads from L2).  Returns this lane's best.
+constexpr int kUnitWarps = 16;
+constexpr float kOver = 1.000002f, kUnder = 0.999998f;
+constexpr float kInf = __builtin_huge_valf();
+
+__device__ __forceinline__ float fast_sqrt(float v) {  // within 2^-22
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+__device__ Best search_rows(const LpArgs &a, int32_t q, const Cell &c, double c0, int warp, int lane,
+                            unsigned *least) {
+  Best b = no_best();
+  const bool right = lane & 1;
+  const int dir = right ? 1 : -1;
+  const float tx = (float)c.tx, ty = (float)c.ty, low = (float)c0 * kUnder;
+  const int rows = max(c.cy, a.H - 1 - c.cy);  // rows on the longer side
+  // a pass covers the rows at distance p0 .. p0 + 8 kUnitWarps - 1; every
+  // row from there on is at least p0 - 1/2 away
+  float most = __uint_as_float(*(volatile unsigned *)least);
+  for (int p0 = 0; p0 <= rows; p0 += 8 * kUnitWarps) {
+    // (most is the same in every thread here: read between the pass's barriers)
+    if (p0 && ((float)p0 - 0.5f) * ((float)p0 - 0.5f) > most) break;
+    // rows m0, -(m0 + 1), m0 + 1, -(m0 + 2), ... of cy, and cy itself once
+    const int k = (lane >> 1) + 2 * (p0 + 8 * warp);
+    const int y = c.cy + ((k & 1) ? -(k + 1) / 2 : k / 2);
+    const float dy = (float)y - ty, dy2 = dy * dy;
+    int x = right ? c.fx + 1 : c.fx;
+    if (low > dy2) {
+      const float d = fast_sqrt(low - dy2) - 0.01f;
+      x = right ? max(x, (int)ceilf(tx + d)) : min(x, (int)floorf(tx - d));
+    }
+    float dx = (float)x - tx;
+    const bool in = y >= 0 && y < a.H && x >= 0 && x < a.W && dx * dx + dy2 <= most;
+    const unsigned side0 = right ? ~0u << (x & 31) : ~0u >> (31 - (x & 31));  // of the first segment
+    const int g0 = x >> 5;
+    const uint2 *row = a.seg + (size_t)y * a.SW;
+    // Sites that nobody holds; late: bit u: the u-th segment of the walk has
+    // a claim of a later cell, bit 31: one from the 31st on has.
+    const bool in1 = in && g0 + dir >= 0 && g0 + dir < a.SW;
+    const uint2 s0 = in ? ld_seg(row + g0) : make_uint2(0u, ~0u);
+    const uint2 s1 = in1 ? ld_seg(row + g0 + dir) : make_uint2(0u, ~0u);
+    unsigned m = s0.x & side0;
+    unsigned late = ((int32_t)s0.y > q ? 1u : 0u) | (!m && (int32_t)s1.y > q ? 2u : 0u);
+    int g = g0;
+    if (!m) {
+      m = s1.x;
+      g += dir;
+    }
+    bool go = in1 && !m;
+    auto site_cost = [&] {  // of the site found, if any
+      x = right ? 32 * g + __ffs(m) - 1 : 32 * g + 31 - __clz(m);
+      dx = (float)x - tx;
+      return m ? dx * dx + dy2 : kInf;
+    };
+    auto bound = [&](float cost) {
+      const unsigned all = __reduce_min_sync(kFull, __float_as_uint(cost * kOver));
+      if (lane == 0 && all < __float_as_uint(most)) atomicMin(least, all);
+    };
+    if (__any_sync(kFull, go)) bound(site_cost());
+    for (int i = 2; __any_sync(kFull, go); ++i) {
+      most = __uint_as_float(*(volatile unsigned *)least);
+      if (go) {
+        g += dir;
+        dx = (float)(right ? 32 * g : 32 * g + 31) - tx;  // the segment's nearest site
+        go = g >= 0 && g < a.SW && dx * dx + dy2 <= most;
+        if (go) {
+          const uint2 s = ld_seg(row + g);
+          if ((int32_t)s.y > q) late |= 1u << min(i, 31);
+          m = s.x;
+          go = !m;
+        }
+      }
+    }
+    const float cost = site_cost();
+    bound(cost);
+    __syncthreads();
+    most = __uint_as_float(*(volatile unsigned *)least);
+    if (cost * kUnder <= most && m) b.take(__dadd_rn(col_dx2(c, x), row_dy2(c, y)), y * a.W + x);
+    // Sites held by later cells, nearest segment first, columns within the bound.
+    const float left = most - dy2;
+    go = in && late && left >= 0.0f;
+    if (__any_sync(kFull, go)) {
+      const float reach = fast_sqrt(fmaxf(left, 0.0f)) + 0.01f;
+      const int last = right ? (int)fminf(floorf(tx + reach), (float)(32 * a.SW - 1))
+                             : (int)fmaxf(ceilf(tx - reach), 0.0f);
+      while (go) {
+        const int i = __ffs(late) - 1;
+        late &= late - 1;
+        for (int j = i; go; ++j) {  // one segment, or all from the 31st on
+          const int at = g0 + j * dir, end = last - 32 * at;  // the bound's column in the segment
+          go = at >= 0 && at < a.SW && (right ? end >= 0 : end <= 31);
+          if (!go) break;
+          const unsigned within = right ? ~0u >> (31 - min(end, 31)) : ~0u << max(end, 0);
+          const unsigned ask = j ? within : within & side0;
+          const unsigned n = ask ? open_sites(own_at(a, 32 * at, y), ask, q) & ask : 0u;
+          if (n) {
+            const int ox = right ? 32 * at + __ffs(n) - 1 : 32 * at + 31 - __clz(n);
+            b.take(__dadd_rn(col_dx2(c, ox), row_dy2(c, y)), y * a.W + ox);
+            go = false;
+          }
+          if (i < 31) break;
+        }
+        go = go && late;
+      }
+      // what was found bounds the next passes
+      const unsigned now = __reduce_min_sync(kFull, __float_as_uint(__double2float_ru(b.cost) * kOver));
+      if (lane == 0 && now < __float_as_uint(most)) atomicMin(least, now);
+    }
+    __syncthreads();
+    most = __uint_as_float(*(volatile unsigned *)least);
+    __syncthreads();  // read before the next pass lowers it
+  }
+  return b;
+}
+
+// Claims site b.tile for q (one thread): kNone: it was free; a later cell: q
+// has it now, and that cell has lost it; an earlier cell: q did not get it.
+__device__ __forceinline__ int32_t claim_site(const LpArgs &a, int32_t q, const Cell &c, const Best &b) {
+  const int x = b.tile % a.W, y = b.tile / a.W;
+  uint2 *s = seg_at(a, x, y);
+  const int32_t top = atomicMax(reinterpret_cast<int32_t *>(&s->y), q);
+  const int32_t held = atomicMin(own_at(a, x, y), q);
+  // the bit goes after both answers are here; one that lost the site clears
+  // it too, so that it does not meet a late bit again
+  if ((held == kNone || held < q) && top != kNone) atomicAnd(&s->x, ~(1u << (x & 31)));
+  put_hint(a, q, c, b.cost);
+  return held;
+}
+
+// A CTA per unit cell, and the cells that its claim displaces one after the
+// other.  What takes the time is the chain of cells that each take a site from
+// the next (about a thousand cells at the rim of a 200k-cell pile), so one
+// search is made short: an answer near the target is found by one warp with
+// no barrier, any other by all 16.  CTAs start in about the order of the
+// cells, so a claim is displaced only by a cell that was under way at the
+// same time; several cells per CTA, or a warp for each, put more cells under
+// way and displace more claims.  Units of a 200k-cell checkpoint whose cells
+// lie in one pile: 7.5 ms and 283k searches of the whole CTA; 2 / 4 / 8 cells
+// per CTA 13.4 / 20 / 30 ms, a warp per cell 27 to 70 ms.
+__global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(const LpArgs a) {
+  __shared__ Best sbest[kUnitWarps];
+  __shared__ unsigned least;
+  // the cell under way: index (-1: done), target, cost below which no site is open
+  __shared__ int32_t sq_;
+  __shared__ float2 spos;
+  __shared__ double sc0;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uchar2 one = make_uchar2(1, 1);
+  bool fresh = true;
+  while (true) {
+    if (warp == 0) {  // while the answer is near the target
+      int32_t q = fresh ? (int32_t)(a.n_mac + blockIdx.x) : sq_;
+      if (q >= 0) {
+        float2 p = fresh ? a.pos[a.order[q]] : spos;
+        Cell c = make_cell(a, p, one);
+        double c0 = fresh ? get_hint(a, q, c) : sc0;
+        while (c0 < 6.25 && placeable(c)) {
+          const Best b = search_near(a, q, c, lane);
+          if (!(b.cost < 6.25)) break;
+          int32_t held = 0;
+          if (lane == 0) held = claim_site(a, q, c, b);
+          held = __shfl_sync(kFull, held, 0);
+          if (held == kNone) {
+            q = -1;
+            break;
+          }
+          if (held > q) {  // go on with the cell that lost it
+            q = held;
+            p = a.pos[a.order[q]];
+            c = make_cell(a, p, one);
+            c0 = c.inside ? __dadd_rn(col_dx2(c, b.tile % a.W), row_dy2(c, b.tile / a.W)) : 0.0;
+          }
+        }
+        if (lane == 0) {
+          spos = p;
+          sc0 = c0;
+        }
+      }
+      if (lane == 0) {
+        sq_ = q;
+        least = __float_as_uint(kInf);
+      }
+    }
+    fresh = false;
+    __syncthreads();
+    const int32_t q = sq_;
+    if (q < 0) return;
+    const Cell c = make_cell(a, spos, one);
+    Best b = no_best();
+    if (placeable(c)) b = search_rows(a, q, c, sc0, warp, lane, &least);
+    b = b.warp_min();
+    if (lane == 0) sbest[warp] = b;
+    __syncthreads();
+    if (warp == 0) {
+      b = (lane < kUnitWarps ? sbest[lane] : no_best()).warp_min();
+      if (lane == 0) {
+        if (b.tile == kNone) {  // no site is open to it
+          atomicMax(&a.st->status, 1);
+          sq_ = -1;
+        } else {
+          const int32_t held = claim_site(a, q, c, b);
+          sc0 = c.inside ? b.cost : 0.0;
+          if (held == kNone) {
+            sq_ = -1;
+          } else if (held > q) {
+            const float2 p = a.pos[a.order[held]];
+            const Cell d = make_cell(a, p, one);
+            sq_ = held;
+            spos = p;
+            sc0 = d.inside ? __dadd_rn(col_dx2(d, b.tile % a.W), row_dy2(d, b.tile / a.W)) : 0.0;
           }
         }
       }
@@ -175,484 +755,172 @@ __device__ void warp_sort(Cand *buf, int n2, int lane) {
   }
 }
 
-// Marks the sites of the w x h block at anchor tile t with min(mark, q).
-__device__ __forceinline__ void mark_block(int32_t *mark, int W, int t, int w, int h, int32_t q) {
-  const int ax = t % W, ay = t / W;
-  for (int dy = 0; dy < h; ++dy)
-    for (int dx = 0; dx < w; ++dx) atomicMin(&mark[(size_t)(ay + dy) * W + ax + dx], q);
-}
-__device__ __forceinline__ bool block_marked_below(const int32_t *mark, int W, int t, int w, int h, int32_t q) {
-  const int ax = t % W, ay = t / W;
-  for (int dy = 0; dy < h; ++dy)
-    for (int dx = 0; dx < w; ++dx)
-      if (__ldcg(&mark[(size_t)(ay + dy) * W + ax + dx]) < q) return true;
-  return false;
-}
-__device__ __forceinline__ void reset_block(int32_t *mark, int W, int t, int w, int h) {
-  const int ax = t % W, ay = t / W;
-  for (int dy = 0; dy < h; ++dy)
-    for (int dx = 0; dx < w; ++dx) mark[(size_t)(ay + dy) * W + ax + dx] = kNoMark;
-}
-
 // ---------------------------------------------------------------------------
-// Kernels
+// Results
 // ---------------------------------------------------------------------------
-__global__ void k_lp_init(const LpArgs a) {
-  const size_t words = (size_t)a.WR * a.H;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < words; i += (size_t)gridDim.x * blockDim.x)
-    a.fm[i] = a.free0[i];
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    LpState *s = a.st;
-    s->pos = 0;
-    s->bcur = a.n < 2048u ? a.n : 2048u;
-    s->stop = 0;
-    s->rounds = 0;
-    s->status = 0;
-    for (int i = 0; i <= kLpPropSteps; ++i) s->changed[i] = 0;
-  }
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < kLpMaxWindow; q += gridDim.x * blockDim.x) {
-    a.dist[q] = 0;
-    a.fresh[q] = 0;
-  }
-}
-
-// One warp per window cell: its candidate list against the frozen map, and
-// its head block entered in hmark.
-__global__ void __launch_bounds__(kListWarps * 32) k_lp_lists(const LpArgs a) {
-  __shared__ Cand sbuf[kListWarps][kCandBuf];
-  __shared__ int scount[kListWarps];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const uint32_t q = blockIdx.x * kListWarps + wib;
-  const LpState *st = a.st;
-  if (blockIdx.x == 0 && threadIdx.x == 0)
-    for (int i = 1; i <= kLpPropSteps; ++i) a.st->changed[i] = 0;
-  const uint32_t bcur = st->bcur, pos = st->pos;
-  if (q >= bcur || pos + q >= a.n) return;
-  const uint32_t cell = a.order[pos + q];
-  const Cell c = load_cell(a, cell);
-  Cand *buf = sbuf[wib];
-  int32_t *out = a.list + (size_t)q * kLpList;
-  if (lane == 0) a.info[q] = c.w | (c.h << 8);
-  if (c.AW <= 0 || c.AH <= 0) {
-    if (lane == 0) a.len[q] = 0;
-    return;
-  }
-  // Threshold: grow until at least kListMin candidates (or the whole chip),
-  // then, if that overshoots the buffer, bisect back into [kListMin, kCandBuf].
-  const double span = (double)a.W + (double)a.H;
-  const double tau_max = span * span;
-  double tau = 2.0, lo = -1.0;
-  int cnt = scan_tau(a, c, tau, lane, nullptr, 0, nullptr);
-  for (int g = 0; cnt < kListMin && tau < tau_max && g < 64; ++g) {
-    lo = tau;
-    tau = fmin(tau * 4.0 + 4.0, tau_max);
-    cnt = scan_tau(a, c, tau, lane, nullptr, 0, nullptr);
-  }
-  int lo_cnt = lo < 0.0 ? 0 : -1;  // count at lo when known
-  for (int it = 0; cnt > kCandBuf && it < 64; ++it) {
-    const double mid = lo < 0.0 ? 0.5 * tau : lo + 0.5 * (tau - lo);
-    if (!(mid > lo && mid < tau)) break;
-    const int m = scan_tau(a, c, mid, lane, nullptr, 0, nullptr);
-    if (m > kCandBuf) {
-      tau = mid;
-      cnt = m;
-    } else if (m >= kListMin) {
-      tau = mid;
-      cnt = m;
-    } else {
-      lo = mid;
-      lo_cnt = m;
-    }
-  }
-  if (cnt > kCandBuf) {  // a tie group wider than the buffer: fall back to lo
-    if (lo >= 0.0) {
-      tau = lo;
-      cnt = lo_cnt >= 0 ? lo_cnt : scan_tau(a, c, lo, lane, nullptr, 0, nullptr);
-    }
-    if (cnt == 0 || cnt > kCandBuf) {
-      if (lane == 0) {
-        a.len[q] = 0;
-        atomicMax(&a.st->status, 3);
-      }
-      return;
-    }
-  }
-  if (cnt == 0) {  // no free anchor anywhere
-    if (lane == 0) a.len[q] = 0;
-    return;
-  }
-  if (lane == 0) scount[wib] = 0;
-  __syncwarp();
-  scan_tau(a, c, tau, lane, buf, kCandBuf, &scount[wib]);
-  __syncwarp();
-  const int n = min(scount[wib], kCandBuf);
-  int n2 = 32;
-  while (n2 < n) n2 <<= 1;
-  for (int i = n + lane; i < n2; i += 32) {
-    buf[i].key = ~0ull;
-    buf[i].tile = 0x7fffffff;
-  }
-  __syncwarp();
-  warp_sort(buf, n2, lane);
-  const int keep = min(n, kLpList);
-  for (int i = lane; i < keep; i += 32) out[i] = buf[i].tile;
-  if (lane == 0) a.len[q] = keep;
-  // head block into hmark (lanes split the block's rows)
-  const int t = buf[0].tile;
+__device__ __forceinline__ void put_result(const LpArgs &a, uint32_t q, int t, bool unit) {
+  const Cell c = load_cell(a, q, unit);
   const int ax = t % a.W, ay = t / a.W;
-  for (int k = lane; k < c.w * c.h; k += 32)
-    atomicMin(&a.hmark[(size_t)(ay + k / c.w) * a.W + ax + k % c.w], (int32_t)q);
+  const uint32_t cell = a.order[q];
+  a.sites[cell] = make_int2(ax, ay);
+  if (a.loc) a.loc[cell] = make_int2(ax + (c.w - 1) / 2, ay + (c.h - 1) / 2);
+  a.cost[q] = __dadd_rn(col_dx2(c, ax), row_dy2(c, ay));
 }
 
-// Disturbance pass `step`: cells whose head block lies under an earlier
-// window cell's head (step 0) or under an earlier disturbed cell's list
-// become disturbed and enter their whole list in dmark.
-__global__ void k_lp_prop(const LpArgs a, int step) {
-  const LpState *st = a.st;
-  if (step > 0 && __ldcg(&st->changed[step]) == 0u) return;
-  const uint32_t bcur = st->bcur, pos = st->pos;
-  bool found = false;
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < bcur && pos + q < a.n;
-       q += gridDim.x * blockDim.x) {
-    const int len = a.len[q];
-    if (len <= 0) continue;
-    const int inf = a.info[q];
-    const uchar2 s = make_uchar2(inf & 255, inf >> 8);
-    const int32_t *lst = a.list + (size_t)q * kLpList;
-    if (!a.dist[q]) {
-      const bool d = step == 0 ? block_marked_below(a.hmark, a.W, lst[0], s.x, s.y, (int32_t)q)
-                               : block_marked_below(a.dmark, a.W, lst[0], s.x, s.y, (int32_t)q);
-      if (d) {
-        a.dist[q] = 1;
-        a.fresh[q] = 1;
-        found = true;
-      }
-    }
-    if (a.fresh[q]) {
-      for (int e = 0; e < len; ++e) mark_block(a.dmark, a.W, lst[e], s.x, s.y, (int32_t)q);
-      a.fresh[q] = 0;
-    }
+__global__ void __launch_bounds__(256) k_lp_result(const LpArgs a) {
+  if (a.st->status != 0) return;
+  const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x, ts = gridDim.x * blockDim.x;
+  for (uint32_t q = t0; q < a.n_mac; q += ts) put_result(a, q, a.choice[q], false);
+  const uint32_t pitch = 32u * (uint32_t)a.SW, sites = pitch * (uint32_t)a.H;
+  for (uint32_t s = t0; s < sites; s += ts) {
+    const int32_t q = a.own[s];
+    if (q < (int32_t)a.n_mac || q == kNone) continue;
+    const uint32_t y = s / pitch;
+    put_result(a, (uint32_t)q, (int)(y * (uint32_t)a.W + (s - y * pitch)), true);
   }
-  if (found) a.st->changed[step + 1] = 1u;
 }
 
-// Sites taken during a round's serial pass, in shared memory: a bitmap of
-// the whole chip when it has at most 2^20 sites, else a hash of the taken
-// sites (keys tile + 1, 0 = empty), whose load caps the window.
-constexpr int kBitmapSites = 1 << 20;
-
-struct TakenBits {
-  uint32_t *w;
-  int W;
-  __device__ __forceinline__ void clear(int tid, int nt, int nsites) {
-    for (int i = tid; i < (nsites + 31) / 32; i += nt) w[i] = 0u;
-  }
-  __device__ __forceinline__ bool block_taken(int t, int bw, int bh) const {
-    // a unit cell's block is its one site, whose bit index is the tile
-    if (bw == 1 && bh == 1) return (reinterpret_cast<const volatile uint32_t *>(w)[t >> 5] >> (t & 31)) & 1u;
-    const int ax = t % W, ay = t / W;
-    for (int dy = 0; dy < bh; ++dy) {
-      const int s0 = (ay + dy) * W + ax, s1 = s0 + bw - 1;
-      const int w0 = s0 >> 5, w1 = s1 >> 5;
-      const volatile uint32_t *vw = w;
-      if (w0 == w1) {
-        const uint32_t m = (bw == 32 ? ~0u : ((1u << bw) - 1u)) << (s0 & 31);
-        if (vw[w0] & m) return true;
-      } else {
-        if (vw[w0] & (~0u << (s0 & 31))) return true;
-        if (vw[w1] & ((2u << (s1 & 31)) - 1u)) return true;
-      }
-    }
-    return false;
-  }
-  __device__ __forceinline__ void put(int t, int bw, int bh) {
-    if (bw == 1 && bh == 1) {
-      atomicOr(&w[t >> 5], 1u << (t & 31));
-      return;
-    }
-    const int ax = t % W, ay = t / W;
-    for (int dy = 0; dy < bh; ++dy)
-      for (int dx = 0; dx < bw; ++dx) {
-        const int s = (ay + dy) * W + ax + dx;
-        atomicOr(&w[s >> 5], 1u << (s & 31));
-      }
-  }
+// A run of additions to a total of t units in the last place: the units added
+// when t is even and when it is odd.  Counts saturate above 2^53, where the
+// total would leave its binade.
+struct AddRun {
+  unsigned long long even, odd;
 };
+constexpr unsigned long long kTop = 1ull << 53;
+__device__ __forceinline__ unsigned long long sat(unsigned long long v) { return v < kTop ? v : kTop; }
+__device__ __forceinline__ AddRun then(const AddRun &f, const AddRun &g) {  // f first
+  return AddRun{sat(f.even + ((f.even & 1) ? g.odd : g.even)), sat(f.odd + ((f.odd & 1) ? g.even : g.odd))};
+}
+// v >= 0 added to a total whose unit in the last place is 1 / scale:
+// v in units is v * scale, exact (a power of two).
+__device__ __forceinline__ AddRun add_one(double v, double scale) {
+  const double u = __dmul_rn(v, scale);
+  if (!(u < 9007199254740992.0)) return AddRun{kTop, kTop};
+  const double fl = floor(u), fr = __dsub_rn(u, fl);
+  const unsigned long long n = (unsigned long long)fl;
+  if (fr < 0.5) return AddRun{n, n};
+  if (fr > 0.5) return AddRun{n + 1, n + 1};
+  return (n & 1) ? AddRun{n + 1, n} : AddRun{n, n + 1};  // half way: to the even total
+}
 
-constexpr int kHashBits = 15;
-constexpr int kHashLimit = 1 << 14;  // sites entered per round (load factor <= 1/2)
+constexpr int kSumThreads = 1024, kSumEach = 8;
 
-struct TakenHash {
-  int *hs;
-  int W;
-  __device__ __forceinline__ static unsigned slot(int key) { return ((unsigned)key * 2654435761u) >> (32 - kHashBits); }
-  __device__ __forceinline__ void clear(int tid, int nt, int) {
-    for (int i = tid; i < (1 << kHashBits); i += nt) hs[i] = 0;
-  }
-  __device__ __forceinline__ bool has(int key) const {
-    const unsigned s = slot(key);
-    for (int p = 0; p < (1 << kHashBits); ++p) {
-      const int v = reinterpret_cast<const volatile int *>(hs)[(s + p) & ((1u << kHashBits) - 1)];
-      if (v == key + 1) return true;
-      if (v == 0) return false;
-    }
-    return false;
-  }
-  __device__ __forceinline__ void add(int key) {
-    const unsigned s = slot(key);
-    for (int p = 0; p < (1 << kHashBits); ++p) {
-      const int prev = atomicCAS(&hs[(s + p) & ((1u << kHashBits) - 1)], 0, key + 1);
-      if (prev == 0 || prev == key + 1) return;
-    }
-  }
-  __device__ __forceinline__ bool block_taken(int t, int bw, int bh) const {
-    const int ax = t % W, ay = t / W;
-    for (int dy = 0; dy < bh; ++dy)
-      for (int dx = 0; dx < bw; ++dx)
-        if (has((ay + dy) * W + ax + dx)) return true;
-    return false;
-  }
-  __device__ __forceinline__ void put(int t, int bw, int bh) {
-    const int ax = t % W, ay = t / W;
-    for (int dy = 0; dy < bh; ++dy)
-      for (int dx = 0; dx < bw; ++dx) add((ay + dy) * W + ax + dx);
-  }
-};
-
-// Inclusive block-wide sum of v (all kSerialThreads threads call it); the
-// block's total is left in wsum[31].
-__device__ __forceinline__ int block_scan(int v, int *wsum) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(kFull, v, o);
-    if (lane >= o) v += t;
-  }
-  if (lane == 31) wsum[w] = v;
-  __syncthreads();
+// The displacement, one CTA: the first costs one after the other (the total
+// soon leaves its binade there), then 8192 a step.  The first addition that
+// leaves the binade (or the first cost that is not zero, while the total is)
+// is made as it stands and the next step starts after it: nine or ten times in
+// 200k costs.  0.4 ms with every cost in steps.
+constexpr uint32_t kSumFirst = 512;
+__global__ void __launch_bounds__(kSumThreads) k_lp_finish(const LpArgs a) {
+  __shared__ AddRun wrun[32];
+  __shared__ double total;
+  __shared__ uint32_t stop;  // first cost of the step that has to be added by itself
+  __shared__ double next;    // the total after it, or after the whole step
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const bool ok = a.st->status == 0;
+  uint32_t at = min(a.n, kSumFirst);
   if (w == 0) {
-    int s = wsum[lane];
+    double t = 0.0;
+    for (uint32_t i = 0; ok && i < at; i += 32) {
+      const double v = i + lane < at ? __ldcg(a.cost + i + lane) : 0.0;  // + 0.0 leaves the total
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(kFull, s, o);
-      if (lane >= o) s += t;
+      for (int l = 0; l < 32; ++l) t = __dadd_rn(t, __shfl_sync(kFull, v, l));
     }
-    wsum[lane] = s;
+    if (lane == 0) total = t;
   }
   __syncthreads();
-  const int r = v + (w ? wsum[w - 1] : 0);
-  __syncthreads();
-  return r;
-}
-
-struct SerialShared {
-  uint16_t didx[kLpMaxWindow];
-  int lbuf[2][kChunk][kLpList];
-  int llen[2][kChunk];
-  int linf[2][kChunk];
-  int wsum[32];
-  int carry, bwin, halt, stop;
-};
-
-template <bool kBits>
-constexpr size_t serial_smem_bytes() {
-  return sizeof(SerialShared) + (kBits ? sizeof(uint32_t) * (kBitmapSites / 32) : sizeof(int) * (1 << kHashBits));
-}
-
-// The serial pass of a round (one CTA).
-template <bool kBits>
-__global__ void __launch_bounds__(kSerialThreads, 1) k_lp_serial(const LpArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  SerialShared &S = *reinterpret_cast<SerialShared *>(smem_raw);
-  using Taken = typename std::conditional<kBits, TakenBits, TakenHash>::type;
-  Taken tk;
-  if constexpr (kBits) tk = TakenBits{reinterpret_cast<uint32_t *>(smem_raw + sizeof(SerialShared)), a.W};
-  else tk = TakenHash{reinterpret_cast<int *>(smem_raw + sizeof(SerialShared)), a.W};
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t pos = a.st->pos;
-  const uint32_t bcur = min(a.st->bcur, a.n - min(pos, a.n));
-  const bool all_serial = __ldcg(&a.st->changed[kLpPropSteps]) != 0u;  // propagation did not settle
-  tk.clear(tid, kSerialThreads, a.W * a.H);
+  while (ok && at < a.n) {
+    const double t0 = total;
+    if (tid == 0) stop = 0xffffffffu;
+    double v[kSumEach];
+    const uint32_t i0 = at + (uint32_t)tid * kSumEach;
+#pragma unroll
+    for (int k = 0; k < kSumEach; ++k) v[k] = i0 + k < a.n ? __ldcg(a.cost + i0 + k) : 0.0;
+    __syncthreads();  // total read, stop set
+    if (t0 == 0.0) {
+#pragma unroll
+      for (int k = kSumEach - 1; k >= 0; --k)
+        if (v[k] != 0.0) atomicMin(&stop, i0 + k);
+      __syncthreads();
+      if (stop != 0xffffffffu && stop - i0 < kSumEach) {
+#pragma unroll
+        for (int k = 0; k < kSumEach; ++k)
+          if (i0 + k == stop) total = v[k];
+      }
+    } else {
+      // unit in the last place of t0: 2^(e - 52) for 2^e <= t0 < 2^(e + 1)
+      const int e = ilogb(t0);
+      const double unit = scalbn(1.0, e - 52), scale = scalbn(1.0, 52 - e);
+      AddRun f[kSumEach];
+      AddRun mine{0, 0};
+#pragma unroll
+      for (int k = 0; k < kSumEach; ++k) {
+        f[k] = add_one(v[k], scale);
+        mine = then(mine, f[k]);
+      }
+      // exclusive scan over the threads, in order
+      AddRun inc = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        AddRun p;
+        p.even = __shfl_up_sync(kFull, inc.even, o);
+        p.odd = __shfl_up_sync(kFull, inc.odd, o);
+        if (lane >= o) inc = then(p, inc);
+      }
+      AddRun ex;
+      ex.even = __shfl_up_sync(kFull, inc.even, 1);
+      ex.odd = __shfl_up_sync(kFull, inc.odd, 1);
+      if (lane == 0) ex = AddRun{0, 0};
+      if (lane == 31) wrun[w] = inc;
+      __syncthreads();
+      if (w == 0) {
+        AddRun x = wrun[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          AddRun p;
+          p.even = __shfl_up_sync(kFull, x.even, o);
+          p.odd = __shfl_up_sync(kFull, x.odd, o);
+          if (lane >= o) x = then(p, x);
+        }
+        wrun[lane] = x;
+      }
+      __syncthreads();
+      if (w) ex = then(wrun[w - 1], ex);
+      const unsigned long long base = (unsigned long long)__dmul_rn(t0, scale);  // 2^52 .. 2^53 - 1
+      unsigned long long t = base + ((base & 1) ? ex.odd : ex.even);
+      unsigned long long before = t;
+      int out = -1;
+#pragma unroll
+      for (int k = 0; k < kSumEach; ++k) {
+        if (out >= 0) continue;
+        before = t;
+        t += (t & 1) ? f[k].odd : f[k].even;
+        if (t >= kTop) out = k;
+      }
+      if (out >= 0) atomicMin(&stop, i0 + out);
+      __syncthreads();
+      if (out >= 0 && i0 + out == stop) {
+        double add = 0.0;
+#pragma unroll
+        for (int k = 0; k < kSumEach; ++k)
+          if (k == out) add = v[k];
+        next = __dadd_rn(__dmul_rn((double)before, unit), add);
+      }
+      if (stop == 0xffffffffu && tid == kSumThreads - 1) next = __dmul_rn((double)t, unit);
+      __syncthreads();
+      if (tid == 0) total = next;
+    }
+    __syncthreads();
+    at = stop != 0xffffffffu ? stop + 1 : at + kSumThreads * kSumEach;
+    __syncthreads();  // stop read before it is set again
+  }
   if (tid == 0) {
-    S.bwin = (int)bcur;
-    S.halt = 0;
-    S.stop = -1;
-    S.carry = 0;
-  }
-  __syncthreads();
-  if constexpr (!kBits) {
-    // Window cap: the prefix whose blocks fit the hash's load limit.
-    for (uint32_t base = 0; base < bcur; base += kSerialThreads) {
-      const uint32_t q = base + tid;
-      int sz = 0;
-      if (q < bcur) {
-        const int inf = a.info[q];
-        sz = (inf & 255) * (inf >> 8);
-      }
-      const int incl = block_scan(sz, S.wsum);
-      if (q < bcur && S.carry + incl > kHashLimit) atomicMin(&S.bwin, (int)q);
-      __syncthreads();
-      if (tid == 0) S.carry += S.wsum[31];
-      __syncthreads();
-      if (S.bwin < (int)bcur) break;
-    }
-  }
-  const int bwin = S.bwin;
-  // Undisturbed heads are taken; disturbed cells are listed in order.
-  int nd = 0;
-  for (int base = 0; base < bwin; base += kSerialThreads) {
-    const int q = base + tid;
-    int dis = 0;
-    if (q < bwin) {
-      const int len = a.len[q];
-      dis = (all_serial || a.dist[q] || len <= 0) ? 1 : 0;
-      if (!dis) {
-        const int inf = a.info[q];
-        tk.put(a.list[(size_t)q * kLpList], inf & 255, inf >> 8);
-      }
-    }
-    const int incl = block_scan(dis, S.wsum);
-    if (dis) S.didx[nd + incl - 1] = (uint16_t)q;
-    nd += S.wsum[31];
-    __syncthreads();
-  }
-  // Stage chunk k of the disturbed cells' lists into buffer k & 1: one warp
-  // per cell, the list read as whole 128-byte lines.
-  auto stage = [&](int k, int wfirst, int nwarps) {
-    const int b = k & 1, c0 = k * kChunk;
-    for (int r = warp - wfirst; r < kChunk; r += nwarps) {
-      if (c0 + r >= nd) break;
-      const int q = S.didx[c0 + r];
-      const int len = __ldcg(&a.len[q]);
-      for (int e = lane; e < len; e += 32) S.lbuf[b][r][e] = __ldcg(&a.list[(size_t)q * kLpList + e]);
-      if (lane == 0) {
-        S.llen[b][r] = len;
-        S.linf[b][r] = __ldcg(&a.info[q]);
-      }
-    }
-  };
-  stage(0, 0, kSerialThreads / 32);
-  __syncthreads();
-  const int nchunks = (nd + kChunk - 1) / kChunk;
-  for (int k = 0; k < nchunks; ++k) {
-    if (warp == 0) {
-      const int b = k & 1;
-      for (int r = 0; r < kChunk && k * kChunk + r < nd; ++r) {
-        const int q = S.didx[k * kChunk + r];
-        const int len = S.llen[b][r];
-        const int inf = S.linf[b][r];
-        const int bw = inf & 255, bh = inf >> 8;
-        int pick = -1;
-        for (int e0 = 0; e0 < len && pick < 0; e0 += 32) {
-          const int e = e0 + lane;
-          bool ok = false;
-          int t = 0;
-          if (e < len) {
-            t = S.lbuf[b][r][e];
-            ok = !tk.block_taken(t, bw, bh);
-          }
-          const unsigned m = __ballot_sync(kFull, ok);
-          if (m) pick = __shfl_sync(kFull, t, __ffs(m) - 1);
-        }
-        if (pick < 0) {  // list exhausted (or empty): the round ends before q
-          if (lane == 0) {
-            S.stop = q;
-            S.halt = 1;
-            if (q == 0) atomicMax(&a.st->status, len <= 0 ? 1 : 3);
-          }
-          break;
-        }
-        if (lane == 0) {
-          tk.put(pick, bw, bh);
-          a.pick[q] = pick;
-        }
-        __syncwarp();
-      }
-    } else if (k + 1 < nchunks) {
-      stage(k + 1, 1, kSerialThreads / 32 - 1);
-    }
-    __syncthreads();
-    if (S.halt) break;
-  }
-  __syncthreads();
-  if (tid == 0) a.st->stop = (uint32_t)(S.stop >= 0 ? S.stop : bwin);
-}
-
-// Commits the round's prefix and clears every mark the round set.
-__global__ void k_lp_commit(const LpArgs a) {
-  const LpState *st = a.st;
-  const uint32_t bcur = st->bcur, pos = st->pos, stop = st->stop;
-  const bool all_serial = st->changed[kLpPropSteps] != 0u;
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < bcur && pos + q < a.n;
-       q += gridDim.x * blockDim.x) {
-    const int len = a.len[q];
-    const uint32_t cell = a.order[pos + q];
-    const int inf = a.info[q];
-    const uchar2 s = make_uchar2(inf & 255, inf >> 8);
-    const int32_t *lst = a.list + (size_t)q * kLpList;
-    if (len > 0) {
-      reset_block(a.hmark, a.W, lst[0], s.x, s.y);
-      if (a.dist[q])
-        for (int e = 0; e < len; ++e) reset_block(a.dmark, a.W, lst[e], s.x, s.y);
-    }
-    if (q < stop) {
-      const int t = (all_serial || a.dist[q]) ? a.pick[q] : lst[0];
-      const int ax = t % a.W, ay = t / a.W;
-      for (int dy = 0; dy < s.y; ++dy)
-        for (int dx = 0; dx < s.x; ++dx) {
-          const int x = ax + dx;
-          atomicAnd(reinterpret_cast<unsigned long long *>(a.fm + (size_t)(ay + dy) * a.WR + (x >> 6)),
-                    ~(1ull << (x & 63)));
-        }
-      a.sites[cell] = make_int2(ax, ay);
-      if (a.loc) a.loc[cell] = make_int2(ax + (s.x - 1) / 2, ay + (s.y - 1) / 2);
-      const Cell c = load_cell(a, cell);
-      a.cost[pos + q] = anchor_cost(c, ax, row_dy2(c, ay));
-    }
-    a.dist[q] = 0;
-    a.fresh[q] = 0;
-  }
-}
-
-__global__ void k_lp_advance(const LpArgs a) {
-  if (threadIdx.x != 0) return;
-  LpState *s = a.st;
-  s->pos += s->stop;
-  s->rounds += 1;
-  const uint32_t left = a.n - min(s->pos, a.n);
-  uint32_t b = 2u * s->stop;
-  b = max(b, 512u);
-  b = min(b, kLpMaxWindow);
-  s->bcur = min(b, left);
-  if (s->status == 0 && left > 0 && s->rounds >= a.max_rounds) s->status = 2;
-  if (left == 0 || s->status != 0) cudaGraphSetConditional(a.handle, 0u);
-}
-
-// Total displacement, summed in order as the sequential loop does, and the
-// status.
-__global__ void k_lp_finish(const LpArgs a) {
-  const int lane = threadIdx.x;
-  double total = 0.0;
-  if (a.st->status == 0) {
-    for (uint32_t base = 0; base < a.n; base += 32) {
-      const uint32_t k = base + lane;
-      const double v = (k < a.n) ? __ldcg(a.cost + k) : 0.0;  // +0.0 leaves a non-negative sum unchanged
-#pragma unroll
-      for (int l = 0; l < 32; ++l) total = __dadd_rn(total, __shfl_sync(kFull, v, l));
-    }
-  }
-  if (lane == 0) {
     *a.disp = total;
     *a.status = a.st->status;
   }
 }
 
 }  // namespace
-
-size_t lp_scratch_bytes(int W, int H) {
-  return 2 * sizeof(int32_t) * (size_t)W * H + sizeof(int32_t) * (size_t)kLpMaxWindow * (kLpList + 3) +
-         2 * (size_t)kLpMaxWindow;
-}
 
 LpGraph::~LpGraph() {
   if (exec) cudaGraphExecDestroy(exec);
@@ -664,63 +932,58 @@ cudaError_t lp_build_graph(LpArgs a, LpGraph &g, cudaStream_t cs) {
   if (g.graph) cudaGraphDestroy(g.graph);
   g.exec = nullptr;
   g.graph = nullptr;
-  const bool bits = (size_t)a.W * a.H <= (size_t)kBitmapSites;
-  const size_t smem = bits ? serial_smem_bytes<true>() : serial_smem_bytes<false>();
-  cudaError_t e = bits ? cudaFuncSetAttribute(k_lp_serial<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                       : cudaFuncSetAttribute(k_lp_serial<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
+  cudaError_t e;
   cudaGraph_t graph = nullptr;
   if ((e = cudaGraphCreate(&graph, 0)) != cudaSuccess) return e;
   g.graph = graph;
-  // Before the loop: map copy and round state, mark arrays cleared.
-  cudaGraphNode_t n_set1, n_set2, n_init, n_loop, n_fin;
-  cudaMemsetParams ms = {};
-  ms.dst = a.hmark;
-  ms.value = 0x7f;
-  ms.elementSize = 1;
-  ms.width = sizeof(int32_t) * (size_t)a.W * a.H;
-  ms.height = 1;
-  ms.pitch = ms.width;
-  if ((e = cudaGraphAddMemsetNode(&n_set1, graph, nullptr, 0, &ms)) != cudaSuccess) return e;
-  ms.dst = a.dmark;
-  if ((e = cudaGraphAddMemsetNode(&n_set2, graph, nullptr, 0, &ms)) != cudaSuccess) return e;
-  cudaKernelNodeParams kp = {};
-  void *args[] = {&a};
-  kp.func = (void *)k_lp_init;
-  kp.gridDim = dim3(256);
-  kp.blockDim = dim3(256);
-  kp.kernelParams = args;
-  cudaGraphNode_t pre[2] = {n_set1, n_set2};
-  if ((e = cudaGraphConditionalHandleCreate(&a.handle, graph, 1, cudaGraphCondAssignDefault)) != cudaSuccess)
+  cudaGraphNode_t tail = nullptr;
+  auto add = [&](const void *func, unsigned grid, unsigned block) -> cudaError_t {
+    void *args[] = {&a};
+    cudaKernelNodeParams kp = {};
+    kp.func = const_cast<void *>(func);
+    kp.gridDim = dim3(grid);
+    kp.blockDim = dim3(block);
+    kp.kernelParams = args;
+    cudaGraphNode_t node;
+    const cudaError_t r = cudaGraphAddKernelNode(&node, graph, tail ? &tail : nullptr, tail ? 1 : 0, &kp);
+    tail = node;
+    return r;
+  };
+  const size_t sites = (size_t)a.W * a.H;
+  const unsigned site_grid = (unsigned)((sites + 255) / 256 < 1184 ? (sites + 255) / 256 : 1184);
+  if (a.n_mac &&
+      (e = cudaGraphConditionalHandleCreate(&a.handle, graph, 1, cudaGraphCondAssignDefault)) != cudaSuccess)
     return e;
-  if ((e = cudaGraphAddKernelNode(&n_init, graph, pre, 2, &kp)) != cudaSuccess) return e;
-  cudaGraphNodeParams cp = {};
-  cp.type = cudaGraphNodeTypeConditional;
-  cp.conditional.handle = a.handle;
-  cp.conditional.type = cudaGraphCondTypeWhile;
-  cp.conditional.size = 1;
-  if ((e = cudaGraphAddNode(&n_loop, graph, &n_init, 1, &cp)) != cudaSuccess) return e;
-  cudaGraph_t body = cp.conditional.phGraph_out[0];
-  // The round, captured into the loop body.
-  if ((e = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
-      cudaSuccess)
-    return e;
-  k_lp_lists<<<kLpMaxWindow / kListWarps, kListWarps * 32, 0, cs>>>(a);
-  for (int i = 0; i < kLpPropSteps; ++i) k_lp_prop<<<kLpMaxWindow / 256, 256, 0, cs>>>(a, i);
-  if (bits) k_lp_serial<true><<<1, kSerialThreads, smem, cs>>>(a);
-  else k_lp_serial<false><<<1, kSerialThreads, smem, cs>>>(a);
-  k_lp_commit<<<kLpMaxWindow / 128, 128, 0, cs>>>(a);
-  k_lp_advance<<<1, 32, 0, cs>>>(a);
-  const cudaError_t launch_err = cudaGetLastError();
-  cudaGraph_t captured = nullptr;
-  e = cudaStreamEndCapture(cs, &captured);
-  if (launch_err != cudaSuccess) return launch_err;
-  if (e != cudaSuccess) return e;
-  // After the loop: displacement and status.
-  kp.func = (void *)k_lp_finish;
-  kp.gridDim = dim3(1);
-  kp.blockDim = dim3(32);
-  if ((e = cudaGraphAddKernelNode(&n_fin, graph, &n_loop, 1, &kp)) != cudaSuccess) return e;
+  if ((e = add((const void *)k_lp_init, site_grid, 256)) != cudaSuccess) return e;
+  if (a.n_mac) {
+    cudaGraphNodeParams cp = {};
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = a.handle;
+    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.size = 1;
+    cudaGraphNode_t loop;
+    if ((e = cudaGraphAddNode(&loop, graph, &tail, 1, &cp)) != cudaSuccess) return e;
+    tail = loop;
+    // The round, captured into the loop body.
+    if ((e = cudaStreamBeginCaptureToGraph(cs, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                           cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
+      return e;
+    const uint32_t most = a.n_mac < kLpWindow ? a.n_mac : kLpWindow;
+    const unsigned grid = (most + kLpWarps - 1) / kLpWarps;
+    k_lp_choose<<<most, kLpWarps * 32, 0, cs>>>(a);
+    k_lp_claim<<<grid, kLpWarps * 32, 0, cs>>>(a);
+    const cudaError_t launch_err = cudaGetLastError();
+    cudaGraph_t captured = nullptr;
+    e = cudaStreamEndCapture(cs, &captured);
+    if (launch_err != cudaSuccess) return launch_err;
+    if (e != cudaSuccess) return e;
+  }
+  if ((e = add((const void *)k_lp_segments, site_grid, 256)) != cudaSuccess) return e;
+  if (a.n > a.n_mac) {
+    if ((e = add((const void *)k_lp_units, a.n - a.n_mac, kUnitWarps * 32)) != cudaSuccess) return e;
+  }
+  if ((e = add((const void *)k_lp_result, site_grid, 256)) != cudaSuccess) return e;
+  if ((e = add((const void *)k_lp_finish, 1, kSumThreads)) != cudaSuccess) return e;
   return cudaGraphInstantiate(&g.exec, graph, 0);
 }
 

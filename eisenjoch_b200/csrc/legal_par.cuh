@@ -7,20 +7,23 @@
 
 namespace eplace {
 
-// Window capacity (cells per round) and candidate-list capacity per cell.
-constexpr uint32_t kLpMaxWindow = 16384;
-constexpr int kLpList = 64;
-constexpr int kLpPropSteps = 16;  // disturbance propagation passes per round
+// Macros that a round works on at once.
+constexpr uint32_t kLpWindow = 2048;
 
-// Round state, in device memory (one per legalisation in flight).
+// State of one legalisation in flight, in device memory.
 struct LpState {
-  uint32_t pos;       // next order index to place
-  uint32_t bcur;      // window size of the current round
-  uint32_t stop;      // window cells committed this round
-  uint32_t rounds;    // rounds run
-  int32_t status;     // 0 ok, 1 no free site for some cell, 2 round cap, 3 tie group beyond the buffer
-  uint32_t changed[kLpPropSteps + 1];  // propagation pass i found new disturbed cells
-  uint32_t pad_;
+  uint32_t base;       // macros [0, base) have their final anchors
+  uint32_t rounds;     // macro rounds run
+  uint32_t first;      // lowest macro whose choice changed in this round
+  uint32_t ticket;     // CTAs of the claim kernel that have finished
+  uint32_t nfreed[2];  // lengths of the two lists of freed blocks
+  int32_t status;      // 0 ok, 1 no free site for some cell, 2 round cap
+  uint32_t next;       // next unit cell to hand out
+};
+
+// A block that a macro gave up in a round.
+struct LpFreed {
+  int32_t q, tile, w, h;
 };
 
 struct LpArgs {
@@ -28,17 +31,16 @@ struct LpArgs {
   const uint32_t *order;   // [n] legalisation order: macros first, then unit cells, solver order within each
   const uchar2 *fsize;     // [N] footprint (w, h) per cell id, or nullptr when every cell is 1x1
   uint32_t n;              // cells to place
+  uint32_t n_mac;          // macros among them (the first of the order)
   int W, H, WR;            // chip sites, 64-bit words per row
+  int SW;                  // 32-site segments per row
   const uint64_t *free0;   // [H * WR] free map with the fixed cells bound (bit set = free)
-  uint64_t *fm;            // [H * WR] working free map
-  int32_t *list;           // [kLpMaxWindow * kLpList] candidate anchors (tile = y * W + x), best first
-  int32_t *len;            // [kLpMaxWindow] list lengths
-  int32_t *info;           // [kLpMaxWindow] w | h << 8 of the window's cells (written with the lists)
-  int32_t *hmark;          // [W * H] lowest window index whose head block covers the site (INT32_MAX: none)
-  int32_t *dmark;          // [W * H] lowest disturbed window index whose list covers the site
-  uint8_t *dist;           // [kLpMaxWindow] cell must take the serial pass
-  uint8_t *fresh;          // [kLpMaxWindow] disturbed in the last pass, lists not marked yet
-  int32_t *pick;           // [kLpMaxWindow] anchor chosen by the serial pass
+  int32_t *own;            // [H][32 SW] lowest order index that claims the site; -1: never free, or no site
+  uint2 *seg;              // [H][SW] what is known of each 32-site segment (see legal_par.cu)
+  int32_t *choice;         // [n_mac] anchor (tile = y * W + x) of each macro; -1: none yet, -2: none free
+  double *mcost;           // [n_mac] its cost
+  LpFreed *freed;          // [2][kLpWindow] blocks given up in the last and in this round
+  unsigned long long *hint;  // [lp_hint_count] radii without an open anchor (see legal_par.cu)
   LpState *st;
   int2 *sites;             // [N] anchor of every cell (out)
   int2 *loc;               // [N] pin location anchor + (size - 1) / 2 (out), or nullptr
@@ -49,16 +51,18 @@ struct LpArgs {
   cudaGraphConditionalHandle handle;
 };
 
-// Chips the device legaliser takes (tile ids and per-site marks sized by
+// The hints: one entry per size class (1 .. 8 sites) and 16 x 16 sites.
+constexpr int kLpHintClasses = 8;
+inline size_t lp_hint_count(int W, int H) { return (size_t)kLpHintClasses * ((W + 15) / 16) * ((H + 15) / 16); }
+
+// Chips the device legaliser takes (tile ids and per-site claims sized by
 // W x H): up to 4096 x 4096 sites.
 inline bool legalize_supported(int W, int H) { return W > 0 && H > 0 && W <= 4096 && H <= 4096; }
 
-// Device bytes of the round buffers (lists, marks, flags) for a W x H chip.
-size_t lp_scratch_bytes(int W, int H);
-
 // A legalisation as one CUDA graph: initialisation, a device-side while
-// loop over rounds, the displacement sum.  Built once per slot and problem
-// load; launched per checkpoint.
+// loop over the macro rounds (when there are macros), the unit cells, the
+// displacement sum.  Built once per slot and problem load; launched per
+// checkpoint.
 struct LpGraph {
   cudaGraphExec_t exec = nullptr;
   cudaGraph_t graph = nullptr;

@@ -167,3 +167,46 @@ def test_device_legalizer_bench_geometry():
     assert np.array_equal(dx, hx) and np.array_equal(dy, hy)
     assert dd == hd
     assert dh == E.hpwl_host(nl, chip, hx, hy)
+
+
+@pytest.mark.parametrize("w,h", [(31, 40), (32, 33), (33, 32), (64, 64), (70, 45), (257, 40)])
+@pytest.mark.parametrize("macros", ["none", "small", "large"])
+def test_device_legalizer_edges(w, h, macros):
+    """Chips whose width is no multiple of the 32-site segments, blocked
+    sites, and footprints on either side of what the word search takes
+    (32 x 16 sites): all cells on one spot, on two corners, and uniform."""
+    rng = np.random.default_rng(w * 100 + h)
+    sizes = {"none": [(1, 1)] * 8, "small": [(2, 2), (8, 8), (3, 5), (1, 9), (12, 1)],
+             "large": [(32, 16), (31, 17), (16, 30), (1, 31), (31, 1)]}[macros]
+    cw, ch, area = [], [], 0
+    for k in range(4 if macros == "large" else 24):
+        a, b = sizes[k % len(sizes)]
+        if a <= w and b <= h and area + 3 * a * b < w * h // 2:
+            cw.append(a)
+            ch.append(b)
+            area += 3 * a * b  # room for the blocks that fragments cost
+    units = (w * h - area) // 2
+    cw, ch = np.array(cw + [1] * units, np.uint8), np.array(ch + [1] * units, np.uint8)
+    n = len(cw)
+    perm = rng.permutation(n)
+    cw, ch = cw[perm], ch[perm]
+    fx, fy = rng.integers(0, w, 5).astype(np.int32), rng.integers(0, h, 5).astype(np.int32)
+    nl = E.Netlist(num_cells=n, net_offsets=np.array([0, 2], np.uint32), pin_cell=np.array([0, 1], np.uint32),
+                   fixed_x=fx, fixed_y=fy, fixed_on_logic=np.ones(5, np.uint8), cell_w=cw, cell_h=ch)
+    chip = E.Chip(w, h)
+    corner = rng.random(n) < 0.5
+    spots = [(np.full(n, 0.37 * w), np.full(n, 0.61 * h)),
+             (np.where(corner, 0.0, w - 1.0), np.where(corner, 0.0, h - 1.0)),
+             (rng.uniform(0, w - 1, n), rng.uniform(0, h - 1, n))]
+    with E.PlacementContext(nl, chip) as ctx:
+        for x, y in spots:
+            try:
+                hx, hy, hd = ctx.legalize(x, y)
+            except E.NoBelsAvailable:
+                with pytest.raises(E.NoBelsAvailable):
+                    ctx.legalize_device(x, y)
+                continue
+            dx, dy, dd, dh = ctx.legalize_device(x, y)
+            assert np.array_equal(dx, hx) and np.array_equal(dy, hy)
+            assert dd == hd
+            assert dh == E.hpwl_host(nl, chip, hx, hy)
