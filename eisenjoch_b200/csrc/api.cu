@@ -34,6 +34,7 @@
 #include "dct_tc.cuh"
 #include "eplace_internal.h"
 #include "fft.cuh"
+#include "host_copy.h"
 #include "init_place.cuh"
 #include "job.h"
 #include "kernels.cuh"
@@ -310,6 +311,9 @@ struct eplace_ctx {
   // wa_pin_ev marks the end of the last upload from it.
   PinBlock wa_pin;
   cudaEvent_t wa_pin_ev = nullptr;
+  // Pinned blocks of the stage entries: the caller's arrays as the device
+  // reads them, the results as it writes them.
+  PinBlock io_in, io_out;
   uint32_t n_mac = 0;
   // state
   DBuf<float2> look;  // [N + F]
@@ -334,6 +338,7 @@ struct eplace_ctx {
   DBuf<GemmOp> hops;
   DBuf<FlyOp> fops;
   DBuf<double> mom, part, part2, part_b;
+  DBuf<double> io_dens;  // [bins] density map of the density entry
   DBuf<DevScalars> sc;
   DBuf<IterLog> log;
   DBuf<unsigned> bar;  // [0..1] grid barrier, [2] finalise ticket, [3] step ticket
@@ -2376,32 +2381,30 @@ struct JobState {
                        (int)(iters_done - 1), last_overlap);
         // Legalisation is a pure function of the positions and the fixed
         // cells, so the final binding is the best checkpoint's own.
-        std::vector<int32_t> fsx(hp.N), fsy(hp.N);
-        std::vector<float> bx(hp.N), by(hp.N);
+        // One pass writes the caller's arrays.
+        auto put = [&](uint32_t i, int32_t sx, int32_t sy, float x, float y) {
+          res->bel_tile[i] = sy * hp.W + sx;
+          if (res->bel_index) res->bel_index[i] = 0;
+          if (res->x) res->x[i] = x;
+          if (res->y) res->y[i] = y;
+        };
         if (best && gpu_legal) {
           LegalSlot &L = *c->lslots[best->slot];
-          std::vector<int2> sites(hp.N);
-          std::vector<float2> pos(hp.N);
-          CK(cudaMemcpyAsync(sites.data(), L.sites.p, sizeof(int2) * hp.N, cudaMemcpyDeviceToHost, L.stream));
-          CK(cudaMemcpyAsync(pos.data(), L.pos.p, sizeof(float2) * hp.N, cudaMemcpyDeviceToHost, L.stream));
+          c->io_out.reserve((sizeof(int2) + sizeof(float2)) * hp.N);
+          int2 *sites = static_cast<int2 *>(c->io_out.p);
+          float2 *pos = reinterpret_cast<float2 *>(sites + hp.N);
+          CK(cudaMemcpyAsync(sites, L.sites.p, sizeof(int2) * hp.N, cudaMemcpyDeviceToHost, L.stream));
+          CK(cudaMemcpyAsync(pos, L.pos.p, sizeof(float2) * hp.N, cudaMemcpyDeviceToHost, L.stream));
           g_d2h += (sizeof(int2) + sizeof(float2)) * hp.N;
           CK(cudaStreamSynchronize(L.stream));
-          for (uint32_t i = 0; i < hp.N; ++i) {
-            fsx[i] = sites[i].x;
-            fsy[i] = sites[i].y;
-            bx[i] = pos[i].x;
-            by[i] = pos[i].y;
-          }
+          for (uint32_t i = 0; i < hp.N; ++i) put(i, sites[i].x, sites[i].y, pos[i].x, pos[i].y);
           res->best_iter = best->iter;
+          res->hpwl = best->hpwl;
         } else if (best) {
           const HostSnap &h = *best->hs;
-          std::copy(h.sx.begin(), h.sx.begin() + hp.N, fsx.begin());
-          std::copy(h.sy.begin(), h.sy.begin() + hp.N, fsy.begin());
-          for (uint32_t i = 0; i < hp.N; ++i) {
-            bx[i] = h.pos[i].x;
-            by[i] = h.pos[i].y;
-          }
+          for (uint32_t i = 0; i < hp.N; ++i) put(i, h.sx[i], h.sy[i], h.pos[i].x, h.pos[i].y);
           res->best_iter = best->iter;
+          res->hpwl = best->hpwl;
         } else {
           if (isx.empty()) {  // the device made the initial placement
             std::vector<int2> site(hp.N);
@@ -2414,10 +2417,8 @@ struct JobState {
               isy[i] = site[i].y;
             }
           }
-          for (uint32_t i = 0; i < hp.N; ++i) {
-            bx[i] = (float)isx[i];
-            by[i] = (float)isy[i];
-          }
+          std::vector<int32_t> fsx(hp.N), fsy(hp.N);
+          std::vector<float> bx(isx.begin(), isx.end()), by(isy.begin(), isy.end());
           double d = 0.0;
           if (!c->lbase) c->lbase.reset(new LegalBase(hp));
           if (c->legal.empty()) c->legal.emplace_back(new Legalizer(hp, *c->lbase));
@@ -2425,16 +2426,10 @@ struct JobState {
           if (ls != EPLACE_OK) {
             final_st = ls;
             set_err(c, "logic");
+          } else {
+            for (uint32_t i = 0; i < hp.N; ++i) put(i, fsx[i], fsy[i], bx[i], by[i]);
+            res->hpwl = hpwl_host(hp, fsx.data(), fsy.data());
           }
-        }
-        if (final_st == EPLACE_OK) {
-          for (uint32_t i = 0; i < hp.N; ++i) {
-            res->bel_tile[i] = fsy[i] * hp.W + fsx[i];
-            if (res->bel_index) res->bel_index[i] = 0;
-            if (res->x) res->x[i] = bx[i];
-            if (res->y) res->y[i] = by[i];
-          }
-          res->hpwl = best ? best->hpwl : hpwl_host(hp, fsx.data(), fsy.data());
         }
       } catch (const CudaError &e) {
         final_st = cuda_fail(c, e);
@@ -2635,7 +2630,7 @@ uint64_t eplace_ctx::device_bytes() const {
   add(half); add(area); add(mflag); add(mac_idx); add(pw); add(look); add(x); add(xp); add(g); add(gprev); add(tmp_wl); add(tmp_den);
   add(acc); add(dens); add(rho); add(T); add(Exh); add(Eyh); add(U); add(V); add(Ex); add(Ey); add(phi);
   add(mB1); add(mL2); add(mB3); add(mL4); add(mB5); add(mL6); add(mB3g); add(mL6g);
-  add(wx); add(gx2); add(wy); add(gy2); add(ops); add(mom); add(part); add(part2); add(part_b);
+  add(wx); add(gx2); add(wy); add(gy2); add(ops); add(mom); add(part); add(part2); add(part_b); add(io_dens);
   add(sc); add(log); add(bar); add(loc); add(hp_total);
   for (const auto &d : snap_pos) add(*d);
   for (const auto &d : snap_sc) add(*d);
@@ -2819,11 +2814,48 @@ eplace_status eplace_profile_stages(eplace_ctx *c, const eplace_cfg *cfg, const 
 // ---------------------------------------------------------------------------
 // Stage entry points (host buffers in/out, one kernel family each).
 // ---------------------------------------------------------------------------
-static void upload_look(eplace_ctx *c, const float *x, const float *y) {
-  AllocOn on_stream(c->stream);
-  std::vector<float2> p(c->hp.N);
-  for (uint32_t i = 0; i < c->hp.N; ++i) p[i] = make_float2(x[i], y[i]);
-  if (c->hp.N) CK(cudaMemcpyAsync(c->look.p, p.data(), sizeof(float2) * c->hp.N, cudaMemcpyHostToDevice, c->stream));
+// Arrays of n 4-byte values in a pinned block, each starting on a 256-byte
+// boundary.
+static size_t io_pitch(size_t n) { return (n + 63) & ~(size_t)63; }
+
+static IoArgs io_args(const eplace_ctx *c, void *host, std::initializer_list<float2 *> pairs) {
+  IoArgs a{};
+  a.n = c->hp.N;
+  a.pitch = io_pitch(c->hp.N);
+  a.host = static_cast<float *>(host);
+  for (float2 *p : pairs) a.pair[a.pairs++] = p;
+  return a;
+}
+
+// The caller's (x, y) arrays into (x, y) pairs on the device: through the
+// pinned block `at`, read there by the device.  acc / scale as launch_io_in.
+static void io_in(eplace_ctx *c, cudaStream_t s, float *at, std::initializer_list<std::pair<const void *, const void *>> xy,
+                  std::initializer_list<float2 *> to, unsigned long long *acc = nullptr, double scale = 0.0) {
+  IoArgs a = io_args(c, at, to);
+  a.acc = acc;
+  a.scale = scale;
+  const size_t bytes = sizeof(float) * c->hp.N;
+  size_t k = 0;
+  for (const auto &p : xy) {
+    HostCopy::get().run({{at + k * a.pitch, p.first, bytes}, {at + (k + 1) * a.pitch, p.second, bytes}});
+    k += 2;
+  }
+  CK(launch_io_in(a, s));
+  g_h2d += 2 * bytes * a.pairs;
+}
+
+// Pairs on the device into the pinned block; the caller waits for the stream
+// and then copies them on.
+static IoArgs io_out(eplace_ctx *c, cudaStream_t s, std::initializer_list<float2 *> from,
+                     unsigned long long *acc = nullptr, double scale = 0.0) {
+  IoArgs a = io_args(c, nullptr, from);
+  c->io_out.reserve(sizeof(float) * 2 * a.pairs * a.pitch + 1024);
+  a.host = static_cast<float *>(c->io_out.p);
+  a.acc = acc;
+  a.scale = scale;
+  CK(launch_io_out(a, s));
+  g_d2h += 2 * sizeof(float) * c->hp.N * a.pairs;
+  return a;
 }
 
 eplace_status eplace_stage_wa_grad(eplace_ctx *c, double wl_coeff, const float *x, const float *y, float *gx,
@@ -2831,22 +2863,13 @@ eplace_status eplace_stage_wa_grad(eplace_ctx *c, double wl_coeff, const float *
   if (!c || (c->hp.N && (!x || !y || !gx || !gy))) return EPLACE_ERR_INVALID;
   try {
     CK(cudaSetDevice(c->device));
-    upload_look(c, x, y);
-    c->acc.zero(c->stream);
+    const size_t bytes = sizeof(float) * c->hp.N;
+    c->io_in.reserve(2 * sizeof(float) * io_pitch(c->hp.N));
+    io_in(c, c->stream, static_cast<float *>(c->io_in.p), {{x, y}}, {c->look.p}, c->acc.p);
     launch_wa_stage(c, (float)wl_coeff);
-    std::vector<unsigned long long> acc((size_t)c->hp.N);
-    if (c->hp.N)
-      CK(cudaMemcpyAsync(acc.data(), c->acc.p, sizeof(unsigned long long) * acc.size(), cudaMemcpyDeviceToHost,
-                         c->stream));
-    c->acc.zero(c->stream);
+    const IoArgs o = io_out(c, c->stream, {nullptr}, c->acc.p, std::ldexp(1.0, -c->grad_k));
     CK(cudaStreamSynchronize(c->stream));
-    const double inv = std::ldexp(1.0, -c->grad_k);
-    for (uint32_t i = 0; i < c->hp.N; ++i) {
-      long long sx, sy;
-      unpack_grad(acc[i], &sx, &sy);
-      gx[i] = (float)((double)sx * inv);
-      gy[i] = (float)((double)sy * inv);
-    }
+    HostCopy::get().run({{gx, o.host, bytes}, {gy, o.host + o.pitch, bytes}});
   } catch (const CudaError &e) {
     return cuda_fail(c, e);
   }
@@ -2859,17 +2882,22 @@ eplace_status eplace_stage_density(eplace_ctx *c, const float *x, const float *y
   try {
     CK(cudaSetDevice(c->device));
     const size_t nb = (size_t)c->hp.BX * c->hp.BY;
-    DBuf<double> dout;
-    dout.alloc(nb);
+    AllocOn on_stream(c->stream);
+    c->io_dens.ensure(nb);
     DevScalars sc{};
     c->sc.upload(&sc, 1, c->stream);
-    upload_look(c, x, y);
+    c->io_in.reserve(2 * sizeof(float) * io_pitch(c->hp.N));
+    io_in(c, c->stream, static_cast<float *>(c->io_in.p), {{x, y}}, {c->look.p});
     c->dens.zero(c->stream);
     launch_scatter_stage(c);
-    launch_final_stage(c, dout.p);
-    CK(cudaMemcpyAsync(density, dout.p, sizeof(double) * nb, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(&sc, c->sc.p, sizeof(sc), cudaMemcpyDeviceToHost, c->stream));
+    launch_final_stage(c, c->io_dens.p);
+    c->io_out.reserve(sizeof(double) * nb + sizeof(sc));
+    double *d = static_cast<double *>(c->io_out.p);
+    CK(cudaMemcpyAsync(d, c->io_dens.p, sizeof(double) * nb, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(d + nb, c->sc.p, sizeof(sc), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    HostCopy::get().run({{density, d, sizeof(double) * nb}});
+    std::memcpy(&sc, d + nb, sizeof(sc));
     if (overlap) *overlap = sc.overlap;
   } catch (const CudaError &e) {
     return cuda_fail(c, e);
@@ -2891,41 +2919,65 @@ eplace_status eplace_stage_field(eplace_ctx *c, const double *density, int32_t d
   c->fft = dct_mode == EPLACE_DCT_FP32_FFT && fft_supported(c->hp.BX, c->hp.BY);
   try {
     CK(cudaSetDevice(c->device));
+    cudaStream_t s = c->stream;
     const size_t nb = (size_t)c->hp.BX * c->hp.BY;
     const double c0 = c->total_area / (double)nb;
-    std::vector<float> rho(nb);
-    for (size_t i = 0; i < nb; ++i) rho[i] = (float)(density[i] - c0);
     if (tc) {
       setup_tc(c);
-      std::vector<__nv_bfloat16> h(nb), l(nb);
-      for (size_t i = 0; i < nb; ++i) {
-        h[i] = __float2bfloat16_rn(rho[i]);
-        l[i] = __float2bfloat16_rn(rho[i] - __bfloat162float(h[i]));
-      }
-      c->rho_h.upload(h.data(), nb, c->stream);
-      c->rho_l.upload(l.data(), nb, c->stream);
       DevScalars sc{};
-      c->sc.upload(&sc, 1, c->stream);
-    } else {
-      c->rho.upload(rho.data(), nb, c->stream);
+      c->sc.upload(&sc, 1, s);
     }
-    DBuf<float> phi;
-    if (phi_hat) phi.alloc(nb);
-    launch_field_stage(c, phi_hat ? phi.p : nullptr, field_mode, tc);
-    CK(cudaMemcpyAsync(ex, c->Ex.p, sizeof(float) * nb, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(ey, c->Ey.p, sizeof(float) * nb, cudaMemcpyDeviceToHost, c->stream));
-    if (phi_hat) CK(cudaMemcpyAsync(phi_hat, phi.p, sizeof(float) * nb, cudaMemcpyDeviceToHost, c->stream));
-    DevScalars sc{};
-    CK(cudaMemcpyAsync(&sc, c->sc.p, sizeof(sc), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    if (tc && sc.err) {
-      set_err(c, "a bounded device wait timed out in the tensor-core transform");
-      return EPLACE_ERR_TIMEOUT;
+    c->io_in.reserve(sizeof(double) * nb);
+    double *d = static_cast<double *>(c->io_in.p);
+    // 2 MB at a time: the device reads one piece while the next is copied
+    constexpr size_t kPiece = 256 << 10;
+    for (size_t at = 0; at < nb; at += kPiece) {
+      const size_t n = std::min(kPiece, nb - at);
+      HostCopy::get().run({{d + at, density + at, sizeof(double) * n}});
+      CK(launch_io_rho(d + at, n, c0, tc ? nullptr : c->rho.p + at, tc ? c->rho_h.p + at : nullptr,
+                       tc ? c->rho_l.p + at : nullptr, s));
+    }
+    g_h2d += sizeof(double) * nb;
+    AllocOn on_stream(s);
+    if (phi_hat) c->phi.ensure(nb);
+    launch_field_stage(c, phi_hat ? c->phi.p : nullptr, field_mode, tc);
+    const size_t bytes = sizeof(float) * nb, pitch = io_pitch(nb);
+    c->io_out.reserve(sizeof(float) * 3 * pitch + sizeof(DevScalars));
+    float *h = static_cast<float *>(c->io_out.p);
+    // Ex is copied on while Ey is on the bus.
+    CK(cudaMemcpyAsync(h, c->Ex.p, bytes, cudaMemcpyDeviceToHost, s));
+    CK(cudaEventRecord(c->ev_fork, s));
+    CK(cudaMemcpyAsync(h + pitch, c->Ey.p, bytes, cudaMemcpyDeviceToHost, s));
+    if (phi_hat) CK(cudaMemcpyAsync(h + 2 * pitch, c->phi.p, bytes, cudaMemcpyDeviceToHost, s));
+    if (tc) CK(cudaMemcpyAsync(h + 3 * pitch, c->sc.p, sizeof(DevScalars), cudaMemcpyDeviceToHost, s));
+    g_d2h += bytes * (phi_hat ? 3 : 2);
+    CK(cudaEventSynchronize(c->ev_fork));
+    HostCopy::get().run({{ex, h, bytes}});
+    CK(cudaStreamSynchronize(s));
+    if (phi_hat) HostCopy::get().run({{ey, h + pitch, bytes}, {phi_hat, h + 2 * pitch, bytes}});
+    else HostCopy::get().run({{ey, h + pitch, bytes}});
+    if (tc) {
+      DevScalars sc;
+      std::memcpy(&sc, h + 3 * pitch, sizeof(sc));
+      if (sc.err) {
+        set_err(c, "a bounded device wait timed out in the tensor-core transform");
+        return EPLACE_ERR_TIMEOUT;
+      }
     }
   } catch (const CudaError &e) {
     return cuda_fail(c, e);
   }
   return EPLACE_OK;
+}
+
+// The field maps of the gather and step entries into Ex and Ey, through the
+// pinned block at h (2 io_pitch(bins) values).
+static void io_field(eplace_ctx *c, float *h, const float *ex, const float *ey) {
+  const size_t nb = (size_t)c->hp.BX * c->hp.BY, bytes = sizeof(float) * nb;
+  HostCopy::get().run({{h, ex, bytes}, {h + io_pitch(nb), ey, bytes}});
+  CK(cudaMemcpyAsync(c->Ex.p, h, bytes, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(c->Ey.p, h + io_pitch(nb), bytes, cudaMemcpyHostToDevice, c->stream));
+  g_h2d += 2 * bytes;
 }
 
 eplace_status eplace_stage_gather(eplace_ctx *c, const float *x, const float *y, const float *ex, const float *ey,
@@ -2936,37 +2988,21 @@ eplace_status eplace_stage_gather(eplace_ctx *c, const float *x, const float *y,
   try {
     CK(cudaSetDevice(c->device));
     const HostProblem &hp = c->hp;
-    const size_t nb = (size_t)hp.BX * hp.BY;
-    upload_look(c, x, y);
-    c->Ex.upload(ex, nb, c->stream);
-    c->Ey.upload(ey, nb, c->stream);
+    const size_t nb = (size_t)hp.BX * hp.BY, bytes = sizeof(float) * hp.N;
+    c->io_in.reserve(2 * sizeof(float) * (io_pitch(nb) + io_pitch(hp.N)));
+    float *h = static_cast<float *>(c->io_in.p);
+    io_field(c, h, ex, ey);
+    io_in(c, c->stream, h + 2 * io_pitch(nb), {{x, y}}, {c->look.p});
     StepArgs a = step_args(c);
     a.mode = 1;
     CK(launch_step(a, c->step_grid, c->stream));
-    std::vector<float2> t(hp.N);
-    if (hp.N) CK(cudaMemcpyAsync(t.data(), c->tmp_den.p, sizeof(float2) * hp.N, cudaMemcpyDeviceToHost, c->stream));
+    const IoArgs o = io_out(c, c->stream, {c->tmp_den.p});
     CK(cudaStreamSynchronize(c->stream));
-    for (uint32_t i = 0; i < hp.N; ++i) {
-      gx[i] = t[i].x;
-      gy[i] = t[i].y;
-    }
+    HostCopy::get().run({{gx, o.host, bytes}, {gy, o.host + o.pitch, bytes}});
   } catch (const CudaError &e) {
     return cuda_fail(c, e);
   }
   return EPLACE_OK;
-}
-
-static std::vector<float2> pack2(const float *a, const float *b, size_t n) {
-  std::vector<float2> v(n);
-  for (size_t i = 0; i < n; ++i) v[i] = make_float2(a[i], b[i]);
-  return v;
-}
-
-static void unpack2(const std::vector<float2> &v, float *a, float *b) {
-  for (size_t i = 0; i < v.size(); ++i) {
-    a[i] = v[i].x;
-    b[i] = v[i].y;
-  }
 }
 
 eplace_status eplace_stage_step(eplace_ctx *c, uint64_t iter, const float *look_x, const float *look_y,
@@ -2986,19 +3022,12 @@ eplace_status eplace_stage_step(eplace_ctx *c, uint64_t iter, const float *look_
     cudaStream_t s = c->stream;
     ensure_log(c, iter + 2);
     upload_momentum(c, iter + 2);
-    upload_look(c, look_x, look_y);
-    c->Ex.upload(ex, nb, s);
-    c->Ey.upload(ey, nb, s);
-    std::vector<unsigned long long> acc((size_t)N);
-    const double scale = std::ldexp(1.0, c->grad_k);
-    for (uint32_t i = 0; i < N; ++i)
-      acc[i] = pack_grad(llrint((double)gwl_x[i] * scale), llrint((double)gwl_y[i] * scale));
-    if (N)
-      CK(cudaMemcpyAsync(c->acc.p, acc.data(), sizeof(unsigned long long) * acc.size(), cudaMemcpyHostToDevice, s));
-    std::vector<float2> vx = pack2(x, y, N), vxp = pack2(x_prev, y_prev, N), vg = pack2(gprev_x, gprev_y, N);
-    c->x.upload(vx.data(), N, s);
-    c->xp.upload(vxp.data(), N, s);
-    c->gprev.upload(vg.data(), N, s);
+    const size_t bytes = sizeof(float) * N;
+    c->io_in.reserve(sizeof(float) * (2 * io_pitch(nb) + 10 * io_pitch(N)));
+    float *h = static_cast<float *>(c->io_in.p);
+    io_in(c, s, h, {{look_x, look_y}, {gwl_x, gwl_y}, {x, y}, {x_prev, y_prev}, {gprev_x, gprev_y}},
+          {c->look.p, nullptr, c->x.p, c->xp.p, c->gprev.p}, c->acc.p, std::ldexp(1.0, c->grad_k));
+    io_field(c, h + 10 * io_pitch(N), ex, ey);
     DevScalars sc{};
     sc.lam = scal[0];
     sc.lam_init = scal[1] != 0.0;
@@ -3008,25 +3037,23 @@ eplace_status eplace_stage_step(eplace_ctx *c, uint64_t iter, const float *look_
     c->sc.upload(&sc, 1, s);
     c->bar.zero(s);
     launch_step_stage(c);
-    std::vector<float2> lk(N);
-    if (N) {
-      CK(cudaMemcpyAsync(vx.data(), c->x.p, sizeof(float2) * N, cudaMemcpyDeviceToHost, s));
-      CK(cudaMemcpyAsync(vxp.data(), c->xp.p, sizeof(float2) * N, cudaMemcpyDeviceToHost, s));
-      CK(cudaMemcpyAsync(vg.data(), c->gprev.p, sizeof(float2) * N, cudaMemcpyDeviceToHost, s));
-      CK(cudaMemcpyAsync(lk.data(), c->look.p, sizeof(float2) * N, cudaMemcpyDeviceToHost, s));
-    }
+    const IoArgs o = io_out(c, s, {c->x.p, c->xp.p, c->gprev.p, c->look.p});
+    // the log entry and the scalars after the arrays (1 KB is kept for them)
+    char *tail = reinterpret_cast<char *>(o.host + 8 * o.pitch);
     IterLog L{};
-    CK(cudaMemcpyAsync(&L, c->log.p + iter, sizeof(L), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(&sc, c->sc.p, sizeof(sc), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(tail, c->log.p + iter, sizeof(L), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(tail + 512, c->sc.p, sizeof(sc), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    std::memcpy(&L, tail, sizeof(L));
+    std::memcpy(&sc, tail + 512, sizeof(sc));
     if (sc.err) {
       set_err(c, "a bounded device wait timed out");
       return EPLACE_ERR_TIMEOUT;
     }
-    unpack2(vx, x, y);
-    unpack2(vxp, x_prev, y_prev);
-    unpack2(vg, gprev_x, gprev_y);
-    unpack2(lk, next_look_x, next_look_y);
+    auto at = [&](int k) { return o.host + k * o.pitch; };
+    HostCopy::get().run({{x, at(0), bytes}, {y, at(1), bytes}, {x_prev, at(2), bytes}, {y_prev, at(3), bytes},
+                         {gprev_x, at(4), bytes}, {gprev_y, at(5), bytes}, {next_look_x, at(6), bytes},
+                         {next_look_y, at(7), bytes}});
     scal[0] = sc.lam;
     scal[1] = sc.lam_init;
     scal[2] = sc.step[0];
@@ -3103,13 +3130,10 @@ eplace_status eplace_stage_initial_placement(eplace_ctx *c, uint64_t seed, int32
       }
     } else if (st == EPLACE_OK && hp.N) {
       ip_device_launch(c, seed);
-      std::vector<int2> site(hp.N);
-      CK(cudaMemcpyAsync(site.data(), c->ip_site.p, sizeof(int2) * hp.N, cudaMemcpyDeviceToHost, c->stream));
+      const IoArgs o = io_out(c, c->stream, {reinterpret_cast<float2 *>(c->ip_site.p)});  // moved as they are
       CK(cudaStreamSynchronize(c->stream));
-      for (uint32_t i = 0; i < hp.N; ++i) {
-        sx[i] = site[i].x;
-        sy[i] = site[i].y;
-      }
+      const size_t bytes = sizeof(int32_t) * hp.N;
+      HostCopy::get().run({{sx, o.host, bytes}, {sy, o.host + o.pitch, bytes}});
     }
     if (st != EPLACE_OK) set_err(c, msg);
     return st;
@@ -3173,23 +3197,18 @@ eplace_status eplace_stage_legalize(eplace_ctx *c, const float *x, const float *
     setup_gpu_legal(c);
     LegalSlot *L = c->lslots.empty() ? new_legal_slot(c) : c->lslots[0].get();
     prepare_slot(c, *L);
-    std::vector<float2> p = pack2(x, y, hp.N);
-    CK(cudaMemcpyAsync(L->pos.p, p.data(), sizeof(float2) * hp.N, cudaMemcpyHostToDevice, L->stream));
-    g_h2d += sizeof(float2) * hp.N;
+    c->io_in.reserve(2 * sizeof(float) * io_pitch(hp.N));
+    io_in(c, L->stream, static_cast<float *>(c->io_in.p), {{x, y}}, {L->pos.p});
     launch_gpu_legal(c, *L);
-    std::vector<int2> s(hp.N);
-    CK(cudaMemcpyAsync(s.data(), L->sites.p, sizeof(int2) * hp.N, cudaMemcpyDeviceToHost, L->stream));
-    g_d2h += sizeof(int2) * hp.N;
+    const IoArgs io = io_out(c, L->stream, {reinterpret_cast<float2 *>(L->sites.p)});  // moved as they are
     CK(cudaStreamSynchronize(L->stream));
     const LegalOut &o = *L->hout.p;
     if (o.status != 0) {
       set_err(c, o.status == 1 ? "logic" : "device legaliser stopped at an internal limit");
       return o.status == 1 ? EPLACE_ERR_NO_BELS : EPLACE_ERR_PLACEMENT_FAILED;
     }
-    for (uint32_t i = 0; i < hp.N; ++i) {
-      sx[i] = s[i].x;
-      sy[i] = s[i].y;
-    }
+    const size_t bytes = sizeof(int32_t) * hp.N;
+    HostCopy::get().run({{sx, io.host, bytes}, {sy, io.host + io.pitch, bytes}});
     if (disp) *disp = o.disp;
     if (hpwl) *hpwl = (int64_t)o.hpwl;
   } catch (const CudaError &e) {

@@ -200,6 +200,29 @@ cudaError_t launch_step_split(const StepArgs &a, int grid, cudaStream_t s);
 int step_max_grid(int device);
 cudaError_t launch_hpwl(const HpwlArgs &a, int grid, cudaStream_t s);
 
+// The stage entries' arrays: x and y apart in pinned host memory, which the
+// kernels read and write over the bus, (x, y) pairs on the device.
+constexpr int kIoPairs = 5;
+struct IoArgs {
+  uint32_t n;
+  size_t pitch;                    // elements from one host array to the next (a multiple of 4)
+  float *host;                     // [2 pairs][pitch]: x and y of pair 0, of pair 1, ...
+  int pairs;
+  float2 *pair[kIoPairs];
+  unsigned long long *acc;         // packed WA gradient, or nullptr (see the launches)
+  double scale;
+};
+// pair[k][i] = (host[2k][i], host[2k + 1][i]).  With acc and scale 0: acc
+// zeroed; with acc and a scale: pair[1] is the WA gradient, packed into acc.
+cudaError_t launch_io_in(const IoArgs &a, cudaStream_t s);
+// The other way.  With acc: pair 0 comes from the packed gradient times scale
+// and acc is zeroed.
+cudaError_t launch_io_out(const IoArgs &a, cudaStream_t s);
+// rho = d - c0 of n density values in pinned host memory, FP32 or as BF16
+// hi / lo planes (rho == nullptr).
+cudaError_t launch_io_rho(const double *d, size_t n, double c0, float *rho, __nv_bfloat16 *hi, __nv_bfloat16 *lo,
+                          cudaStream_t s);
+
 constexpr int kWaBlock = 256;
 constexpr int kScatterBlock = 256;
 constexpr int kFinalBlock = 256;

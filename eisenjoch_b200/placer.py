@@ -364,15 +364,13 @@ class PlacementResult:
 
 class _ResultBuffers:
     def __init__(self, n, width, traj_cap):
-        self.bel_tile = np.zeros(n, np.int32)
-        self.bel_index = np.zeros(n, np.int32)
-        self.x = np.zeros(n, np.float32)
-        self.y = np.zeros(n, np.float32)
+        self.bel_tile = np.empty(n, np.int32)
+        self.x = np.empty(n, np.float32)
+        self.y = np.empty(n, np.float32)
         self.traj = (_abi.TrajEntry * max(1, traj_cap))()
         self.width = width
         r = _abi.Result()
         r.bel_tile = _abi.ptr(self.bel_tile, ctypes.c_int32)
-        r.bel_index = _abi.ptr(self.bel_index, ctypes.c_int32)
         r.x = _abi.ptr(self.x, ctypes.c_float)
         r.y = _abi.ptr(self.y, ctypes.c_float)
         r.traj = ctypes.cast(self.traj, P(_abi.TrajEntry))
@@ -388,12 +386,13 @@ class _ResultBuffers:
                 dict(iter=t.iter, hpwl=t.hpwl, disp=t.displacement, step_x=t.step_x, step_y=t.step_y,
                      density_penalty=t.density_penalty, overlap=t.overlap)
             )
+        bel_y = self.bel_tile // self.width
         return PlacementResult(
-            bel_tile=self.bel_tile.copy(),
-            bel_x=self.bel_tile % self.width,
-            bel_y=self.bel_tile // self.width,
-            x=self.x.copy(),
-            y=self.y.copy(),
+            bel_tile=self.bel_tile,
+            bel_x=self.bel_tile - bel_y * self.width,
+            bel_y=bel_y,
+            x=self.x,
+            y=self.y,
             hpwl=int(r.hpwl),
             overlap=float(r.overlap),
             iters=int(r.iters),
@@ -469,7 +468,7 @@ class PlacementContext:
     def wa_grad(self, x, y, wl_coeff=0.5):
         n = self.netlist.num_cells
         x, y = _abi.f32(x), _abi.f32(y)
-        gx, gy = np.zeros(n, np.float32), np.zeros(n, np.float32)
+        gx, gy = np.empty(n, np.float32), np.empty(n, np.float32)
         F = ctypes.c_float
         self._check(self._lib.eplace_stage_wa_grad(self.handle, wl_coeff, _abi.ptr(x, F), _abi.ptr(y, F),
                                                    _abi.ptr(gx, F), _abi.ptr(gy, F)))
@@ -478,7 +477,7 @@ class PlacementContext:
     def density(self, x, y):
         by, bx = self.bins
         x, y = _abi.f32(x), _abi.f32(y)
-        d = np.zeros((by, bx), np.float64)
+        d = np.empty((by, bx), np.float64)
         ov = ctypes.c_double()
         F = ctypes.c_float
         self._check(self._lib.eplace_stage_density(self.handle, _abi.ptr(x, F), _abi.ptr(y, F),
@@ -488,8 +487,8 @@ class PlacementContext:
     def field(self, density, dct_mode=_abi.EPLACE_DCT_FP32_FFT, want_phi=False, field_mode=_abi.EPLACE_FIELD_REFERENCE):
         by, bx = self.bins
         d = _abi.f64(density).reshape(by, bx)
-        ex, ey = np.zeros((by, bx), np.float32), np.zeros((by, bx), np.float32)
-        phi = np.zeros((by, bx), np.float32) if want_phi else None
+        ex, ey = np.empty((by, bx), np.float32), np.empty((by, bx), np.float32)
+        phi = np.empty((by, bx), np.float32) if want_phi else None
         F = ctypes.c_float
         self._check(self._lib.eplace_stage_field(self.handle, _abi.ptr(d, ctypes.c_double), dct_mode, field_mode,
                                                  _abi.ptr(ex, F), _abi.ptr(ey, F), _abi.ptr(phi, F)))
@@ -499,7 +498,7 @@ class PlacementContext:
         n = self.netlist.num_cells
         F = ctypes.c_float
         x, y, ex, ey = _abi.f32(x), _abi.f32(y), _abi.f32(ex), _abi.f32(ey)
-        gx, gy = np.zeros(n, np.float32), np.zeros(n, np.float32)
+        gx, gy = np.empty(n, np.float32), np.empty(n, np.float32)
         self._check(self._lib.eplace_stage_gather(self.handle, _abi.ptr(x, F), _abi.ptr(y, F), _abi.ptr(ex, F),
                                                   _abi.ptr(ey, F), _abi.ptr(gx, F), _abi.ptr(gy, F)))
         return gx, gy
@@ -512,10 +511,18 @@ class PlacementContext:
         n = self.netlist.num_cells
         F = ctypes.c_float
         arrs = [_abi.f32(a) for a in (look_x, look_y, gwl_x, gwl_y, ex, ey)]
-        st = {k: _abi.f32(state[k]).copy() for k in ("x", "y", "x_prev", "y_prev", "gprev_x", "gprev_y")}
+        # one block for the state that the call updates and the next look-ahead
+        block = np.empty((8, n), np.float32)
+        st = dict(zip(("x", "y", "x_prev", "y_prev", "gprev_x", "gprev_y"), block))
+        for k in st:
+            a = _abi.f32(state[k])
+            if a.shape == (n,):
+                st[k][:] = a
+            else:
+                st[k] = a.copy()
         sc = np.array(scal, np.float64)
         out = np.zeros(4, np.float64)
-        nlx, nly = np.zeros(n, np.float32), np.zeros(n, np.float32)
+        nlx, nly = block[6], block[7]
         self._check(self._lib.eplace_stage_step(
             self.handle, it, *[_abi.ptr(a, F) for a in arrs],
             *[_abi.ptr(st[k], F) for k in ("x", "y", "x_prev", "y_prev", "gprev_x", "gprev_y")],
@@ -557,7 +564,7 @@ class PlacementContext:
         binding: (site_x, site_y, displacement, hpwl)."""
         n = self.netlist.num_cells
         x, y = _abi.f32(x), _abi.f32(y)
-        sx, sy = np.zeros(n, np.int32), np.zeros(n, np.int32)
+        sx, sy = np.empty(n, np.int32), np.empty(n, np.int32)
         d, h = ctypes.c_double(), ctypes.c_int64()
         F = ctypes.c_float
         self._check(self._lib.eplace_stage_legalize(self.handle, _abi.ptr(x, F), _abi.ptr(y, F),
