@@ -341,6 +341,7 @@ struct eplace_ctx {
   DBuf<double> io_dens;  // [bins] density map of the density entry
   DBuf<DevScalars> sc;
   DBuf<IterLog> log;
+  DBuf<unsigned long long> dsum;  // [2] the overlap's sums (zero between launches)
   DBuf<unsigned> bar;  // [0..1] grid barrier, [2] finalise ticket, [3] step ticket
   DBuf<int2> loc;
   DBuf<unsigned long long> hp_total;
@@ -981,12 +982,15 @@ void setup_tc(eplace_ctx *c) {
 
 int *err_ptr(eplace_ctx *c) { return reinterpret_cast<int *>(reinterpret_cast<char *>(c->sc.p) + offsetof(DevScalars, err)); }
 
+// Sites per bin as a fixed-point density.
+unsigned long long cap_fix(const HostProblem &hp) { return (unsigned long long)hp.sx * (unsigned long long)hp.sy << 32; }
+
 void launch_final_stage(eplace_ctx *c, double *dens_out, bool tc = false) {
   const HostProblem &hp = c->hp;
   const int nb = hp.BX * hp.BY;
   const double c0 = c->total_area / (double)nb;
-  FinalArgs a{c->dens.p, nb, (double)hp.sx * hp.sy, c0, tc ? nullptr : c->rho.p, tc ? c->rho_h.p : nullptr,
-              tc ? c->rho_l.p : nullptr, dens_out, 0, c->part.p, c->bar.p + 2, c->sc.p, c->log.p};
+  FinalArgs a{c->dens.p, nb, cap_fix(hp), c0, tc ? nullptr : c->rho.p, tc ? c->rho_h.p : nullptr,
+              tc ? c->rho_l.p : nullptr, dens_out, 0, c->dsum.p, c->bar.p + 2, nullptr, c->sc.p, c->log.p};
   CK(launch_density_final(a, grid_for((nb + 3) / 4, kFinalBlock, c->num_sms * 4), c->stream));
 }
 
@@ -1046,9 +1050,9 @@ void launch_field_gemm(eplace_ctx *c, int g, float *phi, int field_mode, bool tc
         a.out_a = c->T.p;
         if (from_dens) {
           a.dens = c->dens.p;
-          a.cap = (double)c->hp.sx * c->hp.sy;
+          a.cap = cap_fix(c->hp);
           a.c0 = c->total_area / ((double)W * H);
-          a.part = c->part.p;
+          a.sums = c->dsum.p;
           a.ticket = c->bar.p + 2;
           a.sc = c->sc.p;
           a.log = c->log.p;
@@ -1557,6 +1561,7 @@ void load_into(eplace_ctx *c, HostProblem &&hp_in) {
   c->part2.ensure(2 * (size_t)c->step_grid + 8);
   c->part_b.ensure(4 * (size_t)c->step_grid + 8);
   c->bar.zero(s);
+  c->dsum.zero(s);
   c->loc.ensure((size_t)hp.N + hp.F + 1);
   std::vector<int2> floc(hp.F);
   for (uint32_t f = 0; f < hp.F; ++f) floc[f] = make_int2(hp.fx[f], hp.fy[f]);
@@ -1771,6 +1776,7 @@ static int reset_state(eplace_ctx *c, const std::vector<int32_t> &sx, const std:
   sc.spin_cycles = c->spin_cycles;
   c->sc.upload(&sc, 1, s);
   c->bar.zero(s);
+  c->dsum.zero(s);
   int launches = 0;
   if (sx.empty() && hp.N) {
     launches = ip_device_launch(c, cfg->seed);
@@ -2597,6 +2603,7 @@ eplace_ctx *ctx_new(int32_t device, eplace_status *st) {
     CK(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device));
     c->sc.alloc(1);
     c->bar.alloc(4);
+    c->dsum.alloc(2);
     c->hp_total.alloc(1);
     ensure_log(c.get(), 8);
     CK(cudaStreamSynchronize(c->stream));
@@ -2631,7 +2638,7 @@ uint64_t eplace_ctx::device_bytes() const {
   add(acc); add(dens); add(rho); add(T); add(Exh); add(Eyh); add(U); add(V); add(Ex); add(Ey); add(phi);
   add(mB1); add(mL2); add(mB3); add(mL4); add(mB5); add(mL6); add(mB3g); add(mL6g);
   add(wx); add(gx2); add(wy); add(gy2); add(ops); add(mom); add(part); add(part2); add(part_b); add(io_dens);
-  add(sc); add(log); add(bar); add(loc); add(hp_total);
+  add(sc); add(log); add(bar); add(dsum); add(loc); add(hp_total);
   for (const auto &d : snap_pos) add(*d);
   for (const auto &d : snap_sc) add(*d);
   add(rho_h); add(rho_l); add(Tt_h); add(Tt_l); add(Exh_h); add(Exh_l); add(Eyh_h); add(Eyh_l);

@@ -79,23 +79,22 @@ __device__ __forceinline__ void fft_core(float2 *s, int logN, int nf, const floa
   __syncthreads();
 }
 
-// Sum of v over the CTA in a fixed order (a shuffle tree per warp, then the
-// warps in order); the result is valid in thread 0.  red: [2 * warps].
-__device__ __forceinline__ void block_sum2(double (&v)[2], double *red) {
+// Sum of v over the CTA (whole numbers, in any order); valid in thread 0.
+// red: [2 * warps].
+__device__ __forceinline__ void block_sum2(long long (&v)[2], long long *red) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     v[0] += __shfl_down_sync(0xffffffffu, v[0], o);
     v[1] += __shfl_down_sync(0xffffffffu, v[1], o);
   }
   const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  __syncthreads();
   if ((threadIdx.x & 31) == 0) {
     red[2 * w] = v[0];
     red[2 * w + 1] = v[1];
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    v[0] = v[1] = 0.0;
+    v[0] = v[1] = 0;
     for (int k = 0; k < nw; ++k) {
       v[0] += red[2 * k];
       v[1] += red[2 * k + 1];
@@ -186,8 +185,8 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
   // v[N-1-m] = x[2m+1].
   for (int j = threadIdx.x; j < N / 2; j += kFftThreads) tw[j] = __ldg(tb.tw + j);
   for (int j = threadIdx.x; j < N; j += kFftThreads) tq[j] = __ldg(tb.tq + j);
-  __shared__ double red[2 * (kFftThreads / 32)];
-  double ov[2] = {0.0, 0.0};  // sum d, sum max(d - cap, 0) (stage 0 from the map)
+  __shared__ long long red[2 * (kFftThreads / 32)];
+  long long ov[2] = {0, 0};  // sum d, sum max(d - cap, 0) in fixed point (stage 0 from the map)
   if (STAGE == 0 && a.dens) {
     for (int v0 = 0; v0 < nvec; v0 += kBatch * kFftThreads) {
       ulonglong2 q0[kBatch], q1[kBatch];
@@ -215,8 +214,8 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const double d = (double)(long long)qq[c] * (1.0 / 4294967296.0);
-          ov[0] += d;
-          ov[1] += fmax(d - a.cap, 0.0);
+          ov[0] += (long long)qq[c];
+          ov[1] += qq[c] > a.cap ? (long long)(qq[c] - a.cap) : 0;
           sf[2 * pd(b0 + bitrev(vpos(n + c, N), logN))] = (float)(d - a.c0);
         }
       }
@@ -379,29 +378,21 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
     return;
   }
   if (STAGE == 0 && a.dens) {
-    // the overlap: CTA partials, then the last CTA sums them in CTA order
-    __shared__ bool last;
+    // the overlap: whole-number sums, the last CTA forms the quotient
     block_sum2(ov, red);
     if (threadIdx.x == 0) {
-      a.part[2 * blockIdx.x] = ov[0];
-      a.part[2 * blockIdx.x + 1] = ov[1];
+      atomicAdd(&a.sums[0], (unsigned long long)ov[0]);
+      atomicAdd(&a.sums[1], (unsigned long long)ov[1]);
       __threadfence();
-      last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    double t[2] = {0.0, 0.0};
-    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-      t[0] += __ldcg(a.part + 2 * b);
-      t[1] += __ldcg(a.part + 2 * b + 1);
-    }
-    block_sum2(t, red);
-    if (threadIdx.x == 0) {
-      const double ovl = (t[0] < 1e-30) ? 0.0 : t[1] / t[0];  // compute_overlap
-      a.sc->overlap = ovl;
-      a.log[a.sc->iter].overlap = ovl;
-      *a.ticket = 0u;
+      if (atomicAdd(a.ticket, 1u) == gridDim.x - 1) {
+        __threadfence();
+        const unsigned long long sum = atomicExch(&a.sums[0], 0ull), over = atomicExch(&a.sums[1], 0ull);
+        const double inv = 1.0 / 4294967296.0;
+        const double ovl = sum == 0 ? 0.0 : ((double)(long long)over * inv) / ((double)(long long)sum * inv);
+        a.sc->overlap = ovl;  // compute_overlap
+        a.log[a.sc->iter].overlap = ovl;
+        *a.ticket = 0u;
+      }
     }
   }
 }

@@ -55,13 +55,14 @@ struct FftStageArgs {
   float *phi;             // optional [H][W] potential spectrum
   // Stage 0 straight from the fixed-point density map (the finalise fused
   // in): with dens set, the stage reads the map instead of in_a, forms
-  // rho = d - c0, clears the map for the next iteration, and sums the
-  // overlap (density.rs:79-86: sum d and sum max(d - cap, 0)) into part[]
-  // per CTA; the last CTA to finish writes sc->overlap and the iteration's
-  // log entry.
+  // rho = d - c0, clears the map for the next iteration, and adds the two
+  // sums of the overlap (density.rs:79-86: sum d and sum max(d - cap, 0)) in
+  // fixed point to sums[]; the last CTA to finish writes sc->overlap and the
+  // iteration's log entry.
   unsigned long long *dens;
-  double cap, c0;
-  double *part;           // [2 * CTAs of stage 0]
+  unsigned long long cap;
+  double c0;
+  unsigned long long *sums;  // [2], zero between launches
   unsigned *ticket;
   DevScalars *sc;
   IterLog *log;

@@ -388,25 +388,64 @@ __device__ __forceinline__ float overlap_1d(int i, float fr, float h, int b, int
 __device__ __forceinline__ float overlap_x(const Foot &f, int bx, int s) { return overlap_1d(f.ix, f.fx, f.hw, bx, s); }
 __device__ __forceinline__ float overlap_y(const Foot &f, int by, int s) { return overlap_1d(f.iy, f.fy, f.hh, by, s); }
 
+// Adds a footprint's part in a bin to the map.
+__device__ __forceinline__ void add_bin(unsigned long long *dens, const Foot &f, int bx, int by, int BX, int isx,
+                                        int isy) {
+  const float ar = overlap_x(f, bx, isx) * overlap_y(f, by, isy);
+  if (ar > 0.0f) atomicAdd(&dens[(size_t)by * BX + bx], to_fix(ar));
+}
+
+// One cell per lane of the warp (p, hf: centre and half extents; `in`: the
+// lane has one).  A footprint of at most 2 x 2 bins (every unit cell) is
+// unrolled; a larger one is shared out over the warp, a bin per lane, so that
+// 31 lanes don't wait for one macro's bins.
+__device__ __forceinline__ void scatter_warp(const ScatterArgs &a, unsigned long long *dens, float2 p, float2 hf,
+                                             bool in) {
+  const Foot f = make_foot(p, hf.x, hf.y, a.BX, a.BY, a.isx, a.isy);
+  const bool wide = in && (f.bx1 - f.bx0 > 2 || f.by1 - f.by0 > 2);
+  if (in && !wide) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int by = f.by0 + (k >> 1), bx = f.bx0 + (k & 1);
+      if (by < f.by1 && bx < f.bx1) add_bin(dens, f, bx, by, a.BX, a.isx, a.isy);
+    }
+  }
+  unsigned m = __ballot_sync(kFull, wide);
+  while (m) {
+    const int l = __ffs(m) - 1;
+    m &= m - 1;
+    const float2 q = make_float2(__shfl_sync(kFull, p.x, l), __shfl_sync(kFull, p.y, l));
+    const float2 h = make_float2(__shfl_sync(kFull, hf.x, l), __shfl_sync(kFull, hf.y, l));
+    const Foot g = make_foot(q, h.x, h.y, a.BX, a.BY, a.isx, a.isy);
+    const int nx = g.bx1 - g.bx0, bins = nx * (g.by1 - g.by0);
+    for (int k = threadIdx.x & 31; k < bins; k += 32) {
+      const int r = k / nx;
+      add_bin(dens, g, g.bx0 + k - r * nx, g.by0 + r, a.BX, a.isx, a.isy);
+    }
+  }
+}
+
+// Every cell by such warps: 32 cells from `first` on, then `step` further on.
+__device__ __forceinline__ void scatter_all(const ScatterArgs &a, unsigned long long *dens, uint32_t first,
+                                            uint32_t step) {
+  for (uint32_t i0 = first & ~31u; i0 < a.N; i0 += step) {
+    const uint32_t i = i0 + (threadIdx.x & 31);
+    const bool in = i < a.N;
+    scatter_warp(a, dens, in ? a.pos[i] : make_float2(0.f, 0.f),
+                 in && a.half ? a.half[i] : make_float2(0.5f, 0.5f), in);
+  }
+}
+
 // Unit cells first (a 1x1 footprint covers at most 2 x 2 bins: unrolled, no
 // footprint load), then the macros from their own list, so a warp of unit
 // cells never waits for one macro's loop.  Fixed-point atomics make the
 // order irrelevant.  Without a macro list but with footprints, every cell
-// takes the general loop.
+// takes the general form.
 __global__ void __launch_bounds__(kScatterBlock) k_scatter(const ScatterArgs a) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x, ts = gridDim.x * blockDim.x;
   if (a.half && !a.mflag) {
-    for (uint32_t i = t0; i < a.N; i += ts) {
-      const float2 hf = a.half[i];
-      const Foot f = make_foot(a.pos[i], hf.x, hf.y, a.BX, a.BY, a.isx, a.isy);
-      for (int by = f.by0; by < f.by1; ++by) {
-        const float oy = overlap_y(f, by, a.isy);
-        for (int bx = f.bx0; bx < f.bx1; ++bx) {
-          const float ar = overlap_x(f, bx, a.isx) * oy;
-          if (ar > 0.0f) atomicAdd(&a.dens[(size_t)by * a.BX + bx], to_fix(ar));
-        }
-      }
-    }
+    scatter_all(a, a.dens, t0, ts);
     return;
   }
   for (uint32_t i = t0; i < a.N; i += ts) {
@@ -415,46 +454,86 @@ __global__ void __launch_bounds__(kScatterBlock) k_scatter(const ScatterArgs a) 
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int by = f.by0 + (k >> 1), bx = f.bx0 + (k & 1);
-      if (by >= f.by1 || bx >= f.bx1) continue;
-      const float ar = overlap_x(f, bx, a.isx) * overlap_y(f, by, a.isy);
-      if (ar > 0.0f) atomicAdd(&a.dens[(size_t)by * a.BX + bx], to_fix(ar));
+      if (by < f.by1 && bx < f.bx1) add_bin(a.dens, f, bx, by, a.BX, a.isx, a.isy);
     }
   }
   for (uint32_t k = t0; k < a.n_mac; k += ts) {
     const uint32_t i = a.mac_idx[k];
     const float2 hf = a.half[i];
     const Foot f = make_foot(a.pos[i], hf.x, hf.y, a.BX, a.BY, a.isx, a.isy);
-    for (int by = f.by0; by < f.by1; ++by) {
-      const float oy = overlap_y(f, by, a.isy);
-      for (int bx = f.bx0; bx < f.bx1; ++bx) {
-        const float ar = overlap_x(f, bx, a.isx) * oy;
-        if (ar > 0.0f) atomicAdd(&a.dens[(size_t)by * a.BX + bx], to_fix(ar));
-      }
+    for (int by = f.by0; by < f.by1; ++by)
+      for (int bx = f.bx0; bx < f.bx1; ++bx) add_bin(a.dens, f, bx, by, a.BX, a.isx, a.isy);
+  }
+}
+
+// The two sums of the overlap (density.rs:79-86) over the CTA, in fixed point:
+// whole numbers, so their order is free.  Valid in thread 0.
+__device__ __forceinline__ void block_sum_fix(long long (&v)[2], long long *smem /* [2 * warps] */) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    v[0] += __shfl_down_sync(kFull, v[0], o);
+    v[1] += __shfl_down_sync(kFull, v[1], o);
+  }
+  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
+    smem[2 * w] = v[0];
+    smem[2 * w + 1] = v[1];
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int l = threadIdx.x;
+    v[0] = l < nw ? smem[2 * l] : 0;
+    v[1] = l < nw ? smem[2 * l + 1] : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      v[0] += __shfl_down_sync(kFull, v[0], o);
+      v[1] += __shfl_down_sync(kFull, v[1], o);
     }
   }
 }
 
+// compute_overlap of the two sums.
+__device__ __forceinline__ double overlap_of(unsigned long long sum, unsigned long long over) {
+  return sum == 0 ? 0.0 : from_fix(over) / from_fix(sum);
+}
+
+__device__ __forceinline__ void count_bin(unsigned long long q, unsigned long long cap, long long (&v)[2]) {
+  v[0] += (long long)q;
+  v[1] += q > cap ? (long long)(q - cap) : 0;
+}
+
+// Streams the map once (8 bytes read and zeroed, the outputs written), four
+// bins per thread and step, 16-byte accesses where the buffers allow it.  The
+// overlap's sums are whole numbers, so each CTA adds its two with atomics and
+// the last one forms the quotient (FP64 partial sums, which the last CTA read
+// back and added in a fixed order, held the kernel up after its last bin).
+// The launch overlaps the end of the scatter before it (launch_density_final,
+// after).  Scatter and finalise of the allocation-free entry, which also made
+// three clears and a copy, back to back: 64^2 bins, 2k unit cells 14.3 -> 5.1
+// us; 512^2 bins, 200k cells with macros 21.8 -> 10 us (5.3 MB at least: 0.8).
+// A single CTA with the map in its shared memory was slower from 1,000 cells
+// on (2k cells 6.2 us, 8k 14 us).
 __global__ void __launch_bounds__(kFinalBlock) k_density_final(const FinalArgs a) {
-  __shared__ double sm[64];
-  __shared__ bool last;
-  double v[2] = {0.0, 0.0};
+  __shared__ long long sm[2 * kFinalBlock / 32];
+  long long v[2] = {0, 0};
   // Groups of four consecutive bins per thread and step: 16-byte loads and
   // stores (when every pointer is aligned for them; a ragged tail, or
   // unaligned caller buffers, take the scalar loop below).
   const int ng = a.vec4 ? (a.nb >> 2) : 0;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, ts = gridDim.x * blockDim.x;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int gi = t0; gi < ng; gi += ts) {
     ulonglong2 *dp = reinterpret_cast<ulonglong2 *>(a.dens) + 2 * gi;
     const ulonglong2 q0 = dp[0], q1 = dp[1];
     dp[0] = make_ulonglong2(0ull, 0ull);
     dp[1] = make_ulonglong2(0ull, 0ull);
+    const unsigned long long q[4] = {q0.x, q0.y, q1.x, q1.y};
     const double d[4] = {from_fix(q0.x), from_fix(q0.y), from_fix(q1.x), from_fix(q1.y)};
     float r[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       r[k] = (float)(d[k] - a.c0);
-      v[0] += d[k];
-      v[1] += fmax(d[k] - a.cap, 0.0);
+      count_bin(q[k], a.cap, v);
     }
     if (a.rho) reinterpret_cast<float4 *>(a.rho)[gi] = make_float4(r[0], r[1], r[2], r[3]);
     if (a.rho_hi) {
@@ -478,7 +557,8 @@ __global__ void __launch_bounds__(kFinalBlock) k_density_final(const FinalArgs a
     }
   }
   for (int i = 4 * ng + t0; i < a.nb; i += ts) {
-    const double d = from_fix(a.dens[i]);
+    const unsigned long long q = a.dens[i];
+    const double d = from_fix(q);
     a.dens[i] = 0ull;
     const float r = (float)(d - a.c0);
     if (a.rho) a.rho[i] = r;
@@ -488,28 +568,23 @@ __global__ void __launch_bounds__(kFinalBlock) k_density_final(const FinalArgs a
       a.rho_lo[i] = __float2bfloat16_rn(r - __bfloat162float(h));
     }
     if (a.dens_out) a.dens_out[i] = d;
-    v[0] += d;
-    v[1] += fmax(d - a.cap, 0.0);
+    count_bin(q, a.cap, v);
   }
-  block_sum<2>(v, sm);
-  if (threadIdx.x == 0) {
-    a.part[2 * blockIdx.x] = v[0];
-    a.part[2 * blockIdx.x + 1] = v[1];
-    __threadfence();
-    last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last) return;
+  block_sum_fix(v, sm);
+  if (threadIdx.x != 0) return;
+  atomicAdd(&a.sums[0], (unsigned long long)v[0]);
+  atomicAdd(&a.sums[1], (unsigned long long)v[1]);
   __threadfence();
-  double fin[2];
-  sum_partials<2>(a.part, 2, gridDim.x, fin, sm);
-  if (threadIdx.x == 0) {
-    const double s = fin[0], o = fin[1];
-    const double ov = (s < 1e-30) ? 0.0 : o / s;  // compute_overlap
+  if (atomicAdd(a.ticket, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  const double ov = overlap_of(atomicExch(&a.sums[0], 0ull), atomicExch(&a.sums[1], 0ull));
+  if (a.overlap) {
+    *a.overlap = ov;
+  } else {
     a.sc->overlap = ov;
     a.log[a.sc->iter].overlap = ov;
-    *a.ticket = 0u;
   }
+  *a.ticket = 0u;
 }
 
 // ---------------------------------------------------------------------------
@@ -1121,12 +1196,20 @@ cudaError_t launch_scatter(const ScatterArgs &a, int grid, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_density_final(const FinalArgs &a_in, int grid, cudaStream_t s) {
+cudaError_t launch_density_final(const FinalArgs &a_in, int grid, cudaStream_t s, bool after) {
   FinalArgs a = a_in;
   auto al = [](const void *p, uintptr_t m) { return ((uintptr_t)p & (m - 1)) == 0; };
   a.vec4 = al(a.dens, 16) && al(a.rho, 16) && al(a.rho_hi, 8) && al(a.rho_lo, 8) && al(a.dens_out, 16);
-  k_density_final<<<grid, kFinalBlock, 0, s>>>(a);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kFinalBlock);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = after ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k_density_final, a);
 }
 
 // One SIMT GEMM launch: split K four ways over a cluster when 4 * GK

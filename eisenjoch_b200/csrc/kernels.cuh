@@ -94,15 +94,16 @@ struct ScatterArgs {
 struct FinalArgs {
   unsigned long long *dens;
   int nb;
-  double cap;               // capacity per bin (sites per bin)
+  unsigned long long cap;   // capacity per bin (sites per bin), fixed point
   double c0;                // constant removed before the transform
   float *rho;               // FP32 charge map (SIMT transform), or nullptr
   __nv_bfloat16 *rho_hi;    // BF16 hi/lo charge map (tensor-core transform), or nullptr
   __nv_bfloat16 *rho_lo;
   double *dens_out;         // optional FP64 copy (stage entry)
   int vec4;                 // set by launch_density_final: every pointer allows 16-byte groups
-  double *part;             // [2 * grid]
+  unsigned long long *sums; // [2] sum of d, sum of max(d - cap, 0); zero between launches
   unsigned *ticket;
+  double *overlap;          // where the overlap goes, or nullptr: into sc and the log
   DevScalars *sc;
   IterLog *log;
 };
@@ -171,7 +172,9 @@ struct HpwlArgs {
 
 cudaError_t launch_wa(const WaArgs &a, int grid, cudaStream_t s);
 cudaError_t launch_scatter(const ScatterArgs &a, int grid, cudaStream_t s);
-cudaError_t launch_density_final(const FinalArgs &a, int grid, cudaStream_t s);
+// after: whether the launch may start before the kernel ahead of it in the
+// stream has ended (it waits for that kernel's results itself).
+cudaError_t launch_density_final(const FinalArgs &a, int grid, cudaStream_t s, bool after = false);
 // C[b] = A[b] (M x K) * B[b] (K x N), row-major FP32; batches from ops[0..nb).
 // tile: 64 or 32 (CTA tile edge), 0 = pick by grid size.  When 64 divides K
 // the sum is split into four K quarters (a cluster of four CTAs per tile)

@@ -8,7 +8,7 @@
 // code running under a fixed device-memory budget.  They own their inputs
 // and outputs already; what they cannot do is give this library the working
 // memory the density stage needs (the fixed-point accumulation map, the
-// per-block partial sums and the completion counter).  For them the scratch
+// overlap's sums and the completion counter).  For them the scratch
 // lives in one file-scope __device__ array, sized for at most
 // kNoAllocMaxBins bins (512 x 512).  It is part of the library image: every
 // GPU that loads libeplace.so holds it (about 2 MiB) until the process
@@ -30,22 +30,15 @@ namespace eplace {
 namespace {
 
 constexpr size_t kNoAllocMaxBins = 512 * 512;
-constexpr int kNoAllocMaxBlocks = 1024;  // finalise grid cap (partials below)
 
 // Layout of the scratch array (byte offsets, each 256-aligned):
 //   [0, kMapBytes)                fixed-point bin map, must start at zero
-//   [kPartOff, +kPartBytes)       per-block partial sums of the finalise
+//   [kSumOff, +256)               the overlap's two sums, must start at zero
 //   [kTicketOff, +256)            completion counter, must start at zero
-//   [kScalOff, +256)              loop scalars the finalise writes into
-//   [kLogOff, +256)               one per-iteration log record
 constexpr size_t kMapBytes = kNoAllocMaxBins * sizeof(unsigned long long);
-constexpr size_t kPartOff = kMapBytes;
-constexpr size_t kPartBytes = 2 * kNoAllocMaxBlocks * sizeof(double);
-constexpr size_t kTicketOff = kPartOff + kPartBytes;
-constexpr size_t kScalOff = kTicketOff + 256;
-constexpr size_t kLogOff = kScalOff + 256;
-constexpr size_t kScratchBytes = kLogOff + 256;
-static_assert(sizeof(DevScalars) <= 256 && sizeof(IterLog) <= 256, "scratch slots too small");
+constexpr size_t kSumOff = kMapBytes;
+constexpr size_t kTicketOff = kSumOff + 256;
+constexpr size_t kScratchBytes = kTicketOff + 256;
 
 static __device__ __align__(256) unsigned char g_density_scratch[kScratchBytes];
 
@@ -64,6 +57,8 @@ typedef CUresult (*CtxGetIdFn)(CUcontext, unsigned long long *);
 struct ScratchSlot {
   unsigned long long ctx_id = 0;
   void *addr = nullptr;
+  int sms = 0;
+  bool dirty = false;  // a call's launches did not all happen
 };
 
 std::mutex g_mu;
@@ -90,7 +85,7 @@ eplace_status current_context_id(unsigned long long *id) {
   return g_ctx_id(c, id) == CUDA_SUCCESS ? EPLACE_OK : EPLACE_ERR_CUDA;
 }
 
-eplace_status scratch_for_current_device(void **out) {
+eplace_status scratch_for_current_device(void **out, bool *dirty, int *sms) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return EPLACE_ERR_NO_DEVICE;
   if (dev < 0 || dev >= 128) return EPLACE_ERR_NO_DEVICE;
@@ -108,11 +103,23 @@ eplace_status scratch_for_current_device(void **out) {
     st = current_context_id(&id);
     if (st != EPLACE_OK) return st;
     if (id == 0) return EPLACE_ERR_CUDA;
+    if (cudaDeviceGetAttribute(&slot.sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return EPLACE_ERR_CUDA;
     slot.addr = p;
     slot.ctx_id = id;
+    slot.dirty = false;  // a fresh image: all zero
   }
   *out = slot.addr;
+  *dirty = slot.dirty;
+  *sms = slot.sms;
   return EPLACE_OK;
+}
+
+// Whether the next call on the current device has to clear the scratch.
+void scratch_state(bool dirty) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 128) return;
+  std::lock_guard<std::mutex> g(g_mu);
+  g_slot[dev].dirty = dirty;
 }
 
 }  // namespace
@@ -131,43 +138,45 @@ extern "C" eplace_status eplace_density_noalloc(const float *pos_xy, const float
   // doubles: a misaligned pointer would fault the caller's whole context.
   if (((uintptr_t)pos_xy | (uintptr_t)half_wh | (uintptr_t)density | (uintptr_t)overlap) & 7u)
     return EPLACE_ERR_INVALID;
-  void *base = nullptr;
-  eplace_status st = scratch_for_current_device(&base);
-  if (st != EPLACE_OK) return st;
-  int sms = 0, dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return EPLACE_ERR_CUDA;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  unsigned char *b = static_cast<unsigned char *>(base);
-  const int nb = bins_x * bins_y;
-  auto *map = reinterpret_cast<unsigned long long *>(b);
-  auto *part = reinterpret_cast<double *>(b + kPartOff);
-  auto *ticket = reinterpret_cast<unsigned *>(b + kTicketOff);
-  auto *sc = reinterpret_cast<DevScalars *>(b + kScalOff);
-  auto *lg = reinterpret_cast<IterLog *>(b + kLogOff);
-  // The scratch keeps the previous call's contents.  A completed call
-  // leaves the map at zero (the finalise re-zeroes every bin it reads) and
-  // the counter back at zero; the clears below make a call correct also
-  // after an earlier call whose kernels did not all run (a launch error part
-  // way through), and set the scalar slot the finalise reads (iteration 0).
-  if (cudaMemsetAsync(map, 0, (size_t)nb * sizeof(unsigned long long), s) != cudaSuccess ||
-      cudaMemsetAsync(ticket, 0, 256, s) != cudaSuccess || cudaMemsetAsync(sc, 0, 256, s) != cudaSuccess)
-    return EPLACE_ERR_CUDA;
-  const int sx = width / bins_x, sy = height / bins_y;
+  const int nb = bins_x * bins_y, sx = width / bins_x, sy = height / bins_y;
   ScatterArgs a{reinterpret_cast<const float2 *>(pos_xy), reinterpret_cast<const float2 *>(half_wh), nullptr,
-                nullptr, 0u, num_cells, bins_x, bins_y, sx, sy, map};
+                nullptr, 0u, num_cells, bins_x, bins_y, sx, sy, nullptr};
+  FinalArgs f{};
+  f.nb = nb;
+  f.cap = (unsigned long long)sx * (unsigned long long)sy << 32;
+  f.dens_out = density;
+  f.overlap = overlap;
+  void *base = nullptr;
+  bool dirty = false;
+  int sms = 0;
+  eplace_status st = scratch_for_current_device(&base, &dirty, &sms);
+  if (st != EPLACE_OK) return st;
+  unsigned char *b = static_cast<unsigned char *>(base);
+  auto *map = reinterpret_cast<unsigned long long *>(b);
+  a.dens = f.dens = map;
+  f.sums = reinterpret_cast<unsigned long long *>(b + kSumOff);
+  f.ticket = reinterpret_cast<unsigned *>(b + kTicketOff);
+  // The scratch keeps the previous call's contents.  It starts at zero and a
+  // completed call leaves it at zero (the finalise zeroes every bin that it
+  // reads, the sums and the counter); after a call whose second launch failed
+  // it is cleared first.
+  if (dirty && (cudaMemsetAsync(base, 0, kScratchBytes, s) != cudaSuccess)) return EPLACE_ERR_CUDA;
   if (num_cells) {
     long long g = ((long long)num_cells + kScatterBlock - 1) / kScatterBlock;
     if (g > (long long)sms * 16) g = (long long)sms * 16;
-    if (launch_scatter(a, (int)g, s) != cudaSuccess) return EPLACE_ERR_CUDA;
+    if (launch_scatter(a, (int)g, s) != cudaSuccess) {
+      scratch_state(dirty);
+      return EPLACE_ERR_CUDA;
+    }
   }
-  long long fg = ((long long)nb + kFinalBlock - 1) / kFinalBlock;
-  if (fg > (long long)sms * 2) fg = (long long)sms * 2;
-  if (fg > kNoAllocMaxBlocks) fg = kNoAllocMaxBlocks;
-  FinalArgs f{map, nb, (double)sx * (double)sy, 0.0, nullptr, nullptr, nullptr, density, 0, part, ticket, sc, lg};
-  if (launch_density_final(f, (int)fg, s) != cudaSuccess) return EPLACE_ERR_CUDA;
-  if (cudaMemcpyAsync(overlap, &sc->overlap, sizeof(double), cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+  long long fg = ((long long)nb / 4 + kFinalBlock - 1) / kFinalBlock;
+  if (fg > (long long)sms * 4) fg = (long long)sms * 4;
+  if (fg < 1) fg = 1;
+  if (launch_density_final(f, (int)fg, s, num_cells != 0) != cudaSuccess) {
+    scratch_state(true);
     return EPLACE_ERR_CUDA;
+  }
+  if (dirty) scratch_state(false);
   return EPLACE_OK;
 }

@@ -144,3 +144,42 @@ def test_density_noalloc_rejects_bad_arguments():
         st = L.eplace_density_noalloc(ctypes.c_void_p(pos), ctypes.c_void_p(half), 8, 64, 64, 16, 16,
                                       ctypes.c_void_p(dens), ctypes.c_void_p(ov), None)
         assert st == _abi.EPLACE_ERR_INVALID, (pos - base, half, dens - base, ov - base)
+
+
+@pytest.mark.parametrize("cells,w,h,bx,by", [(1, 7, 5, 7, 5), (31, 33, 17, 33, 17), (33, 64, 64, 16, 8),
+                                             (257, 90, 60, 45, 30), (4099, 512, 256, 512, 256)])
+@pytest.mark.parametrize("half", ["unit", "mixed"])
+def test_density_noalloc_shapes(cells, w, h, bx, by, half):
+    """Counts of cells and bins around a warp and around the four-bin groups,
+    footprints within and beyond 2 x 2 bins (0.5 to 6 bins wide, any half
+    extent), some of them partly outside the chip: against the overlaps in
+    FP64, bins within 1e-6 of the largest (a bin is a sum of FP32 areas, each
+    exact to 2^-23, rounded to 2^-32), the overlap within 1e-6."""
+    import torch
+
+    dev = torch.device("cuda:0")
+    torch.cuda.set_device(dev)
+    rng = np.random.default_rng(cells)
+    nl = E.Netlist(num_cells=cells, net_offsets=np.zeros(1, np.uint32), pin_cell=np.zeros(0, np.uint32))
+    chip = E.Chip(w, h, bx, by)
+    x, y = rng.uniform(-1, w, cells).astype(np.float32), rng.uniform(-1, h, cells).astype(np.float32)
+    hf = np.full((cells, 2), 0.5, np.float32)
+    if half == "mixed":
+        hf = np.where(rng.random((cells, 1)) < 0.3, rng.uniform(0.25, 3.0 * w / bx, (cells, 2)), hf).astype(np.float32)
+    half_d = torch.from_numpy(hf).to(dev) if half == "mixed" else None
+    dens_d = torch.full((by, bx), -1.0, dtype=torch.float64, device=dev)
+    ov_d = torch.full((1,), -1.0, dtype=torch.float64, device=dev)
+    sx, sy = w // bx, h // by
+
+    def axis(c, e, s, n):  # [cells, n] lengths in the bins
+        lo, hi = c.astype(np.float64) - e, c.astype(np.float64) + e
+        k = np.arange(n)
+        return np.maximum(np.minimum(hi[:, None], (k + 1) * s) - np.maximum(lo[:, None], k * s), 0.0)
+
+    want = axis(y, hf[:, 1], sy, by).T @ axis(x, hf[:, 0], sx, bx)
+    over = np.maximum(want - sx * sy, 0).sum() / want.sum()
+    for _ in range(2):  # the second call finds the scratch as the first left it
+        st, got, ov = _noalloc(torch, nl, chip, x, y, half_d, dens_d, ov_d)
+        assert st == _abi.EPLACE_OK
+        assert np.abs(got - want).max() <= 1e-6 * want.max()
+        assert abs(ov - over) <= 1e-6
