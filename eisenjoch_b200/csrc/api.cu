@@ -294,7 +294,7 @@ struct eplace_ctx {
   std::string err;
   int num_sms = 0;
   int64_t spin_cycles = 0;  // bound of the step's barrier waits for the current run (0: kernel default)
-  int step_grid = 0;
+  int step_grid = 0, step_threads = 0;
   std::vector<double> pw_host;
   double total_area = 0.0;
 
@@ -393,12 +393,15 @@ struct eplace_ctx {
   DBuf<uint64_t> lg_free0;
   bool lg_macros = false;
   std::vector<std::unique_ptr<LegalSlot>> lslots;
-  int step_grid_full = 0;
   // Step as three ordinary launches instead of one cooperative launch: used
   // whenever other long-running kernels share the device (device legaliser,
   // several jobs at once), where a grid barrier could wait on blocks that
   // cannot become resident.
   bool split_step = false;
+  // The kernels of an iteration may start while the one before them ends (set
+  // while launch_iteration runs; elsewhere copies and event records stand
+  // between them).
+  bool overlap = false;
   bool shared_device = false;  // set by the job engine: other jobs' kernels run beside this one
   int mat_bx = -1, mat_by = -1;  // bin grid the DCT matrices were built for
   uint64_t load_gen = 0;         // bumped by every (re)load of a problem
@@ -982,16 +985,20 @@ void setup_tc(eplace_ctx *c) {
 
 int *err_ptr(eplace_ctx *c) { return reinterpret_cast<int *>(reinterpret_cast<char *>(c->sc.p) + offsetof(DevScalars, err)); }
 
+NormArgs norm_args(const eplace_ctx *c);
+
 // Sites per bin as a fixed-point density.
 unsigned long long cap_fix(const HostProblem &hp) { return (unsigned long long)hp.sx * (unsigned long long)hp.sy << 32; }
 
-void launch_final_stage(eplace_ctx *c, double *dens_out, bool tc = false) {
+// loop: inside an iteration, after the step (whose norms it adds up too).
+void launch_final_stage(eplace_ctx *c, double *dens_out, bool tc = false, bool loop = false) {
   const HostProblem &hp = c->hp;
   const int nb = hp.BX * hp.BY;
   const double c0 = c->total_area / (double)nb;
   FinalArgs a{c->dens.p, nb, cap_fix(hp), c0, tc ? nullptr : c->rho.p, tc ? c->rho_h.p : nullptr,
-              tc ? c->rho_l.p : nullptr, dens_out, 0, c->dsum.p, c->bar.p + 2, nullptr, c->sc.p, c->log.p};
-  CK(launch_density_final(a, grid_for((nb + 3) / 4, kFinalBlock, c->num_sms * 4), c->stream));
+              tc ? c->rho_l.p : nullptr, dens_out, 0, c->dsum.p, c->bar.p + 2, nullptr, c->sc.p, c->log.p, {}};
+  if (loop) a.norms = norm_args(c);
+  CK(launch_density_final(a, grid_for((nb + 3) / 4, kFinalBlock, c->num_sms * 4), c->stream, loop));
 }
 
 // One of the four GEMM launches of a field solve (density.rs:96-166):
@@ -1043,6 +1050,7 @@ void launch_field_gemm(eplace_ctx *c, int g, float *phi, int field_mode, bool tc
     a.H = H;
     a.tx = FftTables{c->fft_twx.p, c->fft_tqx.p};
     a.ty = FftTables{c->fft_twy.p, c->fft_tqy.p};
+    a.after = c->overlap;
     const int sn = fm ? FFT_SG : FFT_S3;  // Ex's transform along x, Ey's along y
     switch (g) {
       case 0:
@@ -1056,6 +1064,7 @@ void launch_field_gemm(eplace_ctx *c, int g, float *phi, int field_mode, bool tc
           a.ticket = c->bar.p + 2;
           a.sc = c->sc.p;
           a.log = c->log.p;
+          a.norms = norm_args(c);
         }
         break;
       case 1:  // forward along y, spectral, then back along y: U, V
@@ -1288,30 +1297,53 @@ StepArgs step_args(eplace_ctx *c) {
   return a;
 }
 
-void launch_step_stage(eplace_ctx *c) {
-  StepArgs a = step_args(c);
-  if (c->split_step) CK(launch_step_split(a, c->step_grid, c->stream));
-  else CK(launch_step(a, c->step_grid, c->stream));
+NormArgs norm_args(const eplace_ctx *c) { return NormArgs{c->part2.p, c->step_grid, c->sc.p, c->log.p}; }
+
+// The interval's positions and scalars into a snapshot; its last iteration's
+// step norms into the log.
+void launch_snapshot_stage(eplace_ctx *c, float2 *pos, DevScalars *sc) {
+  CK(launch_snapshot(SnapArgs{pos ? c->hp.N : 0u, c->x.p, pos, sc, norm_args(c)}, c->stream));
 }
 
-// One iteration.  The WA gradient and the density -> field chain both read
-// only the look-ahead positions and write separate buffers, so WA runs on
-// the side stream beside scatter / finalise / the four GEMMs; the step joins
-// both.  (In a captured graph this is a fork and a join.)
+// scatter: the step also adds the next look-ahead to the density map.
+void launch_step_stage(eplace_ctx *c, bool scatter) {
+  StepArgs a = step_args(c);
+  a.dens = scatter ? c->dens.p : nullptr;
+  if (c->split_step) CK(launch_step_split(a, c->step_grid, c->step_threads, c->stream));
+  else CK(launch_step(a, c->step_grid, c->step_threads, c->stream));
+}
+
+// One iteration from a scattered density map (launch_scatter_stage before the
+// first; then each step scatters its look-ahead).  The WA gradient and the
+// density -> field chain both read only the look-ahead positions and write
+// separate buffers, so WA runs on the side stream beside the finalise and the
+// transform; the step joins both.  (In a captured graph this is a fork and a
+// join.)  The transform's launches overlap the end of the kernel before each.
 void launch_iteration(eplace_ctx *c, float gamma, int field_mode, bool tc) {
   CK(cudaEventRecord(c->ev_fork, c->stream));
   CK(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
   launch_wa_stage(c, gamma, c->side);
   CK(cudaEventRecord(c->ev_join, c->side));
-  launch_scatter_stage(c);
   const bool fuse = final_fused(c, tc);
-  if (!fuse) launch_final_stage(c, nullptr, tc);
-  launch_field_stage(c, nullptr, field_mode, tc, fuse);
+  c->overlap = true;
+  try {
+    if (!fuse) launch_final_stage(c, nullptr, tc, true);
+    launch_field_stage(c, nullptr, field_mode, tc, fuse);
+  } catch (...) {
+    c->overlap = false;
+    throw;
+  }
+  c->overlap = false;
   CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
-  launch_step_stage(c);
+  launch_step_stage(c, true);
 }
 
-constexpr int kLaunchesPerIter = 8;  // with the cooperative step; +2 with the split step, -2 with the FFT form
+// Kernels of one iteration: WA, the step (three when split), the finalise and
+// the transform.
+int launches_per_iteration(const eplace_ctx *c, bool tc) {
+  const int transform = tc ? 5 : c->fft ? 3 : c->fold ? 7 : 5;
+  return 1 + (c->split_step ? 3 : 1) + transform;
+}
 
 void upload_momentum(eplace_ctx *c, uint64_t iters) {
   AllocOn on_stream(c->stream);
@@ -1552,12 +1584,13 @@ void load_into(eplace_ctx *c, HostProblem &&hp_in) {
     c->mat_by = hp.BY;
     c->tc_ready = false;
   }
-  // Two blocks per SM: enough to stream the cells, few arrivals per grid
-  // barrier (the grid must stay co-resident for the cooperative launch).
-  c->step_grid = std::max(1, std::min({step_max_grid(c->device), c->num_sms * 2,
-                                       grid_for((int)hp.N, kStepBlock, 1 << 30)}));
-  c->step_grid_full = c->step_grid;
-  c->part.ensure(4 * (size_t)std::max(c->step_grid, c->num_sms * 4) + 8);
+  // As many threads as cells, up to 1024 an SM: enough to stream the cells,
+  // few arrivals per grid barrier (the grid must stay co-resident for the
+  // cooperative launch).
+  c->step_threads = step_block(c->device, hp.N);
+  c->step_grid = std::max(1, std::min({step_max_grid(c->device, c->step_threads), c->num_sms * 1024 / c->step_threads,
+                                       grid_for((int)hp.N, c->step_threads, 1 << 30)}));
+  c->part.ensure(4 * (size_t)c->step_grid + 8);
   c->part2.ensure(2 * (size_t)c->step_grid + 8);
   c->part_b.ensure(4 * (size_t)c->step_grid + 8);
   c->bar.zero(s);
@@ -1916,6 +1949,7 @@ struct JobState {
       c->spin_cycles = wait_cycles(c->device, opts.wait_limit_us);
       ip_launches = reset_state(c, isx, isy, &cfg);
       autotune_launches(c, gamma, opts.field_mode, tc);
+      launch_scatter_stage(c);  // the first iteration's density; each step scatters the next one's
       mark("device_reset");
       // Host resources persist in the context across runs.
       if (!c->lbase) c->lbase.reset(new LegalBase(hp));
@@ -2254,19 +2288,18 @@ struct JobState {
         cp->slot = acquire_slot();
         LegalSlot &L = *c->lslots[cp->slot];
         CK(cudaStreamWaitEvent(s, L.done, 0));  // a reused slot's last legalisation has finished
-        CK(cudaMemcpyAsync(L.pos.p, c->x.p, sizeof(float2) * hp.N, cudaMemcpyDeviceToDevice, s));
+        launch_snapshot_stage(c, L.pos.p, c->snap_sc[slot]->p);
         CK(cudaEventRecord(L.snap, s));
         CK(cudaStreamWaitEvent(L.stream, L.snap, 0));
         launch_gpu_legal(c, L);
         cps.push_back(std::move(cp));
       } else {
         hs = take_snap();
-        CK(cudaMemcpyAsync(c->snap_pos[slot]->p, c->x.p, sizeof(float2) * hp.N, cudaMemcpyDeviceToDevice, s));
+        launch_snapshot_stage(c, c->snap_pos[slot]->p, c->snap_sc[slot]->p);
       }
       // The interval's outputs leave on the copy stream: positions and
       // scalars from the slot's device copy (the loop overwrites its own),
       // the log entries from their own places (each iteration has one).
-      CK(cudaMemcpyAsync(c->snap_sc[slot]->p, c->sc.p, sizeof(DevScalars), cudaMemcpyDeviceToDevice, s));
       CK(cudaEventRecord(c->snap_ev[slot], s));
       CK(cudaStreamWaitEvent(c->copy, c->snap_ev[slot], 0));
       if (hs) {
@@ -2361,9 +2394,8 @@ struct JobState {
       float ms = 0.f;
       CK(cudaEventElapsedTime(&ms, ev0, ev1));
       res->gpu_seconds = ms * 1e-3;
-      res->gpu_launches = (uint64_t)(kLaunchesPerIter + (c->split_step ? 2 : 0) + (c->fold && !tc && !c->fft ? 2 : 0) -
-                                         (final_fused(c, tc) ? 2 : 0)) *
-                              launched_iters +
+      // one scatter before the first iteration, a snapshot per interval
+      res->gpu_launches = (uint64_t)launches_per_iteration(c, tc) * launched_iters + 1 + (uint64_t)next_chunk +
                           (gpu_legal ? 2 * cps.size() : 0) + (uint64_t)ip_launches;
       res->iters = (uint32_t)iters_done;
       res->converged = converged_chunk < chunks.size() ? 1 : 0;
@@ -2765,7 +2797,7 @@ eplace_status eplace_profile_stages(eplace_ctx *c, const eplace_cfg *cfg, const 
         launch_field_gemm(c, g, nullptr, opts.field_mode, tc, fuse && g == 0);
         rec(ev[4 + g]);
       }
-      launch_step_stage(c);
+      launch_step_stage(c, false);  // the scatter is timed by itself
       rec(ev[8]);
     };
     // The iteration is timed as a CUDA graph (event-record nodes between the
@@ -3002,7 +3034,7 @@ eplace_status eplace_stage_gather(eplace_ctx *c, const float *x, const float *y,
     io_in(c, c->stream, h + 2 * io_pitch(nb), {{x, y}}, {c->look.p});
     StepArgs a = step_args(c);
     a.mode = 1;
-    CK(launch_step(a, c->step_grid, c->stream));
+    CK(launch_step(a, c->step_grid, c->step_threads, c->stream));
     const IoArgs o = io_out(c, c->stream, {c->tmp_den.p});
     CK(cudaStreamSynchronize(c->stream));
     HostCopy::get().run({{gx, o.host, bytes}, {gy, o.host + o.pitch, bytes}});
@@ -3043,7 +3075,8 @@ eplace_status eplace_stage_step(eplace_ctx *c, uint64_t iter, const float *look_
     sc.iter = (int32_t)iter;
     c->sc.upload(&sc, 1, s);
     c->bar.zero(s);
-    launch_step_stage(c);
+    launch_step_stage(c, false);
+    launch_snapshot_stage(c, nullptr, c->sc.p);  // the norms
     const IoArgs o = io_out(c, s, {c->x.p, c->xp.p, c->gprev.p, c->look.p});
     // the log entry and the scalars after the arrays (1 KB is kept for them)
     char *tail = reinterpret_cast<char *>(o.host + 8 * o.pitch);
@@ -3104,7 +3137,7 @@ eplace_status eplace_stage_barrier_timeout(eplace_ctx *c, int32_t wait_limit_us,
     // in the next multiple of the grid waits for arrivals that never come
     const unsigned long long start = phantom;
     CK(cudaMemcpyAsync(c->bar.p, &start, sizeof(start), cudaMemcpyHostToDevice, c->stream));
-    CK(launch_step(step_args(c), c->step_grid, c->stream));
+    CK(launch_step(step_args(c), c->step_grid, c->step_threads, c->stream));
     DevScalars sc{};
     CK(cudaMemcpyAsync(&sc, c->sc.p, sizeof(sc), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));

@@ -162,6 +162,12 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
   const int N = G.N, logN = G.logN, nl = G.lines;
   const FftTables tb = kRows ? a.tx : a.ty;
   const int line0 = blockIdx.x * nl;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (STAGE == 0 && line0 >= G.L) {  // the CTA after the lines'
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (threadIdx.x < 32) finish_norms(a.norms);
+    return;
+  }
   float2 *tw = s + pd(fft_slots(STAGE, G));  // [N/2] e^{-2 pi i j / N}
   float2 *tq = tw + N / 2;              // [N]   (cos, sin)(pi k / 2N)
   float *R = reinterpret_cast<float *>(tq + N);  // stages 1 and 2: R[array][line][pos]
@@ -185,6 +191,7 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
   // v[N-1-m] = x[2m+1].
   for (int j = threadIdx.x; j < N / 2; j += kFftThreads) tw[j] = __ldg(tb.tw + j);
   for (int j = threadIdx.x; j < N; j += kFftThreads) tq[j] = __ldg(tb.tq + j);
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the tables don't change
   __shared__ long long red[2 * (kFftThreads / 32)];
   long long ov[2] = {0, 0};  // sum d, sum max(d - cap, 0) in fixed point (stage 0 from the map)
   if (STAGE == 0 && a.dens) {
@@ -384,7 +391,7 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
       atomicAdd(&a.sums[0], (unsigned long long)ov[0]);
       atomicAdd(&a.sums[1], (unsigned long long)ov[1]);
       __threadfence();
-      if (atomicAdd(a.ticket, 1u) == gridDim.x - 1) {
+      if (atomicAdd(a.ticket, 1u) == (unsigned)((G.L + nl - 1) / nl) - 1) {
         __threadfence();
         const unsigned long long sum = atomicExch(&a.sums[0], 0ull), over = atomicExch(&a.sums[1], 0ull);
         const double inv = 1.0 / 4294967296.0;
@@ -418,29 +425,18 @@ void fft_tables_host(int N, float2 *tw, float2 *tq) {
 
 cudaError_t launch_fft_stage(int stage, const FftStageArgs &a, cudaStream_t s) {
   const FftGeom g = fft_geom(stage, a.W, a.H);
-  const int grid = (g.L + g.lines - 1) / g.lines;
-  const size_t smem = fft_smem(stage, g);
+  const bool norms = stage == 0 && a.dens && a.norms.part2;
+  const int grid = (g.L + g.lines - 1) / g.lines + (norms ? 1 : 0);
   // The shared-memory limit is raised to the stage's largest need (a
   // 1024 x 1024 grid) every time: the same value from every thread, so
   // contexts launching from several host threads never lower it under one
   // another's launch.
   const int cap = (int)fft_smem(stage, fft_geom(stage, 1024, 1024));
-  cudaError_t e = cudaSuccess;
-  switch (stage) {
-    case 0:
-      e = cudaFuncSetAttribute(k_fft<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
-      if (e == cudaSuccess) k_fft<0><<<grid, kFftThreads, smem, s>>>(a);
-      break;
-    case 1:
-      e = cudaFuncSetAttribute(k_fft<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
-      if (e == cudaSuccess) k_fft<1><<<grid, kFftThreads, smem, s>>>(a);
-      break;
-    default:
-      e = cudaFuncSetAttribute(k_fft<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
-      if (e == cudaSuccess) k_fft<2><<<grid, kFftThreads, smem, s>>>(a);
-      break;
-  }
-  return e != cudaSuccess ? e : cudaGetLastError();
+  void (*const k)(FftStageArgs) = stage == 0 ? k_fft<0> : stage == 1 ? k_fft<1> : k_fft<2>;
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
+  if (e != cudaSuccess) return e;
+  Launch l(grid, kFftThreads, s, a.after, fft_smem(stage, g));
+  return cudaLaunchKernelEx(&l.cfg, k, a);
 }
 
 }  // namespace eplace

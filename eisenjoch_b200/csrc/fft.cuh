@@ -66,6 +66,8 @@ struct FftStageArgs {
   unsigned *ticket;
   DevScalars *sc;
   IterLog *log;
+  NormArgs norms;         // with dens and part2 set, one more CTA adds the step norms up
+  bool after;             // the launch may start while the kernel before it ends
 };
 
 bool fft_supported(int W, int H);

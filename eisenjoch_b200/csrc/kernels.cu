@@ -59,49 +59,14 @@ __device__ __forceinline__ double warp_sum_d(double v) {
   return v;
 }
 
-// Deterministic block sum of K doubles (fixed tree for a fixed block size).
-template <int K>
-__device__ __forceinline__ void block_sum(double (&v)[K], double *smem /* [32*K] */) {
+// Deterministic block sum of a double (fixed tree for a fixed block size),
+// valid in thread 0.
+__device__ __forceinline__ double block_sum_d(double v, double *smem /* [32] */) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int k = 0; k < K; ++k) v[k] = warp_sum_d(v[k]);
+  v = warp_sum_d(v);
+  if (lane == 0) smem[wid] = v;
   __syncthreads();
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < K; ++k) smem[wid * K + k] = v[k];
-  __syncthreads();
-  if (wid == 0) {
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      double t = lane < nw ? smem[lane * K + k] : 0.0;
-      v[k] = warp_sum_d(t);
-    }
-  }
-  __syncthreads();
-}
-
-// Deterministic sum over the per-block partials part[stride*b + k], b <
-// nblocks, for k < K, by the whole block: thread t reads blocks t, t +
-// blockDim, ... with L1-bypassing loads (the partials were written by other
-// SMs), then a fixed-tree block reduction; every thread gets the result.
-template <int K>
-__device__ __forceinline__ void sum_partials(const double *part, int stride, unsigned nblocks,
-                                             double (&out)[K], double *smem /* [32*K] */) {
-  double v[K];
-#pragma unroll
-  for (int k = 0; k < K; ++k) v[k] = 0.0;
-  for (unsigned b = threadIdx.x; b < nblocks; b += blockDim.x)
-#pragma unroll
-    for (int k = 0; k < K; ++k) v[k] += __ldcg(part + (size_t)stride * b + k);
-  block_sum<K>(v, smem);
-  __shared__ double bc[K];
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int k = 0; k < K; ++k) bc[k] = v[k];
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < K; ++k) out[k] = bc[k];
-  __syncthreads();
+  return wid == 0 ? warp_sum_d(lane < nw ? smem[lane] : 0.0) : 0.0;
 }
 
 // Per-axis WA terms with max/min shifts.  The reference shifts by the pin
@@ -123,29 +88,6 @@ __device__ __forceinline__ float ex2(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
-}
-
-// Segment max / min over the lanes of `mask` (one mask per segment; the
-// segments partition the warp).
-__device__ __forceinline__ float seg_max(float v, unsigned mask) {
-  float r;
-  asm volatile("redux.sync.max.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "r"(mask));
-  return r;
-}
-__device__ __forceinline__ float seg_min(float v, unsigned mask) {
-  float r;
-  asm volatile("redux.sync.min.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "r"(mask));
-  return r;
-}
-
-// Segment sum over [head, end) with `steps` shuffle rounds (2^steps >= the
-// longest segment of the warp), broadcast from the head lane.
-__device__ __forceinline__ float seg_sum(float v, int lane, int end, int head, int steps) {
-  for (int s = 0, o = 1; s < steps; ++s, o <<= 1) {
-    const float u = __shfl_down_sync(kFull, v, o);
-    if (lane + o < end) v += u;
-  }
-  return __shfl_sync(kFull, v, head);
 }
 
 // Reduction over the g lanes of an aligned lane group (g a power of two,
@@ -520,8 +462,14 @@ __global__ void __launch_bounds__(kFinalBlock) k_density_final(const FinalArgs a
   // stores (when every pointer is aligned for them; a ragged tail, or
   // unaligned caller buffers, take the scalar loop below).
   const int ng = a.vec4 ? (a.nb >> 2) : 0;
-  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, ts = gridDim.x * blockDim.x;
+  const int nblocks = (int)gridDim.x - (a.norms.part2 ? 1 : 0);  // the last one adds the norms up
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, ts = nblocks * blockDim.x;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if ((int)blockIdx.x == nblocks) {
+    if (threadIdx.x < 32) finish_norms(a.norms);
+    return;
+  }
   for (int gi = t0; gi < ng; gi += ts) {
     ulonglong2 *dp = reinterpret_cast<ulonglong2 *>(a.dens) + 2 * gi;
     const ulonglong2 q0 = dp[0], q1 = dp[1];
@@ -575,7 +523,7 @@ __global__ void __launch_bounds__(kFinalBlock) k_density_final(const FinalArgs a
   atomicAdd(&a.sums[0], (unsigned long long)v[0]);
   atomicAdd(&a.sums[1], (unsigned long long)v[1]);
   __threadfence();
-  if (atomicAdd(a.ticket, 1u) != gridDim.x - 1) return;
+  if (atomicAdd(a.ticket, 1u) != (unsigned)nblocks - 1) return;
   __threadfence();
   const double ov = overlap_of(atomicExch(&a.sums[0], 0ull), atomicExch(&a.sums[1], 0ull));
   if (a.overlap) {
@@ -807,51 +755,120 @@ bool sgemm_small_tile(int M, int N, int nb, int K) {
 }
 
 // ---------------------------------------------------------------------------
-// Grid barrier for the cooperative step kernel.  Every wait is bounded: on
-// timeout the block records the error in sc->err and leaves the kernel, so
-// the kernel always terminates, no block computes on partial data, and the
-// host reports EPLACE_ERR_TIMEOUT (the next run resets the device state).
+// The step: field gather, penalty, preconditioner, Barzilai-Borwein step,
+// FISTA, clamp, next look-ahead, and the next iteration's density scatter.
+//
+// Bound by latency: 200k cells are 15.7 MB of L2-resident state (2.4 us at the
+// HBM rate), but the loads of a cell depend on one another (look-ahead ->
+// field), and the step length needs a sum over all cells in between.  So:
+//  * a thread keeps its cells over the whole step: nothing but the block sums
+//    crosses blocks, and the state that the second half needs is loaded while
+//    the block waits for the others;
+//  * a macro (25 bins and more) is gathered by eight lanes, a column of bins
+//    each, four macros a warp, spread over all blocks.  The bins are summed in
+//    the row-major order of one thread, so the bits are the same; one thread
+//    per macro walked its rows one memory latency at a time and held the
+//    barrier up for 8 us at 200k cells (10k macros);
+//  * the block sums are formed with six FP64 shuffles a warp for four sums;
+//  * the next look-ahead is scattered into the density map while it is in
+//    registers (a launch, and a read of the positions, less);
+//  * the step norms, which only the log needs, are left as block sums for the
+//    next iteration's first kernel (finish_norms) instead of a last block.
+// Device time alone / in the loop, before and after: see launch_step.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ bool grid_barrier(unsigned *bar, DevScalars *sc) {
-  // bar[0..1] is one 64-bit arrival count that is never reset inside a run:
-  // every launch on it has the same grid and passes whole barriers, so a
-  // launch starts at a multiple of gridDim.x, and barrier k of the run is
-  // complete when the count reaches (k + 1) * gridDim.x.  The last block's
-  // own add releases the others (no reset, no second word to publish).
-  // The host zeroes the count at every load and run start.  The wait is
-  // bounded (sc->spin_cycles): a block that gives up records sc->err and
-  // returns false, and its caller leaves the kernel.
-  __shared__ int gave_up;
+
+// The four sums v over the block; lane k < 4 of warp 0 gets sum k in v[0].
+// sm: [4 * 16].  One barrier; sm must not be in use before it.
+__device__ __forceinline__ double block_sum4(const double (&v)[4], double *sm) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  // each exchange halves the sums a lane carries: 4 -> 2 -> 1, then three adds
+  const bool up = lane & 16, up2 = lane & 8;
+  double a = up ? v[2] : v[0], b = up ? v[3] : v[1];
+  a += __shfl_xor_sync(kFull, up ? v[0] : v[2], 16);
+  b += __shfl_xor_sync(kFull, up ? v[1] : v[3], 16);
+  double c = up2 ? b : a;
+  c += __shfl_xor_sync(kFull, up2 ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
+  // lanes 8 k .. 8 k + 7 carry sum k
+  if ((lane & 7) == 0) sm[4 * w + (lane >> 3)] = c;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    gave_up = 0;
-    unsigned long long *cnt = reinterpret_cast<unsigned long long *>(bar);
-    const long long limit = sc->spin_cycles > 0 ? sc->spin_cycles : kSpinCycles;
-    __threadfence();  // this block's writes before its arrival
-    const unsigned long long old = atomicAdd(cnt, 1ull);
-    const unsigned long long target = old - old % gridDim.x + gridDim.x;
-    const long long t0 = clock64();
-    while (true) {
-      unsigned long long v;
-      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(cnt) : "memory");
-      if (v >= target) break;
-      if (clock64() - t0 > limit) {
-        atomicExch(&sc->err, 1);
-        gave_up = 1;
-        break;
+  double t = 0.0;
+  if (w == 0) {  // lane: sum lane & 3 of warps lane / 4 and lane / 4 + 8
+    const int k = lane & 3, i = lane >> 2;
+    t = (i < nw ? sm[4 * i + k] : 0.0) + (i + 8 < nw ? sm[4 * (i + 8) + k] : 0.0);
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) t += __shfl_xor_sync(kFull, t, o);
+  }
+  return t;
+}
+
+// The block sums part[4 b + k] of all blocks, by the whole block: every
+// thread gets the four totals (in a fixed order).  sm: [4 * 16], tot: [4].
+__device__ __forceinline__ void total_of(const double *part, unsigned nblocks, double (&out)[4], double *sm,
+                                         double *tot) {
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+  for (unsigned b = threadIdx.x; b < nblocks; b += blockDim.x) {
+    const double2 p = __ldcg(reinterpret_cast<const double2 *>(part) + 2 * b);
+    const double2 q = __ldcg(reinterpret_cast<const double2 *>(part) + 2 * b + 1);
+    v[0] += p.x;
+    v[1] += p.y;
+    v[2] += q.x;
+    v[3] += q.y;
+  }
+  const double t = block_sum4(v, sm);
+  if (threadIdx.x < 4) tot[threadIdx.x] = t;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 4; ++k) out[k] = tot[k];
+}
+
+// Grid barrier of the cooperative step, once the block's sums (lane k < 4 of
+// warp 0: sum t) are in part[].  Every wait is bounded: on timeout the block
+// records the error in sc->err and leaves the kernel, so the kernel always
+// terminates, no block computes on partial data, and the host reports
+// EPLACE_ERR_TIMEOUT (the next run resets the device state).
+// bar[0..1] is one 64-bit arrival count that is never reset inside a run:
+// every launch on it has the same grid and passes whole barriers, so a launch
+// starts at a multiple of gridDim.x, and barrier k of the run is complete when
+// the count reaches (k + 1) * gridDim.x.  The last block's own add releases
+// the others.  The host zeroes the count at every load and run start.
+__device__ __forceinline__ bool publish_and_wait(double *part, double t, unsigned *bar, DevScalars *sc, int *gave_up) {
+  if (threadIdx.x < 32) {
+    if (threadIdx.x < 4) __stcg(part + 4 * blockIdx.x + threadIdx.x, t);
+    __syncwarp();
+    if (threadIdx.x == 0) {
+      *gave_up = 0;
+      unsigned long long *cnt = reinterpret_cast<unsigned long long *>(bar);
+      const long long limit = sc->spin_cycles > 0 ? sc->spin_cycles : kSpinCycles;
+      __threadfence();  // the sums before the arrival
+      const unsigned long long old = atomicAdd(cnt, 1ull);
+      // (a run's arrivals stay far below 2^32: a 64-bit remainder is slow)
+      const unsigned long long target =
+          old < 0xffffffffull ? old - (unsigned)old % gridDim.x + gridDim.x : old - old % gridDim.x + gridDim.x;
+      const long long t0 = clock64();
+      while (true) {
+        unsigned long long v;
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(cnt) : "memory");
+        if (v >= target) break;
+        if (clock64() - t0 > limit) {
+          atomicExch(&sc->err, 1);
+          *gave_up = 1;
+          break;
+        }
       }
-      __nanosleep(32);
+      __threadfence();
     }
-    __threadfence();
   }
   __syncthreads();
-  return !gave_up;
+  return !*gave_up;
 }
 
 // Field gather of a 1x1 footprint: it touches at most 2 x 2 bins (bins are
 // >= 1 site wide); weights first, then all field loads at once, summed in the
-// same row-major order as the general loop of gather_cell.
-__device__ __forceinline__ float2 gather_unit_foot(const StepArgs &a, const Foot &f) {
+// same row-major order as the general form.
+__device__ __forceinline__ float2 gather_unit(const StepArgs &a, float2 p) {
+  const Foot f = make_foot(p, 0.5f, 0.5f, a.BX, a.BY, a.isx, a.isy);
   float fx = 0.f, fy = 0.f, wt = 0.f;
   float w[4];
   size_t id[4];
@@ -883,77 +900,85 @@ __device__ __forceinline__ float2 gather_unit_foot(const StepArgs &a, const Foot
   return g;
 }
 
-// Field gather of a 1x1 cell (no footprint load).
-__device__ __forceinline__ float2 gather_unit(const StepArgs &a, float2 p) {
-  const Foot f = make_foot(p, 0.5f, 0.5f, a.BX, a.BY, a.isx, a.isy);
-  return gather_unit_foot(a, f);
-}
+// A warp's eight-lane groups, one macro each.
+struct Macro {
+  uint32_t i;   // cell
+  bool in;      // the group has one
+  int col;      // this lane's column of the group, 0 .. 7
+  float2 hf;
+  float area;
+};
 
-// Weighted-mean field gather for one cell, scaled by its area
-// (compute_density_gradient, density.rs:171-206).
-__device__ __forceinline__ float2 gather_cell(const StepArgs &a, uint32_t i, float2 p) {
-  const float2 hf = a.half ? a.half[i] : make_float2(0.5f, 0.5f);
-  const Foot f = make_foot(p, hf.x, hf.y, a.BX, a.BY, a.isx, a.isy);
+// Weighted-mean field gather of the groups' macros at p, scaled by the area
+// (compute_density_gradient, density.rs:171-206): each lane loads its column
+// of the footprint's bins, eight columns and up to kRows rows in flight, and
+// every lane of the group sums the bins in row-major order.  All lanes of the
+// warp call it; every lane of a group gets the result.
+__device__ __forceinline__ float2 gather_macro(const StepArgs &a, const Macro &m, float2 p) {
+  constexpr int kRows = 5;
+  const Foot f = make_foot(p, m.hf.x, m.hf.y, a.BX, a.BY, a.isx, a.isy);
+  const int parts = (max(f.bx1 - f.bx0, 0) + 7) >> 3;  // eight-bin parts of a row
+  const int n = m.in ? parts * max(f.by1 - f.by0, 0) : 0;
+  const int most = (int)__reduce_max_sync(kFull, (unsigned)n);
+  const int lead = threadIdx.x & 24;
   float fx = 0.f, fy = 0.f, wt = 0.f;
-  if (hf.x == 0.5f && hf.y == 0.5f) return gather_unit_foot(a, f);
-  // Bins of a row in chunks of 8 with all field loads of a chunk issued
-  // before the sums (a macro spans up to 9 bins per axis), so a footprint
-  // costs one memory latency per row and chunk instead of one per bin; the
-  // sums keep the row-major bin order.
-  for (int by = f.by0; by < f.by1; ++by) {
-    const float oy = overlap_y(f, by, a.isy);
-    for (int b0 = f.bx0; b0 < f.bx1; b0 += 8) {
-      float w[8], e[8], h[8];
+  int by = f.by0, part = 0;
+  for (int r0 = 0; r0 < most; r0 += kRows) {
+    float w[kRows], e[kRows], h[kRows];
+#pragma unroll
+    for (int u = 0; u < kRows; ++u) {
+      const int bx = f.bx0 + 8 * part + m.col;
+      w[u] = (r0 + u < n && bx < f.bx1) ? overlap_x(f, bx, a.isx) * overlap_y(f, by, a.isy) : 0.0f;
+      const size_t idx = w[u] > 0.0f ? (size_t)by * a.BX + bx : 0;
+      e[u] = w[u] > 0.0f ? a.Ex[idx] : 0.0f;
+      h[u] = w[u] > 0.0f ? a.Ey[idx] : 0.0f;
+      if (++part == parts) {
+        part = 0;
+        ++by;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kRows; ++u) {
+      if (r0 + u >= most) break;  // the same in every lane
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const int bx = b0 + k;
-        w[k] = (bx < f.bx1) ? overlap_x(f, bx, a.isx) * oy : 0.0f;
-        const size_t idx = (size_t)by * a.BX + (w[k] > 0.0f ? bx : 0);
-        e[k] = (w[k] > 0.0f) ? a.Ex[idx] : 0.0f;
-        h[k] = (w[k] > 0.0f) ? a.Ey[idx] : 0.0f;
-      }
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (w[k] > 0.0f) {
-          fx = fmaf(w[k], e[k], fx);
-          fy = fmaf(w[k], h[k], fy);
-          wt += w[k];
+        const float wk = __shfl_sync(kFull, w[u], lead + k);
+        const float ek = __shfl_sync(kFull, e[u], lead + k), hk = __shfl_sync(kFull, h[u], lead + k);
+        if (wk > 0.0f) {
+          fx = fmaf(wk, ek, fx);
+          fy = fmaf(wk, hk, fy);
+          wt += wk;
         }
+      }
     }
   }
   float2 g = make_float2(0.f, 0.f);
   if (wt > 1e-10f) {
-    const float ar = a.area ? a.area[i] : 1.0f;
-    g.x = ar * (fx / wt);
-    g.y = ar * (fy / wt);
+    g.x = m.area * (fx / wt);
+    g.y = m.area * (fy / wt);
   }
   return g;
 }
 
 // g = (g_wl + lam g_den) / max(1, pw + lam area)   (mod.rs:145-156)
-// unit: a 1x1 cell, whose area is 1 (no load).
-__device__ __forceinline__ float2 combine(const StepArgs &a, uint32_t i, float2 gw, float2 gd,
-                                          double lam, bool unit) {
-  const double ar = (unit || !a.area) ? 1.0 : (double)a.area[i];
-  const double ipc = 1.0 / fmax((double)a.pw[i] + lam * ar, 1.0);
+__device__ __forceinline__ float2 combine(float2 gw, float2 gd, double lam, float pw, float area) {
+  const double ipc = 1.0 / fmax((double)pw + lam * (double)area, 1.0);
   return make_float2((float)(((double)gw.x + lam * (double)gd.x) * ipc),
                      (float)(((double)gw.y + lam * (double)gd.y) * ipc));
 }
 
-// Phase A of the step for one cell, split into its loads and the rest so
-// that a thread can have the loads of two cells in flight.
-struct CellA {
-  float2 gd, gw;     // density field gather, WA gradient
-  float2 x, xp, gp;  // for the Barzilai-Borwein dots (after the first penalty)
+// What the first half of the step knows of a cell before the gather.
+struct CellIn {
+  float2 look, x, xp, gp;
+  unsigned long long acc;
+  float pw;
 };
 
-// unit: the cell is 1x1 (the 2 x 2-bin gather, no footprint load).
-__device__ __forceinline__ CellA load_a(const StepArgs &a, uint32_t i, bool was_init, bool unit) {
-  CellA c;
-  c.gd = unit ? gather_unit(a, a.look[i]) : gather_cell(a, i, a.look[i]);
-  long long sx, sy;
-  unpack_grad(a.acc[i], &sx, &sy);
-  c.gw = make_float2((float)((double)sx * a.grad_inv), (float)((double)sy * a.grad_inv));
+__device__ __forceinline__ CellIn load_in(const StepArgs &a, uint32_t i, bool was_init) {
+  CellIn c;
+  c.look = a.look[i];
+  c.acc = a.acc[i];
+  c.pw = a.pw[i];
   if (was_init) {
     c.x = a.x[i];
     c.xp = a.xp[i];
@@ -962,29 +987,38 @@ __device__ __forceinline__ CellA load_a(const StepArgs &a, uint32_t i, bool was_
   return c;
 }
 
-__device__ __forceinline__ void finish_a(const StepArgs &a, uint32_t i, const CellA &c, bool was_init, double lam,
-                                         bool unit, double (&v)[4]) {
+__device__ __forceinline__ void bb_terms(double (&v)[4], float2 x, float2 xp, float2 g, float2 gp) {
+  const double dx = (double)x.x - xp.x, dy = (double)x.y - xp.y;
+  v[0] += dx * dx;
+  v[1] += dx * ((double)g.x - gp.x);
+  v[2] += dy * dy;
+  v[3] += dy * ((double)g.y - gp.y);
+}
+
+// The rest of the first half: combined gradient and the terms of the sums
+// (before the first penalty: the two gradients and their norms).
+__device__ __forceinline__ void first_half(const StepArgs &a, uint32_t i, const CellIn &c, float2 gd, float area,
+                                           bool was_init, double lam, double (&v)[4]) {
+  long long sx, sy;
+  unpack_grad(c.acc, &sx, &sy);
+  const float2 gw = make_float2((float)((double)sx * a.grad_inv), (float)((double)sy * a.grad_inv));
   a.acc[i] = 0ull;
   if (was_init) {
-    const float2 g = combine(a, i, c.gw, c.gd, lam, unit);
+    const float2 g = combine(gw, gd, lam, c.pw, area);
     a.g[i] = g;
-    const double dx = (double)c.x.x - c.xp.x, dy = (double)c.x.y - c.xp.y;
-    v[0] += dx * dx;
-    v[1] += dx * ((double)g.x - c.gp.x);
-    v[2] += dy * dy;
-    v[3] += dy * ((double)g.y - c.gp.y);
+    bb_terms(v, c.x, c.xp, g, c.gp);
     return;
   }
-  a.tmp_wl[i] = c.gw;
-  a.tmp_den[i] = c.gd;
-  v[0] += (double)c.gw.x * c.gw.x + (double)c.gw.y * c.gw.y;
-  v[1] += (double)c.gd.x * c.gd.x + (double)c.gd.y * c.gd.y;
+  a.tmp_wl[i] = gw;
+  a.tmp_den[i] = gd;
+  v[0] += (double)gw.x * gw.x + (double)gw.y * gw.y;
+  v[1] += (double)gd.x * gd.x + (double)gd.y * gd.y;
 }
 
 // FISTA step (nesterov.rs:41-64), clamp (:67-72), next look-ahead (:95-101)
-// clamped to the chip (common.rs:410-415), for one cell.
-__device__ __forceinline__ void fista_cell(const StepArgs &a, uint32_t i, float2 x, float2 xp, float2 g, double m,
-                                           double mn, const double (&alpha)[2], double (&nrm)[2]) {
+// clamped to the chip (common.rs:410-415), for one cell; returns the latter.
+__device__ __forceinline__ float2 fista_cell(const StepArgs &a, uint32_t i, float2 x, float2 xp, float2 g, double m,
+                                             double mn, const double (&alpha)[2], double (&nrm)[4]) {
   const double yx = (double)x.x + m * ((double)x.x - xp.x);
   const double yy = (double)x.y + m * ((double)x.y - xp.y);
   const double nx = yx - alpha[0] * g.x, ny = yy - alpha[1] * g.y;
@@ -999,157 +1033,183 @@ __device__ __forceinline__ void fista_cell(const StepArgs &a, uint32_t i, float2
   a.gprev[i] = g;
   const double lx = (double)cx + mn * ((double)cx - px);
   const double ly = (double)cy + mn * ((double)cy - py);
-  a.look[i] = make_float2(fminf(fmaxf((float)lx, 0.0f), a.maxx), fminf(fmaxf((float)ly, 0.0f), a.maxy));
+  const float2 look = make_float2(fminf(fmaxf((float)lx, 0.0f), a.maxx), fminf(fmaxf((float)ly, 0.0f), a.maxy));
+  a.look[i] = look;
+  return look;
 }
 
+// The next iteration's density scatter of a unit cell, and of the groups' macros.
+__device__ __forceinline__ void scatter_unit(const StepArgs &a, float2 p) {
+  const Foot f = make_foot(p, 0.5f, 0.5f, a.BX, a.BY, a.isx, a.isy);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int by = f.by0 + (k >> 1), bx = f.bx0 + (k & 1);
+    if (by < f.by1 && bx < f.bx1) add_bin(a.dens, f, bx, by, a.BX, a.isx, a.isy);
+  }
+}
+__device__ __forceinline__ void scatter_macro(const StepArgs &a, const Macro &m, float2 p) {
+  if (!m.in) return;
+  const Foot f = make_foot(p, m.hf.x, m.hf.y, a.BX, a.BY, a.isx, a.isy);
+  for (int by = f.by0; by < f.by1; ++by)
+    for (int bx = f.bx0 + m.col; bx < f.bx1; bx += 8) add_bin(a.dens, f, bx, by, a.BX, a.isx, a.isy);
+}
+
+// The macros of this warp, four at a time: fn(Macro) with all lanes.  Tasks of
+// four go to the blocks in turn, to a block's last warps first.
+template <typename F>
+__device__ __forceinline__ void each_macro(const StepArgs &a, F fn) {
+  const int nwb = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t tasks = (a.n_mac + 3) / 4;
+  for (uint32_t t = blockIdx.x + gridDim.x * (uint32_t)(nwb - 1 - w); t < tasks; t += gridDim.x * (uint32_t)nwb) {
+    Macro m;
+    const uint32_t k = 4 * t + (lane >> 3);
+    m.in = k < a.n_mac;
+    m.i = a.mac_idx[m.in ? k : 0];
+    m.col = lane & 7;
+    m.hf = a.half[m.i];
+    m.area = a.area[m.i];
+    fn(m);
+  }
+}
+
+// Modes: 0: the whole step in one cooperative launch (grid barriers between
+// its halves); 1: gather only (tmp_den <- density gradient); 2, 3, 4: first
+// half, penalty-initialisation pass and second half as three ordinary launches
+// of the same grid (launch order replaces the barriers, so no block ever waits
+// for another).
 __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
-  __shared__ double sm[32 * 4];
-  __shared__ bool last;
+  __shared__ __align__(16) double sm[64], sm2[64], tot[4];
+  __shared__ int gave_up;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t tid0 = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t gstride = gridDim.x * blockDim.x;
   const int it = a.sc->iter;
   const bool was_init = a.sc->lam_init != 0;
+  double alpha[2] = {a.sc->step[0], a.sc->step[1]};
   double lam = a.sc->lam;
   bool lam_init = was_init;
   if (was_init) lam = (lam < 50.0) ? lam * 1.025 : lam + 1.0;  // mod.rs:139-143
-
   // A bounded wait already gave up in an earlier launch: every block sees the
   // same flag here and leaves before any barrier, so the rest of the
   // interval drains quickly and the host reports EPLACE_ERR_TIMEOUT.
   if (a.sc->err) return;
+
   if (a.mode == 1) {  // gather only: no barrier is reached
-    for (uint32_t i = tid0; i < a.N; i += gstride) a.tmp_den[i] = gather_cell(a, i, a.look[i]);
+    each_macro(a, [&](const Macro &m) {
+      const float2 g = gather_macro(a, m, a.look[m.i]);
+      if (m.in && m.col == 0) a.tmp_den[m.i] = g;
+    });
+    for (uint32_t i = tid0; i < a.N; i += gstride)
+      if (!a.mflag || !a.mflag[i]) a.tmp_den[i] = gather_unit(a, a.look[i]);
     return;
   }
-  // Modes: 0 = whole step in one cooperative launch (grid barriers between
-  // phases); 2, 3, 4 = phase A, the penalty-initialisation pass and phase C
-  // as three ordinary launches of the same grid (kernel boundaries replace
-  // the barriers, so no block ever waits for another).
   const bool coop = a.mode == 0;
-  double v[4] = {0.0, 0.0, 0.0, 0.0};
-  if (a.mode == 0 || a.mode == 2) {
-    // Phase A: gather, read + clear the WA accumulator, combine.  Two cells
-    // per thread and pass (i and i + ustride): every load of both is issued
-    // before the first store, so their latencies overlap.  Macros (w*h > 1)
-    // are skipped here and done afterwards from their own list, so a warp
-    // of unit cells never waits for one macro's multi-bin gather.
-    // When the unit cells still fit one pass of pairs on the other threads,
-    // the last n_mac threads of the grid take macros only (macro k goes to
-    // thread gstride - 1 - k, mod gstride), so a macro's multi-row gather
-    // does not queue behind a unit cell in the same thread (200k cells:
-    // step 29.1 -> 26.9 us); otherwise (800k) every thread takes unit cells.
-    const uint32_t nm =
-        (a.n_mac <= gstride / 4 && (uint64_t)a.N <= 2ull * (gstride - a.n_mac)) ? a.n_mac : 0u;
-    const uint32_t ustride = gstride - nm;
-    if (tid0 < ustride)
-      for (uint32_t i0 = tid0; i0 < a.N; i0 += 2 * ustride) {
-        const uint32_t i1 = i0 + ustride;
-        const bool h1 = i1 < a.N;
-        const bool u0 = !a.mflag || !a.mflag[i0];
-        const bool u1 = h1 && (!a.mflag || !a.mflag[i1]);
-        CellA c0, c1;
-        if (u0) c0 = load_a(a, i0, was_init, true);
-        if (u1) c1 = load_a(a, i1, was_init, true);
-        if (u0) finish_a(a, i0, c0, was_init, lam, true, v);
-        if (u1) finish_a(a, i1, c1, was_init, lam, true, v);
-      }
-    for (uint32_t k = gstride - 1 - tid0; k < a.n_mac; k += gstride) {
-      const uint32_t i = a.mac_idx[k];
-      const CellA c = load_a(a, i, was_init, false);
-      finish_a(a, i, c, was_init, lam, false, v);
+  // The state that the second half needs of this thread's first two cells,
+  // loaded while the block waits for the others.
+  float2 x0, xp0, g0, x1, xp1, g1;
+  const uint32_t j0 = tid0, j1 = tid0 + gstride;
+  const bool in0 = j0 < a.N && (!a.mflag || !a.mflag[j0]), in1 = j1 < a.N && (!a.mflag || !a.mflag[j1]);
+  auto preload = [&] {
+    if (in0) {
+      x0 = a.x[j0];
+      xp0 = a.xp[j0];
+      g0 = a.g[j0];
     }
-    block_sum<4>(v, sm);
-    if (threadIdx.x == 0)
-      for (int k = 0; k < 4; ++k) a.part[4 * blockIdx.x + k] = v[k];
-    if (a.mode == 2) return;
-    if (!grid_barrier(a.bar, a.sc)) return;
+    if (in1) {
+      x1 = a.x[j1];
+      xp1 = a.xp[j1];
+      g1 = a.g[j1];
+    }
+  };
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+  if (coop || a.mode == 2) {
+    each_macro(a, [&](const Macro &m) {
+      CellIn c;
+      c.look = a.look[m.i];
+      if (m.col == 0) c = load_in(a, m.i, was_init);
+      const float2 gd = gather_macro(a, m, c.look);
+      if (m.in && m.col == 0) first_half(a, m.i, c, gd, m.area, was_init, lam, v);
+    });
+    // Two cells per thread and pass, every load of both issued before the
+    // first store, so that their latencies overlap (a macro's are loaded for
+    // nothing: its flag arrives with them).
+    for (uint32_t i0 = tid0; i0 < a.N; i0 += 2 * gstride) {
+      const uint32_t i1 = i0 + gstride;
+      const bool h1 = i1 < a.N;
+      const bool u0 = !a.mflag || !a.mflag[i0];
+      const bool u1 = h1 && (!a.mflag || !a.mflag[i1]);
+      const CellIn c0 = load_in(a, i0, was_init), c1 = load_in(a, h1 ? i1 : i0, was_init);
+      const float2 d0 = gather_unit(a, c0.look), d1 = gather_unit(a, c1.look);
+      if (u0) first_half(a, i0, c0, d0, 1.0f, was_init, lam, v);
+      if (u1) first_half(a, i1, c1, d1, 1.0f, was_init, lam, v);
+    }
+    const double t = block_sum4(v, sm);
+    if (a.mode == 2) {
+      if (threadIdx.x < 4) a.part[4 * blockIdx.x + threadIdx.x] = t;
+      return;
+    }
+    if (was_init) preload();
+    if (!publish_and_wait(a.part, t, a.bar, a.sc, &gave_up)) return;
   }
 
-  // Pass-2 partials: part[] again after a barrier (cooperative), else part_b[].
-  double *part2nd = coop ? a.part : a.part_b;
   if (!was_init) {
     // First penalty: 0.1 * |g_wl| / |g_den| when |g_den| > 1e-30 (mod.rs:132-138).
-    double nr[2];
-    sum_partials<2>(a.part, 4, gridDim.x, nr, sm);
+    double nr[4];
+    total_of(a.part, gridDim.x, nr, sm2, tot);
     const double wl = sqrt(nr[0]);
     const double dn = sqrt(nr[1]);
     if (dn > 1e-30) {
       lam = 0.1 * wl / dn;
       lam_init = true;
     }
-    if (a.mode == 0 || a.mode == 3) {
-      if (coop) if (!grid_barrier(a.bar, a.sc)) return;  // everyone has read part[] before it is reused
+    if (coop || a.mode == 3) {
       for (int k = 0; k < 4; ++k) v[k] = 0.0;
-      for (uint32_t i = tid0; i < a.N; i += gstride) {
-        const float2 g = combine(a, i, a.tmp_wl[i], a.tmp_den[i], lam, false);
+      auto pass = [&](uint32_t i, float area) {
+        const float2 g = combine(a.tmp_wl[i], a.tmp_den[i], lam, a.pw[i], area);
         a.g[i] = g;
-        const float2 x = a.x[i], xp = a.xp[i], gp = a.gprev[i];
-        const double dx = (double)x.x - xp.x, dy = (double)x.y - xp.y;
-        v[0] += dx * dx;
-        v[1] += dx * ((double)g.x - gp.x);
-        v[2] += dy * dy;
-        v[3] += dy * ((double)g.y - gp.y);
+        bb_terms(v, a.x[i], a.xp[i], g, a.gprev[i]);
+      };
+      each_macro(a, [&](const Macro &m) {
+        if (m.in && m.col == 0) pass(m.i, m.area);
+      });
+      for (uint32_t i = tid0; i < a.N; i += gstride)
+        if (!a.mflag || !a.mflag[i]) pass(i, 1.0f);
+      const double t = block_sum4(v, sm);
+      if (a.mode == 3) {
+        if (threadIdx.x < 4) a.part_b[4 * blockIdx.x + threadIdx.x] = t;
+        return;
       }
-      block_sum<4>(v, sm);
-      if (threadIdx.x == 0)
-        for (int k = 0; k < 4; ++k) part2nd[4 * blockIdx.x + k] = v[k];
-      if (a.mode == 3) return;
-      if (!grid_barrier(a.bar, a.sc)) return;
+      preload();
+      if (!publish_and_wait(a.part_b, t, a.bar, a.sc, &gave_up)) return;
     }
   } else if (a.mode == 3) {
     return;
   }
+  if (a.mode == 4) preload();
 
   // Barzilai-Borwein per axis after the first iteration (mod.rs:158-166,
   // nesterov.rs:199-218): |dx.dx / dx.dg| clamped to [1e-4, 1], kept when
   // |dx.dg| < 1e-30.
   double t[4];
-  sum_partials<4>(was_init ? a.part : part2nd, 4, gridDim.x, t, sm);
-  double alpha[2] = {a.sc->step[0], a.sc->step[1]};
+  total_of(was_init ? a.part : a.part_b, gridDim.x, t, sm2, tot);
   if (it > 0) {
     for (int ax = 0; ax < 2; ++ax) {
       const double dxdx = t[2 * ax], dxdg = t[2 * ax + 1];
       if (!(fabs(dxdg) < 1e-30)) alpha[ax] = fmin(fmax(fabs(dxdx / dxdg), 1e-4), 1.0);
     }
   }
-  // FISTA step (nesterov.rs:41-64), clamp (:67-72), next look-ahead
-  // (:95-101) clamped to the chip (common.rs:410-415).
-  const double m = a.mom[it], mn = a.mom[it + 1];
-  double nrm[2] = {0.0, 0.0};
-  for (uint32_t i0 = tid0; i0 < a.N; i0 += 2 * gstride) {  // two cells per pass, loads first
-    const uint32_t i1 = i0 + gstride;
-    const bool h1 = i1 < a.N;
-    const float2 x0 = a.x[i0], xp0 = a.xp[i0], g0 = a.g[i0];
-    float2 x1 = x0, xp1 = xp0, g1 = g0;
-    if (h1) {
-      x1 = a.x[i1];
-      xp1 = a.xp[i1];
-      g1 = a.g[i1];
-    }
-    fista_cell(a, i0, x0, xp0, g0, m, mn, alpha, nrm);
-    if (h1) fista_cell(a, i1, x1, xp1, g1, m, mn, alpha, nrm);
-  }
-  double w2[2] = {nrm[0], nrm[1]};
-  block_sum<2>(w2, sm);
-  // Step norms go to a second partials buffer, so no block has to wait for
-  // the others to finish reading part[]; the last block to arrive sums them.
-  if (threadIdx.x == 0) {
-    a.part2[2 * blockIdx.x] = w2[0];
-    a.part2[2 * blockIdx.x + 1] = w2[1];
+  // Block 0 writes the scalars and the log entry once every block has read the
+  // scalars: after a grid barrier, all have; in mode 4 the last block to get
+  // here does it instead (its whole block is past its reads).
+  bool writer = blockIdx.x == 0;
+  if (!coop && threadIdx.x == 0) {
     __threadfence();
-    last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+    writer = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
   }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double fin[2];
-  sum_partials<2>(a.part2, 2, gridDim.x, fin, sm);
-  if (threadIdx.x == 0) {
-    const double s0 = fin[0], s1 = fin[1];
+  if (writer && threadIdx.x == 0) {
     IterLog &L = a.log[it];
     L.lam = lam;
-    L.step_norm[0] = sqrt(s0);
-    L.step_norm[1] = sqrt(s1);
     L.alpha[0] = alpha[0];
     L.alpha[1] = alpha[1];
     a.sc->lam = lam;
@@ -1159,11 +1219,61 @@ __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
     a.sc->iter = it + 1;
     *a.ticket = 0u;
   }
+  // FISTA step (nesterov.rs:41-64), clamp (:67-72), next look-ahead
+  // (:95-101) clamped to the chip (common.rs:410-415), and its density.
+  const double m = a.mom[it], mn = a.mom[it + 1];
+  double nrm[4] = {0.0, 0.0, 0.0, 0.0};
+  each_macro(a, [&](const Macro &c) {
+    float2 p = make_float2(0.f, 0.f);
+    if (c.in && c.col == 0) p = fista_cell(a, c.i, a.x[c.i], a.xp[c.i], a.g[c.i], m, mn, alpha, nrm);
+    if (a.dens) {
+      const int lead = threadIdx.x & 24;
+      p = make_float2(__shfl_sync(kFull, p.x, lead), __shfl_sync(kFull, p.y, lead));
+      scatter_macro(a, c, p);
+    }
+  });
+  float2 l0, l1;
+  if (in0) l0 = fista_cell(a, j0, x0, xp0, g0, m, mn, alpha, nrm);
+  if (in1) l1 = fista_cell(a, j1, x1, xp1, g1, m, mn, alpha, nrm);
+  if (a.dens) {
+    if (in0) scatter_unit(a, l0);
+    if (in1) scatter_unit(a, l1);
+  }
+  for (uint32_t i0 = tid0 + 2 * gstride; i0 < a.N; i0 += 2 * gstride) {  // two cells per pass, loads first
+    const uint32_t i1 = i0 + gstride;
+    const bool h0 = !a.mflag || !a.mflag[i0], h1 = i1 < a.N && (!a.mflag || !a.mflag[i1]);
+    const float2 xa = a.x[i0], xpa = a.xp[i0], ga = a.g[i0];
+    float2 xb = xa, xpb = xpa, gb = ga;
+    if (h1) {
+      xb = a.x[i1];
+      xpb = a.xp[i1];
+      gb = a.g[i1];
+    }
+    if (h0) l0 = fista_cell(a, i0, xa, xpa, ga, m, mn, alpha, nrm);
+    if (h1) l1 = fista_cell(a, i1, xb, xpb, gb, m, mn, alpha, nrm);
+    if (a.dens) {
+      if (h0) scatter_unit(a, l0);
+      if (h1) scatter_unit(a, l1);
+    }
+  }
+  // The step norms stay block sums; the next iteration's first kernel adds them.
+  const double s = block_sum4(nrm, sm);
+  if (threadIdx.x < 2) a.part2[2 * blockIdx.x + threadIdx.x] = s;
+}
+
+// The end of an interval: the positions and scalars into a snapshot, and the
+// last iteration's step norms into its log entry.
+__global__ void __launch_bounds__(256) k_snapshot(const SnapArgs a) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) a.pos[i] = a.x[i];
+  if (blockIdx.x == 0 && threadIdx.x < 32) {
+    finish_norms(a.norms);
+    if (threadIdx.x == 0) *a.sc_out = *a.norms.sc;
+  }
 }
 
 __global__ void __launch_bounds__(kHpwlBlock) k_hpwl(const HpwlArgs a) {
   __shared__ double sm[32];
-  double v[1] = {0.0};
+  double v = 0.0;
   for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < a.NN; n += gridDim.x * blockDim.x) {
     const uint32_t b = a.net_off[n], e = a.net_off[n + 1];
     if ((a.has_driver && !a.has_driver[n]) || e - b < 2) continue;
@@ -1175,11 +1285,11 @@ __global__ void __launch_bounds__(kHpwlBlock) k_hpwl(const HpwlArgs a) {
       y0 = min(y0, l.y);
       y1 = max(y1, l.y);
     }
-    v[0] += (double)((long long)(x1 - x0) + (long long)(y1 - y0));
+    v += (double)((long long)(x1 - x0) + (long long)(y1 - y0));
   }
   // Per-thread partials are integers below 2^53, so the FP64 block sum is exact.
-  block_sum<1>(v, sm);
-  if (threadIdx.x == 0) atomicAdd(a.total, (unsigned long long)(long long)v[0]);
+  v = block_sum_d(v, sm);
+  if (threadIdx.x == 0) atomicAdd(a.total, (unsigned long long)(long long)v);
 }
 
 }  // namespace
@@ -1200,16 +1310,8 @@ cudaError_t launch_density_final(const FinalArgs &a_in, int grid, cudaStream_t s
   FinalArgs a = a_in;
   auto al = [](const void *p, uintptr_t m) { return ((uintptr_t)p & (m - 1)) == 0; };
   a.vec4 = al(a.dens, 16) && al(a.rho, 16) && al(a.rho_hi, 8) && al(a.rho_lo, 8) && al(a.dens_out, 16);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kFinalBlock);
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = after ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, k_density_final, a);
+  Launch l(grid + (a.norms.part2 ? 1 : 0), kFinalBlock, s, after);
+  return cudaLaunchKernelEx(&l.cfg, k_density_final, a);
 }
 
 // One SIMT GEMM launch: split K four ways over a cluster when 4 * GK
@@ -1283,26 +1385,42 @@ cudaError_t launch_fly_rows(const FlyOp *ops, int nb, int H, int W, cudaStream_t
   return cudaGetLastError();
 }
 
-int step_max_grid(int device) {
+// Threads per block of the step: small designs spread over the SMs (a block
+// of 512 threads per SM issues the FP64 code four times slower than one of
+// 128), large ones keep the barrier's arrivals few.
+int step_block(int device, uint32_t cells) {
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0) sms = 148;
+  return cells <= 128u * (unsigned)sms ? 128 : cells <= 512u * (unsigned)sms ? 256 : kStepBlock;
+}
+
+int step_max_grid(int device, int block) {
   int sms = 0, occ = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_step, kStepBlock, 0) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_step, block, 0) != cudaSuccess) return 0;
   return sms * occ;
 }
 
-cudaError_t launch_step(const StepArgs &a, int grid, cudaStream_t s) {
+cudaError_t launch_step(const StepArgs &a, int grid, int block, cudaStream_t s) {
   void *args[] = {const_cast<StepArgs *>(&a)};
-  return cudaLaunchCooperativeKernel((const void *)k_step, dim3(grid), dim3(kStepBlock), args, 0, s);
+  return cudaLaunchCooperativeKernel((const void *)k_step, dim3(grid), dim3(block), args, 0, s);
 }
-cudaError_t launch_step_split(const StepArgs &a, int grid, cudaStream_t s) {
+cudaError_t launch_step_split(const StepArgs &a, int grid, int block, cudaStream_t s) {
   for (int mode = 2; mode <= 4; ++mode) {
     StepArgs b = a;
     b.mode = mode;
-    k_step<<<grid, kStepBlock, 0, s>>>(b);
-    const cudaError_t e = cudaGetLastError();
+    // the second and third may start while the one before ends (k_step waits)
+    Launch l(grid, block, s, mode > 2);
+    const cudaError_t e = cudaLaunchKernelEx(&l.cfg, k_step, b);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+
+cudaError_t launch_snapshot(const SnapArgs &a, cudaStream_t s) {
+  const unsigned g = (a.n + 255) / 256;
+  k_snapshot<<<g < 1 ? 1 : g < 592 ? g : 592, 256, 0, s>>>(a);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_hpwl(const HpwlArgs &a, int grid, cudaStream_t s) {

@@ -30,6 +30,58 @@ struct IterLog {
   double alpha[2];      // step sizes used by the FISTA step
 };
 
+// The step's block sums of the step norms, and where they go: the log entry
+// of the iteration before sc->iter.
+struct NormArgs {
+  const double *part2;  // [2 * blocks], nullptr: none
+  int blocks;
+  const DevScalars *sc;
+  IterLog *log;
+};
+
+#ifdef __CUDACC__
+// One warp: adds the block sums up in a fixed order and writes the norms.
+__device__ __forceinline__ void finish_norms(const NormArgs &a) {
+  const int it = a.sc->iter - 1;
+  if (it < 0 || a.sc->err) return;
+  double x = 0.0, y = 0.0;
+  for (int b = threadIdx.x & 31; b < a.blocks; b += 32) {
+    const double2 p = __ldcg(reinterpret_cast<const double2 *>(a.part2) + b);
+    x += p.x;
+    y += p.y;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    x += __shfl_xor_sync(0xffffffffu, x, o);
+    y += __shfl_xor_sync(0xffffffffu, y, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    a.log[it].step_norm[0] = sqrt(x);
+    a.log[it].step_norm[1] = sqrt(y);
+  }
+}
+#endif
+
+// A launch that, with `after`, may start before the kernel ahead of it in the
+// stream has ended (that kernel's griddepcontrol.wait keeps the order of the
+// data: every kernel of such a chain executes it in every thread that reads
+// or writes what the one before does).
+struct Launch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  Launch(int grid, int block, cudaStream_t s, bool after, size_t smem = 0) {
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = after ? 1 : 0;
+  }
+  Launch(const Launch &) = delete;
+  Launch &operator=(const Launch &) = delete;
+};
+
 // Degree classes of the WA kernel over the degree-sorted nets: class j holds
 // the nets of degree (kWaDegHi[j-1], kWaDegHi[j]] (class 0 from degree 2;
 // nets of fewer pins have no gradient) and runs kWaGroup[j] lanes per net,
@@ -106,6 +158,7 @@ struct FinalArgs {
   double *overlap;          // where the overlap goes, or nullptr: into sc and the log
   DevScalars *sc;
   IterLog *log;
+  NormArgs norms;           // with part2 set, one more CTA adds the step norms up
 };
 
 // C = A B with leading dimensions lda / ldb / ldc.  a_mir = +1 / -1 reads
@@ -152,13 +205,22 @@ struct StepArgs {
   const double *mom;        // momentum per iteration
   DevScalars *sc;
   IterLog *log;
-  double *part;             // [4 * grid]
-  double *part2;            // [2 * grid] step-norm partials
-  double *part_b;           // [4 * grid] pass-2 partials of the split form
+  double *part;             // [4 * grid] block sums of the first half
+  double *part2;            // [2 * grid] of the step norms
+  double *part_b;           // [4 * grid] of the penalty-initialisation pass
   unsigned *bar;            // grid barrier: words 0-1 are one 64-bit arrival count
   unsigned *ticket;
+  unsigned long long *dens; // density map that takes the next look-ahead, or nullptr
   int mode;                 // 0: full step (cooperative); 1: gather only (tmp_den <- density
-                            // gradient); 2/3/4: phase A / penalty-init pass / phase C
+                            // gradient); 2/3/4: first half / penalty-init pass / second half
+};
+
+struct SnapArgs {
+  uint32_t n;
+  const float2 *x;
+  float2 *pos;         // [n] copy of the positions
+  DevScalars *sc_out;  // copy of the scalars
+  NormArgs norms;
 };
 
 struct HpwlArgs {
@@ -196,11 +258,14 @@ struct FlyOp {
 };
 cudaError_t launch_fly_cols(const FlyOp *ops_dev, int nb, int H, int W, cudaStream_t s);
 cudaError_t launch_fly_rows(const FlyOp *ops_dev, int nb, int H, int W, cudaStream_t s);
-cudaError_t launch_step(const StepArgs &a, int grid, cudaStream_t s);
+// block: step_block; grid: at most step_max_grid for the cooperative form.
+cudaError_t launch_step(const StepArgs &a, int grid, int block, cudaStream_t s);
 // The same step as three ordinary launches (modes 2, 3, 4): no grid barrier,
 // safe beside long-running kernels of other streams.
-cudaError_t launch_step_split(const StepArgs &a, int grid, cudaStream_t s);
-int step_max_grid(int device);
+cudaError_t launch_step_split(const StepArgs &a, int grid, int block, cudaStream_t s);
+int step_block(int device, uint32_t cells);
+int step_max_grid(int device, int block);
+cudaError_t launch_snapshot(const SnapArgs &a, cudaStream_t s);
 cudaError_t launch_hpwl(const HpwlArgs &a, int grid, cudaStream_t s);
 
 // The stage entries' arrays: x and y apart in pinned host memory, which the
