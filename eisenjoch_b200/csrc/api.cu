@@ -2,8 +2,8 @@
 // ElectroPlace loop (electro_place/mod.rs:65-204) and the stage entry points.
 //
 // Loop structure.  Every iteration runs on the device without host round
-// trips: WA gradient -> density scatter -> density finalise -> 4 DCT GEMM
-// launches -> fused gather/penalty/BB/FISTA step.  All loop scalars (penalty,
+// trips: WA gradient beside density finalise -> transform, then the fused
+// gather/penalty/BB/FISTA step, which also scatters the next density.  All loop scalars (penalty,
 // step sizes, iteration counter) live on the device, so one legalisation
 // interval (legalize_interval iterations) is captured once as a CUDA graph
 // and replayed.  After each interval the solver positions are copied to
@@ -1004,8 +1004,8 @@ void launch_final_stage(eplace_ctx *c, double *dens_out, bool tc = false, bool l
 // One of the four GEMM launches of a field solve (density.rs:96-166):
 //   0: T = rho * B1 (row DCT-II)          1: Coef = L2 * T + spectral epilogue
 //   2: U = Ex^ * B3, V = Ey^ * B5          3: Ex = L4 * U, Ey = L6 * V
-// from_dens (FFT form, stage 0): read the fixed-point density map itself,
-// with the finalise (charge, map clear, overlap) fused into the stage.
+// from_dens (FFT form): stage 0 reads the fixed-point density map itself, with
+// the finalise (charge, map clear, overlap) fused into the stages.
 void launch_field_gemm(eplace_ctx *c, int g, float *phi, int field_mode, bool tc, bool from_dens = false) {
   const int W = c->hp.BX, H = c->hp.BY;
   const int fm = field_mode == EPLACE_FIELD_POTENTIAL_GRADIENT ? 1 : 0;
@@ -1061,10 +1061,6 @@ void launch_field_gemm(eplace_ctx *c, int g, float *phi, int field_mode, bool tc
           a.cap = cap_fix(c->hp);
           a.c0 = c->total_area / ((double)W * H);
           a.sums = c->dsum.p;
-          a.ticket = c->bar.p + 2;
-          a.sc = c->sc.p;
-          a.log = c->log.p;
-          a.norms = norm_args(c);
         }
         break;
       case 1:  // forward along y, spectral, then back along y: U, V
@@ -1079,6 +1075,12 @@ void launch_field_gemm(eplace_ctx *c, int g, float *phi, int field_mode, bool tc
         a.gy2 = c->gy2.p;
         a.scale = (float)(4.0 / ((double)W * H));
         a.phi = phi;
+        if (from_dens) {
+          a.sums = c->dsum.p;
+          a.sc = c->sc.p;
+          a.log = c->log.p;
+          a.norms = norm_args(c);
+        }
         break;
       case 2:
         a.in_a = c->U.p;
@@ -1138,7 +1140,7 @@ void launch_field_gemm(eplace_ctx *c, int g, float *phi, int field_mode, bool tc
 }
 
 void launch_field_stage(eplace_ctx *c, float *phi, int field_mode, bool tc = false, bool from_dens = false) {
-  for (int g = 0; g < 4; ++g) launch_field_gemm(c, g, phi, field_mode, tc, from_dens && g == 0);
+  for (int g = 0; g < 4; ++g) launch_field_gemm(c, g, phi, field_mode, tc, from_dens);
 }
 
 // The FFT form takes the density finalise into its first stage.
@@ -2794,7 +2796,7 @@ eplace_status eplace_profile_stages(eplace_ctx *c, const eplace_cfg *cfg, const 
       if (!fuse) launch_final_stage(c, nullptr, tc);
       rec(ev[3]);
       for (int g = 0; g < 4; ++g) {
-        launch_field_gemm(c, g, nullptr, opts.field_mode, tc, fuse && g == 0);
+        launch_field_gemm(c, g, nullptr, opts.field_mode, tc, fuse);
         rec(ev[4 + g]);
       }
       launch_step_stage(c, false);  // the scatter is timed by itself

@@ -6,7 +6,9 @@
 // and stored once per stage, as 16-byte vectors (four positions of a row, or
 // the four columns of a CTA at one row), with the lines staged in shared
 // memory; the working set of a 1024^2 grid (4 MB per array) stays in L2
-// across the three stages.
+// across the three stages.  In a loop each stage is launched while the kernel
+// before it ends, and loads its twiddles before it waits for that kernel's
+// results.
 #include <cmath>
 
 #include "fft.cuh"
@@ -14,7 +16,7 @@
 namespace eplace {
 namespace {
 
-constexpr int kFftThreads = 256;
+constexpr int kFftThreads = 256;  // at most
 constexpr int kColLines = 4;  // columns per CTA of the column stages: one 16-byte vector a row
 constexpr int kBatch = 4;     // vector loads a thread issues before using them
 
@@ -79,29 +81,6 @@ __device__ __forceinline__ void fft_core(float2 *s, int logN, int nf, const floa
   __syncthreads();
 }
 
-// Sum of v over the CTA (whole numbers, in any order); valid in thread 0.
-// red: [2 * warps].
-__device__ __forceinline__ void block_sum2(long long (&v)[2], long long *red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v[0] += __shfl_down_sync(0xffffffffu, v[0], o);
-    v[1] += __shfl_down_sync(0xffffffffu, v[1], o);
-  }
-  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    red[2 * w] = v[0];
-    red[2 * w + 1] = v[1];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    v[0] = v[1] = 0;
-    for (int k = 0; k < nw; ++k) {
-      v[0] += red[2 * k];
-      v[1] += red[2 * k + 1];
-    }
-  }
-}
-
 // Index in the line of X'[k] for a stage-2/3 kind (-1: the value is 0).
 __device__ __forceinline__ int pre_index(int kind, int k, int N) {
   if (kind == FFT_C3) return k;
@@ -119,7 +98,7 @@ __device__ __forceinline__ float post_sign(int kind, int n) {
 // Geometry of a stage: N the transform length, L the lines of the stage,
 // lines and FFTs per CTA.
 struct FftGeom {
-  int N, logN, L, lines, per, ffts;
+  int N, logN, L, lines, per, ffts, threads;
 };
 
 __host__ __device__ inline FftGeom fft_geom(int stage, int W, int H) {
@@ -130,11 +109,18 @@ __host__ __device__ inline FftGeom fft_geom(int stage, int W, int H) {
   g.logN = 0;
   while ((1 << g.logN) < g.N) ++g.logN;
   g.per = stage <= 1 ? 2 : 1;  // lines per FFT
-  // rows: 1024 points (256 radix-4 butterflies a pass) per CTA; columns:
-  // four adjacent columns per CTA, one 16-byte vector per row and array
-  g.lines = rows ? g.per * (g.N >= 1024 ? 1 : 1024 / g.N) : kColLines;
+  // rows: up to 1024 points (256 radix-4 butterflies a pass) per CTA, but no
+  // more than leave about a CTA for each SM, since a stage lasts as long as one
+  // CTA takes for its lines (64^2 and 128^2 bins: 16 to 128 CTAs in place of 2
+  // to 16; iterations of 2k and 5k cells 24.9 -> 23.5 and 23.9 -> 23.1 us);
+  // columns: four adjacent columns per CTA, one 16-byte vector per row and array
+  const int many = (g.L + 128 * g.per - 1) / (128 * g.per);
+  g.lines = rows ? g.per * (g.N >= 1024 ? 1 : (1024 / g.N < many ? 1024 / g.N : many)) : kColLines;
   if (g.lines > g.L) g.lines = g.L;
   g.ffts = g.lines / g.per;
+  // a thread per radix-4 butterfly of a pass
+  g.threads = (stage == 1 ? g.lines : g.ffts) * g.N / 4;
+  g.threads = g.threads < 64 ? 64 : g.threads > kFftThreads ? kFftThreads : g.threads;
   return g;
 }
 
@@ -144,31 +130,42 @@ __host__ __device__ inline int fft_slots(int stage, const FftGeom &g) {
   return (stage == 1 ? g.lines : g.ffts) * g.N;
 }
 
+// Their padded length, even: what follows them (3N/2 twiddles, then vectors of
+// four floats) starts on a 16-byte boundary.
+__host__ __device__ inline int fft_padded(int pts) { return (pts + (pts >> 4) + 1) & ~1; }
+
 // Dynamic shared memory of a stage: the FFTs (padded), the twiddles (N/2 +
 // N), then (stages 1 and 2) two arrays of the CTA's lines.
 __host__ __device__ inline size_t fft_smem(int stage, const FftGeom &g) {
   const int arrays = stage == 0 ? 0 : 2;
-  const size_t pts = (size_t)fft_slots(stage, g);
-  return sizeof(float2) * (pts + pts / 16 + g.N / 2 + g.N) + sizeof(float) * (size_t)arrays * g.lines * g.N;
+  const size_t pts = (size_t)fft_padded(fft_slots(stage, g));
+  return sizeof(float2) * (pts + g.N / 2 + g.N) + sizeof(float) * (size_t)arrays * g.lines * g.N;
 }
 
 template <int STAGE>
 __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
-  extern __shared__ float2 s[];
+  extern __shared__ __align__(16) float2 s[];
   constexpr bool kRows = STAGE != 1;
   constexpr bool kFwd = STAGE <= 1;
   constexpr int kArrays = kFwd ? 1 : 2;
   const FftGeom G = fft_geom(STAGE, a.W, a.H);
-  const int N = G.N, logN = G.logN, nl = G.lines;
+  const int N = G.N, logN = G.logN, nl = G.lines, nt = (int)blockDim.x;
   const FftTables tb = kRows ? a.tx : a.ty;
   const int line0 = blockIdx.x * nl;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (STAGE == 0 && line0 >= G.L) {  // the CTA after the lines'
+  if (STAGE == 1 && line0 >= G.L) {  // the CTA after the lines': what the loop logs
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (threadIdx.x < 32) finish_norms(a.norms);
+    if (threadIdx.x == 32) {
+      const unsigned long long sum = atomicExch(&a.sums[0], 0ull), over = atomicExch(&a.sums[1], 0ull);
+      const double inv = 1.0 / 4294967296.0;
+      const double ovl = sum == 0 ? 0.0 : ((double)(long long)over * inv) / ((double)(long long)sum * inv);
+      a.sc->overlap = ovl;  // compute_overlap
+      a.log[a.sc->iter].overlap = ovl;
+    }
     return;
   }
-  float2 *tw = s + pd(fft_slots(STAGE, G));  // [N/2] e^{-2 pi i j / N}
+  float2 *tw = s + fft_padded(fft_slots(STAGE, G));  // [N/2] e^{-2 pi i j / N}
   float2 *tq = tw + N / 2;              // [N]   (cos, sin)(pi k / 2N)
   float *R = reinterpret_cast<float *>(tq + N);  // stages 1 and 2: R[array][line][pos]
   // 16-byte vectors: rows hold 4 consecutive positions of one line, columns
@@ -189,17 +186,16 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
   // at its bit-reversed slot: lines 2p and 2p + 1 are the real and imaginary
   // parts of FFT p, position n of a line goes to v[m], v[m] = x[2m],
   // v[N-1-m] = x[2m+1].
-  for (int j = threadIdx.x; j < N / 2; j += kFftThreads) tw[j] = __ldg(tb.tw + j);
-  for (int j = threadIdx.x; j < N; j += kFftThreads) tq[j] = __ldg(tb.tq + j);
+  for (int j = threadIdx.x; j < N / 2; j += nt) tw[j] = __ldg(tb.tw + j);
+  for (int j = threadIdx.x; j < N; j += nt) tq[j] = __ldg(tb.tq + j);
   asm volatile("griddepcontrol.wait;" ::: "memory");  // the tables don't change
-  __shared__ long long red[2 * (kFftThreads / 32)];
   long long ov[2] = {0, 0};  // sum d, sum max(d - cap, 0) in fixed point (stage 0 from the map)
   if (STAGE == 0 && a.dens) {
-    for (int v0 = 0; v0 < nvec; v0 += kBatch * kFftThreads) {
+    for (int v0 = 0; v0 < nvec; v0 += kBatch * nt) {
       ulonglong2 q0[kBatch], q1[kBatch];
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) {
-        const int v = v0 + u * kFftThreads + threadIdx.x;
+        const int v = v0 + u * nt + threadIdx.x;
         int l, n;
         const size_t g = vec_at(v < nvec ? v : 0, l, n);
         const ulonglong2 *dp = reinterpret_cast<const ulonglong2 *>(a.dens + g);
@@ -208,7 +204,7 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
       }
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) {
-        const int v = v0 + u * kFftThreads + threadIdx.x;
+        const int v = v0 + u * nt + threadIdx.x;
         if (v >= nvec) break;
         int l, n;
         const size_t g = vec_at(v, l, n);
@@ -227,13 +223,24 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
         }
       }
     }
+    // whole numbers: added up in any order, and nobody waits for them (a last
+    // CTA that summed them held the stage up for 1.8 us)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      ov[0] += __shfl_xor_sync(0xffffffffu, ov[0], o);
+      ov[1] += __shfl_xor_sync(0xffffffffu, ov[1], o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd(&a.sums[0], (unsigned long long)ov[0]);
+      if (ov[1]) atomicAdd(&a.sums[1], (unsigned long long)ov[1]);
+    }
   } else {
     const float *src[2] = {a.in_a, a.in_b};
-    for (int v0 = 0; v0 < nvec; v0 += kBatch * kFftThreads) {
+    for (int v0 = 0; v0 < nvec; v0 += kBatch * nt) {
       float4 q[kArrays][kBatch];
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) {
-        const int v = v0 + u * kFftThreads + threadIdx.x;
+        const int v = v0 + u * nt + threadIdx.x;
         int l, n;
         const size_t g = vec_at(v < nvec ? v : 0, l, n);
 #pragma unroll
@@ -242,7 +249,7 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
       }
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) {
-        const int v = v0 + u * kFftThreads + threadIdx.x;
+        const int v = v0 + u * nt + threadIdx.x;
         if (v >= nvec) break;
         int l, n;
         vec_at(v, l, n);
@@ -280,7 +287,7 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
   // and of array b (R) -> real and imaginary parts of FFT l.
   auto inv_build = [&]() {
     const float *Ra = R, *Rb = R + (size_t)nl * N;
-    for (int e = threadIdx.x; e < nl * N; e += kFftThreads) {
+    for (int e = threadIdx.x; e < nl * N; e += nt) {
       const int l = e >> logN, k = e & (N - 1);
       const float *ra = Ra + (l << logN), *rb = Rb + (l << logN);
       const int ia = pre_index(a.kind_a, k, N), ib = pre_index(a.kind_b, k, N);
@@ -304,7 +311,7 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
   };
   // the inverse outputs, one 16-byte vector per thread and array
   auto inv_out = [&]() {
-    for (int v = threadIdx.x; v < nvec; v += kFftThreads) {
+    for (int v = threadIdx.x; v < nvec; v += nt) {
       int l0, n0;
       const size_t g = vec_at(v, l0, n0);
       float o[2][4];
@@ -332,7 +339,7 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
   // epilogue, writes phi (when asked), keeps Ex^ and Ey^ of its columns in R
   // and transforms them back along y (Ex: C3, Ey: S3 or SG) before writing.
   float *Rx = R, *Ry = R + (size_t)nl * N;
-  for (int v = threadIdx.x; v < nvec; v += kFftThreads) {
+  for (int v = threadIdx.x; v < nvec; v += nt) {
     int l0, n0;
     const size_t g = vec_at(v, l0, n0);
     float o[2][4];
@@ -384,24 +391,6 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
     inv_out();
     return;
   }
-  if (STAGE == 0 && a.dens) {
-    // the overlap: whole-number sums, the last CTA forms the quotient
-    block_sum2(ov, red);
-    if (threadIdx.x == 0) {
-      atomicAdd(&a.sums[0], (unsigned long long)ov[0]);
-      atomicAdd(&a.sums[1], (unsigned long long)ov[1]);
-      __threadfence();
-      if (atomicAdd(a.ticket, 1u) == (unsigned)((G.L + nl - 1) / nl) - 1) {
-        __threadfence();
-        const unsigned long long sum = atomicExch(&a.sums[0], 0ull), over = atomicExch(&a.sums[1], 0ull);
-        const double inv = 1.0 / 4294967296.0;
-        const double ovl = sum == 0 ? 0.0 : ((double)(long long)over * inv) / ((double)(long long)sum * inv);
-        a.sc->overlap = ovl;  // compute_overlap
-        a.log[a.sc->iter].overlap = ovl;
-        *a.ticket = 0u;
-      }
-    }
-  }
 }
 
 }  // namespace
@@ -425,7 +414,7 @@ void fft_tables_host(int N, float2 *tw, float2 *tq) {
 
 cudaError_t launch_fft_stage(int stage, const FftStageArgs &a, cudaStream_t s) {
   const FftGeom g = fft_geom(stage, a.W, a.H);
-  const bool norms = stage == 0 && a.dens && a.norms.part2;
+  const bool norms = stage == 1 && a.sums;
   const int grid = (g.L + g.lines - 1) / g.lines + (norms ? 1 : 0);
   // The shared-memory limit is raised to the stage's largest need (a
   // 1024 x 1024 grid) every time: the same value from every thread, so
@@ -435,7 +424,7 @@ cudaError_t launch_fft_stage(int stage, const FftStageArgs &a, cudaStream_t s) {
   void (*const k)(FftStageArgs) = stage == 0 ? k_fft<0> : stage == 1 ? k_fft<1> : k_fft<2>;
   const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
   if (e != cudaSuccess) return e;
-  Launch l(grid, kFftThreads, s, a.after, fft_smem(stage, g));
+  Launch l(grid, g.threads, s, a.after, fft_smem(stage, g));
   return cudaLaunchKernelEx(&l.cfg, k, a);
 }
 

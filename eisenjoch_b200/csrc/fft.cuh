@@ -57,16 +57,16 @@ struct FftStageArgs {
   // in): with dens set, the stage reads the map instead of in_a, forms
   // rho = d - c0, clears the map for the next iteration, and adds the two
   // sums of the overlap (density.rs:79-86: sum d and sum max(d - cap, 0)) in
-  // fixed point to sums[]; the last CTA to finish writes sc->overlap and the
-  // iteration's log entry.
+  // fixed point to sums[].  Stage 1, with sums set, has one more CTA, which
+  // forms the overlap, writes sc->overlap and the iteration's log entry, and
+  // adds the last step's norms up: neither holds the transform up.
   unsigned long long *dens;
   unsigned long long cap;
   double c0;
-  unsigned long long *sums;  // [2], zero between launches
-  unsigned *ticket;
+  unsigned long long *sums;  // [2], zero between iterations
   DevScalars *sc;
   IterLog *log;
-  NormArgs norms;         // with dens and part2 set, one more CTA adds the step norms up
+  NormArgs norms;
   bool after;             // the launch may start while the kernel before it ends
 };
 

@@ -6,12 +6,12 @@
 //                   to a warp per net), deterministic fixed-point scatter.
 //   k_scatter       cell -> bin overlap areas (electro_place/density.rs:54-76),
 //                   fixed-point atomics (order independent, bit-reproducible).
-//   k_density_final FP64 sum / overflow (density.rs:79-86), FP32 charge map
+//   k_density_final sums for the overlap (density.rs:79-86), FP32 charge map
 //                   for the transform, resets the accumulator.
 //   k_sgemm         FP32 DCT-matrix GEMMs (density.rs:96-166), spectral
 //                   Poisson scaling fused into the second GEMM's epilogue.
 //   k_step          field gather + penalty + preconditioner + Barzilai-
-//                   Borwein + FISTA + clamp + next look-ahead in one
+//                   Borwein + FISTA + clamp + next look-ahead and its scatter in one
 //                   cooperative kernel (density.rs:171-206,
 //                   electro_place/mod.rs:131-173, solver/nesterov.rs:41-101,
 //                   :199-218).
@@ -767,14 +767,22 @@ bool sgemm_small_tile(int M, int N, int nb, int K) {
 //  * a macro (25 bins and more) is gathered by eight lanes, a column of bins
 //    each, four macros a warp, spread over all blocks.  The bins are summed in
 //    the row-major order of one thread, so the bits are the same; one thread
-//    per macro walked its rows one memory latency at a time and held the
+//    per macro walked its rows one memory latency at a time, and held the
 //    barrier up for 8 us at 200k cells (10k macros);
 //  * the block sums are formed with six FP64 shuffles a warp for four sums;
 //  * the next look-ahead is scattered into the density map while it is in
 //    registers (a launch, and a read of the positions, less);
-//  * the step norms, which only the log needs, are left as block sums for the
-//    next iteration's first kernel (finish_norms) instead of a last block.
-// Device time alone / in the loop, before and after: see launch_step.
+//  * the step norms, which only the log needs, are left as block sums for a
+//    kernel of the next iteration (finish_norms) instead of a last block;
+//  * there is one copy of the code of a cell in each half, in a loop over the
+//    thread's cells with the next one's loads under way: two cells side by side
+//    doubled the instructions, and a block runs them once, so that waiting for
+//    their fetch was its longest stall.
+// Inside one launch (5k / 200k / 800k cells), first half done 3 / 9 / 33 us,
+// sums known 5 / 12 / 36, end 8 / 20 / 67 (with the scatter; before, without
+// it: 200k 14, 20, 25).  Whole iterations with the FFT transform, reference
+// field: 5k cells 30.9 -> 21.5 us, 30k 52.7 -> 44.9, 200k 111.6 -> 98.2, 800k
+// 229 -> 213.
 // ---------------------------------------------------------------------------
 
 // The four sums v over the block; lane k < 4 of warp 0 gets sum k in v[0].
@@ -864,27 +872,37 @@ __device__ __forceinline__ bool publish_and_wait(double *part, double t, unsigne
   return !*gave_up;
 }
 
-// Field gather of a 1x1 footprint: it touches at most 2 x 2 bins (bins are
-// >= 1 site wide); weights first, then all field loads at once, summed in the
-// same row-major order as the general form.
-__device__ __forceinline__ float2 gather_unit(const StepArgs &a, float2 p) {
+// The at most 2 x 2 bins of a 1x1 footprint (bins are >= 1 site wide): the
+// lower left one and the lengths along x and y, 0 outside the chip.
+struct UnitFoot {
+  int at;           // bin (bx0, by0); bins bx0 + 1, by0 + 1 only where ox[1], oy[1] > 0
+  float ox[2], oy[2];
+};
+__device__ __forceinline__ UnitFoot unit_foot(const StepArgs &a, float2 p) {
   const Foot f = make_foot(p, 0.5f, 0.5f, a.BX, a.BY, a.isx, a.isy);
+  UnitFoot u;
+  u.at = f.by0 * a.BX + f.bx0;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    u.ox[k] = f.bx0 + k < f.bx1 ? overlap_x(f, f.bx0 + k, a.isx) : 0.0f;
+    u.oy[k] = f.by0 + k < f.by1 ? overlap_y(f, f.by0 + k, a.isy) : 0.0f;
+  }
+  return u;
+}
+
+// Field gather of a 1x1 footprint: all field loads at once, summed in the
+// row-major order of the general form.
+__device__ __forceinline__ float2 gather_unit(const StepArgs &a, float2 p) {
+  const UnitFoot u = unit_foot(a, p);
+  float w[4], e[4], h[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    w[k] = u.ox[k & 1] * u.oy[k >> 1];
+    const int at = u.at + (k >> 1) * a.BX + (k & 1);
+    e[k] = w[k] > 0.0f ? a.Ex[at] : 0.0f;
+    h[k] = w[k] > 0.0f ? a.Ey[at] : 0.0f;
+  }
   float fx = 0.f, fy = 0.f, wt = 0.f;
-  float w[4];
-  size_t id[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int by = f.by0 + (k >> 1), bx = f.bx0 + (k & 1);
-    const bool in = by < f.by1 && bx < f.bx1;
-    w[k] = in ? overlap_x(f, bx, a.isx) * overlap_y(f, by, a.isy) : 0.0f;
-    id[k] = (w[k] > 0.0f) ? (size_t)by * a.BX + bx : 0;
-  }
-  float e[4], h[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    e[k] = (w[k] > 0.0f) ? a.Ex[id[k]] : 0.0f;
-    h[k] = (w[k] > 0.0f) ? a.Ey[id[k]] : 0.0f;
-  }
 #pragma unroll
   for (int k = 0; k < 4; ++k)
     if (w[k] > 0.0f) {
@@ -917,9 +935,10 @@ struct Macro {
 __device__ __forceinline__ float2 gather_macro(const StepArgs &a, const Macro &m, float2 p) {
   constexpr int kRows = 5;
   const Foot f = make_foot(p, m.hf.x, m.hf.y, a.BX, a.BY, a.isx, a.isy);
-  const int parts = (max(f.bx1 - f.bx0, 0) + 7) >> 3;  // eight-bin parts of a row
+  const int nx = max(f.bx1 - f.bx0, 0), parts = (nx + 7) >> 3;  // eight-bin parts of a row
   const int n = m.in ? parts * max(f.by1 - f.by0, 0) : 0;
   const int most = (int)__reduce_max_sync(kFull, (unsigned)n);
+  const int cols = (int)__reduce_max_sync(kFull, (unsigned)min(nx, 8));
   const int lead = threadIdx.x & 24;
   float fx = 0.f, fy = 0.f, wt = 0.f;
   int by = f.by0, part = 0;
@@ -929,9 +948,9 @@ __device__ __forceinline__ float2 gather_macro(const StepArgs &a, const Macro &m
     for (int u = 0; u < kRows; ++u) {
       const int bx = f.bx0 + 8 * part + m.col;
       w[u] = (r0 + u < n && bx < f.bx1) ? overlap_x(f, bx, a.isx) * overlap_y(f, by, a.isy) : 0.0f;
-      const size_t idx = w[u] > 0.0f ? (size_t)by * a.BX + bx : 0;
-      e[u] = w[u] > 0.0f ? a.Ex[idx] : 0.0f;
-      h[u] = w[u] > 0.0f ? a.Ey[idx] : 0.0f;
+      const int at = by * a.BX + bx;
+      e[u] = w[u] > 0.0f ? a.Ex[at] : 0.0f;
+      h[u] = w[u] > 0.0f ? a.Ey[at] : 0.0f;
       if (++part == parts) {
         part = 0;
         ++by;
@@ -939,9 +958,8 @@ __device__ __forceinline__ float2 gather_macro(const StepArgs &a, const Macro &m
     }
 #pragma unroll
     for (int u = 0; u < kRows; ++u) {
-      if (r0 + u >= most) break;  // the same in every lane
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
+#pragma unroll 1
+      for (int k = 0; k < cols; ++k) {
         const float wk = __shfl_sync(kFull, w[u], lead + k);
         const float ek = __shfl_sync(kFull, e[u], lead + k), hk = __shfl_sync(kFull, h[u], lead + k);
         if (wk > 0.0f) {
@@ -1040,11 +1058,11 @@ __device__ __forceinline__ float2 fista_cell(const StepArgs &a, uint32_t i, floa
 
 // The next iteration's density scatter of a unit cell, and of the groups' macros.
 __device__ __forceinline__ void scatter_unit(const StepArgs &a, float2 p) {
-  const Foot f = make_foot(p, 0.5f, 0.5f, a.BX, a.BY, a.isx, a.isy);
+  const UnitFoot u = unit_foot(a, p);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const int by = f.by0 + (k >> 1), bx = f.bx0 + (k & 1);
-    if (by < f.by1 && bx < f.bx1) add_bin(a.dens, f, bx, by, a.BX, a.isx, a.isy);
+    const float ar = u.ox[k & 1] * u.oy[k >> 1];
+    if (ar > 0.0f) atomicAdd(&a.dens[u.at + (k >> 1) * a.BX + (k & 1)], to_fix(ar));
   }
 }
 __device__ __forceinline__ void scatter_macro(const StepArgs &a, const Macro &m, float2 p) {
@@ -1054,13 +1072,29 @@ __device__ __forceinline__ void scatter_macro(const StepArgs &a, const Macro &m,
     for (int bx = f.bx0 + m.col; bx < f.bx1; bx += 8) add_bin(a.dens, f, bx, by, a.BX, a.isx, a.isy);
 }
 
-// The macros of this warp, four at a time: fn(Macro) with all lanes.  Tasks of
-// four go to the blocks in turn, to a block's last warps first.
+// How a block's warps share the cells: the last `macro` warps take macros, the
+// first `unit` warps unit cells.  Four macros make a task; with few enough
+// tasks they get warps of their own (a macro costs a warp about as long as two
+// passes of unit cells, and a warp with both held the block's sum up), else
+// every warp takes both.
+struct Shares {
+  int unit, macro;
+};
+__device__ __forceinline__ Shares shares(const StepArgs &a) {
+  const int nwb = blockDim.x >> 5;
+  const uint32_t per = ((a.n_mac + 3) / 4 + gridDim.x - 1) / gridDim.x;  // tasks of a block, at most
+  if (per == 0 || per > (uint32_t)(3 * nwb / 4)) return Shares{nwb, nwb};
+  return Shares{nwb - (int)per, (int)per};
+}
+
+// The macros of this warp, four at a time: fn(Macro) with all lanes.
 template <typename F>
-__device__ __forceinline__ void each_macro(const StepArgs &a, F fn) {
-  const int nwb = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+__device__ __forceinline__ void each_macro(const StepArgs &a, const Shares &sh, F fn) {
+  const int k0 = (int)(blockDim.x >> 5) - 1 - (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (k0 >= sh.macro) return;
   const uint32_t tasks = (a.n_mac + 3) / 4;
-  for (uint32_t t = blockIdx.x + gridDim.x * (uint32_t)(nwb - 1 - w); t < tasks; t += gridDim.x * (uint32_t)nwb) {
+#pragma unroll 1
+  for (uint32_t t = blockIdx.x + gridDim.x * (uint32_t)k0; t < tasks; t += gridDim.x * (uint32_t)sh.macro) {
     Macro m;
     const uint32_t k = 4 * t + (lane >> 3);
     m.in = k < a.n_mac;
@@ -1080,10 +1114,14 @@ __device__ __forceinline__ void each_macro(const StepArgs &a, F fn) {
 __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
   __shared__ __align__(16) double sm[64], sm2[64], tot[4];
   __shared__ int gave_up;
+
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const uint32_t tid0 = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t gstride = gridDim.x * blockDim.x;
+  // this thread's unit cells: tid0, tid0 + gstride, ...
+  const Shares sh = shares(a);
+  const bool units = (int)(threadIdx.x >> 5) < sh.unit;
+  const uint32_t gstride = gridDim.x * (uint32_t)sh.unit * 32;
+  const uint32_t tid0 = units ? blockIdx.x * (uint32_t)sh.unit * 32 + threadIdx.x : a.N;
   const int it = a.sc->iter;
   const bool was_init = a.sc->lam_init != 0;
   double alpha[2] = {a.sc->step[0], a.sc->step[1]};
@@ -1096,7 +1134,7 @@ __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
   if (a.sc->err) return;
 
   if (a.mode == 1) {  // gather only: no barrier is reached
-    each_macro(a, [&](const Macro &m) {
+    each_macro(a, sh, [&](const Macro &m) {
       const float2 g = gather_macro(a, m, a.look[m.i]);
       if (m.in && m.col == 0) a.tmp_den[m.i] = g;
     });
@@ -1105,51 +1143,45 @@ __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
     return;
   }
   const bool coop = a.mode == 0;
-  // The state that the second half needs of this thread's first two cells,
-  // loaded while the block waits for the others.
-  float2 x0, xp0, g0, x1, xp1, g1;
-  const uint32_t j0 = tid0, j1 = tid0 + gstride;
-  const bool in0 = j0 < a.N && (!a.mflag || !a.mflag[j0]), in1 = j1 < a.N && (!a.mflag || !a.mflag[j1]);
-  auto preload = [&] {
-    if (in0) {
-      x0 = a.x[j0];
-      xp0 = a.xp[j0];
-      g0 = a.g[j0];
-    }
-    if (in1) {
-      x1 = a.x[j1];
-      xp1 = a.xp[j1];
-      g1 = a.g[j1];
-    }
+  // The state that the second half needs of this thread's first cell, loaded
+  // while the block waits for the others.
+  struct State {
+    float2 x, xp, g;
   };
+  auto unit_at = [&](uint32_t i) { return i < a.N && (!a.mflag || !a.mflag[i]); };
+  auto state_of = [&](uint32_t i) {
+    State c{};
+    if (i < a.N) c = State{a.x[i], a.xp[i], a.g[i]};
+    return c;
+  };
+  State s0{};
   double v[4] = {0.0, 0.0, 0.0, 0.0};
   if (coop || a.mode == 2) {
-    each_macro(a, [&](const Macro &m) {
+    each_macro(a, sh, [&](const Macro &m) {
       CellIn c;
       c.look = a.look[m.i];
       if (m.col == 0) c = load_in(a, m.i, was_init);
       const float2 gd = gather_macro(a, m, c.look);
       if (m.in && m.col == 0) first_half(a, m.i, c, gd, m.area, was_init, lam, v);
     });
-    // Two cells per thread and pass, every load of both issued before the
-    // first store, so that their latencies overlap (a macro's are loaded for
-    // nothing: its flag arrives with them).
-    for (uint32_t i0 = tid0; i0 < a.N; i0 += 2 * gstride) {
-      const uint32_t i1 = i0 + gstride;
-      const bool h1 = i1 < a.N;
-      const bool u0 = !a.mflag || !a.mflag[i0];
-      const bool u1 = h1 && (!a.mflag || !a.mflag[i1]);
-      const CellIn c0 = load_in(a, i0, was_init), c1 = load_in(a, h1 ? i1 : i0, was_init);
-      const float2 d0 = gather_unit(a, c0.look), d1 = gather_unit(a, c1.look);
-      if (u0) first_half(a, i0, c0, d0, 1.0f, was_init, lam, v);
-      if (u1) first_half(a, i1, c1, d1, 1.0f, was_init, lam, v);
+    // One cell at a time, the next one's state on the way (a macro's is loaded
+    // for nothing: its flag arrives with it).
+    CellIn c = load_in(a, min(tid0, a.N - 1), was_init);
+#pragma unroll 1
+    for (uint32_t i = tid0; i < a.N; i += gstride) {
+      const bool unit = !a.mflag || !a.mflag[i];
+      CellIn next = c;
+      if (i + gstride < a.N) next = load_in(a, i + gstride, was_init);
+      const float2 gd = gather_unit(a, c.look);
+      if (unit) first_half(a, i, c, gd, 1.0f, was_init, lam, v);
+      c = next;
     }
     const double t = block_sum4(v, sm);
     if (a.mode == 2) {
       if (threadIdx.x < 4) a.part[4 * blockIdx.x + threadIdx.x] = t;
       return;
     }
-    if (was_init) preload();
+    if (was_init) s0 = state_of(tid0);
     if (!publish_and_wait(a.part, t, a.bar, a.sc, &gave_up)) return;
   }
 
@@ -1170,7 +1202,7 @@ __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
         a.g[i] = g;
         bb_terms(v, a.x[i], a.xp[i], g, a.gprev[i]);
       };
-      each_macro(a, [&](const Macro &m) {
+      each_macro(a, sh, [&](const Macro &m) {
         if (m.in && m.col == 0) pass(m.i, m.area);
       });
       for (uint32_t i = tid0; i < a.N; i += gstride)
@@ -1180,13 +1212,13 @@ __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
         if (threadIdx.x < 4) a.part_b[4 * blockIdx.x + threadIdx.x] = t;
         return;
       }
-      preload();
+      s0 = state_of(tid0);
       if (!publish_and_wait(a.part_b, t, a.bar, a.sc, &gave_up)) return;
     }
   } else if (a.mode == 3) {
     return;
   }
-  if (a.mode == 4) preload();
+  if (a.mode == 4) s0 = state_of(tid0);
 
   // Barzilai-Borwein per axis after the first iteration (mod.rs:158-166,
   // nesterov.rs:199-218): |dx.dx / dx.dg| clamped to [1e-4, 1], kept when
@@ -1223,7 +1255,7 @@ __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
   // (:95-101) clamped to the chip (common.rs:410-415), and its density.
   const double m = a.mom[it], mn = a.mom[it + 1];
   double nrm[4] = {0.0, 0.0, 0.0, 0.0};
-  each_macro(a, [&](const Macro &c) {
+  each_macro(a, sh, [&](const Macro &c) {
     float2 p = make_float2(0.f, 0.f);
     if (c.in && c.col == 0) p = fista_cell(a, c.i, a.x[c.i], a.xp[c.i], a.g[c.i], m, mn, alpha, nrm);
     if (a.dens) {
@@ -1232,29 +1264,15 @@ __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
       scatter_macro(a, c, p);
     }
   });
-  float2 l0, l1;
-  if (in0) l0 = fista_cell(a, j0, x0, xp0, g0, m, mn, alpha, nrm);
-  if (in1) l1 = fista_cell(a, j1, x1, xp1, g1, m, mn, alpha, nrm);
-  if (a.dens) {
-    if (in0) scatter_unit(a, l0);
-    if (in1) scatter_unit(a, l1);
-  }
-  for (uint32_t i0 = tid0 + 2 * gstride; i0 < a.N; i0 += 2 * gstride) {  // two cells per pass, loads first
-    const uint32_t i1 = i0 + gstride;
-    const bool h0 = !a.mflag || !a.mflag[i0], h1 = i1 < a.N && (!a.mflag || !a.mflag[i1]);
-    const float2 xa = a.x[i0], xpa = a.xp[i0], ga = a.g[i0];
-    float2 xb = xa, xpb = xpa, gb = ga;
-    if (h1) {
-      xb = a.x[i1];
-      xpb = a.xp[i1];
-      gb = a.g[i1];
+#pragma unroll 1
+  for (uint32_t i = tid0; i < a.N; i += gstride) {
+    const bool unit = unit_at(i);
+    const State next = state_of(i + gstride);
+    if (unit) {
+      const float2 look = fista_cell(a, i, s0.x, s0.xp, s0.g, m, mn, alpha, nrm);
+      if (a.dens) scatter_unit(a, look);
     }
-    if (h0) l0 = fista_cell(a, i0, xa, xpa, ga, m, mn, alpha, nrm);
-    if (h1) l1 = fista_cell(a, i1, xb, xpb, gb, m, mn, alpha, nrm);
-    if (a.dens) {
-      if (h0) scatter_unit(a, l0);
-      if (h1) scatter_unit(a, l1);
-    }
+    s0 = next;
   }
   // The step norms stay block sums; the next iteration's first kernel adds them.
   const double s = block_sum4(nrm, sm);
@@ -1385,9 +1403,10 @@ cudaError_t launch_fly_rows(const FlyOp *ops, int nb, int H, int W, cudaStream_t
   return cudaGetLastError();
 }
 
-// Threads per block of the step: small designs spread over the SMs (a block
-// of 512 threads per SM issues the FP64 code four times slower than one of
-// 128), large ones keep the barrier's arrivals few.
+// Threads per block of the step: small designs spread over the SMs (one block
+// of 512 threads takes four times as long for its instructions as one of 128
+// on an SM of its own: 5k cells, ten blocks of 512 threads 15.9 us a step),
+// large ones keep the barrier's arrivals few.
 int step_block(int device, uint32_t cells) {
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0) sms = 148;
