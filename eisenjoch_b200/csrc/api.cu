@@ -244,7 +244,7 @@ struct LegalOut {
   unsigned long long hpwl;  // HPWL accumulator (k_hpwl)
   double disp;
   int32_t status;           // 0 ok, 1 no free site
-  int32_t pad_;
+  int32_t cancel;           // set by the host while it runs: the result is not wanted
 };
 
 // Device resources of one legalisation in flight: its own copy of the
@@ -257,10 +257,11 @@ struct LegalSlot {
   DBuf<LegalOut> out;
   PinBuf<LegalOut> hout;
   // working state of the parallel legaliser (legal_par.cu)
-  DBuf<int32_t> own, choice;
+  DBuf<int32_t> own, choice, cand;
   DBuf<uint2> seg;
   DBuf<double> mcost;
   DBuf<LpFreed> freed;
+  DBuf<uint32_t> work, queued;
   DBuf<unsigned long long> hint;
   DBuf<LpState> lst;
   LpGraph graph;        // the whole legalisation: rounds in a device-side loop
@@ -1412,7 +1413,10 @@ void prepare_slot(eplace_ctx *c, LegalSlot &L) {
   L.seg.ensure((size_t)SW * hp.H);
   L.choice.ensure(std::max<size_t>(n_mac, 1));
   L.mcost.ensure(std::max<size_t>(n_mac, 1));
-  L.freed.ensure(2 * (size_t)kLpWindow);
+  L.cand.ensure(std::max<size_t>(order.size() - n_mac, 1) * kLpCand);
+  L.freed.ensure(kLpWindow);
+  L.work.ensure(2 * (size_t)kLpWindow);
+  L.queued.ensure(std::max<size_t>(n_mac, 1));
   L.hint.ensure(lp_hint_count(hp.W, hp.H));
   L.lst.ensure(1);
   std::vector<int2> floc(hp.F);
@@ -1437,13 +1441,17 @@ void prepare_slot(eplace_ctx *c, LegalSlot &L) {
   a.choice = L.choice.p;
   a.mcost = L.mcost.p;
   a.freed = L.freed.p;
+  a.work = L.work.p;
+  a.queued = L.queued.p;
   a.hint = L.hint.p;
+  a.cand = L.cand.p;
   a.st = L.lst.p;
   a.sites = L.sites.p;
   a.loc = L.loc.p;
   a.cost = L.cost.p;
   a.disp = &L.out.p->disp;
   a.status = &L.out.p->status;
+  a.cancel = &L.out.p->cancel;
   a.max_rounds = 2 * n_mac + 64;
   CK(lp_build_graph(a, L.graph, L.stream));
   L.gen = c->load_gen;
@@ -1892,6 +1900,8 @@ struct JobState {
     while (outstanding.load(std::memory_order_acquire) != 0) std::this_thread::sleep_for(std::chrono::microseconds(50));
     for (auto &l : c->lslots)
       if (l && l->stream) cudaStreamSynchronize(l->stream);
+    if (discarded) cudaStreamSynchronize(c->copy);  // a cancel mark must not reach the slot's next use
+    discarded = false;
   }
 
   void mark(const char *what) {
@@ -2043,6 +2053,14 @@ struct JobState {
       return final_st;
     }
     return EPLACE_OK;
+  }
+
+  // A checkpoint past the end of the run: its legalisation on the device stops
+  // at the next kernel or block of cells (the run waits for it before it ends).
+  void discard(Checkpoint *cp) {
+    cp->discard = discarded = true;
+    LegalSlot &L = *c->lslots[cp->slot];
+    CK(cudaMemsetAsync(&L.out.p->cancel, 1, sizeof(int32_t), c->copy));
   }
 
   bool slot_available() const { return !free_slots.empty() || (int)c->lslots.size() < kMaxLegalSlots; }
@@ -2331,7 +2349,7 @@ struct JobState {
       progressed = true;
       processed = ci + 1;
       if (stop) {  // ran ahead of convergence: discard
-        if (gpu_legal) cps[ci]->discard = true;
+        if (gpu_legal) discard(cps[ci].get());
         give_snap(hs);
         continue;
       }
@@ -2340,7 +2358,7 @@ struct JobState {
         set_err(c, "a bounded device wait timed out");
         final_st = EPLACE_ERR_TIMEOUT;
         stop = true;
-        if (gpu_legal) cps[ci]->discard = true;
+        if (gpu_legal) discard(cps[ci].get());
         give_snap(hs);
         continue;
       }
@@ -2516,6 +2534,7 @@ struct JobState {
   std::vector<Chunk> chunks;
   int inflight = 1;
   std::vector<int> free_slots;
+  bool discarded = false;  // a legalisation has been cancelled
   uint64_t launched_iters = 0;
   struct Pending {
     size_t chunk;
@@ -2681,7 +2700,7 @@ uint64_t eplace_ctx::device_bytes() const {
   add(B3gt_h); add(B3gt_l); add(L6g_h); add(L6g_l); add(lg_order); add(lg_fsize); add(lg_free0);
   for (const auto &l : lslots) {
     add(l->pos); add(l->sites); add(l->loc); add(l->cost); add(l->out); add(l->own); add(l->seg); add(l->choice);
-    add(l->mcost); add(l->freed); add(l->hint); add(l->lst);
+    add(l->mcost); add(l->freed); add(l->work); add(l->queued); add(l->hint); add(l->cand); add(l->lst);
   }
   return b;
 }

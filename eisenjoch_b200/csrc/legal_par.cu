@@ -11,9 +11,9 @@
 // Unit cells: the greedy is a serial dictatorship, which is the stable
 // matching in which every site prefers the lower order index, and a stable
 // matching with strict preferences is reached by deferred acceptance whatever
-// the order of the proposals.  A warp takes a cell q, finds the open site of
+// the order of the proposals.  A CTA takes a cell q, finds the open site of
 // least (cost, tile) and claims it with atomicMin(own, q).  If the site was
-// held by a later cell, the warp goes on with the cell it displaced; if an
+// held by a later cell, the CTA goes on with the cell it displaced; if an
 // earlier cell got there first, it looks again.  own[s] only ever falls, so
 // a site once closed to q stays closed: no waiting, no rounds, and every
 // lost or won claim lowers some own[s], so it ends.
@@ -38,7 +38,7 @@
 // A 200k-cell checkpoint (5 % macros, half of the cells in six piles): 150 to
 // 200 ms as rounds of candidate lists, disturbance passes and one CTA's serial
 // pass over the cells whose lists interact (a hundred rounds and more of 20
-// launches), 11 ms in this form.
+// launches), 8.4 ms in this form (macros 2.8 ms in 54 rounds, units 4.9).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -51,7 +51,7 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int32_t kNone = 0x7fffffff;  // own[] of a site nobody claims
 constexpr int kInfHi = 0x7ff00000;     // high word of +infinity
-constexpr int kLpWarps = 8;            // warps per CTA of the macro kernels
+constexpr int kLpWarps = 16;           // warps per CTA of the macro kernels (a power of two)
 
 __device__ __forceinline__ double sq(double d) { return __dmul_rn(d, d); }
 
@@ -154,9 +154,19 @@ struct Best {
     return Best{__hiloint2double((int)mh, (int)ml), t};
   }
 };
-// High word of a cost; a larger word means a larger cost.
-__device__ __forceinline__ unsigned hi(double cost) { return (unsigned)__double2hiint(cost); }
 __device__ __forceinline__ Best no_best() { return Best{__hiloint2double(kInfHi, 0), kNone}; }
+
+// FP32 costs, to rule rows, segments and most sites out: coordinates are whole
+// or FP32 numbers (halves, for a block's centre), so such a cost is within
+// 2^-21 of the exact one; kOver and kUnder cover twice that.
+constexpr float kOver = 1.000002f, kUnder = 0.999998f;
+constexpr float kInf = __builtin_huge_valf();
+
+__device__ __forceinline__ float fast_sqrt(float v) {  // within 2^-22
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
 
 // Hints.  When cell k has its place, every anchor cheaper than its own was
 // closed to it, and what is closed to k is closed to every later cell of the
@@ -187,10 +197,12 @@ __device__ __forceinline__ void put_hint(const LpArgs &a, int32_t q, const Cell 
 __device__ __forceinline__ double get_hint(const LpArgs &a, int32_t q, const Cell &c) {
   if (!c.inside) return 0.0;
   float r = 0.0f;
-  for (int size = min(min(c.w, c.h), kLpHintClasses); size >= 1; --size) {
-    const unsigned long long e = __ldcg(hint_at(a, c, size));
-    if ((int32_t)(unsigned)e < q) r = fmaxf(r, __uint_as_float((unsigned)(e >> 32)));
-  }
+  unsigned long long e[kLpHintClasses];  // what was closed to a smaller footprint is closed to this one
+#pragma unroll
+  for (int k = 0; k < kLpHintClasses; ++k) e[k] = k < min(c.w, c.h) ? __ldcg(hint_at(a, c, k + 1)) : 0ull;
+#pragma unroll
+  for (int k = 0; k < kLpHintClasses; ++k)
+    if ((int32_t)(unsigned)e[k] < q) r = fmaxf(r, __uint_as_float((unsigned)(e[k] >> 32)));
   r = (r - hint_dist(c)) * 0.9999f;
   return r > 0.0f ? (double)r * (double)r : 0.0;
 }
@@ -209,20 +221,26 @@ __device__ __forceinline__ unsigned open_word(const LpArgs &a, int32_t q, int y,
 }
 
 // The open anchor of least (cost, tile) for macro q of at most 32 x 16 sites,
-// none of cost below c0 being open: bands of 33 - h anchor rows outward from
-// the target, a lane per site row, in a band the segments outward from the
-// target (from the circle of cost c0), each tested as bit words (a run of w
-// open sites along the row, then h such rows), stopped by the least cost so
-// far, which the CTA's warps share through *least; the warps take the bands in
-// turn.  Latency bound (a word per lane and segment from L2, four segments in
-// flight).
+// none of cost below c0 being open, by the CTA: bands of 33 - h anchor rows
+// outward from the target, a lane per site row, in a band the segments outward
+// from the circle of cost c0, to the right and to the left by different warps,
+// each segment tested as bit words (a run of w open sites along the row, then
+// h such rows), stopped by the least cost so far (*least, shared, FP32).
+// Latency bound (a word per lane and segment from L2, four segments in flight,
+// and own[] of the words that need it).  Returns this lane's best.
 __device__ Best search_block(const LpArgs &a, int32_t q, const Cell &c, double c0, int warp, int lane,
                              unsigned *least) {
   Best b = no_best();
-  unsigned bhi = kInfHi;  // high word of the least cost so far
   const int nb = 33 - c.h;
+  const float tx = (float)c.tx, ty = (float)c.ty, ox = (float)c.ox, oy = (float)c.oy;
+  float most = kInf;
+  auto d2 = [](float at, float off, float t) {
+    const float d = at + off - t;
+    return d * d;
+  };
   // anchors of segment g whose block is open: wc, wn the words of segments g, g + 1
   auto eval = [&](int g, int a0, unsigned wc, unsigned wn) {
+    most = __uint_as_float(*(volatile unsigned *)least);
     if (!__any_sync(kFull, wc != 0)) return;
     uint64_t t = (uint64_t)wc | ((uint64_t)wn << 32);
     for (int s = 1; s < c.w;) {
@@ -237,38 +255,39 @@ __device__ Best search_block(const LpArgs &a, int32_t q, const Cell &c, double c
       s += d;
     }
     if (lane >= nb) v = 0;  // its rows below the band are not here
+    float mine = kInf;
     if (v) {
-      const int ay = a0 + lane, f = c.fx - 32 * g;
       // (split at the target, not at the nearest column: two columns half a
       // site away on either side are a tie for the lower one)
-      const double dy2 = row_dy2(c, ay);
+      const int ay = a0 + lane, f = c.fx - 32 * g;
+      const float dy2 = d2((float)ay, oy, ty);
       const unsigned left = f < 0 ? 0u : (f >= 31 ? ~0u : (2u << f) - 1u);
       const unsigned vl = v & left, vr = v & ~left;
-      if (vl) {
-        const int ax = 32 * g + 31 - __clz(vl);
-        b.take(__dadd_rn(col_dx2(c, ax), dy2), ay * a.W + ax);
-      }
-      if (vr) {
-        const int ax = 32 * g + __ffs(vr) - 1;
-        b.take(__dadd_rn(col_dx2(c, ax), dy2), ay * a.W + ax);
-      }
+      const int xl = 32 * g + 31 - __clz(vl), xr = 32 * g + __ffs(vr) - 1;
+      const float cl = vl ? d2((float)xl, ox, tx) + dy2 : kInf, cr = vr ? d2((float)xr, ox, tx) + dy2 : kInf;
+      mine = fminf(cl, cr);
+      const float bound = fminf(most, mine * kOver) * kOver;
+      if (vl && cl <= bound) b.take(__dadd_rn(col_dx2(c, xl), row_dy2(c, ay)), ay * a.W + xl);
+      if (vr && cr <= bound) b.take(__dadd_rn(col_dx2(c, xr), row_dy2(c, ay)), ay * a.W + xr);
     }
-    bhi = __reduce_min_sync(kFull, (unsigned)__double2hiint(b.cost));
-    if (lane == 0) bhi = min(atomicMin(least, bhi), bhi);
-    bhi = __shfl_sync(kFull, bhi, 0);
+    const unsigned all = __reduce_min_sync(kFull, __float_as_uint(mine * kOver));
+    if (lane == 0 && all < __float_as_uint(most)) atomicMin(least, all);
+    most = fminf(most, __uint_as_float(all));
   };
   const int base0 = c.cy - nb / 2;
   for (int k = 0;; ++k) {
     bool any = false;
+    most = __uint_as_float(*(volatile unsigned *)least);
     for (int side = 0; side < (k ? 2 : 1); ++side) {
       const int a0 = base0 + (side ? -k * nb : k * nb);
       const int r0 = max(a0, 0), r1 = min(a0 + nb, c.AH) - 1;
       if (r0 > r1) continue;
-      const double dmin = row_dy2(c, min(max(c.cy, r0), r1));
-      if (hi(dmin) > bhi) continue;
+      const float dmin = d2((float)min(max(c.cy, r0), r1), oy, ty);
+      if (dmin > most) continue;
       any = true;
-      if ((2 * k + side) % kLpWarps != warp) continue;  // another warp's band
-      bhi = min(bhi, *(volatile unsigned *)least);
+      const int part = (2 * (2 * k + side) - warp) & (kLpWarps - 1);  // 0: right, 1: left is this warp's
+      const bool right = part == 0, left = ((part + 1) & (kLpWarps - 1)) == 0;
+      if (!right && !left) continue;
       const int y = a0 + lane;
       const bool row = y >= 0 && y < a.H;
       auto raw = [&](int g) {
@@ -279,51 +298,53 @@ __device__ Best search_block(const LpArgs &a, int32_t q, const Cell &c, double c
       const int skip = c0 > far ? max((int)sqrtf((float)__dsub_rn(c0, far)) - 2, 0) : 0;
       const int gr = min(max(c.fx + skip, 0), c.AW - 1) >> 5, gl = max(c.fx - skip, 0) >> 5;
       uint2 p[5];
+      if (right) {
 #pragma unroll
-      for (int u = 0; u < 5; ++u) p[u] = raw(gr + u);
-      unsigned cur = open_word(a, q, y, gr, p[0]);
-      const unsigned w0 = cur;
-      for (int g = gr;; g += 4) {
-        bool done = false;
+        for (int u = 0; u < 5; ++u) p[u] = raw(gr + u);
+        unsigned cur = open_word(a, q, y, gr, p[0]);
+        for (int g = gr;; g += 4) {
+          bool done = false;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int at = g + u;
-          if (!done && (32 * at >= c.AW ||
-                        (at > gr && hi(__dadd_rn(col_dx2(c, 32 * at), dmin)) > bhi)))
-            done = true;
-          if (!done) {
-            const unsigned nxt = open_word(a, q, y, at + 1, p[u + 1]);
-            eval(at, a0, cur, nxt);
-            cur = nxt;
+          for (int u = 0; u < 4; ++u) {
+            const int at = g + u;
+            done = done || 32 * at >= c.AW || (at > gr && d2((float)(32 * at), ox, tx) + dmin > most);
+            if (!done) {
+              const unsigned nxt = open_word(a, q, y, at + 1, p[u + 1]);
+              eval(at, a0, cur, nxt);
+              cur = nxt;
+            }
           }
+          if (done) break;
+#pragma unroll
+          for (int u = 1; u < 5; ++u) p[u] = raw(g + 4 + u);
         }
-        if (done) break;
+      } else {
+        const int g0 = gl == gr ? gl - 1 : gl;  // the other warp has the segment they share
+        if (g0 < 0) continue;
+        p[4] = raw(g0 + 1);
+        unsigned nxt = 0, cur;
+        for (int g = g0; g >= 0; g -= 4) {
 #pragma unroll
-        for (int u = 1; u < 5; ++u) p[u] = raw(g + 4 + u);
-      }
-      unsigned nxt = gl == gr ? w0 : open_word(a, q, y, gl + 1, raw(gl + 1));
-      for (int g = gl == gr ? gl - 1 : gl; g >= 0; g -= 4) {
+          for (int u = 0; u < 4; ++u) p[u] = raw(g - u);
+          if (g == g0) nxt = open_word(a, q, y, g0 + 1, p[4]);
+          bool done = false;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) p[u] = raw(g - u);
-        bool done = false;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int at = g - u;
-          if (!done && (at < 0 || (at < (c.cx >> 5) &&
-                                   hi(__dadd_rn(col_dx2(c, 32 * at + 31), dmin)) > bhi)))
-            done = true;
-          if (!done) {
-            cur = open_word(a, q, y, at, p[u]);
-            eval(at, a0, cur, nxt);
-            nxt = cur;
+          for (int u = 0; u < 4; ++u) {
+            const int at = g - u;
+            done = done || at < 0 || (at < (c.cx >> 5) && d2((float)(32 * at + 31), ox, tx) + dmin > most);
+            if (!done) {
+              cur = open_word(a, q, y, at, p[u]);
+              eval(at, a0, cur, nxt);
+              nxt = cur;
+            }
           }
+          if (done) break;
         }
-        if (done) break;
       }
     }
     if (!any) break;  // outside the chip or too far on both sides, and the next bands too
   }
-  return b;  // this lane's
+  return b;
 }
 
 // The same for any footprint (wider or higher ones): a lane per anchor.
@@ -367,90 +388,91 @@ __global__ void __launch_bounds__(256) k_lp_init(const LpArgs a) {
     const unsigned m = __ballot_sync(kFull, open);
     if (lane == 0) a.seg[i] = make_uint2(m, 0u);
   }
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < a.n_mac; q += gridDim.x * blockDim.x) a.choice[q] = -1;
+  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < a.n_mac; q += gridDim.x * blockDim.x) {
+    a.choice[q] = -1;
+    const bool in = q < kLpWindow;  // the first round's
+    a.queued[q] = in ? 1u : 0u;
+    if (in) a.work[q] = q;
+  }
   const uint32_t hints = kLpHintClasses * (uint32_t)((a.W + 15) / 16) * (uint32_t)((a.H + 15) / 16);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < hints; i += gridDim.x * blockDim.x) a.hint[i] = 0ull;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *a.st = LpState{0u, 0u, (uint32_t)kNone, 0u, {0u, 0u}, 0, 0u};
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n - a.n_mac; i += gridDim.x * blockDim.x)
+    a.cand[(size_t)kLpCand * i] = -1;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.st = LpState{0u, 0u, (uint32_t)kNone, 0u, 0u, {min(a.n_mac, kLpWindow), 0u}, 0};
 }
 
-// A round, first half: each macro of the window whose choice may have become
-// wrong chooses again; the blocks given up are entered in this round's list
-// and leave own[].  (A macro that reads own[] while another leaves it sees
-// some sites of the old block open and some not; the block is in the list, so
-// it is looked at again in the next round if that could matter to it.)
-// A CTA per macro: a round lasts as long as its longest search, and only some
-// of the window's macros search at all.
+// A round, first half: each macro of the work list (whose choice may have
+// become wrong) chooses again; the blocks given up are entered in the round's
+// list and leave own[].  (A macro that reads own[] while another leaves it
+// sees some sites of the old block open and some not; the block is in the
+// list, so it is looked at again in the next round if that could matter to it.)
+// A CTA per macro: a round lasts as long as its longest search.
 __global__ void __launch_bounds__(kLpWarps * 32) k_lp_choose(const LpArgs a) {
   __shared__ Best sbest[kLpWarps];
   __shared__ unsigned least;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   LpState *st = a.st;
-  const uint32_t base = st->base, par = st->rounds & 1u;
-  const uint32_t qi = base + blockIdx.x;
-  if (qi >= a.n_mac) return;
-  const int32_t q = (int32_t)qi;
-  const Cell c = load_cell(a, qi, false);
-  const int32_t old = a.choice[q];
-  const int oldx = old % a.W, oldy = old / a.W;
-  double c0 = 0.0;  // no anchor of a lower cost is open
-  if (tid == 0) least = kInfHi;
-  if (old != -1) {
-    bool lost = false, freed = false;
-    if (old >= 0)
-      for (int s = tid; s < c.w * c.h; s += kLpWarps * 32)
-        lost |= ld_own(own_at(a, oldx + s % c.w, oldy + s / c.w)) < q;
-    const double mine = old >= 0 ? a.mcost[q] : __hiloint2double(kInfHi, 0);
-    const uint32_t nf = st->nfreed[par];
-    for (uint32_t e = tid; e < nf; e += kLpWarps * 32) {
-      const LpFreed f = a.freed[par * kLpWindow + e];
-      if (f.q >= q) continue;
-      // the least cost of an anchor whose block meets the freed one
-      const int fx = f.tile % a.W, fy = f.tile / a.W;
-      const int x0 = max(fx - c.w + 1, 0), x1 = min(fx + f.w - 1, c.AW - 1);
-      const int y0 = max(fy - c.h + 1, 0), y1 = min(fy + f.h - 1, c.AH - 1);
-      if (x0 > x1 || y0 > y1) continue;
-      freed |= __dadd_rn(col_dx2(c, min(max(c.cx, x0), x1)), row_dy2(c, min(max(c.cy, y0), y1))) <= mine;
+  const uint32_t par = st->rounds & 1u, nwork = st->nwork[par];
+  for (uint32_t item = blockIdx.x; item < nwork; item += gridDim.x) {
+    const uint32_t qi = a.work[par * kLpWindow + item];
+    const int32_t q = (int32_t)qi;
+    const Cell c = load_cell(a, qi, false);
+    const int32_t old = a.choice[q];
+    // nothing of a lower cost than its own is open when only its own block was lost
+    double c0 = old >= 0 && !(a.queued[q] & 2) && c.inside ? a.mcost[q] : 0.0;
+    c0 = fmax(c0, get_hint(a, q, c));
+    if (tid == 0) least = __float_as_uint(kInf);
+    __syncthreads();
+    Best b = no_best();
+    if (placeable(c)) {
+      if (c.w <= 32 && c.h <= 16) b = search_block(a, q, c, c0, warp, lane, &least);
+      else if (warp == 0) b = search_any(a, q, c, lane);
     }
-    lost = __syncthreads_or(lost);
-    freed = __syncthreads_or(freed);
-    if (!lost && !freed) return;
-    if (!freed && old >= 0 && c.inside) c0 = mine;
-  }
-  c0 = fmax(c0, get_hint(a, q, c));
-  __syncthreads();  // least
-  Best b = no_best();
-  if (placeable(c)) {
-    if (c.w <= 32 && c.h <= 16) b = search_block(a, q, c, c0, warp, lane, &least);
-    else if (warp == 0) b = search_any(a, q, c, lane);
-  }
-  b = b.warp_min();
-  if (lane == 0) sbest[warp] = b;
-  __syncthreads();
-  if (warp != 0) return;
-  b = (lane < kLpWarps ? sbest[lane] : no_best()).warp_min();
-  const int32_t now = b.tile == kNone ? -2 : b.tile;
-  if (now == old) return;
-  if (old >= 0) {
-    for (int s = lane; s < c.w * c.h; s += 32) {
-      const int x = oldx + s % c.w, y = oldy + s / c.w;
-      int32_t *o = own_at(a, x, y);
-      if (ld_own(o) == q) {  // nobody else writes a site that q holds
-        *o = kNone;
-        atomicAnd(&seg_at(a, x, y)->y, ~(1u << (x & 31)));
+    b = b.warp_min();
+    if (lane == 0) sbest[warp] = b;
+    __syncthreads();
+    if (warp == 0) {
+      b = (lane < kLpWarps ? sbest[lane] : no_best()).warp_min();
+      const int32_t now = b.tile == kNone ? -2 : b.tile;
+      if (lane == 0) a.queued[q] = 0;
+      if (now != old) {
+        if (old >= 0) {
+          const int oldx = old % a.W, oldy = old / a.W;
+          for (int s = lane; s < c.w * c.h; s += 32) {
+            const int x = oldx + s % c.w, y = oldy + s / c.w;
+            int32_t *o = own_at(a, x, y);
+            if (ld_own(o) == q) {  // nobody else writes a site that q holds
+              *o = kNone;
+              atomicAnd(&seg_at(a, x, y)->y, ~(1u << (x & 31)));
+            }
+          }
+        }
+        if (lane == 0) {
+          atomicMin(&st->first, qi);
+          if (old >= 0) a.freed[atomicAdd(&st->nfreed, 1u)] = LpFreed{q, old, c.w, c.h};
+          a.choice[q] = now;
+          a.mcost[q] = b.cost;
+        }
       }
     }
-  }
-  if (lane == 0) {
-    atomicMin(&st->first, qi);
-    if (old >= 0) a.freed[(par ^ 1u) * kLpWindow + atomicAdd(&st->nfreed[par ^ 1u], 1u)] = LpFreed{q, old, c.w, c.h};
-    a.choice[q] = now;
-    a.mcost[q] = b.cost;
+    __syncthreads();  // sbest and least are free again
   }
 }
 
-// Second half: every macro of the window enters its claim again (a macro that
-// left may have covered a later one's), and the last CTA moves the window to
-// the first macro that changed.
+// Enters macro q in the next round's work list, once; why: 1: its block was
+// lost, 2: something was given up that may be better.
+__device__ __forceinline__ void queue_macro(const LpArgs &a, uint32_t q, unsigned why) {
+  if (atomicOr(&a.queued[q], why) != 0u) return;
+  const uint32_t par = (a.st->rounds + 1) & 1u;
+  a.work[par * kLpWindow + atomicAdd(&a.st->nwork[par], 1u)] = q;
+}
+
+// Second half, a warp per macro of the window: every macro enters its claim
+// again (a macro that left may have covered a later one's); who finds an
+// earlier claim on its block, or loses a site to one here, and who could gain
+// from a block given up in this round, chooses again in the next.  The last
+// CTA moves the window to the first macro that changed; those that enter it
+// choose for the first time.
 __global__ void __launch_bounds__(kLpWarps * 32) k_lp_claim(const LpArgs a) {
   __shared__ bool last;
   const int lane = threadIdx.x & 31;
@@ -460,21 +482,42 @@ __global__ void __launch_bounds__(kLpWarps * 32) k_lp_claim(const LpArgs a) {
   const uint32_t q = base + blockIdx.x * kLpWarps + (threadIdx.x >> 5);
   if (q < end) {
     const int32_t t = a.choice[q];
+    const Cell c = load_cell(a, q, false);
     if (t >= 0) {
-      const uchar2 s = a.fsize[a.order[q]];
       const int ax = t % a.W, ay = t / a.W;
-      for (int k = lane; k < s.x * s.y; k += 32) {
-        const int x = ax + k % s.x, y = ay + k / s.x;
+      bool lost = false;
+      for (int k = lane; k < c.w * c.h; k += 32) {
+        const int x = ax + k % c.w, y = ay + k / c.w;
         int32_t *o = own_at(a, x, y);
-        if (ld_own(o) > (int32_t)q) {
-          atomicMin(o, (int32_t)q);
+        int32_t was = ld_own(o);
+        if (was > (int32_t)q) {
+          was = atomicMin(o, (int32_t)q);
           atomicOr(&seg_at(a, x, y)->y, 1u << (x & 31));
+          if (was > (int32_t)q && was < (int32_t)end) queue_macro(a, (uint32_t)was, 1u);
         }
+        lost |= was < (int32_t)q;
         if (q < stop) atomicAnd(&seg_at(a, x, y)->x, ~(1u << (x & 31)));  // final
       }
-      if (q < stop && lane == 0) put_hint(a, (int32_t)q, load_cell(a, q, false), a.mcost[q]);
+      if (__any_sync(kFull, lost) && lane == 0) queue_macro(a, q, 1u);
+      if (q < stop && lane == 0) put_hint(a, (int32_t)q, c, a.mcost[q]);
     } else if (q < stop && lane == 0) {
       atomicMax(&st->status, 1);  // final, and no anchor was open
+    }
+    if (q >= stop) {
+      const double mine = t >= 0 ? a.mcost[q] : __hiloint2double(kInfHi, 0);
+      bool gain = false;
+      const uint32_t nf = __ldcg(&st->nfreed);
+      for (uint32_t e = lane; e < nf; e += 32) {
+        const LpFreed f = a.freed[e];
+        if (f.q >= (int32_t)q) continue;
+        // the least cost of an anchor whose block meets the freed one
+        const int fx = f.tile % a.W, fy = f.tile / a.W;
+        const int x0 = max(fx - c.w + 1, 0), x1 = min(fx + f.w - 1, c.AW - 1);
+        const int y0 = max(fy - c.h + 1, 0), y1 = min(fy + f.h - 1, c.AH - 1);
+        if (x0 > x1 || y0 > y1) continue;
+        gain |= __dadd_rn(col_dx2(c, min(max(c.cx, x0), x1)), row_dy2(c, min(max(c.cy, y0), y1))) <= mine;
+      }
+      if (__any_sync(kFull, gain) && lane == 0) queue_macro(a, q, 2u);
     }
   }
   __syncthreads();
@@ -483,14 +526,19 @@ __global__ void __launch_bounds__(kLpWarps * 32) k_lp_claim(const LpArgs a) {
     last = atomicAdd(&st->ticket, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (!last || threadIdx.x != 0) return;
+  if (!last) return;
   __threadfence();
+  for (uint32_t i = end + threadIdx.x; i < min(stop + kLpWindow, a.n_mac); i += blockDim.x) queue_macro(a, i, 1u);
+  __syncthreads();
+  if (threadIdx.x != 0) return;
   st->base = stop;
   st->first = (uint32_t)kNone;
-  st->nfreed[st->rounds & 1u] = 0;
+  st->nfreed = 0;
+  st->nwork[st->rounds & 1u] = 0;
   st->rounds += 1;
   st->ticket = 0;
   if (stop < a.n_mac && st->rounds >= a.max_rounds) atomicMax(&st->status, 2);
+  if (ld_own(a.cancel)) atomicMax(&st->status, 4);
   if (stop >= a.n_mac || atomicAdd(&st->status, 0) != 0) cudaGraphSetConditional(a.handle, 0u);
 }
 
@@ -532,20 +580,9 @@ __device__ Best search_near(const LpArgs &a, int32_t q, const Cell &c, int lane)
 // (their bits alone); the least of these bounds the cost for the whole CTA
 // (*least).  Then it looks for a site held by a later cell that is cheaper
 // still, in the segments where there can be one, within the bound.  Bounds
-// are FP32 costs: coordinates are whole or FP32 numbers, so such a cost is
-// within 2^-21 of the exact one, and kOver covers twice that; the few sites
-// within the bound are costed in FP64.  Bound by the latency of a pass (a few
+// are FP32 costs; the few sites within them are costed in FP64.  Bound by the latency of a pass (a few
 // hundred instructions, two or three loads from L2).  Returns this lane's best.
 constexpr int kUnitWarps = 16;
-constexpr float kOver = 1.000002f, kUnder = 0.999998f;
-constexpr float kInf = __builtin_huge_valf();
-
-__device__ __forceinline__ float fast_sqrt(float v) {  // within 2^-22
-  float r;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-  return r;
-}
-
 __device__ Best search_rows(const LpArgs &a, int32_t q, const Cell &c, double c0, int warp, int lane,
                             unsigned *least) {
   Best b = no_best();
@@ -652,75 +689,178 @@ __device__ Best search_rows(const LpArgs &a, int32_t q, const Cell &c, double c0
   return b;
 }
 
-// Claims site b.tile for q (one thread): kNone: it was free; a later cell: q
+// The open sites of cost `best` (the least) to best + ring_of, by the whole CTA,
+// unsorted: the next answers of this cell, should it be displaced.  Sites
+// cheaper than `best` are closed, so only the few columns of each row between
+// the two circles are looked at.  *count may exceed kLpRingMax: too many to
+// keep.
+constexpr int kLpRingMax = 64;
+// Wide enough for some ten to thirty sites: a cell at the rim of a pile of
+// radius r has open sites on one side only, in a ring of 1 to 2 sites' width.
+__device__ __forceinline__ float ring_of(double best) { return 60.0f + 2.4f * fast_sqrt((float)best); }
+
+__device__ void list_ring(const LpArgs &a, int32_t q, const Cell &c, double best, int warp, int lane, Best *list,
+                          int *count) {
+  const bool right = lane & 1;
+  const int dir = right ? 1 : -1;
+  const float tx = (float)c.tx, ty = (float)c.ty, low = (float)best * kUnder;
+  const float ring = ring_of(best), most = (float)best * kOver + ring;
+  const int rows = max(c.cy, a.H - 1 - c.cy);
+  for (int p0 = 0; p0 <= rows; p0 += 8 * kUnitWarps) {
+    if (p0 && ((float)p0 - 0.5f) * ((float)p0 - 0.5f) > most) break;
+    const int k = (lane >> 1) + 2 * (p0 + 8 * warp);
+    const int y = c.cy + ((k & 1) ? -(k + 1) / 2 : k / 2);
+    const float dy = (float)y - ty, dy2 = dy * dy, left = most - dy2;
+    if (y < 0 || y >= a.H || left < 0.0f) continue;
+    int x = right ? c.fx + 1 : c.fx;
+    if (low > dy2) {
+      const float d = fast_sqrt(low - dy2) - 0.01f;
+      x = right ? max(x, (int)ceilf(tx + d)) : min(x, (int)floorf(tx - d));
+    }
+    const float reach = fast_sqrt(left) + 0.01f;
+    const int last = right ? (int)fminf(floorf(tx + reach), (float)(a.W - 1)) : (int)fmaxf(ceilf(tx - reach), 0.0f);
+    if (right ? x > last || x >= a.W : x < last || x < 0) continue;
+    for (int g = x >> 5; right ? g <= last >> 5 : g >= last >> 5; g += dir) {
+      const int lo = max((right ? x : last) - 32 * g, 0), hi = min((right ? last : x) - 32 * g, 31);
+      const unsigned ask = (~0u << lo) & (~0u >> (31 - hi));
+      const uint2 s = ld_seg(a.seg + (size_t)y * a.SW + g);
+      unsigned m = ((int32_t)s.y > q ? open_sites(own_at(a, 32 * g, y), ask, q) : s.x) & ask;
+      while (m) {
+        const int at = 32 * g + __ffs(m) - 1;
+        m &= m - 1;
+        const double cost = __dadd_rn(col_dx2(c, at), row_dy2(c, y));
+        if (cost > best + (double)ring) continue;
+        const int n = atomicAdd(count, 1);
+        if (n < kLpRingMax) list[n] = Best{cost, y * a.W + at};
+      }
+    }
+  }
+}
+
+// Sorts the (at most 32) entries, one per lane; lane l then has the l-th.
+__device__ __forceinline__ Best warp_sorted(Best b) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      Best o;
+      o.cost = __shfl_xor_sync(kFull, b.cost, j);
+      o.tile = __shfl_xor_sync(kFull, b.tile, j);
+      const bool less = o.cost < b.cost || (o.cost == b.cost && o.tile < b.tile);
+      const bool low = ((lane & j) == 0) == ((lane & k) == 0);  // this lane keeps the smaller one
+      if (less == low) b = o;
+    }
+  return b;
+}
+
+// Claims site (x, y) for q (one thread): kNone: it was free; a later cell: q
 // has it now, and that cell has lost it; an earlier cell: q did not get it.
-__device__ __forceinline__ int32_t claim_site(const LpArgs &a, int32_t q, const Cell &c, const Best &b) {
-  const int x = b.tile % a.W, y = b.tile / a.W;
+__device__ __forceinline__ int32_t claim_site(const LpArgs &a, int32_t q, int x, int y) {
   uint2 *s = seg_at(a, x, y);
   const int32_t top = atomicMax(reinterpret_cast<int32_t *>(&s->y), q);
   const int32_t held = atomicMin(own_at(a, x, y), q);
   // the bit goes after both answers are here; one that lost the site clears
   // it too, so that it does not meet a late bit again
   if ((held == kNone || held < q) && top != kNone) atomicAnd(&s->x, ~(1u << (x & 31)));
-  put_hint(a, q, c, b.cost);
   return held;
 }
 
 // A CTA per unit cell, and the cells that its claim displaces one after the
 // other.  What takes the time is the chain of cells that each take a site from
 // the next (about a thousand cells at the rim of a 200k-cell pile), so one
-// search is made short: an answer near the target is found by one warp with
-// no barrier, any other by all 16.  CTAs start in about the order of the
-// cells, so a claim is displaced only by a cell that was under way at the
-// same time; several cells per CTA, or a warp for each, put more cells under
-// way and displace more claims.  Units of a 200k-cell checkpoint whose cells
-// lie in one pile: 7.5 ms and 283k searches of the whole CTA; 2 / 4 / 8 cells
-// per CTA 13.4 / 20 / 30 ms, a warp per cell 27 to 70 ms.
+// answer is made short: one warp, with no barrier, finds an answer near the
+// target, and that of a displaced cell in the list its search left (closed
+// sites stay closed, so the first one still open is the best); any other
+// search takes all 16 warps, and lists the sites next in cost for a later
+// displacement.  CTAs start in about the order of the cells, so a claim is
+// displaced only by a cell that was under way at the same time; several cells
+// per CTA, or a warp for each, put more cells under way and displace more
+// claims.  Units of a 200k-cell checkpoint whose cells lie in one pile:
+// 4.9 ms and 117k searches of the whole CTA; without the lists 7.5 ms and 283k;
+// without them and with 2 / 4 / 8 cells per CTA 13.4 / 20 / 30 ms, with a warp
+// per cell 27 to 70 ms.
 __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(const LpArgs a) {
-  __shared__ Best sbest[kUnitWarps];
+  __shared__ Best sbest[kUnitWarps], slist[kLpRingMax];
   __shared__ unsigned least;
+  __shared__ int scount;
   // the cell under way: index (-1: done), target, cost below which no site is open
   __shared__ int32_t sq_;
   __shared__ float2 spos;
   __shared__ double sc0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uchar2 one = make_uchar2(1, 1);
-  bool fresh = true;
+  int32_t next = (int32_t)(a.n_mac + blockIdx.x);  // warp 0: the cell to place
+  bool listed = false;                             // it may have a list
+  int px = 0, py = 0;                              // a displaced cell: the site it lost
+  if (warp == 0) {  // nothing to do for a legalisation that failed or is not wanted
+    const bool off = ld_own(a.cancel) != 0;
+    if (off && lane == 0) atomicMax(&a.st->status, 4);
+    if (off || ld_own(&a.st->status) != 0) next = -1;
+  }
   while (true) {
-    if (warp == 0) {  // while the answer is near the target
-      int32_t q = fresh ? (int32_t)(a.n_mac + blockIdx.x) : sq_;
-      if (q >= 0) {
-        float2 p = fresh ? a.pos[a.order[q]] : spos;
-        Cell c = make_cell(a, p, one);
-        double c0 = fresh ? get_hint(a, q, c) : sc0;
-        while (c0 < 6.25 && placeable(c)) {
-          const Best b = search_near(a, q, c, lane);
-          if (!(b.cost < 6.25)) break;
-          int32_t held = 0;
-          if (lane == 0) held = claim_site(a, q, c, b);
-          held = __shfl_sync(kFull, held, 0);
-          if (held == kNone) {
-            q = -1;
-            break;
+    if (warp == 0) {  // while one warp can tell
+      int32_t q = next;
+      while (q >= 0) {
+        int32_t held = 0;
+        double c0 = 0.0;
+        float2 p;
+        if (listed) {
+          const int32_t *l = a.cand + (size_t)kLpCand * (q - (int32_t)a.n_mac);
+          const int32_t t = lane < kLpCand ? ld_own(l + lane) : -1;
+          const unsigned ends = __ballot_sync(kFull, t < 0);  // the list ends at its first -1
+          const int len = __ffs(ends) - 1;
+          const int x = t % a.W, y = t / a.W;
+          const unsigned open = __ballot_sync(kFull, lane < len && ld_own(own_at(a, x, y)) > q);
+          if (open) {
+            const int l0 = __ffs(open) - 1;
+            px = __shfl_sync(kFull, x, l0);
+            py = __shfl_sync(kFull, y, l0);
+            if (lane == 0) held = claim_site(a, q, px, py);
+            held = __shfl_sync(kFull, held, 0);
+            if (held == kNone) q = -1;
+            else if (held > q) q = held;
+            continue;  // (an earlier cell was faster: the list again)
           }
-          if (held > q) {  // go on with the cell that lost it
-            q = held;
-            p = a.pos[a.order[q]];
-            c = make_cell(a, p, one);
-            c0 = c.inside ? __dadd_rn(col_dx2(c, b.tile % a.W), row_dy2(c, b.tile / a.W)) : 0.0;
+          p = a.pos[a.order[q]];
+          const Cell c = make_cell(a, p, one);
+          if (len > 0) {  // all of it closed, as everything cheaper
+            px = __shfl_sync(kFull, x, len - 1);
+            py = __shfl_sync(kFull, y, len - 1);
+          }
+          if (c.inside) c0 = __dadd_rn(col_dx2(c, px), row_dy2(c, py));
+        } else {
+          p = a.pos[a.order[q]];
+          c0 = get_hint(a, q, make_cell(a, p, one));
+        }
+        listed = false;
+        const Cell c = make_cell(a, p, one);
+        if (c0 < 6.25 && placeable(c)) {
+          const Best b = search_near(a, q, c, lane);
+          if (b.cost < 6.25) {
+            px = b.tile % a.W;
+            py = b.tile / a.W;
+            if (lane == 0) held = claim_site(a, q, px, py);
+            held = __shfl_sync(kFull, held, 0);
+            if (held == kNone) {
+              q = -1;
+            } else if (held > q) {
+              q = held;
+              listed = true;
+            }
+            continue;
           }
         }
         if (lane == 0) {
           spos = p;
           sc0 = c0;
+          least = __float_as_uint(kInf);
+          scount = 0;
         }
+        break;  // the whole CTA
       }
-      if (lane == 0) {
-        sq_ = q;
-        least = __float_as_uint(kInf);
-      }
+      if (lane == 0) sq_ = q;
     }
-    fresh = false;
     __syncthreads();
     const int32_t q = sq_;
     if (q < 0) return;
@@ -730,27 +870,50 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
     b = b.warp_min();
     if (lane == 0) sbest[warp] = b;
     __syncthreads();
+    b = (lane < kUnitWarps ? sbest[lane] : no_best()).warp_min();
+    if (b.tile == kNone) {  // no site is open to it
+      if (tid == 0) atomicMax(&a.st->status, 1);
+      return;
+    }
+    list_ring(a, q, c, b.cost, warp, lane, slist, &scount);
+    __syncthreads();
     if (warp == 0) {
-      b = (lane < kUnitWarps ? sbest[lane] : no_best()).warp_min();
-      if (lane == 0) {
-        if (b.tile == kNone) {  // no site is open to it
-          atomicMax(&a.st->status, 1);
-          sq_ = -1;
-        } else {
-          const int32_t held = claim_site(a, q, c, b);
-          sc0 = c.inside ? b.cost : 0.0;
-          if (held == kNone) {
-            sq_ = -1;
-          } else if (held > q) {
-            const float2 p = a.pos[a.order[held]];
-            const Cell d = make_cell(a, p, one);
-            sq_ = held;
-            spos = p;
-            sc0 = d.inside ? __dadd_rn(col_dx2(d, b.tile % a.W), row_dy2(d, b.tile / a.W)) : 0.0;
-          }
-        }
+      const int n = scount;
+      const bool keep = n <= kLpRingMax;
+      // the cheapest 32 or fewer: the ring halved until they are
+      Best e0 = lane < n ? slist[lane] : no_best(), e1 = lane + 32 < n ? slist[lane + 32] : no_best();
+      double ring = (double)ring_of(b.cost);
+      unsigned m0, m1;
+      while (true) {
+        m0 = __ballot_sync(kFull, e0.cost <= b.cost + ring);
+        m1 = __ballot_sync(kFull, e1.cost <= b.cost + ring);
+        if (__popc(m0) + __popc(m1) <= 32 || ring < 1e-3) break;
+        ring *= 0.5;
       }
+      const unsigned below = (1u << lane) - 1;
+      const int i0 = __popc(m0 & below), i1 = __popc(m0) + __popc(m1 & below);
       __syncwarp();
+      if ((m0 >> lane & 1) && i0 < 32) slist[i0] = e0;
+      if ((m1 >> lane & 1) && i1 < 32) slist[i1] = e1;
+      __syncwarp();
+      const int m = __popc(m0) + __popc(m1);
+      const bool some = keep && m <= 32;
+      const Best e = some ? warp_sorted(lane < m ? slist[lane] : no_best()) : no_best();
+      if (lane < kLpCand)
+        a.cand[(size_t)kLpCand * (q - (int32_t)a.n_mac) + lane] =
+            some && e.tile != kNone ? e.tile : lane == 0 && !some ? b.tile : -1;
+      px = b.tile % a.W;
+      py = b.tile / a.W;
+      int32_t held = 0;
+      __syncwarp();
+      if (lane == 0) {
+        put_hint(a, q, c, b.cost);
+        __threadfence();  // the list before the claim: who displaces q reads it
+        held = claim_site(a, q, px, py);
+      }
+      held = __shfl_sync(kFull, held, 0);
+      next = held == kNone ? -1 : held > q ? held : q;
+      listed = true;
     }
   }
 }
@@ -970,7 +1133,7 @@ cudaError_t lp_build_graph(LpArgs a, LpGraph &g, cudaStream_t cs) {
       return e;
     const uint32_t most = a.n_mac < kLpWindow ? a.n_mac : kLpWindow;
     const unsigned grid = (most + kLpWarps - 1) / kLpWarps;
-    k_lp_choose<<<most, kLpWarps * 32, 0, cs>>>(a);
+    k_lp_choose<<<most < 592 ? most : 592, kLpWarps * 32, 0, cs>>>(a);
     k_lp_claim<<<grid, kLpWarps * 32, 0, cs>>>(a);
     const cudaError_t launch_err = cudaGetLastError();
     cudaGraph_t captured = nullptr;

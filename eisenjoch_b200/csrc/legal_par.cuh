@@ -10,15 +10,18 @@ namespace eplace {
 // Macros that a round works on at once.
 constexpr uint32_t kLpWindow = 2048;
 
+// Sites kept of a unit cell's search.
+constexpr int kLpCand = 16;
+
 // State of one legalisation in flight, in device memory.
 struct LpState {
   uint32_t base;       // macros [0, base) have their final anchors
   uint32_t rounds;     // macro rounds run
   uint32_t first;      // lowest macro whose choice changed in this round
   uint32_t ticket;     // CTAs of the claim kernel that have finished
-  uint32_t nfreed[2];  // lengths of the two lists of freed blocks
-  int32_t status;      // 0 ok, 1 no free site for some cell, 2 round cap
-  uint32_t next;       // next unit cell to hand out
+  uint32_t nfreed;     // blocks given up in this round
+  uint32_t nwork[2];   // macros to choose in this and in the next round
+  int32_t status;      // 0 ok, 1 no free site for some cell, 2 round cap, 4 cancelled
 };
 
 // A block that a macro gave up in a round.
@@ -39,7 +42,10 @@ struct LpArgs {
   uint2 *seg;              // [H][SW] what is known of each 32-site segment (see legal_par.cu)
   int32_t *choice;         // [n_mac] anchor (tile = y * W + x) of each macro; -1: none yet, -2: none free
   double *mcost;           // [n_mac] its cost
-  LpFreed *freed;          // [2][kLpWindow] blocks given up in the last and in this round
+  LpFreed *freed;          // [kLpWindow] blocks given up in this round
+  uint32_t *work;          // [2][kLpWindow] macros to choose in this and in the next round
+  uint32_t *queued;        // [n_mac] why a macro is in the next list: 1: block lost or none yet, 2: may gain
+  int32_t *cand;           // [n - n_mac][kLpCand] next best sites of a unit cell, best first; -1: no more
   unsigned long long *hint;  // [lp_hint_count] radii without an open anchor (see legal_par.cu)
   LpState *st;
   int2 *sites;             // [N] anchor of every cell (out)
@@ -47,6 +53,7 @@ struct LpArgs {
   double *cost;            // [n] cost of each placement, by order index (out)
   double *disp;            // [1] total displacement, summed in order (out)
   int32_t *status;         // [1] 0 ok, 1 no free site, else an internal limit (out)
+  const int32_t *cancel;   // [1] set by the host: the result is no longer wanted, and what there is is not one
   uint32_t max_rounds;
   cudaGraphConditionalHandle handle;
 };
