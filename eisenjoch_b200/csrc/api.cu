@@ -1103,20 +1103,18 @@ void launch_field_gemm(eplace_ctx *c, int g, float *phi, int field_mode, bool tc
     const int hw = W / 2, hh = H / 2;
     switch (g) {
       case 0:
-        CK(launch_sgemm(h + 0, 2, H, hw, hw, c->stream, c->gemm_tile[0]));
+        CK(launch_sgemm(h + 0, 2, H, hw, hw, c->stream, c->gemm_tile[0], c->overlap));
         break;
       case 1: {
         SpectralArgs sp{c->wx.p, c->gx2.p, c->wy.p, c->gy2.p, (float)(4.0 / ((double)W * H)), phi};
-        CK(launch_sgemm_spectral(h + 2, 2, hh, W, hh, sp, c->stream, c->gemm_tile[1]));
+        CK(launch_sgemm_spectral(h + 2, 2, hh, W, hh, sp, c->stream, c->gemm_tile[1], c->overlap));
         break;
       }
       case 2:
-        CK(launch_sgemm(h + 4, 4, H, hw, hw, c->stream, c->gemm_tile[2]));
-        CK(launch_fly_cols(f, 2, H, W, c->stream));
+        CK(launch_sgemm_fly(h + 4, f, 4, H, hw, hw, true, c->stream, c->gemm_tile[2], c->overlap));
         break;
       default:
-        CK(launch_sgemm(h + 8, 4, hh, W, hh, c->stream, c->gemm_tile[3]));
-        CK(launch_fly_rows(f + 2, 2, H, W, c->stream));
+        CK(launch_sgemm_fly(h + 8, f + 2, 4, hh, W, hh, false, c->stream, c->gemm_tile[3], c->overlap));
         break;
     }
     return;
@@ -1124,18 +1122,18 @@ void launch_field_gemm(eplace_ctx *c, int g, float *phi, int field_mode, bool tc
   const GemmOp *ops = c->ops.p + (fm ? 6 : 0);
   switch (g) {
     case 0:
-      CK(launch_sgemm(ops + 0, 1, H, W, W, c->stream, c->gemm_tile[0]));
+      CK(launch_sgemm(ops + 0, 1, H, W, W, c->stream, c->gemm_tile[0], c->overlap));
       break;
     case 1: {
       SpectralArgs sp{c->wx.p, c->gx2.p, c->wy.p, c->gy2.p, (float)(4.0 / ((double)W * H)), phi};
-      CK(launch_sgemm_spectral(ops + 1, 1, H, W, H, sp, c->stream, c->gemm_tile[1]));
+      CK(launch_sgemm_spectral(ops + 1, 1, H, W, H, sp, c->stream, c->gemm_tile[1], c->overlap));
       break;
     }
     case 2:
-      CK(launch_sgemm(ops + 2, 2, H, W, W, c->stream, c->gemm_tile[2]));
+      CK(launch_sgemm(ops + 2, 2, H, W, W, c->stream, c->gemm_tile[2], c->overlap));
       break;
     default:
-      CK(launch_sgemm(ops + 4, 2, H, W, H, c->stream, c->gemm_tile[3]));
+      CK(launch_sgemm(ops + 4, 2, H, W, H, c->stream, c->gemm_tile[3], c->overlap));
       break;
   }
 }
@@ -1234,6 +1232,8 @@ void autotune_launches(eplace_ctx *c, float gamma, int field_mode, bool tc) {
     if (!tc && !c->fft) {
       for (int g = 0; g < 4; ++g) {
         float bt = 1e30f;
+        const int K = (g % 2 ? hp.BY : hp.BX) / (c->fold ? 2 : 1);
+        if (K % 64) continue;  // the launch's own rule
         for (int tile : {64, 32}) {
           c->gemm_tile[g] = tile;
           const float t = timed([&] { launch_field_gemm(c, g, nullptr, field_mode, false); });
@@ -1344,7 +1344,11 @@ void launch_iteration(eplace_ctx *c, float gamma, int field_mode, bool tc) {
 // Kernels of one iteration: WA, the step (three when split), the finalise and
 // the transform.
 int launches_per_iteration(const eplace_ctx *c, bool tc) {
-  const int transform = tc ? 5 : c->fft ? 3 : c->fold ? 7 : 5;
+  int transform = tc ? 5 : c->fft ? 3 : 5;
+  if (!tc && !c->fft && c->fold) {  // the butterflies of the forms that don't write them themselves
+    const int hw = c->hp.BX / 2, hh = c->hp.BY / 2;
+    transform += !sgemm_panel(c->hp.BY, hw, 4, hw, c->gemm_tile[2]) + !sgemm_panel(hh, c->hp.BX, 4, hh, c->gemm_tile[3]);
+  }
   return 1 + (c->split_step ? 3 : 1) + transform;
 }
 

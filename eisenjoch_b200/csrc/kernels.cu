@@ -8,7 +8,8 @@
 //                   fixed-point atomics (order independent, bit-reproducible).
 //   k_density_final sums for the overlap (density.rs:79-86), FP32 charge map
 //                   for the transform, resets the accumulator.
-//   k_sgemm         FP32 DCT-matrix GEMMs (density.rs:96-166), spectral
+//   k_sgemm, k_sgemm_panel
+//                   FP32 DCT-matrix GEMMs (density.rs:96-166), spectral
 //                   Poisson scaling fused into the second GEMM's epilogue.
 //   k_step          field gather + penalty + preconditioner + Barzilai-
 //                   Borwein + FISTA + clamp + next look-ahead and its scatter in one
@@ -579,6 +580,11 @@ __device__ __forceinline__ void gemm_store(const GemmOp &op, const SpectralArgs 
   }
 }
 
+// a + m b, m = +-1
+__device__ __forceinline__ float4 fold4(float4 a, float m, float4 b) {
+  return make_float4(a.x + m * b.x, a.y + m * b.y, a.z + m * b.z, a.w + m * b.w);
+}
+
 template <bool SPECTRAL, int TM, int TN, int S>
 __global__ void __launch_bounds__((TM / 4) * (TN / 4)) k_sgemm(const GemmOp *ops, int M, int N, int K,
                                                                SpectralArgs sp) {
@@ -594,66 +600,72 @@ __global__ void __launch_bounds__((TM / 4) * (TN / 4)) k_sgemm(const GemmOp *ops
   const int bm = blockIdx.y * TM, bn = blockIdx.x * TN;
   const bool vec = ((K & 3) == 0) && ((N & 3) == 0) && ((op.lda & 3) == 0) && ((op.ldb & 3) == 0) &&
                    ((op.a_full & 3) == 0);
-  const float am = (float)op.a_mir, bmir = (float)op.b_mir;
-  float ra[LA][4], rb[LB][4];
+  const float mir = (float)(op.a_mir ? op.a_mir : op.b_mir);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  // Loads of a step are all in flight together: what a folded operand adds
+  // (u: one operand of a product is folded, and folded grids take the float4
+  // path) is added when the step is stored.
+  float4 ra[LA], rb[LB], u[LA > LB ? LA : LB];
   auto load = [&](int k0) {
 #pragma unroll
     for (int l = 0; l < LA; ++l) {
       const int f = tid + l * T;
       const int gr = bm + f / (GK / 4), gk = k0 + (f % (GK / 4)) * 4;
-      const float *arow = op.A + (size_t)gr * op.lda;
-      if (vec && gr < M && gk + 3 < K) {
-        float4 t = *reinterpret_cast<const float4 *>(arow + gk);
-        if (op.a_mir) {  // columns a_full-1-gk-j, j = 0..3: the block below, reversed
-          const float4 u = *reinterpret_cast<const float4 *>(arow + (op.a_full - 4 - gk));
-          t.x += am * u.w; t.y += am * u.z; t.z += am * u.y; t.w += am * u.x;
-        }
-        ra[l][0] = t.x; ra[l][1] = t.y; ra[l][2] = t.z; ra[l][3] = t.w;
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float v = (gr < M && gk + j < K) ? arow[gk + j] : 0.0f;
-          if (op.a_mir && gr < M && gk + j < K) v += am * arow[op.a_full - 1 - (gk + j)];
-          ra[l][j] = v;
-        }
-      }
+      const float *p = op.A + (size_t)gr * op.lda + gk;
+      if (vec) ra[l] = gr < M && gk < K ? *reinterpret_cast<const float4 *>(p) : zero;
+      else
+        ra[l] = make_float4(gr < M && gk < K ? p[0] : 0.f, gr < M && gk + 1 < K ? p[1] : 0.f,
+                            gr < M && gk + 2 < K ? p[2] : 0.f, gr < M && gk + 3 < K ? p[3] : 0.f);
     }
 #pragma unroll
     for (int l = 0; l < LB; ++l) {
       const int f = tid + l * T;
       const int gk = k0 + f / (TN / 4), gc = bn + (f % (TN / 4)) * 4;
-      const float *brow = op.B + (size_t)gk * op.ldb;
-      const float *bmrow = op.b_mir ? op.B + (size_t)(op.b_full - 1 - gk) * op.ldb : brow;
-      if (vec && gk < K && gc + 3 < N) {
-        float4 t = *reinterpret_cast<const float4 *>(brow + gc);
-        if (op.b_mir) {
-          const float4 u = *reinterpret_cast<const float4 *>(bmrow + gc);
-          t.x += bmir * u.x; t.y += bmir * u.y; t.z += bmir * u.z; t.w += bmir * u.w;
-        }
-        rb[l][0] = t.x; rb[l][1] = t.y; rb[l][2] = t.z; rb[l][3] = t.w;
-      } else {
+      const float *p = op.B + (size_t)gk * op.ldb + gc;
+      if (vec) rb[l] = gk < K && gc < N ? *reinterpret_cast<const float4 *>(p) : zero;
+      else
+        rb[l] = make_float4(gk < K && gc < N ? p[0] : 0.f, gk < K && gc + 1 < N ? p[1] : 0.f,
+                            gk < K && gc + 2 < N ? p[2] : 0.f, gk < K && gc + 3 < N ? p[3] : 0.f);
+    }
+    if (op.a_mir) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float v = (gk < K && gc + j < N) ? brow[gc + j] : 0.0f;
-          if (op.b_mir && gk < K && gc + j < N) v += bmir * bmrow[gc + j];
-          rb[l][j] = v;
-        }
+      for (int l = 0; l < LA; ++l) {  // columns a_full-1-gk-j, j = 0..3: the block below, reversed
+        const int f = tid + l * T;
+        const int gr = bm + f / (GK / 4), gk = k0 + (f % (GK / 4)) * 4;
+        u[l] = gr < M && gk < K
+                   ? *reinterpret_cast<const float4 *>(op.A + (size_t)gr * op.lda + (op.a_full - 4 - gk)) : zero;
+      }
+    } else if (op.b_mir) {
+#pragma unroll
+      for (int l = 0; l < LB; ++l) {
+        const int f = tid + l * T;
+        const int gk = k0 + f / (TN / 4), gc = bn + (f % (TN / 4)) * 4;
+        u[l] = gk < K && gc < N
+                   ? *reinterpret_cast<const float4 *>(op.B + (size_t)(op.b_full - 1 - gk) * op.ldb + gc) : zero;
       }
     }
   };
   auto store = [&](int buf) {
+    if (op.a_mir) {
+#pragma unroll
+      for (int l = 0; l < LA; ++l) ra[l] = fold4(ra[l], mir, make_float4(u[l].w, u[l].z, u[l].y, u[l].x));
+    } else if (op.b_mir) {
+#pragma unroll
+      for (int l = 0; l < LB; ++l) rb[l] = fold4(rb[l], mir, u[l]);
+    }
 #pragma unroll
     for (int l = 0; l < LA; ++l) {
       const int f = tid + l * T;
       const int r = f / (GK / 4), k = (f % (GK / 4)) * 4;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) As[buf][k + j][r] = ra[l][j];
+      As[buf][k][r] = ra[l].x;
+      As[buf][k + 1][r] = ra[l].y;
+      As[buf][k + 2][r] = ra[l].z;
+      As[buf][k + 3][r] = ra[l].w;
     }
 #pragma unroll
     for (int l = 0; l < LB; ++l) {
       const int f = tid + l * T;
-      const int k = f / (TN / 4), c = (f % (TN / 4)) * 4;
-      *reinterpret_cast<float4 *>(&Bs[buf][k][c]) = make_float4(rb[l][0], rb[l][1], rb[l][2], rb[l][3]);
+      *reinterpret_cast<float4 *>(&Bs[buf][f / (TN / 4)][(f % (TN / 4)) * 4]) = rb[l];
     }
   };
   float acc[4][4];
@@ -733,6 +745,183 @@ __global__ void __launch_bounds__((TM / 4) * (TN / 4)) k_sgemm(const GemmOp *ops
   }
 }
 
+// ---------------------------------------------------------------------------
+// k_sgemm_panel: the same products where K has no split in four (the side, half
+// of it when folded, is not a multiple of 64).
+//
+// Bound by latency: such a product is a few hundred kFMA to some MFMA, and
+// tiles of 64 x 64 leave most SMs without one and go through K in steps of 16
+// with a barrier and an L2 round trip each.  Here a tile is 16 or 32 x 32, a
+// step is 64 of K, loaded by 128 threads while the step before is multiplied,
+// and a thread has 2 x 2 or 2 x 4 outputs.  With PAIR a CTA has both halves E
+// and O of a folded transform, 128 threads each, and writes the butterfly
+// E + O, sig (E - O) itself (cols: about the middle column, else about the
+// middle row): E and O never go to memory and the butterfly's launch goes.
+// Each output sums k = 0 .. K-1 in order as in k_sgemm: the same bits.
+// The four products (with butterflies) of a square grid back to back, before
+// -> now: side 69 36.9 -> 15.0 us, 72 34.8 -> 10.2, 133 59.5 -> 21.6, 200
+// 54.9 -> 23.1, 269 106 -> 55, 533 223 -> 131; an iteration of 1k cells on 69^2
+// bins 53.3 -> 26.7 us, of 10k on 133^2 80.7 -> 37.3, of 200k on 533^2 312 -> 196.
+// ---------------------------------------------------------------------------
+constexpr int PN = 32, PK = 64;
+
+template <bool SPECTRAL, bool PAIR, int PM>
+__global__ void __launch_bounds__(PAIR ? 256 : 128)
+    k_sgemm_panel(const GemmOp *ops, const FlyOp *fly, int cols, int M, int N, int K, SpectralArgs sp) {
+  constexpr int TC = PM / 8;  // columns of a thread; it has two rows
+  constexpr int LA = PM * PK / 128, LB = PK * PN / 128;
+  __shared__ __align__(16) float as_[PAIR ? 2 : 1][PM][PK + 4];
+  __shared__ __align__(16) float bs_[PAIR ? 2 : 1][PK][PN];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int half = PAIR ? (int)threadIdx.x >> 7 : 0, tid = threadIdx.x & 127;
+  const GemmOp op = ops[PAIR ? 2 * blockIdx.z + half : blockIdx.z];
+  auto As = as_[half];
+  auto Bs = bs_[half];
+  const int tx = tid % (PN / TC), ty = tid / (PN / TC);
+  const int bm = blockIdx.y * PM, bn = blockIdx.x * PN;
+  const bool vec = ((K & 3) == 0) && ((N & 3) == 0) && ((op.lda & 3) == 0) && ((op.ldb & 3) == 0) &&
+                   ((op.a_full & 3) == 0);
+  const float mir = (float)(op.a_mir ? op.a_mir : op.b_mir);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  // float4 l of a thread: elements 4 (tid + 128 l) .. + 3 (vec), or elements
+  // tid + 512 l + 128 j, j = 0 .. 3.  u as in k_sgemm.
+  float4 ra[LA / 4], rb[LB / 4], u[LB / 4];
+  auto load = [&](int k0) {
+    if (vec) {
+#pragma unroll
+      for (int l = 0; l < LA / 4; ++l) {
+        const int f = tid + 128 * l, gr = bm + f / (PK / 4), gk = k0 + (f % (PK / 4)) * 4;
+        ra[l] = gr < M && gk < K ? *reinterpret_cast<const float4 *>(op.A + (size_t)gr * op.lda + gk) : zero;
+      }
+#pragma unroll
+      for (int l = 0; l < LB / 4; ++l) {
+        const int f = tid + 128 * l, gk = k0 + f / (PN / 4), gc = bn + (f % (PN / 4)) * 4;
+        rb[l] = gk < K && gc < N ? *reinterpret_cast<const float4 *>(op.B + (size_t)gk * op.ldb + gc) : zero;
+      }
+      if (op.a_mir) {
+#pragma unroll
+        for (int l = 0; l < LA / 4; ++l) {  // columns a_full-1-gk-j, j = 0..3: the block below, reversed
+          const int f = tid + 128 * l, gr = bm + f / (PK / 4), gk = k0 + (f % (PK / 4)) * 4;
+          u[l] = gr < M && gk < K
+                     ? *reinterpret_cast<const float4 *>(op.A + (size_t)gr * op.lda + (op.a_full - 4 - gk)) : zero;
+        }
+      } else if (op.b_mir) {
+#pragma unroll
+        for (int l = 0; l < LB / 4; ++l) {
+          const int f = tid + 128 * l, gk = k0 + f / (PN / 4), gc = bn + (f % (PN / 4)) * 4;
+          u[l] = gk < K && gc < N
+                     ? *reinterpret_cast<const float4 *>(op.B + (size_t)(op.b_full - 1 - gk) * op.ldb + gc) : zero;
+        }
+      }
+    } else {
+      const int ak = k0 + tid % PK, ar = bm + tid / PK, bk = k0 + tid / PN, bc = bn + tid % PN;
+      const float *pa = op.A + (size_t)ar * op.lda + ak, *pb = op.B + (size_t)bk * op.ldb + bc;
+      constexpr int SA = 128 / PK, SB = 128 / PN;  // rows between a thread's elements
+      auto ea = [&](int i) { return ak < K && ar + SA * i < M ? pa[(size_t)(SA * i) * op.lda] : 0.f; };
+      auto eb = [&](int i) { return bc < N && bk + SB * i < K ? pb[(size_t)(SB * i) * op.ldb] : 0.f; };
+#pragma unroll
+      for (int l = 0; l < LA / 4; ++l) ra[l] = make_float4(ea(4 * l), ea(4 * l + 1), ea(4 * l + 2), ea(4 * l + 3));
+#pragma unroll
+      for (int l = 0; l < LB / 4; ++l) rb[l] = make_float4(eb(4 * l), eb(4 * l + 1), eb(4 * l + 2), eb(4 * l + 3));
+    }
+  };
+  auto store = [&]() {
+    float *af = &As[tid / PK][tid % PK], *bf = &Bs[tid / PN][tid % PN];
+    if (vec) {
+      if (op.a_mir) {
+#pragma unroll
+        for (int l = 0; l < LA / 4; ++l) ra[l] = fold4(ra[l], mir, make_float4(u[l].w, u[l].z, u[l].y, u[l].x));
+      } else if (op.b_mir) {
+#pragma unroll
+        for (int l = 0; l < LB / 4; ++l) rb[l] = fold4(rb[l], mir, u[l]);
+      }
+#pragma unroll
+      for (int l = 0; l < LA / 4; ++l) {
+        const int f = tid + 128 * l;
+        *reinterpret_cast<float4 *>(&As[f / (PK / 4)][(f % (PK / 4)) * 4]) = ra[l];
+      }
+#pragma unroll
+      for (int l = 0; l < LB / 4; ++l) {
+        const int f = tid + 128 * l;
+        *reinterpret_cast<float4 *>(&Bs[f / (PN / 4)][(f % (PN / 4)) * 4]) = rb[l];
+      }
+    } else {
+      constexpr int SA = 128 / PK * (PK + 4), SB = 128;
+#pragma unroll
+      for (int l = 0; l < LA / 4; ++l) {
+        af[4 * l * SA] = ra[l].x;
+        af[(4 * l + 1) * SA] = ra[l].y;
+        af[(4 * l + 2) * SA] = ra[l].z;
+        af[(4 * l + 3) * SA] = ra[l].w;
+      }
+#pragma unroll
+      for (int l = 0; l < LB / 4; ++l) {
+        bf[4 * l * SB] = rb[l].x;
+        bf[(4 * l + 1) * SB] = rb[l].y;
+        bf[(4 * l + 2) * SB] = rb[l].z;
+        bf[(4 * l + 3) * SB] = rb[l].w;
+      }
+    }
+  };
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  float acc[2][TC] = {};
+  load(0);
+  for (int k0 = 0; k0 < K; k0 += PK) {
+    store();
+    __syncthreads();
+    if (k0 + PK < K) load(k0 + PK);
+    const int kn = min(PK, (K - k0 + 3) & ~3);  // the rest of the step is zeros
+#pragma unroll 4
+    for (int k = 0; k < kn; k += 4) {
+      const float4 a0 = *reinterpret_cast<const float4 *>(&As[2 * ty][k]);
+      const float4 a1 = *reinterpret_cast<const float4 *>(&As[2 * ty + 1][k]);
+      const float av[2][4] = {{a0.x, a0.y, a0.z, a0.w}, {a1.x, a1.y, a1.z, a1.w}};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float b[TC];
+        if constexpr (TC == 2) {
+          const float2 t = *reinterpret_cast<const float2 *>(&Bs[k + j][2 * tx]);
+          b[0] = t.x, b[1] = t.y;
+        } else {
+          const float4 t = *reinterpret_cast<const float4 *>(&Bs[k + j][4 * tx]);
+          b[0] = t.x, b[1] = t.y, b[2] = t.z, b[3] = t.w;
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int c = 0; c < TC; ++c) acc[i][c] = fmaf(av[i][j], b[c], acc[i][c]);
+      }
+    }
+    __syncthreads();
+  }
+  if constexpr (PAIR) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int c = 0; c < TC; ++c) Bs[2 * ty + i][TC * tx + c] = acc[i][c];
+    __syncthreads();
+    const FlyOp f = fly[blockIdx.z];
+    const int W = cols ? 2 * N : N;
+    for (int q = tid; q < PM * PN; q += 128) {
+      const int lr = q / PN, lc = q % PN, r = bm + lr, c = bn + lc;
+      if (r >= M || c >= N) continue;
+      const float e = bs_[0][lr][lc], o = bs_[1][lr][lc];
+      if (half == 0) f.out[(size_t)r * W + c] = e + o;
+      else f.out[(size_t)(cols ? r : 2 * M - 1 - r) * W + (cols ? W - 1 - c : c)] = f.sig * (e - o);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = bm + 2 * ty + i;
+#pragma unroll
+      for (int j = 0; j < TC; ++j) {
+        const int c = bn + TC * tx + j;
+        if (r < M && c < N) gemm_store<SPECTRAL>(op, sp, r, c, N, acc[i][j]);
+      }
+    }
+  }
+}
+
 // SMs of the current device (cached per device).
 int device_sms() {
   static int sms[64] = {0};
@@ -746,12 +935,11 @@ int device_sms() {
   return sms[dev];
 }
 
-// The small tile when the 64 x 64 grid would leave more than half the SMs
-// without a CTA (measured: 64 CTAs of 512^3 gain from the small tile, 128
+// Split K: the small tile when the 64 x 64 grid would leave more than half the
+// SMs without a CTA (measured: 64 CTAs of 512^3 gain from the small tile, 128
 // CTAs do not).
-bool sgemm_small_tile(int M, int N, int nb, int K) {
-  const long ctas = (long)((N + 63) / 64) * ((M + 63) / 64) * nb * (K % 64 == 0 ? 4 : 1);  // split K: 4 CTAs a tile
-  return 2L * ctas < device_sms();
+bool sgemm_small_tile(int M, int N, int nb) {
+  return 2L * ((N + 63) / 64) * ((M + 63) / 64) * nb * 4 < device_sms();
 }
 
 // ---------------------------------------------------------------------------
@@ -1332,20 +1520,16 @@ cudaError_t launch_density_final(const FinalArgs &a_in, int grid, cudaStream_t s
   return cudaLaunchKernelEx(&l.cfg, k_density_final, a);
 }
 
-// One SIMT GEMM launch: split K four ways over a cluster when 4 * GK
-// divides K (every transform of a power-of-two bin grid of at least 64),
-// else one CTA per tile.  Which form runs depends on K alone, never on the
-// tile, so the tile stays a choice of time only.
+// One SIMT GEMM launch.  K that is a multiple of 4 * GK (every transform of a
+// power-of-two bin grid of at least 64) is split four ways over a cluster;
+// which sums run in which order depends on K alone, never on the tile, so the
+// tile stays a choice of time only.
 constexpr int kSplitK = 4;
 
 template <bool SPECTRAL, int TM, int TN>
 cudaError_t sgemm_launch(const GemmOp *ops, int nb, int M, int N, int K, const SpectralArgs &sp, cudaStream_t s) {
   const dim3 tiles((N + TN - 1) / TN, (M + TM - 1) / TM, nb);
   constexpr int T = (TM / 4) * (TN / 4);
-  if (K % (kSplitK * GK) != 0) {
-    k_sgemm<SPECTRAL, TM, TN, 1><<<tiles, T, 0, s>>>(ops, M, N, K, sp);
-    return cudaGetLastError();
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles.x, tiles.y, tiles.z * kSplitK);
   cfg.blockDim = dim3(T);
@@ -1361,17 +1545,49 @@ cudaError_t sgemm_launch(const GemmOp *ops, int nb, int M, int N, int K, const S
   return cudaLaunchKernelEx(&cfg, k_sgemm<SPECTRAL, TM, TN, kSplitK>, ops, M, N, K, sp);
 }
 
-cudaError_t launch_sgemm(const GemmOp *ops, int nb, int M, int N, int K, cudaStream_t s, int tile) {
-  if (tile == 32 || (tile == 0 && sgemm_small_tile(M, N, nb, K)))
-    return sgemm_launch<false, 32, 32>(ops, nb, M, N, K, SpectralArgs{}, s);
-  return sgemm_launch<false, 64, 64>(ops, nb, M, N, K, SpectralArgs{}, s);
+// Rows of the panels that a product runs as, 0 for none.  Measured (us a
+// product, rows 16 / rows 32 / 64 x 64 tiles; the folded third product of a
+// square grid, in brackets the CTAs of the first and of the last form): side
+// 264 6.9 / 9.8 / 14.4 (340, 60); 400 14.0 / 13.5 / 18.4 (700, 112); 600 35.1 /
+// 28.9 / 34.8 (1520, 200); 808 70.6 / 60.8 / 56.9 (2652, 364).
+int sgemm_panel(int M, int N, int nb, int K, int tile) {
+  if (K % (kSplitK * GK) == 0) return 0;
+  if (tile) return tile == 64 ? 0 : tile;
+  const long ctas = (long)((N + PN - 1) / PN) * ((M + 15) / 16) * nb;
+  const long large = (long)((N + 63) / 64) * ((M + 63) / 64) * nb;
+  return ctas <= 5L * device_sms() ? 16 : 2 * large <= 3L * device_sms() ? 32 : 0;
+}
+
+template <bool SPECTRAL, bool PAIR>
+cudaError_t panel_launch(const GemmOp *ops, const FlyOp *fly, bool cols, int nb, int M, int N, int K, int rows,
+                         const SpectralArgs &sp, cudaStream_t s, bool after) {
+  Launch l(1, PAIR ? 256 : 128, s, after);
+  l.cfg.gridDim = dim3((N + PN - 1) / PN, (M + rows - 1) / rows, PAIR ? nb / 2 : nb);
+  auto kernel = rows == 16 ? k_sgemm_panel<SPECTRAL, PAIR, 16> : k_sgemm_panel<SPECTRAL, PAIR, 32>;
+  return cudaLaunchKernelEx(&l.cfg, kernel, ops, fly, (int)cols, M, N, K, sp);
+}
+
+template <bool SPECTRAL>
+cudaError_t sgemm_any(const GemmOp *ops, int nb, int M, int N, int K, const SpectralArgs &sp, cudaStream_t s, int tile,
+                      bool after) {
+  if (const int rows = sgemm_panel(M, N, nb, K, tile))
+    return panel_launch<SPECTRAL, false>(ops, nullptr, false, nb, M, N, K, rows, sp, s, after);
+  if (K % (kSplitK * GK) != 0) {
+    k_sgemm<SPECTRAL, 64, 64, 1><<<dim3((N + 63) / 64, (M + 63) / 64, nb), 256, 0, s>>>(ops, M, N, K, sp);
+    return cudaGetLastError();
+  }
+  if (tile == 32 || (tile == 0 && sgemm_small_tile(M, N, nb)))
+    return sgemm_launch<SPECTRAL, 32, 32>(ops, nb, M, N, K, sp, s);
+  return sgemm_launch<SPECTRAL, 64, 64>(ops, nb, M, N, K, sp, s);
+}
+
+cudaError_t launch_sgemm(const GemmOp *ops, int nb, int M, int N, int K, cudaStream_t s, int tile, bool after) {
+  return sgemm_any<false>(ops, nb, M, N, K, SpectralArgs{}, s, tile, after);
 }
 
 cudaError_t launch_sgemm_spectral(const GemmOp *ops, int nb, int M, int N, int K, const SpectralArgs &sp,
-                                  cudaStream_t s, int tile) {
-  if (tile == 32 || (tile == 0 && sgemm_small_tile(M, N, nb, K)))
-    return sgemm_launch<true, 32, 32>(ops, nb, M, N, K, sp, s);
-  return sgemm_launch<true, 64, 64>(ops, nb, M, N, K, sp, s);
+                                  cudaStream_t s, int tile, bool after) {
+  return sgemm_any<true>(ops, nb, M, N, K, sp, s, tile, after);
 }
 
 namespace {
@@ -1394,12 +1610,14 @@ __global__ void k_fly_rows(const FlyOp *ops, int H, int W) {
 }
 }  // namespace
 
-cudaError_t launch_fly_cols(const FlyOp *ops, int nb, int H, int W, cudaStream_t s) {
-  k_fly_cols<<<dim3((W / 2 + 127) / 128, H, nb), 128, 0, s>>>(ops, H, W);
-  return cudaGetLastError();
-}
-cudaError_t launch_fly_rows(const FlyOp *ops, int nb, int H, int W, cudaStream_t s) {
-  k_fly_rows<<<dim3((W + 127) / 128, H / 2, nb), 128, 0, s>>>(ops, H, W);
+cudaError_t launch_sgemm_fly(const GemmOp *ops, const FlyOp *fly, int nb, int M, int N, int K, bool cols,
+                             cudaStream_t s, int tile, bool after) {
+  if (const int rows = sgemm_panel(M, N, nb, K, tile))
+    return panel_launch<false, true>(ops, fly, cols, nb, M, N, K, rows, SpectralArgs{}, s, after);
+  const cudaError_t e = launch_sgemm(ops, nb, M, N, K, s, tile, after);
+  if (e != cudaSuccess) return e;
+  if (cols) k_fly_cols<<<dim3((N + 127) / 128, M, nb / 2), 128, 0, s>>>(fly, M, 2 * N);
+  else k_fly_rows<<<dim3((N + 127) / 128, M, nb / 2), 128, 0, s>>>(fly, 2 * M, N);
   return cudaGetLastError();
 }
 

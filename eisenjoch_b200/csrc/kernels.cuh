@@ -238,26 +238,33 @@ cudaError_t launch_scatter(const ScatterArgs &a, int grid, cudaStream_t s);
 // stream has ended (it waits for that kernel's results itself).
 cudaError_t launch_density_final(const FinalArgs &a, int grid, cudaStream_t s, bool after = false);
 // C[b] = A[b] (M x K) * B[b] (K x N), row-major FP32; batches from ops[0..nb).
-// tile: 64 or 32 (CTA tile edge), 0 = pick by grid size.  When 64 divides K
-// the sum is split into four K quarters (a cluster of four CTAs per tile)
-// added in quarter order; either way both tiles sum every output in the
-// same order, so the tile never changes the bits.
-cudaError_t launch_sgemm(const GemmOp *ops_dev, int nb, int M, int N, int K, cudaStream_t s, int tile = 0);
+// tile: 64 (CTA tile edge), 32 (where 64 doesn't divide K: panels of 32 x 32)
+// or, where 64 doesn't divide K, 16 (panels of 16 x 32), 0 = pick by grid size.  When 64 divides K the sum is
+// split into four K quarters (a cluster of four CTAs per tile) added in
+// quarter order; either way all tiles sum every output in the same order, so
+// the tile never changes the bits.  after: the panels may launch while the
+// kernel before them ends.
+cudaError_t launch_sgemm(const GemmOp *ops_dev, int nb, int M, int N, int K, cudaStream_t s, int tile = 0,
+                         bool after = false);
 // As above with the spectral epilogue: C = Ex_hat, C2 = Ey_hat.
 cudaError_t launch_sgemm_spectral(const GemmOp *ops_dev, int nb, int M, int N, int K,
-                                  const SpectralArgs &sp, cudaStream_t s, int tile = 0);
-// The butterflies that complete a folded transform (see api.cu):
-// cols: out[r][x] = E[r][x] + O[r][x], out[r][W-1-x] = sig (E - O), x < W/2,
-//       E / O: [H][W/2]; nb products (blockIdx.z), each its own E, O, out, sig.
-// rows: out[y][x] = E[y][x] + O[y][x], out[H-1-y][x] = sig (E - O), y < H/2,
-//       E / O: [H/2][W].
+                                  const SpectralArgs &sp, cudaStream_t s, int tile = 0, bool after = false);
+// Products 2j and 2j+1 are the halves E and O (fly[j].E, fly[j].O: M x N) of a
+// folded transform; as above, with the butterfly that completes it (see
+// api.cu):
+// cols: out[r][x] = E[r][x] + O[r][x], out[r][2N-1-x] = sig (E - O);
+// rows: out[y][x] = E[y][x] + O[y][x], out[2M-1-y][x] = sig (E - O).
+// The panels write the result alone, the other forms E and O too.
 struct FlyOp {
   const float *E, *O;
   float *out;
   float sig;
 };
-cudaError_t launch_fly_cols(const FlyOp *ops_dev, int nb, int H, int W, cudaStream_t s);
-cudaError_t launch_fly_rows(const FlyOp *ops_dev, int nb, int H, int W, cudaStream_t s);
+cudaError_t launch_sgemm_fly(const GemmOp *ops_dev, const FlyOp *fly_dev, int nb, int M, int N, int K, bool cols,
+                             cudaStream_t s, int tile = 0, bool after = false);
+// Rows of the panels that a product runs as (one launch, with the butterfly),
+// 0 for none.
+int sgemm_panel(int M, int N, int nb, int K, int tile);
 // block: step_block; grid: at most step_max_grid for the cooperative form.
 cudaError_t launch_step(const StepArgs &a, int grid, int block, cudaStream_t s);
 // The same step as three ordinary launches (modes 2, 3, 4): no grid barrier,
