@@ -73,3 +73,33 @@ def test_step_in_one_launch_and_in_three(n):
         b, _ = srv.wait(srv.submit(nl, chip, cfg))
     assert np.array_equal(a.x, b.x) and np.array_equal(a.y, b.y) and np.array_equal(a.bel_tile, b.bel_tile)
     assert a.trajectory == b.trajectory
+
+
+@pytest.mark.parametrize("n,side,bins,macros", [(100, 32, 16, 0.0), (1000, 64, 64, 0.05), (5000, 128, 128, 0.05),
+                                                (21000, 256, 64, 0.0)])
+@pytest.mark.parametrize("it", [16, 30])
+def test_scatter_of_cells_piled_up_in_a_bin(n, side, bins, macros, it):
+    """The reference's field drives the cells to the edges and into the
+    corners.  The density that step `it` scatters (lanes of one bin add
+    together) against the density entry point's (each cell adds its own) at
+    the same look-ahead, by the overlap of the next checkpoint: sums of whole
+    numbers on both sides, a few FP64 operations after them."""
+    nl, chip = E.synth_netlist(E.SynthSpec(seed=n, num_cells=n, num_nets=n, num_pads=40, width=side, height=side,
+                                           bins_x=bins, bins_y=bins, cluster_size=32, macro_fraction=macros))
+    opts = E.RunOptions(field_mode=0)
+    with E.PlacementContext(nl, chip) as ctx:
+        before, now, after = (ctx.run(E.ElectroPlaceCfg(max_iters=k + 1, legalize_interval=k), opts)
+                              for k in (it - 1, it, it + 1))
+        assert before.best_iter == it - 1 and now.best_iter == it
+        a = [1.0]
+        while len(a) < it + 3:
+            a.append((1 + np.sqrt(1 + 4 * a[-1] ** 2)) / 2)
+        m = (a[it + 1] - 1) / a[it + 2]
+
+        def look(p, q):
+            p, q = p.astype(np.float64), q.astype(np.float64)
+            return np.clip((p + m * (p - q)).astype(np.float32), 0, np.float32(side - 1))
+
+        d, ov = ctx.density(look(now.x, before.x), look(now.y, before.y))
+    got = next(t["overlap"] for t in after.trajectory if t["iter"] == it + 1)
+    assert abs(got - ov) <= 1e-12
