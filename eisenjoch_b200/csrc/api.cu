@@ -1018,29 +1018,30 @@ void launch_field_gemm(eplace_ctx *c, int g, float *phi, int field_mode, bool tc
     e.wy = c->wy.p;
     e.gy2 = c->gy2.p;
     e.scale = (float)(4.0 / ((double)W * H));
+    e.a_fixed = g & 1;
     switch (g) {
       case 0:
         e.mode = TC_EPI_SPLIT_T;
         e.out[0] = TcEpiOut{nullptr, c->Tt_h.p, c->Tt_l.p, nullptr, nullptr};
-        CK(launch_tc_gemm(c->tm1, e, 1, H, W, W, c->stream));
+        CK(launch_tc_gemm(c->tm1, e, 1, H, W, W, c->stream, c->overlap));
         break;
       case 1:
         e.mode = TC_EPI_SPECTRAL;
         e.phi = phi;
         e.out[0] = TcEpiOut{nullptr, c->Exh_h.p, c->Exh_l.p, c->Eyh_h.p, c->Eyh_l.p};
-        CK(launch_tc_gemm(c->tm2, e, 1, H, W, H, c->stream));
+        CK(launch_tc_gemm(c->tm2, e, 1, H, W, H, c->stream, c->overlap));
         break;
       case 2:
         e.mode = TC_EPI_SPLIT_T;
         e.out[0] = TcEpiOut{nullptr, c->Ut_h.p, c->Ut_l.p, nullptr, nullptr};
         e.out[1] = TcEpiOut{nullptr, c->Vt_h.p, c->Vt_l.p, nullptr, nullptr};
-        CK(launch_tc_gemm(c->tm3[fm], e, 2, H, W, W, c->stream));
+        CK(launch_tc_gemm(c->tm3[fm], e, 2, H, W, W, c->stream, c->overlap));
         break;
       default:
         e.mode = TC_EPI_F32;
         e.out[0] = TcEpiOut{c->Ex.p, nullptr, nullptr, nullptr, nullptr};
         e.out[1] = TcEpiOut{c->Ey.p, nullptr, nullptr, nullptr, nullptr};
-        CK(launch_tc_gemm(c->tm4[fm], e, 2, H, W, H, c->stream));
+        CK(launch_tc_gemm(c->tm4[fm], e, 2, H, W, H, c->stream, c->overlap));
         break;
     }
     return;
@@ -1137,6 +1138,16 @@ void launch_field_gemm(eplace_ctx *c, int g, float *phi, int field_mode, bool tc
       break;
   }
 }
+
+// While it lives, the transform's launches overlap the end of the kernel
+// before each.
+struct OverlapOn {
+  eplace_ctx *c;
+  explicit OverlapOn(eplace_ctx *ctx) : c(ctx) { c->overlap = true; }
+  ~OverlapOn() { c->overlap = false; }
+  OverlapOn(const OverlapOn &) = delete;
+  OverlapOn &operator=(const OverlapOn &) = delete;
+};
 
 void launch_field_stage(eplace_ctx *c, float *phi, int field_mode, bool tc = false, bool from_dens = false) {
   for (int g = 0; g < 4; ++g) launch_field_gemm(c, g, phi, field_mode, tc, from_dens);
@@ -1328,15 +1339,11 @@ void launch_iteration(eplace_ctx *c, float gamma, int field_mode, bool tc) {
   launch_wa_stage(c, gamma, c->side);
   CK(cudaEventRecord(c->ev_join, c->side));
   const bool fuse = final_fused(c, tc);
-  c->overlap = true;
-  try {
+  {
+    OverlapOn on(c);
     if (!fuse) launch_final_stage(c, nullptr, tc, true);
     launch_field_stage(c, nullptr, field_mode, tc, fuse);
-  } catch (...) {
-    c->overlap = false;
-    throw;
   }
-  c->overlap = false;
   CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
   launch_step_stage(c, true);
 }
@@ -3004,7 +3011,10 @@ eplace_status eplace_stage_field(eplace_ctx *c, const double *density, int32_t d
     g_h2d += sizeof(double) * nb;
     AllocOn on_stream(s);
     if (phi_hat) c->phi.ensure(nb);
-    launch_field_stage(c, phi_hat ? c->phi.p : nullptr, field_mode, tc);
+    {
+      OverlapOn on(c);
+      launch_field_stage(c, phi_hat ? c->phi.p : nullptr, field_mode, tc);
+    }
     const size_t bytes = sizeof(float) * nb, pitch = io_pitch(nb);
     c->io_out.reserve(sizeof(float) * 3 * pitch + sizeof(DevScalars));
     float *h = static_cast<float *>(c->io_out.p);

@@ -38,10 +38,12 @@ struct TcGemmEpi {
   float scale;
   float *phi;                        // optional scaled potential spectrum
   int *err;                          // set non-zero when a bounded wait gives up
+  bool a_fixed;                      // A is the transform matrix (else B): no kernel writes it
 };
 
 bool tc_shape_ok(int M, int N, int K);
+// after: may launch while the kernel before it ends.
 cudaError_t launch_tc_gemm(const TcGemmMaps &maps, const TcGemmEpi &epi, int nbatch, int M, int N, int K,
-                           cudaStream_t s);
+                           cudaStream_t s, bool after);
 
 }  // namespace eplace
