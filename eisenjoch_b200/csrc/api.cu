@@ -257,11 +257,11 @@ struct LegalSlot {
   DBuf<LegalOut> out;
   PinBuf<LegalOut> hout;
   // working state of the parallel legaliser (legal_par.cu)
-  DBuf<int32_t> own, choice, cand;
+  DBuf<int32_t> own, choice, cand, near;
   DBuf<uint2> seg;
   DBuf<double> mcost;
   DBuf<LpFreed> freed;
-  DBuf<uint32_t> work, queued;
+  DBuf<uint32_t> work, queued, pend, left;
   DBuf<unsigned long long> hint;
   DBuf<LpState> lst;
   LpGraph graph;        // the whole legalisation: rounds in a device-side loop
@@ -1429,6 +1429,10 @@ void prepare_slot(eplace_ctx *c, LegalSlot &L) {
   L.work.ensure(2 * (size_t)kLpWindow);
   L.queued.ensure(std::max<size_t>(n_mac, 1));
   L.hint.ensure(lp_hint_count(hp.W, hp.H));
+  const size_t units = std::max<size_t>(order.size() - n_mac, 1);
+  L.near.ensure(units);
+  L.pend.ensure(units);
+  L.left.ensure(lp_chunks(units));
   L.lst.ensure(1);
   std::vector<int2> floc(hp.F);
   for (uint32_t f = 0; f < hp.F; ++f) floc[f] = make_int2(hp.fx[f], hp.fy[f]);
@@ -1456,6 +1460,9 @@ void prepare_slot(eplace_ctx *c, LegalSlot &L) {
   a.queued = L.queued.p;
   a.hint = L.hint.p;
   a.cand = L.cand.p;
+  a.near = L.near.p;
+  a.pend = L.pend.p;
+  a.left = L.left.p;
   a.st = L.lst.p;
   a.sites = L.sites.p;
   a.loc = L.loc.p;
@@ -2711,7 +2718,7 @@ uint64_t eplace_ctx::device_bytes() const {
   add(B3gt_h); add(B3gt_l); add(L6g_h); add(L6g_l); add(lg_order); add(lg_fsize); add(lg_free0);
   for (const auto &l : lslots) {
     add(l->pos); add(l->sites); add(l->loc); add(l->cost); add(l->out); add(l->own); add(l->seg); add(l->choice);
-    add(l->mcost); add(l->freed); add(l->work); add(l->queued); add(l->hint); add(l->cand); add(l->lst);
+    add(l->mcost); add(l->freed); add(l->work); add(l->queued); add(l->hint); add(l->cand); add(l->near); add(l->pend); add(l->left); add(l->lst);
   }
   return b;
 }

@@ -398,7 +398,8 @@ __global__ void __launch_bounds__(256) k_lp_init(const LpArgs a) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < hints; i += gridDim.x * blockDim.x) a.hint[i] = 0ull;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n - a.n_mac; i += gridDim.x * blockDim.x)
     a.cand[(size_t)kLpCand * i] = -1;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *a.st = LpState{0u, 0u, (uint32_t)kNone, 0u, 0u, {min(a.n_mac, kLpWindow), 0u}, 0};
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    *a.st = LpState{0u, 0u, (uint32_t)kNone, 0u, 0u, {min(a.n_mac, kLpWindow), 0u}, 0u, 0u, 0};
 }
 
 // A round, first half: each macro of the work list (whose choice may have
@@ -571,6 +572,112 @@ __device__ Best search_near(const LpArgs &a, int32_t q, const Cell &c, int lane)
       b.take(__dadd_rn(col_dx2(c, x), row_dy2(c, y)), y * a.W + x);
   }
   return b.warp_min();
+}
+
+// Claims site (x, y) for q (one thread): kNone: it was free; a later cell: q
+// has it now, and that cell has lost it; an earlier cell: q did not get it.
+__device__ __forceinline__ int32_t claim_site(const LpArgs &a, int32_t q, int x, int y) {
+  uint2 *s = seg_at(a, x, y);
+  const int32_t top = atomicMax(reinterpret_cast<int32_t *>(&s->y), q);
+  const int32_t held = atomicMin(own_at(a, x, y), q);
+  // the bit goes after both answers are here; one that lost the site clears
+  // it too, so that it does not meet a late bit again
+  if ((held == kNone || held < q) && top != kNone) atomicAnd(&s->x, ~(1u << (x & 31)));
+  return held;
+}
+
+// First all unit cells at once, a warp each: the best open site near the
+// target, claimed.  A cell that finds none, or is displaced by an earlier one
+// that was under way at the same time, is left over: the answer doesn't depend
+// on the order of the proposals.  But the work does, where many cells want the
+// same sites: a claim made too early is displaced again.  So with more than one
+// cell in kLeftMost left over, the claims are undone (0.1 ms for 200k cells) and
+// k_lp_units takes all cells, nearly in order.
+// Units of a 200k-cell checkpoint at the end of a run, 0.65 % left over: 1.74 ->
+// 0.22 ms; of 30k cells, 4.8 % left over: 0.30 -> 0.20.  Half of the cells in
+// six piles, 41 % left over: 70 ms, against 4.9 in order; trying it first costs
+// 0.15 of 7.6 ms there.  Below kNearFrom cells the attempt costs about what it
+// saves (3k cells in piles 0.15 -> 0.18 ms, 10k with macros 0.75 -> 0.81).
+constexpr uint32_t kLeftMost = 12, kNearFrom = 16384;
+__device__ __forceinline__ bool few_left(const LpArgs &a) { return kLeftMost * (uint64_t)a.st->npend <= a.n - a.n_mac; }
+
+constexpr int kNearTries = 4;
+__global__ void __launch_bounds__(256) k_lp_near(const LpArgs a) {
+  if (a.st->status != 0) return;
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (i >= a.n - a.n_mac) return;
+  const int lane = threadIdx.x & 31;
+  const int32_t q = (int32_t)(a.n_mac + i);
+  const Cell c = load_cell(a, (uint32_t)q, true);
+  int32_t site = -1;
+  for (int k = 0; k < kNearTries && placeable(c); ++k) {
+    const Best b = search_near(a, q, c, lane);
+    if (!(b.cost < 6.25)) break;
+    int32_t held = 0;
+    if (lane == 0) held = claim_site(a, q, b.tile % a.W, b.tile / a.W);
+    held = __shfl_sync(kFull, held, 0);
+    if (held > q) {  // (kNone too)
+      site = b.tile;
+      break;
+    }
+  }
+  if (lane == 0) a.near[i] = site;
+}
+
+// Whether unit cell i has not kept a site.
+__device__ __forceinline__ bool left_over(const LpArgs &a, uint32_t i) {
+  if (i >= a.n - a.n_mac) return false;
+  const int32_t t = a.near[i];
+  return t < 0 || *own_at(a, t % a.W, t / a.W) != (int32_t)(a.n_mac + i);
+}
+
+// The cells left over, in order: counted by a CTA for each kLpChunk of them,
+// then listed behind those of the chunks before.
+// (Nothing was taken, and near[] is not written, where the macros failed or
+// the result is no longer wanted; the status doesn't change in between.)
+__global__ void __launch_bounds__(kLpChunk) k_lp_count(const LpArgs a) {
+  if (a.st->status != 0) return;
+  const int n = __syncthreads_count(left_over(a, blockIdx.x * kLpChunk + threadIdx.x));
+  if (threadIdx.x == 0) a.left[blockIdx.x] = (uint32_t)n;
+}
+__global__ void __launch_bounds__(kLpChunk) k_lp_pending(const LpArgs a) {
+  __shared__ uint32_t part[kLpChunk / 32];
+  if (a.st->status != 0) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto block_sum = [&](uint32_t v) {
+    v = __reduce_add_sync(kFull, v);
+    if (lane == 0) part[warp] = v;
+    __syncthreads();
+    v = __reduce_add_sync(kFull, part[lane]);
+    __syncthreads();
+    return v;
+  };
+  uint32_t v = 0;
+  for (uint32_t j = threadIdx.x; j < blockIdx.x; j += kLpChunk) v += a.left[j];
+  const uint32_t before = block_sum(v);
+  const uint32_t i = blockIdx.x * kLpChunk + threadIdx.x;
+  const bool left = left_over(a, i);
+  const unsigned m = __ballot_sync(kFull, left);
+  if (lane == 0) part[warp] = __popc(m);
+  __syncthreads();
+  const uint32_t mine = __reduce_add_sync(kFull, lane < warp ? part[lane] : 0u);
+  if (left) a.pend[before + mine + __popc(m & ((1u << lane) - 1u))] = a.n_mac + i;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kLpChunk - 1) {
+    a.st->npend = before + mine + __popc(m);
+    if (!few_left(a)) cudaGraphSetConditional(a.many, 1u);
+  }
+}
+
+// Undoes the claims of the unit cells when too many are left over.
+__global__ void __launch_bounds__(256) k_lp_undo(const LpArgs a) {
+  const int lane = threadIdx.x & 31;
+  const int nseg = a.SW * a.H;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nseg; i += (gridDim.x * blockDim.x) >> 5) {
+    const bool open = a.own[(size_t)32 * i + lane] >= (int32_t)a.n_mac;  // (kNone too)
+    if (open) a.own[(size_t)32 * i + lane] = kNone;
+    const unsigned m = __ballot_sync(kFull, open);
+    if (lane == 0) a.seg[i] = make_uint2(m, ~0u);
+  }
 }
 
 // The search over the whole chip by the CTA, none of cost below c0 being
@@ -754,20 +861,8 @@ __device__ __forceinline__ Best warp_sorted(Best b) {
   return b;
 }
 
-// Claims site (x, y) for q (one thread): kNone: it was free; a later cell: q
-// has it now, and that cell has lost it; an earlier cell: q did not get it.
-__device__ __forceinline__ int32_t claim_site(const LpArgs &a, int32_t q, int x, int y) {
-  uint2 *s = seg_at(a, x, y);
-  const int32_t top = atomicMax(reinterpret_cast<int32_t *>(&s->y), q);
-  const int32_t held = atomicMin(own_at(a, x, y), q);
-  // the bit goes after both answers are here; one that lost the site clears
-  // it too, so that it does not meet a late bit again
-  if ((held == kNone || held < q) && top != kNone) atomicAnd(&s->x, ~(1u << (x & 31)));
-  return held;
-}
-
-// A CTA per unit cell, and the cells that its claim displaces one after the
-// other.  What takes the time is the chain of cells that each take a site from
+// A CTA per unit cell (kAll: each CTA has one; else those left over, taken up
+// in order), and the cells that its claim displaces one after the other.  What takes the time is the chain of cells that each take a site from
 // the next (about a thousand cells at the rim of a 200k-cell pile), so one
 // answer is made short: one warp, with no barrier, finds an answer near the
 // target, and that of a displaced cell in the list its search left (closed
@@ -780,25 +875,36 @@ __device__ __forceinline__ int32_t claim_site(const LpArgs &a, int32_t q, int x,
 // 4.9 ms and 117k searches of the whole CTA; without the lists 7.5 ms and 283k;
 // without them and with 2 / 4 / 8 cells per CTA 13.4 / 20 / 30 ms, with a warp
 // per cell 27 to 70 ms.
+template <bool kAll>
 __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(const LpArgs a) {
   __shared__ Best sbest[kUnitWarps], slist[kLpRingMax];
   __shared__ unsigned least;
   __shared__ int scount;
-  // the cell under way: index (-1: done), target, cost below which no site is open
+  // the cell under way: index (-1: done, -2: none, take up the next), target, cost below which no site is open
   __shared__ int32_t sq_;
   __shared__ float2 spos;
   __shared__ double sc0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uchar2 one = make_uchar2(1, 1);
-  int32_t next = (int32_t)(a.n_mac + blockIdx.x);  // warp 0: the cell to place
-  bool listed = false;                             // it may have a list
-  int px = 0, py = 0;                              // a displaced cell: the site it lost
-  if (warp == 0) {  // nothing to do for a legalisation that failed or is not wanted
-    const bool off = ld_own(a.cancel) != 0;
-    if (off && lane == 0) atomicMax(&a.st->status, 4);
-    if (off || ld_own(&a.st->status) != 0) next = -1;
-  }
+  int32_t next = -1;    // warp 0: the cell to place, -1: none
+  bool listed = false;  // it may have a list
+  int px = 0, py = 0;   // a displaced cell: the site it lost
+  if (!kAll && !few_left(a)) return;
+  bool fresh = true;  // no cell under way
   while (true) {
+    if (warp == 0 && fresh) {
+      uint32_t item = blockIdx.x;
+      if (!kAll) {
+        if (lane == 0) item = atomicAdd(&a.st->taken, 1u);
+        item = __shfl_sync(kFull, item, 0);
+      }
+      next = kAll ? (int32_t)(a.n_mac + item) : item < a.st->npend ? (int32_t)a.pend[item] : -1;
+      listed = false;
+      // nothing to do for a legalisation that failed or is not wanted
+      const bool off = ld_own(a.cancel) != 0;
+      if (off && lane == 0) atomicMax(&a.st->status, 4);
+      if (off || ld_own(&a.st->status) != 0) next = -1;
+    }
     if (warp == 0) {  // while one warp can tell
       int32_t q = next;
       while (q >= 0) {
@@ -859,11 +965,18 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
         }
         break;  // the whole CTA
       }
-      if (lane == 0) sq_ = q;
+      // none left to take up, or (kAll) this CTA's one has its place
+      const bool last = kAll || (fresh && next < 0);
+      if (lane == 0) sq_ = q >= 0 ? q : last ? -1 : -2;
     }
     __syncthreads();
     const int32_t q = sq_;
-    if (q < 0) return;
+    if (q == -1) return;
+    fresh = q < 0;
+    if (fresh) {
+      __syncthreads();  // read before it changes
+      continue;
+    }
     const Cell c = make_cell(a, spos, one);
     Best b = no_best();
     if (placeable(c)) b = search_rows(a, q, c, sc0, warp, lane, &least);
@@ -1112,38 +1225,66 @@ cudaError_t lp_build_graph(LpArgs a, LpGraph &g, cudaStream_t cs) {
     tail = node;
     return r;
   };
+  auto add_cond = [&](cudaGraphConditionalHandle handle, cudaGraphConditionalNodeType type, cudaGraph_t *body) {
+    cudaGraphNodeParams cp = {};
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = handle;
+    cp.conditional.type = type;
+    cp.conditional.size = 1;
+    cudaGraphNode_t node;
+    const cudaError_t r = cudaGraphAddNode(&node, graph, tail ? &tail : nullptr, tail ? 1 : 0, &cp);
+    tail = node;
+    if (r == cudaSuccess) *body = cp.conditional.phGraph_out[0];
+    return r;
+  };
+  auto end_body = [&] {  // of a body captured from cs
+    const cudaError_t launched = cudaGetLastError();
+    cudaGraph_t captured = nullptr;
+    const cudaError_t r = cudaStreamEndCapture(cs, &captured);
+    return launched != cudaSuccess ? launched : r;
+  };
   const size_t sites = (size_t)a.W * a.H;
   const unsigned site_grid = (unsigned)((sites + 255) / 256 < 1184 ? (sites + 255) / 256 : 1184);
   if (a.n_mac &&
       (e = cudaGraphConditionalHandleCreate(&a.handle, graph, 1, cudaGraphCondAssignDefault)) != cudaSuccess)
     return e;
+  const uint32_t units = a.n - a.n_mac;
+  const bool at_once = units >= kNearFrom;
+  if (at_once &&
+      (e = cudaGraphConditionalHandleCreate(&a.many, graph, 0, cudaGraphCondAssignDefault)) != cudaSuccess)
+    return e;
   if ((e = add((const void *)k_lp_init, site_grid, 256)) != cudaSuccess) return e;
   if (a.n_mac) {
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = a.handle;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    cudaGraphNode_t loop;
-    if ((e = cudaGraphAddNode(&loop, graph, &tail, 1, &cp)) != cudaSuccess) return e;
-    tail = loop;
+    cudaGraph_t body;
+    if ((e = add_cond(a.handle, cudaGraphCondTypeWhile, &body)) != cudaSuccess) return e;
     // The round, captured into the loop body.
-    if ((e = cudaStreamBeginCaptureToGraph(cs, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                           cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
+    if ((e = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
+        cudaSuccess)
       return e;
     const uint32_t most = a.n_mac < kLpWindow ? a.n_mac : kLpWindow;
     const unsigned grid = (most + kLpWarps - 1) / kLpWarps;
     k_lp_choose<<<most < 592 ? most : 592, kLpWarps * 32, 0, cs>>>(a);
     k_lp_claim<<<grid, kLpWarps * 32, 0, cs>>>(a);
-    const cudaError_t launch_err = cudaGetLastError();
-    cudaGraph_t captured = nullptr;
-    e = cudaStreamEndCapture(cs, &captured);
-    if (launch_err != cudaSuccess) return launch_err;
-    if (e != cudaSuccess) return e;
+    if ((e = end_body()) != cudaSuccess) return e;
   }
   if ((e = add((const void *)k_lp_segments, site_grid, 256)) != cudaSuccess) return e;
-  if (a.n > a.n_mac) {
-    if ((e = add((const void *)k_lp_units, a.n - a.n_mac, kUnitWarps * 32)) != cudaSuccess) return e;
+  if (units && !at_once) {
+    if ((e = add((const void *)k_lp_units<true>, units, kUnitWarps * 32)) != cudaSuccess) return e;
+  } else if (units) {
+    const uint32_t chunks = (uint32_t)lp_chunks(units);
+    if ((e = add((const void *)k_lp_near, (units + 7) / 8, 256)) != cudaSuccess) return e;
+    if ((e = add((const void *)k_lp_count, chunks, kLpChunk)) != cudaSuccess) return e;
+    if ((e = add((const void *)k_lp_pending, chunks, kLpChunk)) != cudaSuccess) return e;
+    cudaGraph_t body;
+    if ((e = add_cond(a.many, cudaGraphCondTypeIf, &body)) != cudaSuccess) return e;
+    if ((e = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
+        cudaSuccess)
+      return e;
+    k_lp_undo<<<site_grid, 256, 0, cs>>>(a);
+    k_lp_units<true><<<units, kUnitWarps * 32, 0, cs>>>(a);
+    if ((e = end_body()) != cudaSuccess) return e;
+    if ((e = add((const void *)k_lp_units<false>, 296, kUnitWarps * 32)) != cudaSuccess)
+      return e;
   }
   if ((e = add((const void *)k_lp_result, site_grid, 256)) != cudaSuccess) return e;
   if ((e = add((const void *)k_lp_finish, 1, kSumThreads)) != cudaSuccess) return e;

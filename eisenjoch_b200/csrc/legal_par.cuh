@@ -21,6 +21,8 @@ struct LpState {
   uint32_t ticket;     // CTAs of the claim kernel that have finished
   uint32_t nfreed;     // blocks given up in this round
   uint32_t nwork[2];   // macros to choose in this and in the next round
+  uint32_t npend;      // unit cells left to k_lp_units
+  uint32_t taken;      // of them, those that a CTA has taken up
   int32_t status;      // 0 ok, 1 no free site for some cell, 2 round cap, 4 cancelled
 };
 
@@ -47,6 +49,9 @@ struct LpArgs {
   uint32_t *queued;        // [n_mac] why a macro is in the next list: 1: block lost or none yet, 2: may gain
   int32_t *cand;           // [n - n_mac][kLpCand] next best sites of a unit cell, best first; -1: no more
   unsigned long long *hint;  // [lp_hint_count] radii without an open anchor (see legal_par.cu)
+  int32_t *near;           // [n - n_mac] site a unit cell took near its target, -1: none
+  uint32_t *pend;          // [n - n_mac] order indices of the cells left to k_lp_units, ascending
+  uint32_t *left;          // [lp_chunks] how many of them in each kLpChunk unit cells
   LpState *st;
   int2 *sites;             // [N] anchor of every cell (out)
   int2 *loc;               // [N] pin location anchor + (size - 1) / 2 (out), or nullptr
@@ -55,20 +60,26 @@ struct LpArgs {
   int32_t *status;         // [1] 0 ok, 1 no free site, else an internal limit (out)
   const int32_t *cancel;   // [1] set by the host: the result is no longer wanted, and what there is is not one
   uint32_t max_rounds;
-  cudaGraphConditionalHandle handle;
+  cudaGraphConditionalHandle handle;  // of the loop over the macro rounds
+  cudaGraphConditionalHandle many;    // of the pass over all unit cells in order
 };
 
 // The hints: one entry per size class (1 .. 8 sites) and 16 x 16 sites.
 constexpr int kLpHintClasses = 8;
 inline size_t lp_hint_count(int W, int H) { return (size_t)kLpHintClasses * ((W + 15) / 16) * ((H + 15) / 16); }
 
+// Unit cells that a CTA looks through for ones that are left.
+constexpr uint32_t kLpChunk = 1024;
+inline size_t lp_chunks(size_t units) { return (units + kLpChunk - 1) / kLpChunk; }
+
 // Chips the device legaliser takes (tile ids and per-site claims sized by
 // W x H): up to 4096 x 4096 sites.
 inline bool legalize_supported(int W, int H) { return W > 0 && H > 0 && W <= 4096 && H <= 4096; }
 
 // A legalisation as one CUDA graph: initialisation, a device-side while
-// loop over the macro rounds (when there are macros), the unit cells, the
-// displacement sum.  Built once per slot and problem load; launched per
+// loop over the macro rounds (when there are macros), the unit cells (all at
+// once and the few left over, or, where too many are, all in order: an if
+// node), the displacement sum.  Built once per slot and problem load; launched per
 // checkpoint.
 struct LpGraph {
   cudaGraphExec_t exec = nullptr;
@@ -76,7 +87,7 @@ struct LpGraph {
   ~LpGraph();
 };
 
-// Builds the graph for args `a` (the handle field is filled in).
+// Builds the graph for args `a` (the handles are filled in).
 cudaError_t lp_build_graph(LpArgs a, LpGraph &g, cudaStream_t capture_stream);
 
 }  // namespace eplace

@@ -210,3 +210,47 @@ def test_device_legalizer_edges(w, h, macros):
             assert np.array_equal(dx, hx) and np.array_equal(dy, hy)
             assert dd == hd
             assert dh == E.hpwl_host(nl, chip, hx, hy)
+
+
+@pytest.mark.parametrize("n,side", [(16383, 256), (16384, 256), (17408, 256), (17409, 140), (16900, 130)])
+@pytest.mark.parametrize("macros", [0, 12])
+def test_device_legalizer_all_at_once(n, side, macros):
+    """Unit cells that are placed all at once and those left over: counts
+    around where that starts and around the chunks they are listed by, from
+    hardly any left over to all of them, on an open and on a full chip."""
+    rng = np.random.default_rng(n + macros)
+    cw = np.ones(n, np.uint8)
+    cw[rng.permutation(n)[:macros]] = 4  # 4 x 1
+    if n + 3 * macros > side * side:
+        n -= 3 * macros
+        cw = np.sort(cw)[::-1][:n].copy()
+    nl = E.Netlist(num_cells=n, net_offsets=np.array([0, 2], np.uint32), pin_cell=np.array([0, 1], np.uint32),
+                   cell_w=cw, cell_h=np.ones(n, np.uint8))
+    chip = E.Chip(side, side)
+    grid = np.arange(n) * (side * side // n)
+    own_site = np.stack([grid % side, grid // side]).astype(np.float64)
+    uniform = rng.uniform(0, side - 1, (2, n))
+    with E.PlacementContext(nl, chip) as ctx:
+        for piled in (0.0, 0.05, 0.12, 1.0):
+            p = own_site if piled == 0.0 else uniform.copy()
+            m = rng.random(n) < piled
+            p = np.where(m, side * 0.4 + rng.normal(0, side * 0.02, (2, n)), p)
+            x, y = np.clip(p, 0, side - 1).astype(np.float32)
+            hx, hy, hd = ctx.legalize(x, y)
+            dx, dy, dd, _ = ctx.legalize_device(x, y)
+            assert np.array_equal(dx, hx) and np.array_equal(dy, hy), piled
+            assert dd == hd
+
+
+@pytest.mark.parametrize("field_mode", [0, 1])
+def test_run_with_device_legalizer_all_at_once(field_mode):
+    """A run long enough to legalise checkpoints that are no longer wanted."""
+    nl, chip = E.synth_netlist(E.SynthSpec(seed=11, num_cells=24000, num_nets=26000, num_pads=200, width=256,
+                                           height=256, bins_x=128, bins_y=128, cluster_size=64, macro_fraction=0.02))
+    cfg = E.ElectroPlaceCfg(max_iters=60)
+    a = E.place_electro(nl, chip, cfg, E.RunOptions(field_mode=field_mode, legal_mode=0))
+    for _ in range(2):
+        b = E.place_electro(nl, chip, cfg, E.RunOptions(field_mode=field_mode, legal_mode=1))
+        assert a.hpwl == b.hpwl and a.best_iter == b.best_iter
+        assert np.array_equal(a.bel_tile, b.bel_tile)
+        assert a.trajectory == b.trajectory
