@@ -38,7 +38,9 @@
 // A 200k-cell checkpoint (5 % macros, half of the cells in six piles): 150 to
 // 200 ms as rounds of candidate lists, disturbance passes and one CTA's serial
 // pass over the cells whose lists interact (a hundred rounds and more of 20
-// launches), 8.4 ms in this form (macros 2.8 ms in 54 rounds, units 4.9).
+// launches), 7.6 ms in this form (macros 2.8 ms in 54 rounds, units 4.9).  The
+// checkpoint at the end of such a run, cells spread: 1.3 ms (macros 0.7 in 17
+// rounds, units 0.2, the displacement's sum 0.24).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -596,7 +598,7 @@ __device__ __forceinline__ int32_t claim_site(const LpArgs &a, int32_t q, int x,
 // Units of a 200k-cell checkpoint at the end of a run, 0.65 % left over: 1.74 ->
 // 0.22 ms; of 30k cells, 4.8 % left over: 0.30 -> 0.20.  Half of the cells in
 // six piles, 41 % left over: 70 ms, against 4.9 in order; trying it first costs
-// 0.15 of 7.6 ms there.  Below kNearFrom cells the attempt costs about what it
+// 0.04 of 7.6 ms there.  Below kNearFrom cells the attempt costs about what it
 // saves (3k cells in piles 0.15 -> 0.18 ms, 10k with macros 0.75 -> 0.81).
 constexpr uint32_t kLeftMost = 12, kNearFrom = 16384;
 __device__ __forceinline__ bool few_left(const LpArgs &a) { return kLeftMost * (uint64_t)a.st->npend <= a.n - a.n_mac; }
@@ -890,20 +892,21 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
   bool listed = false;  // it may have a list
   int px = 0, py = 0;   // a displaced cell: the site it lost
   if (!kAll && !few_left(a)) return;
+  // nothing to do for a legalisation that failed or is not wanted
+  auto wanted = [&] {
+    const bool off = ld_own(a.cancel) != 0;
+    if (off && lane == 0) atomicMax(&a.st->status, 4);
+    return !off && ld_own(&a.st->status) == 0;
+  };
   bool fresh = true;  // no cell under way
+  if (kAll && warp == 0 && wanted()) next = (int32_t)(a.n_mac + blockIdx.x);
   while (true) {
-    if (warp == 0 && fresh) {
-      uint32_t item = blockIdx.x;
-      if (!kAll) {
-        if (lane == 0) item = atomicAdd(&a.st->taken, 1u);
-        item = __shfl_sync(kFull, item, 0);
-      }
-      next = kAll ? (int32_t)(a.n_mac + item) : item < a.st->npend ? (int32_t)a.pend[item] : -1;
+    if (!kAll && warp == 0 && fresh) {
+      uint32_t item = 0;
+      if (lane == 0) item = atomicAdd(&a.st->taken, 1u);
+      item = __shfl_sync(kFull, item, 0);
+      next = item < a.st->npend && wanted() ? (int32_t)a.pend[item] : -1;
       listed = false;
-      // nothing to do for a legalisation that failed or is not wanted
-      const bool off = ld_own(a.cancel) != 0;
-      if (off && lane == 0) atomicMax(&a.st->status, 4);
-      if (off || ld_own(&a.st->status) != 0) next = -1;
     }
     if (warp == 0) {  // while one warp can tell
       int32_t q = next;
@@ -965,17 +968,18 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
         }
         break;  // the whole CTA
       }
-      // none left to take up, or (kAll) this CTA's one has its place
-      const bool last = kAll || (fresh && next < 0);
-      if (lane == 0) sq_ = q >= 0 ? q : last ? -1 : -2;
+      // (-2: there may be others to take up)
+      if (lane == 0) sq_ = q >= 0 || kAll || (fresh && next < 0) ? q : -2;
     }
     __syncthreads();
     const int32_t q = sq_;
-    if (q == -1) return;
-    fresh = q < 0;
-    if (fresh) {
-      __syncthreads();  // read before it changes
-      continue;
+    if (kAll ? q < 0 : q == -1) return;
+    if (!kAll) {
+      fresh = q < 0;
+      if (fresh) {
+        __syncthreads();  // read before it changes
+        continue;
+      }
     }
     const Cell c = make_cell(a, spos, one);
     Best b = no_best();
