@@ -125,17 +125,22 @@ __device__ __forceinline__ Cell load_cell(const LpArgs &a, uint32_t q, bool unit
   return make_cell(a, a.pos[cell], unit ? make_uchar2(1, 1) : a.fsize[cell]);
 }
 
-// A cell with no finite target has no site of least cost.
-__device__ __forceinline__ bool placeable(const Cell &c) {
-  return isfinite(c.tx) && isfinite(c.ty) && c.AW > 0 && c.AH > 0;
-}
-
 // Cost of anchor (ax, ay), formed as the host legaliser forms it.
 __device__ __forceinline__ double axis2(double at, double off, double target) {
   return sq(__dsub_rn(__dadd_rn(at, off), target));
 }
 __device__ __forceinline__ double col_dx2(const Cell &c, int ax) { return axis2((double)ax, c.ox, c.tx); }
 __device__ __forceinline__ double row_dy2(const Cell &c, int ay) { return axis2((double)ay, c.oy, c.ty); }
+
+// A cell whose target is no number, infinite, or more than 2^24 sites from its
+// nearest anchor finds no site.  Up to there the costs of two sites in a row on
+// the same side of the target differ in FP64 (whole sites apart, an ulp of
+// 2^-5), and FP32 bounds on them stay far from overflow; from 2^26.5 on sites
+// of one row tie, and past 2^64 a cost in FP32 is infinite.
+constexpr double kFarCost = 281474976710656.0;  // (2^24)^2
+__device__ __forceinline__ bool placeable(const Cell &c) {
+  return c.AW > 0 && c.AH > 0 && __dadd_rn(col_dx2(c, c.cx), row_dy2(c, c.cy)) <= kFarCost;
+}
 
 // The least (cost, tile) seen; tile kNone: none.  Costs are >= 0, so the
 // words of a cost order like the cost.
@@ -997,11 +1002,11 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
     if (warp == 0) {
       const int n = scount;
       const bool keep = n <= kLpRingMax;
-      // the cheapest 32 or fewer: the ring halved until they are
+      // the cheapest 32 or fewer: the ring (below 2^26) halved until they are
       Best e0 = lane < n ? slist[lane] : no_best(), e1 = lane + 32 < n ? slist[lane + 32] : no_best();
       double ring = (double)ring_of(b.cost);
-      unsigned m0, m1;
-      while (true) {
+      unsigned m0 = 0, m1 = 0;
+      for (int k = 0; k < 37; ++k) {
         m0 = __ballot_sync(kFull, e0.cost <= b.cost + ring);
         m1 = __ballot_sync(kFull, e1.cost <= b.cost + ring);
         if (__popc(m0) + __popc(m1) <= 32 || ring < 1e-3) break;

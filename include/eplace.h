@@ -296,8 +296,8 @@ eplace_status eplace_legalize(eplace_ctx *ctx, const float *x, const float *y,
  * to eplace_legalize), followed by the device HPWL of the binding.  Replaces
  * legalize_electro (electro_place/mod.rs:206-255) + total_hpwl
  * (metrics/wirelength.rs:10-51).  Returns EPLACE_ERR_NO_BELS when a cell
- * finds no free site; EPLACE_ERR_INVALID for chips larger than 4096 x 4096
- * sites. */
+ * finds no free site, or its position is not finite or more than 2^24 sites
+ * from the chip; EPLACE_ERR_INVALID for chips larger than 4096 x 4096 sites. */
 eplace_status eplace_stage_legalize(eplace_ctx *ctx, const float *x, const float *y,
                                     int32_t *site_x, int32_t *site_y, double *displacement,
                                     int64_t *hpwl);

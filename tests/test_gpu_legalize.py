@@ -254,3 +254,48 @@ def test_run_with_device_legalizer_all_at_once(field_mode):
         assert a.hpwl == b.hpwl and a.best_iter == b.best_iter
         assert np.array_equal(a.bel_tile, b.bel_tile)
         assert a.trajectory == b.trajectory
+
+
+@pytest.mark.parametrize("macros", [False, True])
+@pytest.mark.parametrize("far", [1e2, 1e4, 1e6, 1.1e7])
+def test_device_legalizer_targets_off_the_chip(far, macros):
+    """Targets beside, above and diagonally off the chip, some of them one on
+    another (the displaced cells' lists), up to 2^24 sites away."""
+    rng = np.random.default_rng(int(far))
+    n, w, h = 300, 70, 40
+    cw = np.ones(n, np.uint8)
+    if macros:
+        cw[rng.permutation(n)[:20]] = 3
+    nl = E.Netlist(num_cells=n, net_offsets=np.array([0, 2], np.uint32), pin_cell=np.array([0, 1], np.uint32),
+                   cell_w=cw, cell_h=cw if macros else None)
+    with E.PlacementContext(nl, E.Chip(w, h)) as ctx:
+        for dx, dy in ((1, 0), (-1, 0), (0, 1), (0, -1), (1, 1), (-1, 0.3)):
+            x, y = rng.uniform(0, w - 1, n), rng.uniform(0, h - 1, n)
+            off = rng.random(n) < 0.5
+            x, y = np.where(off, 0.4 * w + dx * far, x), np.where(off, 0.6 * h + dy * far, y)
+            hx, hy, hd = ctx.legalize(x, y)
+            gx, gy, gd, _ = ctx.legalize_device(x, y)
+            assert np.array_equal(gx, hx) and np.array_equal(gy, hy)
+            assert gd == hd
+
+
+@pytest.mark.parametrize("cells", [40, 16384])
+@pytest.mark.parametrize("bad", [(2.0 ** 25, 5.0), (5.0, -(2.0 ** 25)), (1e19, 5.0), (5.0, 2e19), (-3e38, 3e38),
+                                 (np.inf, 5.0), (5.0, -np.inf), (np.nan, 5.0), (5.0, np.nan)])
+def test_device_legalizer_refuses_targets_without_a_site(cells, bad):
+    """A target that is no number, infinite or too far away (FP32 costs of its
+    sites are infinite from 2^64 sites on): the call ends with an error, and the
+    next one is right."""
+    side = 8 if cells == 40 else 160
+    rng = np.random.default_rng(cells)
+    nl = E.Netlist(num_cells=cells, net_offsets=np.array([0, 2], np.uint32), pin_cell=np.array([0, 1], np.uint32))
+    x, y = rng.uniform(0, side - 1, (2, cells)).astype(np.float32)
+    with E.PlacementContext(nl, E.Chip(side, side)) as ctx:
+        for which in (0, cells // 2, cells - 1):
+            fx, fy = x.copy(), y.copy()
+            fx[which], fy[which] = bad
+            with pytest.raises(E.NoBelsAvailable):
+                ctx.legalize_device(fx, fy)
+        hx, hy, hd = ctx.legalize(x, y)
+        gx, gy, gd, _ = ctx.legalize_device(x, y)
+        assert np.array_equal(gx, hx) and np.array_equal(gy, hy) and gd == hd
