@@ -342,7 +342,7 @@ struct eplace_ctx {
   DBuf<double> io_dens;  // [bins] density map of the density entry
   DBuf<DevScalars> sc;
   DBuf<IterLog> log;
-  DBuf<unsigned long long> dsum;  // [2] the overlap's sums (zero between launches)
+  DBuf<unsigned long long> dsum;  // [kOverlapWords] the overlap's sums (zero between launches)
   DBuf<unsigned> bar;  // [0..1] grid barrier, [2] finalise ticket, [3] step ticket
   DBuf<int2> loc;
   DBuf<unsigned long long> hp_total;
@@ -988,8 +988,7 @@ int *err_ptr(eplace_ctx *c) { return reinterpret_cast<int *>(reinterpret_cast<ch
 
 NormArgs norm_args(const eplace_ctx *c);
 
-// Sites per bin as a fixed-point density.
-unsigned long long cap_fix(const HostProblem &hp) { return (unsigned long long)hp.sx * (unsigned long long)hp.sy << 32; }
+long long cap_fix(const HostProblem &hp) { return fixed_capacity((long long)hp.sx * hp.sy); }
 
 // loop: inside an iteration, after the step (whose norms it adds up too).
 void launch_final_stage(eplace_ctx *c, double *dens_out, bool tc = false, bool loop = false) {
@@ -2674,7 +2673,7 @@ eplace_ctx *ctx_new(int32_t device, eplace_status *st) {
     CK(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device));
     c->sc.alloc(1);
     c->bar.alloc(4);
-    c->dsum.alloc(2);
+    c->dsum.alloc(kOverlapWords);
     c->hp_total.alloc(1);
     ensure_log(c.get(), 8);
     CK(cudaStreamSynchronize(c->stream));

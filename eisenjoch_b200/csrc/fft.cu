@@ -157,9 +157,7 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (threadIdx.x < 32) finish_norms(a.norms);
     if (threadIdx.x == 32) {
-      const unsigned long long sum = atomicExch(&a.sums[0], 0ull), over = atomicExch(&a.sums[1], 0ull);
-      const double inv = 1.0 / 4294967296.0;
-      const double ovl = sum == 0 ? 0.0 : ((double)(long long)over * inv) / ((double)(long long)sum * inv);
+      const double ovl = take_overlap(a.sums);
       a.sc->overlap = ovl;  // compute_overlap
       a.log[a.sc->iter].overlap = ovl;
     }
@@ -189,7 +187,7 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
   for (int j = threadIdx.x; j < N / 2; j += nt) tw[j] = __ldg(tb.tw + j);
   for (int j = threadIdx.x; j < N; j += nt) tq[j] = __ldg(tb.tq + j);
   asm volatile("griddepcontrol.wait;" ::: "memory");  // the tables don't change
-  long long ov[2] = {0, 0};  // sum d, sum max(d - cap, 0) in fixed point (stage 0 from the map)
+  long long ov[kOverlapWords] = {};  // of the overlap (stage 0 from the map)
   if (STAGE == 0 && a.dens) {
     for (int v0 = 0; v0 < nvec; v0 += kBatch * nt) {
       ulonglong2 q0[kBatch], q1[kBatch];
@@ -217,23 +215,15 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const double d = (double)(long long)qq[c] * (1.0 / 4294967296.0);
-          ov[0] += (long long)qq[c];
-          ov[1] += qq[c] > a.cap ? (long long)(qq[c] - a.cap) : 0;
+          count_bin(qq[c], a.cap, ov);
           sf[2 * pd(b0 + bitrev(vpos(n + c, N), logN))] = (float)(d - a.c0);
         }
       }
     }
     // whole numbers: added up in any order, and nobody waits for them (a last
     // CTA that summed them held the stage up for 1.8 us)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      ov[0] += __shfl_xor_sync(0xffffffffu, ov[0], o);
-      ov[1] += __shfl_xor_sync(0xffffffffu, ov[1], o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      atomicAdd(&a.sums[0], (unsigned long long)ov[0]);
-      if (ov[1]) atomicAdd(&a.sums[1], (unsigned long long)ov[1]);
-    }
+    const long long c = warp_sum_words(ov);
+    if ((threadIdx.x & 7) == 0 && c) atomicAdd(&a.sums[(threadIdx.x & 31) >> 3], (unsigned long long)c);
   } else {
     const float *src[2] = {a.in_a, a.in_b};
     for (int v0 = 0; v0 < nvec; v0 += kBatch * nt) {

@@ -55,15 +55,14 @@ struct FftStageArgs {
   float *phi;             // optional [H][W] potential spectrum
   // Stage 0 straight from the fixed-point density map (the finalise fused
   // in): with dens set, the stage reads the map instead of in_a, forms
-  // rho = d - c0, clears the map for the next iteration, and adds the two
-  // sums of the overlap (density.rs:79-86: sum d and sum max(d - cap, 0)) in
-  // fixed point to sums[].  Stage 1, with sums set, has one more CTA, which
-  // forms the overlap, writes sc->overlap and the iteration's log entry, and
-  // adds the last step's norms up: neither holds the transform up.
+  // rho = d - c0, clears the map for the next iteration, and adds its bins to
+  // the overlap's sums[] (count_bin).  Stage 1, with sums set, has one more
+  // CTA, which forms the overlap, writes sc->overlap and the iteration's log
+  // entry, and adds the last step's norms up: neither holds the transform up.
   unsigned long long *dens;
-  unsigned long long cap;
+  long long cap;          // fixed_capacity
   double c0;
-  unsigned long long *sums;  // [2], zero between iterations
+  unsigned long long *sums;  // [kOverlapWords], zero between iterations
   DevScalars *sc;
   IterLog *log;
   NormArgs norms;

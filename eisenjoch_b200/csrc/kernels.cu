@@ -409,45 +409,9 @@ __global__ void __launch_bounds__(kScatterBlock) k_scatter(const ScatterArgs a) 
   }
 }
 
-// The two sums of the overlap (density.rs:79-86) over the CTA, in fixed point:
-// whole numbers, so their order is free.  Valid in thread 0.
-__device__ __forceinline__ void block_sum_fix(long long (&v)[2], long long *smem /* [2 * warps] */) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v[0] += __shfl_down_sync(kFull, v[0], o);
-    v[1] += __shfl_down_sync(kFull, v[1], o);
-  }
-  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    smem[2 * w] = v[0];
-    smem[2 * w + 1] = v[1];
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    const int l = threadIdx.x;
-    v[0] = l < nw ? smem[2 * l] : 0;
-    v[1] = l < nw ? smem[2 * l + 1] : 0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      v[0] += __shfl_down_sync(kFull, v[0], o);
-      v[1] += __shfl_down_sync(kFull, v[1], o);
-    }
-  }
-}
-
-// compute_overlap of the two sums.
-__device__ __forceinline__ double overlap_of(unsigned long long sum, unsigned long long over) {
-  return sum == 0 ? 0.0 : from_fix(over) / from_fix(sum);
-}
-
-__device__ __forceinline__ void count_bin(unsigned long long q, unsigned long long cap, long long (&v)[2]) {
-  v[0] += (long long)q;
-  v[1] += q > cap ? (long long)(q - cap) : 0;
-}
-
 // Streams the map once (8 bytes read and zeroed, the outputs written), four
 // bins per thread and step, 16-byte accesses where the buffers allow it.  The
-// overlap's sums are whole numbers, so each CTA adds its two with atomics and
+// overlap's sums are whole numbers, so each CTA adds its own with atomics and
 // the last one forms the quotient (FP64 partial sums, which the last CTA read
 // back and added in a fixed order, held the kernel up after its last bin).
 // The launch overlaps the end of the scatter before it (launch_density_final,
@@ -457,8 +421,8 @@ __device__ __forceinline__ void count_bin(unsigned long long q, unsigned long lo
 // A single CTA with the map in its shared memory was slower from 1,000 cells
 // on (2k cells 6.2 us, 8k 14 us).
 __global__ void __launch_bounds__(kFinalBlock) k_density_final(const FinalArgs a) {
-  __shared__ long long sm[2 * kFinalBlock / 32];
-  long long v[2] = {0, 0};
+  __shared__ long long sm[kOverlapWords * kFinalBlock / 32];
+  long long v[kOverlapWords] = {};
   // Groups of four consecutive bins per thread and step: 16-byte loads and
   // stores (when every pointer is aligned for them; a ragged tail, or
   // unaligned caller buffers, take the scalar loop below).
@@ -519,14 +483,20 @@ __global__ void __launch_bounds__(kFinalBlock) k_density_final(const FinalArgs a
     if (a.dens_out) a.dens_out[i] = d;
     count_bin(q, a.cap, v);
   }
-  block_sum_fix(v, sm);
-  if (threadIdx.x != 0) return;
-  atomicAdd(&a.sums[0], (unsigned long long)v[0]);
-  atomicAdd(&a.sums[1], (unsigned long long)v[1]);
+  const int lane = threadIdx.x & 31;
+  const long long c = warp_sum_words(v);
+  if ((lane & 7) == 0) sm[kOverlapWords * (threadIdx.x >> 5) + (lane >> 3)] = c;
+  __syncthreads();
+  if (threadIdx.x >= kOverlapWords) return;
+  long long t = 0;
+#pragma unroll
+  for (int w = 0; w < kFinalBlock / 32; ++w) t += sm[kOverlapWords * w + threadIdx.x];
+  if (t) atomicAdd(&a.sums[threadIdx.x], (unsigned long long)t);
   __threadfence();
-  if (atomicAdd(a.ticket, 1u) != (unsigned)nblocks - 1) return;
+  __syncwarp((1u << kOverlapWords) - 1u);
+  if (threadIdx.x != 0 || atomicAdd(a.ticket, 1u) != (unsigned)nblocks - 1) return;
   __threadfence();
-  const double ov = overlap_of(atomicExch(&a.sums[0], 0ull), atomicExch(&a.sums[1], 0ull));
+  const double ov = take_overlap(a.sums);
   if (a.overlap) {
     *a.overlap = ov;
   } else {

@@ -61,6 +61,53 @@ __device__ __forceinline__ void finish_norms(const NormArgs &a) {
 }
 #endif
 
+// The overlap (density.rs:79-86) from the fixed-point map: the sum of d and of
+// max(d - cap, 0) over all bins, each in two 64-bit words, whole sites and
+// 2^-32 sites: {sum, sum's fraction, over, over's fraction}.  A bin holds less
+// than 2^31 sites, but all bins together may hold more, and one 64-bit word of
+// 2^-32 sites wraps there.  Whole numbers: their order is free.
+constexpr int kOverlapWords = 4;
+
+// A bin's capacity in the map's unit; no bin reaches one of 2^31 sites and more.
+inline long long fixed_capacity(long long sites) { return sites < (1ll << 31) ? sites << 32 : 0x7fffffffffffffffll; }
+
+#ifdef __CUDACC__
+__device__ __forceinline__ void count_bin(unsigned long long q, long long cap, long long (&v)[kOverlapWords]) {
+  const long long d = (long long)q, over = d > cap ? d - cap : 0;
+  v[0] += d >> 32;
+  v[1] += (unsigned)d;
+  v[2] += over >> 32;
+  v[3] += (unsigned)over;
+}
+
+// The warp's four sums: lanes 8 k .. 8 k + 7 get sum k.  Each exchange halves
+// the sums that a lane carries, 4 -> 2 -> 1.
+__device__ __forceinline__ long long warp_sum_words(const long long (&v)[kOverlapWords]) {
+  const bool up = threadIdx.x & 16, up2 = threadIdx.x & 8;
+  long long a = up ? v[2] : v[0], b = up ? v[3] : v[1];
+  a += __shfl_xor_sync(0xffffffffu, up ? v[0] : v[2], 16);
+  b += __shfl_xor_sync(0xffffffffu, up ? v[1] : v[3], 16);
+  long long c = up2 ? b : a;
+  c += __shfl_xor_sync(0xffffffffu, up2 ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  return c;
+}
+
+// compute_overlap of the sums, which are zero again (one thread).
+__device__ __forceinline__ double take_overlap(unsigned long long *sums) {
+  long long w[kOverlapWords];
+#pragma unroll
+  for (int k = 0; k < kOverlapWords; ++k) w[k] = (long long)atomicExch(sums + k, 0ull);
+  // carried first, so that each sum is rounded once
+  const auto value = [](long long sites, long long frac) {
+    return (double)(sites + (frac >> 32)) + (double)(frac & 0xffffffffll) * (1.0 / 4294967296.0);
+  };
+  const double sum = value(w[0], w[1]);
+  return sum < 1e-30 ? 0.0 : value(w[2], w[3]) / sum;
+}
+#endif
+
 // A launch that, with `after`, may start before the kernel ahead of it in the
 // stream has ended (that kernel's griddepcontrol.wait keeps the order of the
 // data: every kernel of such a chain executes it in every thread that reads
@@ -146,14 +193,14 @@ struct ScatterArgs {
 struct FinalArgs {
   unsigned long long *dens;
   int nb;
-  unsigned long long cap;   // capacity per bin (sites per bin), fixed point
+  long long cap;            // capacity per bin (sites per bin), fixed_capacity
   double c0;                // constant removed before the transform
   float *rho;               // FP32 charge map (SIMT transform), or nullptr
   __nv_bfloat16 *rho_hi;    // BF16 hi/lo charge map (tensor-core transform), or nullptr
   __nv_bfloat16 *rho_lo;
   double *dens_out;         // optional FP64 copy (stage entry)
   int vec4;                 // set by launch_density_final: every pointer allows 16-byte groups
-  unsigned long long *sums; // [2] sum of d, sum of max(d - cap, 0); zero between launches
+  unsigned long long *sums; // [kOverlapWords], zero between launches
   unsigned *ticket;
   double *overlap;          // where the overlap goes, or nullptr: into sc and the log
   DevScalars *sc;

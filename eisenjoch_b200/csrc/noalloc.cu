@@ -33,7 +33,7 @@ constexpr size_t kNoAllocMaxBins = 512 * 512;
 
 // Layout of the scratch array (byte offsets, each 256-aligned):
 //   [0, kMapBytes)                fixed-point bin map, must start at zero
-//   [kSumOff, +256)               the overlap's two sums, must start at zero
+//   [kSumOff, +256)               the overlap's sums, must start at zero
 //   [kTicketOff, +256)            completion counter, must start at zero
 constexpr size_t kMapBytes = kNoAllocMaxBins * sizeof(unsigned long long);
 constexpr size_t kSumOff = kMapBytes;
@@ -144,7 +144,7 @@ extern "C" eplace_status eplace_density_noalloc(const float *pos_xy, const float
                 nullptr, 0u, num_cells, bins_x, bins_y, sx, sy, nullptr};
   FinalArgs f{};
   f.nb = nb;
-  f.cap = (unsigned long long)sx * (unsigned long long)sy << 32;
+  f.cap = fixed_capacity((long long)sx * sy);
   f.dens_out = density;
   f.overlap = overlap;
   void *base = nullptr;

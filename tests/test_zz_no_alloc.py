@@ -183,3 +183,60 @@ def test_density_noalloc_shapes(cells, w, h, bx, by, half):
         assert st == _abi.EPLACE_OK
         assert np.abs(got - want).max() <= 1e-6 * want.max()
         assert abs(ov - over) <= 1e-6
+
+
+def _axis(c, e, s, n):  # [cells, n] lengths of [c - e, c + e] in n bins of s sites
+    lo, hi = c.astype(np.float64) - e, c.astype(np.float64) + e
+    k = np.arange(n)
+    return np.maximum(np.minimum(hi[:, None], (k + 1) * s) - np.maximum(lo[:, None], k * s), 0.0)
+
+
+@pytest.mark.parametrize("cells,side,bins,extent", [
+    (200, 4096, 512, 2000.0),     # 2^31 sites and more of footprints in all, a bin far below
+    (900, 4096, 512, 2000.0),     # 2^32 and more
+    (3, 16384, 1, 8192.0),        # one bin of 2^28 sites, three times over
+    (5, 46341, 1, 700.0),         # bins of 2^31 sites and of 2^32: cells fill little of them
+    (5, 65536, 1, 700.0),
+    (5, 131072, 2, 700.0),
+])
+def test_density_noalloc_large_areas(cells, side, bins, extent):
+    """Areas beyond 2^31 sites, in all bins together or as a bin's capacity:
+    bins and overlap within 1e-6 as for small ones."""
+    import torch
+
+    dev = torch.device("cuda:0")
+    torch.cuda.set_device(dev)
+    rng = np.random.default_rng(cells)
+    nl = E.Netlist(num_cells=cells, net_offsets=np.zeros(1, np.uint32), pin_cell=np.zeros(0, np.uint32))
+    chip = E.Chip(side, side, bins, bins)
+    x, y = rng.uniform(0.45 * side, 0.55 * side, (2, cells)).astype(np.float32)
+    hf = np.full((cells, 2), extent, np.float32)
+    half_d = torch.from_numpy(hf).to(dev)
+    dens_d = torch.full((bins, bins), -1.0, dtype=torch.float64, device=dev)
+    ov_d = torch.full((1,), -1.0, dtype=torch.float64, device=dev)
+    s = side // bins
+    want = _axis(y, hf[:, 1], s, bins).T @ _axis(x, hf[:, 0], s, bins)
+    over = np.maximum(want - float(s) * s, 0).sum() / want.sum()
+    assert want.max() < 2.0 ** 31  # what a bin holds
+    st, got, ov = _noalloc(torch, nl, chip, x, y, half_d, dens_d, ov_d)
+    assert st == _abi.EPLACE_OK
+    assert np.abs(got - want).max() <= 1e-6 * want.max()
+    assert abs(ov - over) <= 1e-6
+
+
+def test_density_stage_large_areas():
+    """The same through the regular density entry: 60,000 macros of 255 x 255
+    sites, 3.4e9 sites of footprints in all."""
+    n, side, bins = 60000, 4096, 256
+    rng = np.random.default_rng(1)
+    w = np.full(n, 255, np.uint8)
+    nl = E.Netlist(num_cells=n, net_offsets=np.zeros(1, np.uint32), pin_cell=np.zeros(0, np.uint32), cell_w=w, cell_h=w)
+    x, y = rng.uniform(0.1 * side, 0.9 * side, (2, n)).astype(np.float32)
+    half = np.full(n, 127.5)
+    s = side // bins
+    want = _axis(y, half, s, bins).T @ _axis(x, half, s, bins)
+    over = np.maximum(want - float(s) * s, 0).sum() / want.sum()
+    with E.PlacementContext(nl, E.Chip(side, side, bins, bins)) as ctx:
+        got, ov = ctx.density(x, y)
+    assert np.abs(got - want).max() <= 1e-6 * want.max()
+    assert abs(ov - over) <= 1e-6
