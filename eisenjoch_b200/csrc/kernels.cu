@@ -1362,7 +1362,8 @@ __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
     });
     // One cell at a time, the next one's state on the way (a macro's is loaded
     // for nothing: its flag arrives with it).
-    CellIn c = load_in(a, min(tid0, a.N - 1), was_init);
+    CellIn c{};
+    if (tid0 < a.N) c = load_in(a, tid0, was_init);
 #pragma unroll 1
     for (uint32_t i = tid0; i < a.N; i += gstride) {
       const bool unit = !a.mflag || !a.mflag[i];

@@ -103,3 +103,26 @@ def test_scatter_of_cells_piled_up_in_a_bin(n, side, bins, macros, it):
         d, ov = ctx.density(look(now.x, before.x), look(now.y, before.y))
     got = next(t["overlap"] for t in after.trajectory if t["iter"] == it + 1)
     assert abs(got - ov) <= 1e-12
+
+
+@pytest.mark.parametrize("it,lam", [(0, 0.0), (0, 2.5), (5, 2.5)])
+def test_entries_on_an_empty_design(it, lam):
+    """No movable cell: every stage entry takes it, and reads no cell."""
+    nl = E.Netlist(num_cells=0, net_offsets=np.array([0, 2], np.uint32), pin_cell=np.array([0, 1], np.uint32),
+                   fixed_x=np.array([3, 20], np.int32), fixed_y=np.array([5, 9], np.int32))
+    chip = E.Chip(32, 32)
+    z = np.zeros(0, np.float32)
+    rng = np.random.default_rng(0)
+    ex, ey = rng.normal(0, 1, (2, 32, 32)).astype(np.float32)
+    with E.PlacementContext(nl, chip) as ctx:
+        state = {k: z for k in ("x", "y", "x_prev", "y_prev", "gprev_x", "gprev_y")}
+        scal = [lam, float(lam > 0), 0.1, 0.2]
+        nx, ny, ax, ay, lx, ly = ctx.step(it, z, z, z, z, ex, ey, state, scal)
+        assert nx == 0.0 and ny == 0.0 and ax == 0.1 and ay == 0.2 and len(lx) == len(ly) == 0
+        gx, gy = ctx.gather(z, z, ex, ey)
+        wx, wy = ctx.wa_grad(z, z)
+        assert len(gx) == len(gy) == len(wx) == len(wy) == 0
+        d, ov = ctx.density(z, z)
+        assert not d.any() and ov == 0.0
+        sx, sy, disp, _ = ctx.legalize_device(z, z)
+        assert len(sx) == len(sy) == 0 and disp == 0.0
