@@ -235,7 +235,9 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(const FftStageArgs a) {
         const size_t g = vec_at(v < nvec ? v : 0, l, n);
 #pragma unroll
         for (int r = 0; r < kArrays; ++r)
-          q[r][u] = v < nvec ? __ldg(reinterpret_cast<const float4 *>(src[r] + g)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          // (a plain load: the stage before may still be writing these while
+          // this one runs, so they aren't read-only data of this kernel)
+          q[r][u] = v < nvec ? *reinterpret_cast<const float4 *>(src[r] + g) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) {

@@ -46,7 +46,7 @@ __device__ __forceinline__ void finish_norms(const NormArgs &a) {
   if (it < 0 || a.sc->err) return;
   double x = 0.0, y = 0.0;
   for (int b = threadIdx.x & 31; b < a.blocks; b += 32) {
-    const double2 p = __ldcg(reinterpret_cast<const double2 *>(a.part2) + b);
+    const double2 p = reinterpret_cast<const double2 *>(a.part2)[b];
     x += p.x;
     y += p.y;
   }
