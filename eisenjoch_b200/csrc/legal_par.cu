@@ -593,6 +593,18 @@ __device__ __forceinline__ int32_t claim_site(const LpArgs &a, int32_t q, int x,
   return held;
 }
 
+// The same by a warp, whose lanes read the displaced cell's list next: its
+// writer's fence and claim are paired with a fence here (claims are relaxed).
+__device__ __forceinline__ int32_t claim_and_acquire(const LpArgs &a, int32_t q, int x, int y, int lane) {
+  int32_t held = 0;
+  if (lane == 0) {
+    held = claim_site(a, q, x, y);
+    if (held > q && held != kNone) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  }
+  __syncwarp();
+  return __shfl_sync(kFull, held, 0);
+}
+
 // First all unit cells at once, a warp each: the best open site near the
 // target, claimed.  A cell that finds none, or is displaced by an earlier one
 // that was under way at the same time, is left over: the answer doesn't depend
@@ -916,7 +928,6 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
     if (warp == 0) {  // while one warp can tell
       int32_t q = next;
       while (q >= 0) {
-        int32_t held = 0;
         double c0 = 0.0;
         float2 p;
         if (listed) {
@@ -930,8 +941,7 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
             const int l0 = __ffs(open) - 1;
             px = __shfl_sync(kFull, x, l0);
             py = __shfl_sync(kFull, y, l0);
-            if (lane == 0) held = claim_site(a, q, px, py);
-            held = __shfl_sync(kFull, held, 0);
+            const int32_t held = claim_and_acquire(a, q, px, py, lane);
             if (held == kNone) q = -1;
             else if (held > q) q = held;
             continue;  // (an earlier cell was faster: the list again)
@@ -954,8 +964,7 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
           if (b.cost < 6.25) {
             px = b.tile % a.W;
             py = b.tile / a.W;
-            if (lane == 0) held = claim_site(a, q, px, py);
-            held = __shfl_sync(kFull, held, 0);
+            const int32_t held = claim_and_acquire(a, q, px, py, lane);
             if (held == kNone) {
               q = -1;
             } else if (held > q) {
@@ -1026,14 +1035,12 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
             some && e.tile != kNone ? e.tile : lane == 0 && !some ? b.tile : -1;
       px = b.tile % a.W;
       py = b.tile / a.W;
-      int32_t held = 0;
       __syncwarp();
       if (lane == 0) {
         put_hint(a, q, c, b.cost);
         __threadfence();  // the list before the claim: who displaces q reads it
-        held = claim_site(a, q, px, py);
       }
-      held = __shfl_sync(kFull, held, 0);
+      const int32_t held = claim_and_acquire(a, q, px, py, lane);
       next = held == kNone ? -1 : held > q ? held : q;
       listed = true;
     }

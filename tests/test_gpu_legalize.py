@@ -299,3 +299,20 @@ def test_device_legalizer_refuses_targets_without_a_site(cells, bad):
         hx, hy, hd = ctx.legalize(x, y)
         gx, gy, gd, _ = ctx.legalize_device(x, y)
         assert np.array_equal(gx, hx) and np.array_equal(gy, hy) and gd == hd
+
+
+@pytest.mark.parametrize("n,piles", [(3000, 1), (15000, 3), (30000, 1), (30000, 8)])
+def test_device_legalizer_long_chains(n, piles):
+    """Piles whose cells displace one another in long chains, each displaced
+    cell going by the list that another CTA wrote: the same binding every time."""
+    rng = np.random.default_rng(n + piles)
+    side = 256
+    nl = E.Netlist(num_cells=n, net_offsets=np.array([0, 2], np.uint32), pin_cell=np.array([0, 1], np.uint32))
+    k = rng.integers(0, piles, n)
+    c = rng.uniform(0.3 * side, 0.7 * side, (2, piles))
+    x, y = np.clip(c[:, k] + rng.normal(0, 1.5, (2, n)), 0, side - 1).astype(np.float32)
+    with E.PlacementContext(nl, E.Chip(side, side)) as ctx:
+        hx, hy, hd = ctx.legalize(x, y)
+        for _ in range(3):
+            gx, gy, gd, _ = ctx.legalize_device(x, y)
+            assert np.array_equal(gx, hx) and np.array_equal(gy, hy) and gd == hd
