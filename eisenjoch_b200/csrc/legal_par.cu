@@ -57,7 +57,10 @@ constexpr int kLpWarps = 16;           // warps per CTA of the macro kernels (a 
 
 __device__ __forceinline__ double sq(double d) { return __dmul_rn(d, d); }
 
-// own[] and seg[] change under the readers: L2 loads, never kept in L1.
+// own[] and seg[] change under the readers: L2 loads, never kept in L1.  A
+// segment's two words change in an order that its readers rely on, so where
+// they are read while they change, every access is of the 64-bit pair: those to
+// one location keep their order.
 __device__ __forceinline__ int32_t ld_own(const int32_t *p) {
   int32_t v;
   asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -67,6 +70,20 @@ __device__ __forceinline__ uint2 ld_seg(const uint2 *p) {
   unsigned long long v;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return make_uint2((unsigned)v, (unsigned)(v >> 32));
+}
+// Clears a bit of the first word and raises the second, as a signed number, to
+// q, in one; s: what the pair was at some time.  (Bits only go, so one that is
+// clear in s has gone; ends, since a pair that changed under it has fewer bits
+// or a higher second word.)
+__device__ __forceinline__ void take_bit(uint2 *p, uint2 s, unsigned bit, int32_t q) {
+  while (s.x & bit) {
+    const unsigned y = (unsigned)max((int32_t)s.y, q);
+    const unsigned long long was = ((unsigned long long)s.y << 32) | s.x;
+    const unsigned long long is = atomicCAS(reinterpret_cast<unsigned long long *>(p), was,
+                                            ((unsigned long long)y << 32) | (s.x & ~bit));
+    if (is == was) break;
+    s = make_uint2((unsigned)is, (unsigned)(is >> 32));
+  }
 }
 // Bit b set: site b of the segment has a claim of q or later, or none; only
 // the groups of four sites with a bit in `ask` are looked at.
@@ -451,7 +468,7 @@ __global__ void __launch_bounds__(kLpWarps * 32) k_lp_choose(const LpArgs a) {
             int32_t *o = own_at(a, x, y);
             if (ld_own(o) == q) {  // nobody else writes a site that q holds
               *o = kNone;
-              atomicAnd(&seg_at(a, x, y)->y, ~(1u << (x & 31)));
+              atomicAnd(reinterpret_cast<unsigned long long *>(seg_at(a, x, y)), ~(1ull << (32 + (x & 31))));
             }
           }
         }
@@ -556,8 +573,7 @@ __global__ void __launch_bounds__(kLpWarps * 32) k_lp_claim(const LpArgs a) {
 
 // seg[] while the unit cells are placed: x has a bit for each site that
 // nobody has claimed yet (cleared after the claim, so a bit may be late), y
-// the largest order index that ever claimed a free site of the segment
-// (raised before the claim's bit goes).  A segment with x == 0 and y < q has
+// the largest order index that cleared one of them.  A segment with x == 0 and y < q has
 // no site open to q; with y < q the bits of x are the open sites.
 __global__ void __launch_bounds__(256) k_lp_segments(const LpArgs a) {
   const int lane = threadIdx.x & 31;
@@ -570,35 +586,49 @@ __global__ void __launch_bounds__(256) k_lp_segments(const LpArgs a) {
 
 // Search of the sites around unit cell q's target by one warp: the 5 x 5 sites
 // around the nearest one, a lane each.  A site outside costs at least 2.5^2,
-// so a cheaper one inside is the answer.
-__device__ Best search_near(const LpArgs &a, int32_t q, const Cell &c, int lane) {
+// so a cheaper one inside is the answer.  seen: the answer's segment, if asked for.
+__device__ __forceinline__ Best search_near(const LpArgs &a, int32_t q, const Cell &c, int lane, uint2 *seen) {
   Best b = no_best();
-  if (lane < 25) {
-    const int x = c.cx - 2 + lane % 5, y = c.cy - 2 + lane / 5;
-    if (x >= 0 && x < a.W && y >= 0 && y < a.H && ld_own(own_at(a, x, y)) > q)
-      b.take(__dadd_rn(col_dx2(c, x), row_dy2(c, y)), y * a.W + x);
+  const int x = c.cx - 2 + lane % 5, y = c.cy - 2 + lane / 5;
+  uint2 s = make_uint2(0u, 0u);
+  if (lane < 25 && x >= 0 && x < a.W && y >= 0 && y < a.H) {
+    const int32_t held = ld_own(own_at(a, x, y));
+    if (seen) s = ld_seg(seg_at(a, x, y));
+    if (held > q) b.take(__dadd_rn(col_dx2(c, x), row_dy2(c, y)), y * a.W + x);
   }
-  return b.warp_min();
+  const Best all = b.warp_min();
+  if (seen) {
+    const int l = __ffs(__ballot_sync(kFull, b.tile == all.tile)) - 1;  // (any lane where there is none)
+    *seen = make_uint2(__shfl_sync(kFull, s.x, l), __shfl_sync(kFull, s.y, l));
+  }
+  return all;
 }
 
 // Claims site (x, y) for q (one thread): kNone: it was free; a later cell: q
 // has it now, and that cell has lost it; an earlier cell: q did not get it.
-__device__ __forceinline__ int32_t claim_site(const LpArgs &a, int32_t q, int x, int y) {
+// The first to claim it takes its bit, or whoever meets a bit that is late;
+// the site's holder is never later than the one that took the bit.  (The two
+// atomics are under way together: whichever is first, the claim will stand.)
+// seen: the segment as it was at some time; nullptr while nobody reads any.
+__device__ __forceinline__ int32_t claim_site(const LpArgs &a, int32_t q, int x, int y, const uint2 *seen) {
   uint2 *s = seg_at(a, x, y);
-  const int32_t top = atomicMax(reinterpret_cast<int32_t *>(&s->y), q);
+  const unsigned bit = 1u << (x & 31);
   const int32_t held = atomicMin(own_at(a, x, y), q);
-  // the bit goes after both answers are here; one that lost the site clears
-  // it too, so that it does not meet a late bit again
-  if ((held == kNone || held < q) && top != kNone) atomicAnd(&s->x, ~(1u << (x & 31)));
+  if (seen) {
+    take_bit(s, *seen, bit, q);
+  } else if (held == kNone || held < q) {
+    atomicMax(reinterpret_cast<int32_t *>(&s->y), q);
+    atomicAnd(&s->x, ~bit);
+  }
   return held;
 }
 
 // The same by a warp, whose lanes read the displaced cell's list next: its
 // writer's fence and claim are paired with a fence here (claims are relaxed).
-__device__ __forceinline__ int32_t claim_and_acquire(const LpArgs &a, int32_t q, int x, int y, int lane) {
+__device__ __forceinline__ int32_t claim_and_acquire(const LpArgs &a, int32_t q, int x, int y, uint2 seen, int lane) {
   int32_t held = 0;
   if (lane == 0) {
-    held = claim_site(a, q, x, y);
+    held = claim_site(a, q, x, y, &seen);
     if (held > q && held != kNone) asm volatile("fence.acq_rel.gpu;" ::: "memory");
   }
   __syncwarp();
@@ -630,10 +660,10 @@ __global__ void __launch_bounds__(256) k_lp_near(const LpArgs a) {
   const Cell c = load_cell(a, (uint32_t)q, true);
   int32_t site = -1;
   for (int k = 0; k < kNearTries && placeable(c); ++k) {
-    const Best b = search_near(a, q, c, lane);
+    const Best b = search_near(a, q, c, lane, nullptr);
     if (!(b.cost < 6.25)) break;
     int32_t held = 0;
-    if (lane == 0) held = claim_site(a, q, b.tile % a.W, b.tile / a.W);
+    if (lane == 0) held = claim_site(a, q, b.tile % a.W, b.tile / a.W, nullptr);
     held = __shfl_sync(kFull, held, 0);
     if (held > q) {  // (kNone too)
       site = b.tile;
@@ -936,12 +966,15 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
           const unsigned ends = __ballot_sync(kFull, t < 0);  // the list ends at its first -1
           const int len = __ffs(ends) - 1;
           const int x = t % a.W, y = t / a.W;
-          const unsigned open = __ballot_sync(kFull, lane < len && ld_own(own_at(a, x, y)) > q);
+          const int32_t on = lane < len ? ld_own(own_at(a, x, y)) : -1;
+          const uint2 s = lane < len ? ld_seg(seg_at(a, x, y)) : make_uint2(0u, 0u);
+          const unsigned open = __ballot_sync(kFull, on > q);
           if (open) {
             const int l0 = __ffs(open) - 1;
             px = __shfl_sync(kFull, x, l0);
             py = __shfl_sync(kFull, y, l0);
-            const int32_t held = claim_and_acquire(a, q, px, py, lane);
+            const uint2 seen = make_uint2(__shfl_sync(kFull, s.x, l0), __shfl_sync(kFull, s.y, l0));
+            const int32_t held = claim_and_acquire(a, q, px, py, seen, lane);
             if (held == kNone) q = -1;
             else if (held > q) q = held;
             continue;  // (an earlier cell was faster: the list again)
@@ -960,11 +993,12 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
         listed = false;
         const Cell c = make_cell(a, p, one);
         if (c0 < 6.25 && placeable(c)) {
-          const Best b = search_near(a, q, c, lane);
+          uint2 seen;
+          const Best b = search_near(a, q, c, lane, &seen);
           if (b.cost < 6.25) {
             px = b.tile % a.W;
             py = b.tile / a.W;
-            const int32_t held = claim_and_acquire(a, q, px, py, lane);
+            const int32_t held = claim_and_acquire(a, q, px, py, seen, lane);
             if (held == kNone) {
               q = -1;
             } else if (held > q) {
@@ -1009,6 +1043,9 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
     list_ring(a, q, c, b.cost, warp, lane, slist, &scount);
     __syncthreads();
     if (warp == 0) {
+      px = b.tile % a.W;
+      py = b.tile / a.W;
+      const uint2 seen = ld_seg(seg_at(a, px, py));
       const int n = scount;
       const bool keep = n <= kLpRingMax;
       // the cheapest 32 or fewer: the ring (below 2^26) halved until they are
@@ -1033,14 +1070,12 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
       if (lane < kLpCand)
         a.cand[(size_t)kLpCand * (q - (int32_t)a.n_mac) + lane] =
             some && e.tile != kNone ? e.tile : lane == 0 && !some ? b.tile : -1;
-      px = b.tile % a.W;
-      py = b.tile / a.W;
       __syncwarp();
       if (lane == 0) {
         put_hint(a, q, c, b.cost);
         __threadfence();  // the list before the claim: who displaces q reads it
       }
-      const int32_t held = claim_and_acquire(a, q, px, py, lane);
+      const int32_t held = claim_and_acquire(a, q, px, py, seen, lane);
       next = held == kNone ? -1 : held > q ? held : q;
       listed = true;
     }
