@@ -387,6 +387,10 @@ __device__ __forceinline__ void scatter_all(const ScatterArgs &a, unsigned long 
 __global__ void __launch_bounds__(kScatterBlock) k_scatter(const ScatterArgs a) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x, ts = gridDim.x * blockDim.x;
+  if (a.sums) {
+    if (t0 < kOverlapWords) a.sums[t0] = 0ull;
+    if (t0 == 0) *a.ticket = 0u;
+  }
   if (a.half && !a.mflag) {
     scatter_all(a, a.dens, t0, ts);
     return;

@@ -188,6 +188,8 @@ struct ScatterArgs {
   int BX, BY;
   int isx, isy;              // sites per bin along x / y
   unsigned long long *dens; // [BY * BX] fixed point
+  unsigned long long *sums = nullptr;  // of the finalise behind it: cleared here, with its ticket
+  unsigned *ticket = nullptr;
 };
 
 struct FinalArgs {

@@ -33,8 +33,8 @@ constexpr size_t kNoAllocMaxBins = 512 * 512;
 
 // Layout of the scratch array (byte offsets, each 256-aligned):
 //   [0, kMapBytes)                fixed-point bin map, must start at zero
-//   [kSumOff, +256)               the overlap's sums, must start at zero
-//   [kTicketOff, +256)            completion counter, must start at zero
+//   [kSumOff, +256)               the overlap's sums, cleared by each call
+//   [kTicketOff, +256)            completion counter, cleared by each call
 constexpr size_t kMapBytes = kNoAllocMaxBins * sizeof(unsigned long long);
 constexpr size_t kSumOff = kMapBytes;
 constexpr size_t kTicketOff = kSumOff + 256;
@@ -157,18 +157,20 @@ extern "C" eplace_status eplace_density_noalloc(const float *pos_xy, const float
   a.dens = f.dens = map;
   f.sums = reinterpret_cast<unsigned long long *>(b + kSumOff);
   f.ticket = reinterpret_cast<unsigned *>(b + kTicketOff);
-  // The scratch keeps the previous call's contents.  It starts at zero and a
-  // completed call leaves it at zero (the finalise zeroes every bin that it
-  // reads, the sums and the counter); after a call whose second launch failed
-  // it is cleared first.
+  // The scratch keeps the previous call's contents.  Its map starts at zero and
+  // is zero again when every call has run (a call's finalise zeroes every bin
+  // that its scatter may have added to); after a call whose second launch
+  // failed it is cleared first.  Sums and counter are cleared by the scatter:
+  // calls that overlapped by mistake may leave them anyhow.
   if (dirty && (cudaMemsetAsync(base, 0, kScratchBytes, s) != cudaSuccess)) return EPLACE_ERR_CUDA;
-  if (num_cells) {
+  if (!num_cells) {
+    if (cudaMemsetAsync(f.sums, 0, kScratchBytes - kSumOff, s) != cudaSuccess) return EPLACE_ERR_CUDA;
+  } else {
+    a.sums = f.sums;
+    a.ticket = f.ticket;
     long long g = ((long long)num_cells + kScatterBlock - 1) / kScatterBlock;
     if (g > (long long)sms * 16) g = (long long)sms * 16;
-    if (launch_scatter(a, (int)g, s) != cudaSuccess) {
-      scratch_state(dirty);
-      return EPLACE_ERR_CUDA;
-    }
+    if (launch_scatter(a, (int)g, s) != cudaSuccess) return EPLACE_ERR_CUDA;
   }
   long long fg = ((long long)nb / 4 + kFinalBlock - 1) / kFinalBlock;
   if (fg > (long long)sms * 4) fg = (long long)sms * 4;

@@ -339,7 +339,8 @@ eplace_status eplace_pin_weights(const eplace_netlist *nl, const eplace_chip *ch
  * array's device address up in the current context; make that first call
  * before any stream capture.  All calls share the one array: calls that
  * overlap on the GPU (other streams, other threads) race, so serialise
- * them.  Nothing is allocated or freed. */
+ * them; the results of calls that did overlap are undefined, those of calls
+ * after them are not affected.  Nothing is allocated or freed. */
 eplace_status eplace_density_noalloc(const float *pos_xy, const float *half_wh,
                                      uint32_t num_cells, int32_t width, int32_t height,
                                      int32_t bins_x, int32_t bins_y, double *density,

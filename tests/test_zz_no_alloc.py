@@ -240,3 +240,41 @@ def test_density_stage_large_areas():
         got, ov = ctx.density(x, y)
     assert np.abs(got - want).max() <= 1e-6 * want.max()
     assert abs(ov - over) <= 1e-6
+
+
+def test_density_noalloc_after_overlapping_calls():
+    """Calls that overlap on the GPU spoil each other's results, but no later
+    call's: the next ones are right, map and overlap."""
+    import torch
+
+    L = _abi.lib()
+    dev = torch.device("cuda:0")
+    torch.cuda.set_device(dev)
+    torch.cuda.synchronize(dev)
+    rng = np.random.default_rng(4)
+    streams = [torch.cuda.Stream(dev) for _ in range(3)]
+    work = []
+    for k, (cells, side, bins) in enumerate(((150000, 1024, 512), (2000, 128, 64), (0, 96, 96))):
+        nl = E.Netlist(num_cells=cells, net_offsets=np.zeros(1, np.uint32), pin_cell=np.zeros(0, np.uint32))
+        x, y = rng.uniform(0, side - 1, (2, cells)).astype(np.float32)
+        pos = torch.from_numpy(np.ascontiguousarray(np.stack([x, y], axis=1))).to(dev)
+        work.append((nl, E.Chip(side, side, bins, bins), x, y, pos,
+                     torch.zeros((bins, bins), dtype=torch.float64, device=dev),
+                     torch.zeros(1, dtype=torch.float64, device=dev)))
+    torch.cuda.synchronize(dev)
+    for _ in range(3):
+        for _ in range(200):
+            for s, (nl, chip, x, y, pos, dens, ov) in zip(streams, work):
+                st = L.eplace_density_noalloc(
+                    ctypes.c_void_p(pos.data_ptr() if nl.num_cells else 0), None, nl.num_cells, chip.width, chip.height,
+                    chip.bins_x, chip.bins_y, ctypes.c_void_p(dens.data_ptr()), ctypes.c_void_p(ov.data_ptr()),
+                    ctypes.c_void_p(s.cuda_stream))
+                assert st == _abi.EPLACE_OK
+        torch.cuda.synchronize(dev)
+        for nl, chip, x, y, pos, dens, ov in work:
+            ov.fill_(-1.0)
+            with E.PlacementContext(nl, chip) as ctx:
+                want, ref = ctx.density(x, y)
+            st, got, o = _noalloc(torch, nl, chip, x, y, None, dens, ov)
+            assert st == _abi.EPLACE_OK
+            assert np.array_equal(got, want) and abs(o - ref) <= 1e-12
