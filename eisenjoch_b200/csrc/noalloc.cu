@@ -162,7 +162,14 @@ extern "C" eplace_status eplace_density_noalloc(const float *pos_xy, const float
   // that its scatter may have added to); after a call whose second launch
   // failed it is cleared first.  Sums and counter are cleared by the scatter:
   // calls that overlapped by mistake may leave them anyhow.
-  if (dirty && (cudaMemsetAsync(base, 0, kScratchBytes, s) != cudaSuccess)) return EPLACE_ERR_CUDA;
+  const bool clear = dirty;
+  if (clear) {
+    // a clear that is captured into a graph has not run yet: the mark stays
+    cudaStreamCaptureStatus capture;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) return EPLACE_ERR_CUDA;
+    if (cudaMemsetAsync(base, 0, kScratchBytes, s) != cudaSuccess) return EPLACE_ERR_CUDA;
+    dirty = capture != cudaStreamCaptureStatusNone;
+  }
   if (!num_cells) {
     if (cudaMemsetAsync(f.sums, 0, kScratchBytes - kSumOff, s) != cudaSuccess) return EPLACE_ERR_CUDA;
   } else {
@@ -179,6 +186,6 @@ extern "C" eplace_status eplace_density_noalloc(const float *pos_xy, const float
     scratch_state(true);
     return EPLACE_ERR_CUDA;
   }
-  if (dirty) scratch_state(false);
+  if (clear) scratch_state(dirty);
   return EPLACE_OK;
 }
