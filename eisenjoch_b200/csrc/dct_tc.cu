@@ -131,6 +131,15 @@ struct Smem {
   static constexpr int TOTAL = STAGE_BYTES * STAGES + 1024 /* align */ + 256 /* barriers */;
 };
 
+// CTAs of the next product start while this one's may not have their tensor
+// memory yet, and hold theirs until this one has ended.  So all that shared
+// memory lets onto an SM at once must find room: columns in proportion to bytes
+// of shared memory stay below 512 columns to 228 KB, whatever the tile shapes.
+template <int BN, int STAGES>
+constexpr bool tmem_never_waits() {
+  return (size_t)BN * 228 * 1024 <= (size_t)512 * Smem<BN, STAGES>::TOTAL;
+}
+
 template <int BN, int STAGES>
 __global__ void __launch_bounds__(128, 1)
     k_tc_gemm(const __grid_constant__ TcGemmMaps maps, const TcGemmEpi epi, int M, int N, int K) {
@@ -332,6 +341,7 @@ template <int BN, int STAGES>
 cudaError_t launch_cfg(const TcGemmMaps &maps, const TcGemmEpi &epi, int nbatch, int M, int N, int K,
                        cudaStream_t s, bool after) {
   using S = Smem<BN, STAGES>;
+  static_assert(tmem_never_waits<BN, STAGES>(), "a CTA could wait for tensor memory held by one that waits for it");
   // The shared-memory opt-in is per device: set it once on each.
   static std::atomic<bool> attr[64];
   int dev = 0;
