@@ -226,6 +226,7 @@ __global__ void __launch_bounds__(128, 1)
     // MMA issuer: M = 128, N = BN, BF16 x BF16 -> FP32, both K-major.
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
                            ((uint32_t)(BM >> 4) << 24);
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the bound on the waits is for this kernel's loads alone
     bool ok = true;
     for (int kb = 0; kb < nk; ++kb) {
       const int s = kb % STAGES;
