@@ -213,6 +213,8 @@ struct PinBlock {
   void reserve(size_t need) {
     if (p && need <= bytes) return;
     PinArena::get().put(p, cls);
+    p = nullptr;  // given back: not ours any more if the next line throws
+    bytes = 0;
     p = PinArena::get().take(std::max<size_t>(need, 1), &cls);
     bytes = (size_t)1 << cls;
   }
