@@ -264,7 +264,9 @@ struct LegalSlot {
   DBuf<double> mcost;
   DBuf<LpFreed> freed;
   DBuf<uint32_t> work, queued, pend, left;
-  DBuf<unsigned long long> hint;
+  DBuf<unsigned long long> hint, tie_key;
+  DBuf<uint32_t> tie_count;
+  DBuf<int32_t> list;
   DBuf<LpState> lst;
   LpGraph graph;        // the whole legalisation: rounds in a device-side loop
   uint64_t gen = ~0ull;  // problem load this slot is prepared for
@@ -1434,6 +1436,10 @@ void prepare_slot(eplace_ctx *c, LegalSlot &L) {
   L.near.ensure(units);
   L.pend.ensure(units);
   L.left.ensure(lp_chunks(units));
+  const size_t ties = lp_tie_entries(units);
+  L.tie_key.ensure(ties);
+  L.tie_count.ensure(ties);
+  L.list.ensure((size_t)kUnitWindow * (kLpRingMax + 1));
   L.lst.ensure(1);
   std::vector<int2> floc(hp.F);
   for (uint32_t f = 0; f < hp.F; ++f) floc[f] = make_int2(hp.fx[f], hp.fy[f]);
@@ -1464,6 +1470,11 @@ void prepare_slot(eplace_ctx *c, LegalSlot &L) {
   a.near = L.near.p;
   a.pend = L.pend.p;
   a.left = L.left.p;
+  a.tie_key = L.tie_key.p;
+  a.tie_count = L.tie_count.p;
+  a.list = L.list.p;
+  a.list_len = L.list.p + (size_t)kUnitWindow * kLpRingMax;
+  a.tie_mask = (uint32_t)ties - 1;
   a.st = L.lst.p;
   a.sites = L.sites.p;
   a.loc = L.loc.p;
@@ -2719,7 +2730,8 @@ uint64_t eplace_ctx::device_bytes() const {
   add(B3gt_h); add(B3gt_l); add(L6g_h); add(L6g_l); add(lg_order); add(lg_fsize); add(lg_free0);
   for (const auto &l : lslots) {
     add(l->pos); add(l->sites); add(l->loc); add(l->cost); add(l->out); add(l->own); add(l->seg); add(l->choice);
-    add(l->mcost); add(l->freed); add(l->work); add(l->queued); add(l->hint); add(l->cand); add(l->near); add(l->pend); add(l->left); add(l->lst);
+    add(l->mcost); add(l->freed); add(l->work); add(l->queued); add(l->hint); add(l->cand); add(l->near); add(l->pend); add(l->left); add(l->tie_key); add(l->tie_count);
+    add(l->list); add(l->lst);
   }
   return b;
 }

@@ -16,7 +16,9 @@
 // held by a later cell, the CTA goes on with the cell it displaced; if an
 // earlier cell got there first, it looks again.  own[s] only ever falls, so
 // a site once closed to q stays closed: no waiting, no rounds, and every
-// lost or won claim lowers some own[s], so it ends.
+// lost or won claim lowers some own[s], so it ends.  (Where many unit cells have
+// one target they are placed in windows instead: lists against the map as it
+// stands, then each takes what the cells before it leave.  See k_lp_lists.)
 //
 // Macros (several sites per claim, and a macro that moves opens sites again)
 // reach their fixed point in rounds over a window of the next kLpWindow
@@ -38,9 +40,9 @@
 // A 200k-cell checkpoint (5 % macros, half of the cells in six piles): 150 to
 // 200 ms as rounds of candidate lists, disturbance passes and one CTA's serial
 // pass over the cells whose lists interact (a hundred rounds and more of 20
-// launches), 7.6 ms in this form (macros 2.8 ms in 54 rounds, units 4.9).  The
-// checkpoint at the end of such a run, cells spread: 1.3 ms (macros 0.7 in 17
-// rounds, units 0.2, the displacement's sum 0.24).
+// launches), 7.3 ms in this form (macros 2.2 ms in 54 rounds, units 4.7, the
+// displacement's sum 0.33).  The checkpoint at the end of such a run, cells
+// spread: 1.3 to 3 ms (macros 0.6, units 0.2 to 2.1 by the design, sum 0.26).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -402,6 +404,15 @@ __device__ Best search_any(const LpArgs &a, int32_t q, const Cell &c, int lane) 
   return b.warp_min();
 }
 
+// Targets in the same square of 1 / tie_scale sites have one key.
+constexpr unsigned long long kNoTie = 1ull << 63;  // none: the column of no target within 2^25 sites
+__device__ __forceinline__ unsigned long long tie_key(const LpArgs &a, float2 p) {
+  constexpr float kMost = 33554432.0f;  // 2^25 (farther ones find no site)
+  if (!(fabsf(p.x) < kMost && fabsf(p.y) < kMost)) return kNoTie;
+  return ((unsigned long long)(unsigned)(int)floorf(p.x * a.tie_scale) << 32) |
+         (unsigned)(int)floorf(p.y * a.tie_scale);
+}
+
 __global__ void __launch_bounds__(256) k_lp_init(const LpArgs a) {
   const int lane = threadIdx.x & 31;
   const int nseg = a.SW * a.H;
@@ -422,8 +433,12 @@ __global__ void __launch_bounds__(256) k_lp_init(const LpArgs a) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < hints; i += gridDim.x * blockDim.x) a.hint[i] = 0ull;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n - a.n_mac; i += gridDim.x * blockDim.x)
     a.cand[(size_t)kLpCand * i] = -1;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= a.tie_mask; i += gridDim.x * blockDim.x) {
+    a.tie_key[i] = kNoTie;
+    a.tie_count[i] = 0u;
+  }
   if (blockIdx.x == 0 && threadIdx.x == 0)
-    *a.st = LpState{0u, 0u, (uint32_t)kNone, 0u, 0u, {min(a.n_mac, kLpWindow), 0u}, 0u, 0u, 0};
+    *a.st = LpState{0u, 0u, (uint32_t)kNone, 0u, 0u, {min(a.n_mac, kLpWindow), 0u}, 0u, 0u, 0u, 0u, 0u, 0};
 }
 
 // A round, first half: each macro of the work list (whose choice may have
@@ -575,8 +590,35 @@ __global__ void __launch_bounds__(kLpWarps * 32) k_lp_claim(const LpArgs a) {
 // nobody has claimed yet (cleared after the claim, so a bit may be late), y
 // the largest order index that cleared one of them.  A segment with x == 0 and y < q has
 // no site open to q; with y < q the bits of x are the open sites.
+//
+// Counts the unit cells of each key (the table has twice as many entries or
+// more; a warp adds those of one key together), and those of the keys that have
+// tie_least or more; of the cells that k_lp_near left over, where it is tried.
+__device__ void count_tie(const LpArgs &a, uint32_t i, bool in) {  // a warp; in: unit cell i counts
+  const unsigned long long key = in ? tie_key(a, a.pos[a.order[a.n_mac + i]]) : kNoTie;
+  const unsigned same = __match_any_sync(kFull, key);
+  if (key == kNoTie || (int)(threadIdx.x & 31) != __ffs(same) - 1) return;
+  uint32_t h = (uint32_t)((key * 0x9e3779b97f4a7c15ull) >> 32) & a.tie_mask;
+  for (uint32_t k = 0; k <= a.tie_mask; ++k, h = (h + 1) & a.tie_mask) {
+    const unsigned long long was = atomicCAS(a.tie_key + h, kNoTie, key);
+    if (was != kNoTie && was != key) continue;
+    const uint32_t n = (uint32_t)__popc(same), had = atomicAdd(a.tie_count + h, n);
+    if (had + n < a.tie_least) return;
+    const uint32_t add = had >= a.tie_least ? n : had + n, ties = atomicAdd(&a.st->ties, add);
+    if (ties < a.tie_limit && ties + add >= a.tie_limit) {
+      a.st->tied = 1u;
+      cudaGraphSetConditional(a.windows, 1u);
+    }
+    return;
+  }
+}
+
 __global__ void __launch_bounds__(256) k_lp_segments(const LpArgs a) {
   const int lane = threadIdx.x & 31;
+  const uint32_t units = a.n - a.n_mac;
+  if (a.tie_limit)
+    for (uint32_t i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; i0 < units; i0 += gridDim.x * blockDim.x)
+      count_tie(a, i0 + lane, i0 + lane < units);
   const int nseg = a.SW * a.H;
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nseg; i += (gridDim.x * blockDim.x) >> 5) {
     const unsigned m = __ballot_sync(kFull, a.own[(size_t)32 * i + lane] == kNone);
@@ -686,7 +728,10 @@ __device__ __forceinline__ bool left_over(const LpArgs &a, uint32_t i) {
 // the result is no longer wanted; the status doesn't change in between.)
 __global__ void __launch_bounds__(kLpChunk) k_lp_count(const LpArgs a) {
   if (a.st->status != 0) return;
-  const int n = __syncthreads_count(left_over(a, blockIdx.x * kLpChunk + threadIdx.x));
+  const uint32_t i = blockIdx.x * kLpChunk + threadIdx.x;
+  const bool left = left_over(a, i);
+  if (__any_sync(kFull, left)) count_tie(a, i, left);
+  const int n = __syncthreads_count(left);
   if (threadIdx.x == 0) a.left[blockIdx.x] = (uint32_t)n;
 }
 __global__ void __launch_bounds__(kLpChunk) k_lp_pending(const LpArgs a) {
@@ -712,8 +757,14 @@ __global__ void __launch_bounds__(kLpChunk) k_lp_pending(const LpArgs a) {
   const uint32_t mine = __reduce_add_sync(kFull, lane < warp ? part[lane] : 0u);
   if (left) a.pend[before + mine + __popc(m & ((1u << lane) - 1u))] = a.n_mac + i;
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kLpChunk - 1) {
-    a.st->npend = before + mine + __popc(m);
-    if (!few_left(a)) cudaGraphSetConditional(a.many, 1u);
+    const uint32_t npend = before + mine + __popc(m), ties = a.st->ties, units = a.n - a.n_mac;
+    a.st->npend = npend;
+    const bool tied = 64ull * ties >= units && 5ull * ties >= npend;  // (the rule: at k_lp_lists)
+    if (tied) {
+      a.st->tied = 1u;
+      cudaGraphSetConditional(a.windows, 1u);
+    }
+    if (tied || !few_left(a)) cudaGraphSetConditional(a.many, 1u);
   }
 }
 
@@ -850,17 +901,16 @@ __device__ Best search_rows(const LpArgs &a, int32_t q, const Cell &c, double c0
 // cheaper than `best` are closed, so only the few columns of each row between
 // the two circles are looked at.  *count may exceed kLpRingMax: too many to
 // keep.
-constexpr int kLpRingMax = 64;
 // Wide enough for some ten to thirty sites: a cell at the rim of a pile of
 // radius r has open sites on one side only, in a ring of 1 to 2 sites' width.
 __device__ __forceinline__ float ring_of(double best) { return 60.0f + 2.4f * fast_sqrt((float)best); }
 
-__device__ void list_ring(const LpArgs &a, int32_t q, const Cell &c, double best, int warp, int lane, Best *list,
-                          int *count) {
+__device__ void list_ring(const LpArgs &a, int32_t q, const Cell &c, double best, float ring, int warp, int lane,
+                          Best *list, int *count) {
   const bool right = lane & 1;
   const int dir = right ? 1 : -1;
   const float tx = (float)c.tx, ty = (float)c.ty, low = (float)best * kUnder;
-  const float ring = ring_of(best), most = (float)best * kOver + ring;
+  const float most = (float)best * kOver + ring;
   const int rows = max(c.cy, a.H - 1 - c.cy);
   for (int p0 = 0; p0 <= rows; p0 += 8 * kUnitWarps) {
     if (p0 && ((float)p0 - 0.5f) * ((float)p0 - 0.5f) > most) break;
@@ -911,8 +961,9 @@ __device__ __forceinline__ Best warp_sorted(Best b) {
 }
 
 // A CTA per unit cell (kAll: each CTA has one; else those left over, taken up
-// in order), and the cells that its claim displaces one after the other.  What takes the time is the chain of cells that each take a site from
-// the next (about a thousand cells at the rim of a 200k-cell pile), so one
+// in order), and the cells that its claim displaces one after the other.  What
+// takes the time is the chain of cells that each take a site from the next
+// (about a thousand cells at the rims of a 200k-cell design's piles), so one
 // answer is made short: one warp, with no barrier, finds an answer near the
 // target, and that of a displaced cell in the list its search left (closed
 // sites stay closed, so the first one still open is the best); any other
@@ -920,107 +971,178 @@ __device__ __forceinline__ Best warp_sorted(Best b) {
 // displacement.  CTAs start in about the order of the cells, so a claim is
 // displaced only by a cell that was under way at the same time; several cells
 // per CTA, or a warp for each, put more cells under way and displace more
-// claims.  Units of a 200k-cell checkpoint whose cells lie in one pile:
+// claims.  Units of a 200k-cell checkpoint, half of the cells in six piles:
 // 4.9 ms and 117k searches of the whole CTA; without the lists 7.5 ms and 283k;
 // without them and with 2 / 4 / 8 cells per CTA 13.4 / 20 / 30 ms, with a warp
 // per cell 27 to 70 ms.
+struct UnitShared {
+  Best best[kUnitWarps], list[kLpRingMax];
+  unsigned least;
+  int count;
+  // the cell under way: index, target, cost below which no site is open
+  int32_t q;
+  float2 pos;
+  double c0;
+};
+
+// Nothing to do for a legalisation that failed or is not wanted (a warp).
+__device__ __forceinline__ bool wanted(const LpArgs &a, int lane) {
+  const bool off = ld_own(a.cancel) != 0;
+  if (off && lane == 0) atomicMax(&a.st->status, 4);
+  return !off && ld_own(&a.st->status) == 0;
+}
+
+// Warp 0: cell q and the cells that its claims displace, one after the other,
+// while one warp can tell; listed: q has lost site (px, py) and may have a
+// list.  Returns -1 when all have a site, else the cell that needs a search of
+// the whole CTA (its target and c0 are entered).
+__device__ __forceinline__ int32_t settle(const LpArgs &a, UnitShared &sh, int32_t q, bool &listed, int &px, int &py,
+                                          int lane) {
+  while (q >= 0) {
+    double c0 = 0.0;
+    float2 p;
+    if (listed) {
+      const int32_t *l = a.cand + (size_t)kLpCand * (q - (int32_t)a.n_mac);
+      const int32_t t = lane < kLpCand ? ld_own(l + lane) : -1;
+      const unsigned ends = __ballot_sync(kFull, t < 0);  // the list ends at its first -1
+      const int len = __ffs(ends) - 1;
+      const int x = t % a.W, y = t / a.W;
+      const int32_t on = lane < len ? ld_own(own_at(a, x, y)) : -1;
+      const uint2 s = lane < len ? ld_seg(seg_at(a, x, y)) : make_uint2(0u, 0u);
+      const unsigned open = __ballot_sync(kFull, on > q);
+      if (open) {
+        const int l0 = __ffs(open) - 1;
+        px = __shfl_sync(kFull, x, l0);
+        py = __shfl_sync(kFull, y, l0);
+        const uint2 seen = make_uint2(__shfl_sync(kFull, s.x, l0), __shfl_sync(kFull, s.y, l0));
+        const int32_t held = claim_and_acquire(a, q, px, py, seen, lane);
+        if (held == kNone) q = -1;
+        else if (held > q) q = held;
+        continue;  // (an earlier cell was faster: the list again)
+      }
+      p = a.pos[a.order[q]];
+      const Cell c = make_cell(a, p, make_uchar2(1, 1));
+      if (len > 0) {  // all of it closed, as everything cheaper
+        px = __shfl_sync(kFull, x, len - 1);
+        py = __shfl_sync(kFull, y, len - 1);
+      }
+      if (c.inside) c0 = __dadd_rn(col_dx2(c, px), row_dy2(c, py));
+    } else {
+      p = a.pos[a.order[q]];
+      c0 = get_hint(a, q, make_cell(a, p, make_uchar2(1, 1)));
+    }
+    listed = false;
+    const Cell c = make_cell(a, p, make_uchar2(1, 1));
+    if (c0 < 6.25 && placeable(c)) {
+      uint2 seen;
+      const Best b = search_near(a, q, c, lane, &seen);
+      if (b.cost < 6.25) {
+        px = b.tile % a.W;
+        py = b.tile / a.W;
+        const int32_t held = claim_and_acquire(a, q, px, py, seen, lane);
+        if (held == kNone) {
+          q = -1;
+        } else if (held > q) {
+          q = held;
+          listed = true;
+        }
+        continue;
+      }
+    }
+    if (lane == 0) {
+      sh.pos = p;
+      sh.c0 = c0;
+      sh.least = __float_as_uint(kInf);
+      sh.count = 0;
+    }
+    break;
+  }
+  return q;
+}
+
+// The search for cell q by the whole CTA, and the sites next in cost listed.
+__device__ __forceinline__ Best search_cta(const LpArgs &a, UnitShared &sh, int32_t q, const Cell &c, float &ring,
+                                           int warp, int lane) {
+  Best b = no_best();
+  if (placeable(c)) b = search_rows(a, q, c, sh.c0, warp, lane, &sh.least);
+  b = b.warp_min();
+  if (lane == 0) sh.best[warp] = b;
+  __syncthreads();
+  b = (lane < kUnitWarps ? sh.best[lane] : no_best()).warp_min();
+  if (ring == 0.0f) ring = ring_of(b.cost);
+  if (b.tile != kNone) list_ring(a, q, c, b.cost, ring, warp, lane, sh.list, &sh.count);
+  __syncthreads();
+  return b;
+}
+
+// Warp 0: leaves the cheapest 32 or fewer entries of the list, the ring (below
+// 2^26) halved until they are.  Returns how many; -1: no list.
+__device__ __forceinline__ int shrink_list(UnitShared &sh, const Best &b, int lane, double &ring) {
+  const int n = sh.count;
+  Best e0 = lane < n ? sh.list[lane] : no_best(), e1 = lane + 32 < n ? sh.list[lane + 32] : no_best();
+  unsigned m0 = 0, m1 = 0;
+  for (int k = 0; k < 37; ++k) {
+    m0 = __ballot_sync(kFull, e0.cost <= b.cost + ring);
+    m1 = __ballot_sync(kFull, e1.cost <= b.cost + ring);
+    if (__popc(m0) + __popc(m1) <= 32 || ring < 1e-3) break;
+    ring *= 0.5;
+  }
+  const unsigned below = (1u << lane) - 1;
+  const int i0 = __popc(m0 & below), i1 = __popc(m0) + __popc(m1 & below);
+  __syncwarp();
+  if ((m0 >> lane & 1) && i0 < 32) sh.list[i0] = e0;
+  if ((m1 >> lane & 1) && i1 < 32) sh.list[i1] = e1;
+  __syncwarp();
+  const int m = __popc(m0) + __popc(m1);
+  return n <= kLpRingMax && m <= 32 ? m : -1;
+}
+
+// Warp 0: q's list and claim of its best site b.  Returns the cell to go on
+// with (displaced, or q itself where an earlier cell was faster), -1: none.
+__device__ __forceinline__ int32_t list_and_claim(const LpArgs &a, UnitShared &sh, int32_t q, const Cell &c,
+                                                  const Best &b, double ring, int &px, int &py, int lane) {
+  px = b.tile % a.W;
+  py = b.tile / a.W;
+  const uint2 seen = ld_seg(seg_at(a, px, py));
+  const int m = shrink_list(sh, b, lane, ring);
+  const Best e = m >= 0 ? warp_sorted(lane < m ? sh.list[lane] : no_best()) : no_best();
+  if (lane < kLpCand)
+    a.cand[(size_t)kLpCand * (q - (int32_t)a.n_mac) + lane] =
+        m >= 0 && e.tile != kNone ? e.tile : lane == 0 && m < 0 ? b.tile : -1;
+  __syncwarp();
+  if (lane == 0) {
+    put_hint(a, q, c, b.cost);
+    __threadfence();  // the list before the claim: who displaces q reads it
+  }
+  const int32_t held = claim_and_acquire(a, q, px, py, seen, lane);
+  return held == kNone ? -1 : held > q ? held : q;
+}
+
 template <bool kAll>
 __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(const LpArgs a) {
-  __shared__ Best sbest[kUnitWarps], slist[kLpRingMax];
-  __shared__ unsigned least;
-  __shared__ int scount;
-  // the cell under way: index (-1: done, -2: none, take up the next), target, cost below which no site is open
-  __shared__ int32_t sq_;
-  __shared__ float2 spos;
-  __shared__ double sc0;
+  __shared__ UnitShared sh;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uchar2 one = make_uchar2(1, 1);
   int32_t next = -1;    // warp 0: the cell to place, -1: none
   bool listed = false;  // it may have a list
   int px = 0, py = 0;   // a displaced cell: the site it lost
-  if (!kAll && !few_left(a)) return;
-  // nothing to do for a legalisation that failed or is not wanted
-  auto wanted = [&] {
-    const bool off = ld_own(a.cancel) != 0;
-    if (off && lane == 0) atomicMax(&a.st->status, 4);
-    return !off && ld_own(&a.st->status) == 0;
-  };
+  if (a.st->tied || (!kAll && !few_left(a))) return;
   bool fresh = true;  // no cell under way
-  if (kAll && warp == 0 && wanted()) next = (int32_t)(a.n_mac + blockIdx.x);
+  if (kAll && warp == 0 && wanted(a, lane)) next = (int32_t)(a.n_mac + blockIdx.x);
   while (true) {
     if (!kAll && warp == 0 && fresh) {
       uint32_t item = 0;
       if (lane == 0) item = atomicAdd(&a.st->taken, 1u);
       item = __shfl_sync(kFull, item, 0);
-      next = item < a.st->npend && wanted() ? (int32_t)a.pend[item] : -1;
+      next = item < a.st->npend && wanted(a, lane) ? (int32_t)a.pend[item] : -1;
       listed = false;
     }
-    if (warp == 0) {  // while one warp can tell
-      int32_t q = next;
-      while (q >= 0) {
-        double c0 = 0.0;
-        float2 p;
-        if (listed) {
-          const int32_t *l = a.cand + (size_t)kLpCand * (q - (int32_t)a.n_mac);
-          const int32_t t = lane < kLpCand ? ld_own(l + lane) : -1;
-          const unsigned ends = __ballot_sync(kFull, t < 0);  // the list ends at its first -1
-          const int len = __ffs(ends) - 1;
-          const int x = t % a.W, y = t / a.W;
-          const int32_t on = lane < len ? ld_own(own_at(a, x, y)) : -1;
-          const uint2 s = lane < len ? ld_seg(seg_at(a, x, y)) : make_uint2(0u, 0u);
-          const unsigned open = __ballot_sync(kFull, on > q);
-          if (open) {
-            const int l0 = __ffs(open) - 1;
-            px = __shfl_sync(kFull, x, l0);
-            py = __shfl_sync(kFull, y, l0);
-            const uint2 seen = make_uint2(__shfl_sync(kFull, s.x, l0), __shfl_sync(kFull, s.y, l0));
-            const int32_t held = claim_and_acquire(a, q, px, py, seen, lane);
-            if (held == kNone) q = -1;
-            else if (held > q) q = held;
-            continue;  // (an earlier cell was faster: the list again)
-          }
-          p = a.pos[a.order[q]];
-          const Cell c = make_cell(a, p, one);
-          if (len > 0) {  // all of it closed, as everything cheaper
-            px = __shfl_sync(kFull, x, len - 1);
-            py = __shfl_sync(kFull, y, len - 1);
-          }
-          if (c.inside) c0 = __dadd_rn(col_dx2(c, px), row_dy2(c, py));
-        } else {
-          p = a.pos[a.order[q]];
-          c0 = get_hint(a, q, make_cell(a, p, one));
-        }
-        listed = false;
-        const Cell c = make_cell(a, p, one);
-        if (c0 < 6.25 && placeable(c)) {
-          uint2 seen;
-          const Best b = search_near(a, q, c, lane, &seen);
-          if (b.cost < 6.25) {
-            px = b.tile % a.W;
-            py = b.tile / a.W;
-            const int32_t held = claim_and_acquire(a, q, px, py, seen, lane);
-            if (held == kNone) {
-              q = -1;
-            } else if (held > q) {
-              q = held;
-              listed = true;
-            }
-            continue;
-          }
-        }
-        if (lane == 0) {
-          spos = p;
-          sc0 = c0;
-          least = __float_as_uint(kInf);
-          scount = 0;
-        }
-        break;  // the whole CTA
-      }
-      // (-2: there may be others to take up)
-      if (lane == 0) sq_ = q >= 0 || kAll || (fresh && next < 0) ? q : -2;
+    if (warp == 0) {
+      const int32_t q = settle(a, sh, next, listed, px, py, lane);
+      // (-1: done; -2: there may be others to take up)
+      if (lane == 0) sh.q = q >= 0 || kAll || (fresh && next < 0) ? q : -2;
     }
     __syncthreads();
-    const int32_t q = sq_;
+    const int32_t q = sh.q;
     if (kAll ? q < 0 : q == -1) return;
     if (!kAll) {
       fresh = q < 0;
@@ -1029,57 +1151,155 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
         continue;
       }
     }
-    const Cell c = make_cell(a, spos, one);
-    Best b = no_best();
-    if (placeable(c)) b = search_rows(a, q, c, sc0, warp, lane, &least);
-    b = b.warp_min();
-    if (lane == 0) sbest[warp] = b;
-    __syncthreads();
-    b = (lane < kUnitWarps ? sbest[lane] : no_best()).warp_min();
+    const Cell c = make_cell(a, sh.pos, make_uchar2(1, 1));
+    float ring = 0.0f;
+    const Best b = search_cta(a, sh, q, c, ring, warp, lane);
     if (b.tile == kNone) {  // no site is open to it
       if (tid == 0) atomicMax(&a.st->status, 1);
       return;
     }
-    list_ring(a, q, c, b.cost, warp, lane, slist, &scount);
-    __syncthreads();
     if (warp == 0) {
-      px = b.tile % a.W;
-      py = b.tile / a.W;
-      const uint2 seen = ld_seg(seg_at(a, px, py));
-      const int n = scount;
-      const bool keep = n <= kLpRingMax;
-      // the cheapest 32 or fewer: the ring (below 2^26) halved until they are
-      Best e0 = lane < n ? slist[lane] : no_best(), e1 = lane + 32 < n ? slist[lane + 32] : no_best();
-      double ring = (double)ring_of(b.cost);
-      unsigned m0 = 0, m1 = 0;
-      for (int k = 0; k < 37; ++k) {
-        m0 = __ballot_sync(kFull, e0.cost <= b.cost + ring);
-        m1 = __ballot_sync(kFull, e1.cost <= b.cost + ring);
-        if (__popc(m0) + __popc(m1) <= 32 || ring < 1e-3) break;
-        ring *= 0.5;
-      }
-      const unsigned below = (1u << lane) - 1;
-      const int i0 = __popc(m0 & below), i1 = __popc(m0) + __popc(m1 & below);
-      __syncwarp();
-      if ((m0 >> lane & 1) && i0 < 32) slist[i0] = e0;
-      if ((m1 >> lane & 1) && i1 < 32) slist[i1] = e1;
-      __syncwarp();
-      const int m = __popc(m0) + __popc(m1);
-      const bool some = keep && m <= 32;
-      const Best e = some ? warp_sorted(lane < m ? slist[lane] : no_best()) : no_best();
-      if (lane < kLpCand)
-        a.cand[(size_t)kLpCand * (q - (int32_t)a.n_mac) + lane] =
-            some && e.tile != kNone ? e.tile : lane == 0 && !some ? b.tile : -1;
-      __syncwarp();
-      if (lane == 0) {
-        put_hint(a, q, c, b.cost);
-        __threadfence();  // the list before the claim: who displaces q reads it
-      }
-      const int32_t held = claim_and_acquire(a, q, px, py, seen, lane);
-      next = held == kNone ? -1 : held > q ? held : q;
+      next = list_and_claim(a, sh, q, c, b, ring, px, py, lane);
       listed = true;
     }
   }
+}
+
+// Cells on one target.  Above, those under way want the same site: all but the
+// first lose it and search again, and so does who is displaced from it (13 us
+// each).  So where many share a target (positions clamped into a corner of the
+// chip, as the reference's field leaves them), the unit cells are placed in
+// windows of the next ones in order instead, whose searches see a map that does
+// not change: first each cell's list, then each takes of its list what the
+// cells before it leave.  A window ends early at the first cell whose list is
+// used up: after some 50 cells of one target.
+// ms, in the order without windows -> with (before deferred acceptance, as
+// rounds of lists and a serial pass), unit cells alone: all on one spot 1k 11.0
+// -> 0.9 (2.2), 30k 419 -> 27 (87), 200k 3697 -> 192 (1173); 40 % in a corner,
+// the others spread: 5k 17 -> 2.1 (6.5), 60k 308 -> 24 (84).  Runs with the
+// reference's field, 5k cells, 300 iterations 1297 -> 32 (48), 30k, 100
+// iterations, 4568 -> 290 (285).  Bound by the list kernel: two dependent
+// passes over the rows, 20 us a window, and two launches.
+// The rule (lp_build_graph, k_lp_pending): ties (cells of a target that has
+// tie_least or more) are at least 1/64 of the unit cells and 1/5 of those left
+// over by k_lp_near, or, where that isn't tried, 1/10 of all.  The line lies
+// where both ways take about as long: 200k cells, 2 % in a corner 29 -> 18 ms,
+// 30k 2.8 -> 2.6; 16 spots of 30k cells 23 -> 3.4; but a wide pile of 30k cells
+// of which 10 % are on one spot would take 14 -> 70 (40 %: 86 -> 64): its other
+// cells use up their lists too.  A loop that is not entered costs a graph
+// without other conditional nodes 15 us (3k spread cells 135 -> 150 us).
+
+// A CTA per cell of the window: the open sites of least cost, in order.
+__global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_lists(const LpArgs a) {
+  __shared__ UnitShared sh;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t i = a.st->wbase + blockIdx.x;
+  if (i >= a.n - a.n_mac || a.st->status != 0) return;
+  const int32_t q = (int32_t)(a.n_mac + i);
+  const Cell c = load_cell(a, (uint32_t)q, true);
+  if (tid == 0) {
+    sh.c0 = get_hint(a, q, c);
+    sh.least = __float_as_uint(kInf);
+    sh.count = 0;
+  }
+  __syncthreads();
+  // A ring of cost w round the best site holds about pi w open sites, half or a
+  // quarter of that at an edge or in a corner: another width where too few or
+  // too many are found.
+  float ring = 16.0f;
+  const Best b = search_cta(a, sh, q, c, ring, warp, lane);
+  int n = sh.count;
+  for (int k = 0; k < 3 && b.tile != kNone && (n > kLpRingMax || n < 24); ++k) {
+    __syncthreads();
+    if (tid == 0) sh.count = 0;
+    __syncthreads();
+    ring *= 44.0f / (float)max(n, 1);
+    list_ring(a, q, c, b.cost, ring, warp, lane, sh.list, &sh.count);
+    __syncthreads();
+    n = sh.count;
+  }
+  if (n > kLpRingMax) {  // too many sites tie
+    __syncthreads();
+    if (tid == 0) sh.list[0] = b;
+    __syncthreads();
+    n = 1;
+  }
+  if (b.tile == kNone) n = 0;
+  if (tid < n) {
+    const Best e = sh.list[tid];
+    int k = 0;
+    for (int t = 0; t < n; ++t) {
+      const Best o = sh.list[t];
+      k += o.cost < e.cost || (o.cost == e.cost && o.tile < e.tile) ? 1 : 0;
+    }
+    a.list[kLpRingMax * blockIdx.x + k] = e.tile;
+  }
+  if (tid == 0) a.list_len[blockIdx.x] = n;
+}
+
+// One CTA, a thread per cell of the window: each onto the first entry of its
+// list that no earlier cell of the window takes (everything cheaper was closed,
+// everything off the list costs more), again by deferred acceptance: who has
+// lost its site to an earlier cell goes on to its next entry.  The cells before
+// the first whose entries are all lost are final; the next window begins there.
+constexpr int kTakenBits = kUnitWindowBits + 2;  // table of the sites proposed to (each is held by some cell)
+__global__ void __launch_bounds__(kUnitWindow) k_lp_take(const LpArgs a) {
+  extern __shared__ int32_t list[];  // [kUnitWindow][kLpRingMax + 1]: no two cells' entries in one bank
+  __shared__ int32_t site[1 << kTakenBits], holder[1 << kTakenBits];
+  __shared__ int done;
+  LpState *st = a.st;
+  const int tid = threadIdx.x;
+  const uint32_t units = a.n - a.n_mac, base = st->wbase;
+  const int count = (int)min(kUnitWindow, units - base);
+  if (st->status == 0) {
+    for (int k = tid; k < 1 << kTakenBits; k += kUnitWindow) {
+      site[k] = -1;
+      holder[k] = kNone;
+    }
+    for (int k = tid; k < count * kLpRingMax; k += kUnitWindow)
+      list[k + k / kLpRingMax] = a.list[k];
+    if (tid == 0) done = count;
+    const int len = tid < count ? a.list_len[tid] : 0;
+    __syncthreads();
+    int at = 0;          // entry of the list
+    int32_t where = -1;  // its place in the table
+    bool propose = tid < count;
+    while (true) {
+      if (propose && at < len) {
+        const int32_t t = list[tid * (kLpRingMax + 1) + at];
+        uint32_t h = ((uint32_t)t * 2654435761u) >> (32 - kTakenBits);
+        while (true) {
+          const int32_t was = atomicCAS(&site[h], -1, t);
+          if (was == -1 || was == t) break;
+          h = (h + 1) & ((1u << kTakenBits) - 1u);
+        }
+        where = (int32_t)h;
+        atomicMin(&holder[h], tid);
+      }
+      __syncthreads();
+      propose = tid < count && at < len && holder[where] != tid;
+      if (propose) ++at;
+      if (!__syncthreads_or(propose)) break;
+    }
+    if (tid < count && at >= len) atomicMin(&done, tid);
+    __syncthreads();
+    if (tid < done) {
+      const int32_t q = (int32_t)(a.n_mac + base) + tid, t = site[where];
+      const int x = t % a.W, y = t / a.W;
+      const Cell c = load_cell(a, (uint32_t)q, true);
+      *own_at(a, x, y) = q;
+      atomicAnd(&seg_at(a, x, y)->x, ~(1u << (x & 31)));
+      put_hint(a, q, c, __dadd_rn(col_dx2(c, x), row_dy2(c, y)));
+    }
+    if (tid == 0) {
+      st->wbase = base + (uint32_t)done;
+      if (done == 0) atomicMax(&st->status, 1);  // the first cell's list is empty: no site is open to it
+    }
+  }
+  __syncthreads();
+  if (tid != 0) return;
+  if (ld_own(a.cancel)) atomicMax(&st->status, 4);
+  if (st->wbase >= units || atomicAdd(&st->status, 0) != 0) cudaGraphSetConditional(a.windows, 0u);
 }
 
 // ---------------------------------------------------------------------------
@@ -1300,9 +1520,19 @@ cudaError_t lp_build_graph(LpArgs a, LpGraph &g, cudaStream_t cs) {
       (e = cudaGraphConditionalHandleCreate(&a.handle, graph, 1, cudaGraphCondAssignDefault)) != cudaSuccess)
     return e;
   const uint32_t units = a.n - a.n_mac;
+  constexpr int kTakeShared = (int)(sizeof(int32_t) * kUnitWindow * (kLpRingMax + 1));
+  if ((e = cudaFuncSetAttribute(k_lp_take, cudaFuncAttributeMaxDynamicSharedMemorySize, kTakeShared)) != cudaSuccess)
+    return e;
   const bool at_once = units >= kNearFrom;
+  // Few cells: targets that differ by less than a tenth of a site crowd like equal
+  // ones (5k in a pile of sigma 0.1: 13.7 -> 7.0 ms, but 60k 135 -> 230).
+  a.tie_scale = at_once ? 64.0f : 16.0f;
+  a.tie_least = units / (at_once ? 64 : 32) > 32 ? units / (at_once ? 64 : 32) : 32;
+  a.tie_limit = at_once ? 0 : units / 10 > 32 ? units / 10 : 32;
   if (at_once &&
       (e = cudaGraphConditionalHandleCreate(&a.many, graph, 0, cudaGraphCondAssignDefault)) != cudaSuccess)
+    return e;
+  if (units && (e = cudaGraphConditionalHandleCreate(&a.windows, graph, 0, cudaGraphCondAssignDefault)) != cudaSuccess)
     return e;
   if ((e = add((const void *)k_lp_init, site_grid, 256)) != cudaSuccess) return e;
   if (a.n_mac) {
@@ -1319,8 +1549,21 @@ cudaError_t lp_build_graph(LpArgs a, LpGraph &g, cudaStream_t cs) {
     if ((e = end_body()) != cudaSuccess) return e;
   }
   if ((e = add((const void *)k_lp_segments, site_grid, 256)) != cudaSuccess) return e;
+  // the loop over the windows
+  auto add_windows = [&]() -> cudaError_t {
+    cudaGraph_t body;
+    cudaError_t r;
+    if ((r = add_cond(a.windows, cudaGraphCondTypeWhile, &body)) != cudaSuccess) return r;
+    if ((r = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
+        cudaSuccess)
+      return r;
+    k_lp_lists<<<units < kUnitWindow ? units : kUnitWindow, kUnitWarps * 32, 0, cs>>>(a);
+    k_lp_take<<<1, kUnitWindow, kTakeShared, cs>>>(a);
+    return end_body();
+  };
   if (units && !at_once) {
     if ((e = add((const void *)k_lp_units<true>, units, kUnitWarps * 32)) != cudaSuccess) return e;
+    if ((e = add_windows()) != cudaSuccess) return e;
   } else if (units) {
     const uint32_t chunks = (uint32_t)lp_chunks(units);
     if ((e = add((const void *)k_lp_near, (units + 7) / 8, 256)) != cudaSuccess) return e;
@@ -1334,6 +1577,7 @@ cudaError_t lp_build_graph(LpArgs a, LpGraph &g, cudaStream_t cs) {
     k_lp_undo<<<site_grid, 256, 0, cs>>>(a);
     k_lp_units<true><<<units, kUnitWarps * 32, 0, cs>>>(a);
     if ((e = end_body()) != cudaSuccess) return e;
+    if ((e = add_windows()) != cudaSuccess) return e;
     if ((e = add((const void *)k_lp_units<false>, 296, kUnitWarps * 32)) != cudaSuccess)
       return e;
   }

@@ -10,6 +10,14 @@ namespace eplace {
 // Macros that a round works on at once.
 constexpr uint32_t kLpWindow = 2048;
 
+// Unit cells of a window (a power of two; with two CTAs per SM their searches
+// run in one wave).
+constexpr int kUnitWindowBits = 8;
+constexpr uint32_t kUnitWindow = 1u << kUnitWindowBits;
+
+// Sites that a search lists at most.
+constexpr int kLpRingMax = 64;
+
 // Sites kept of a unit cell's search.
 constexpr int kLpCand = 16;
 
@@ -23,6 +31,9 @@ struct LpState {
   uint32_t nwork[2];   // macros to choose in this and in the next round
   uint32_t npend;      // unit cells left to k_lp_units
   uint32_t taken;      // of them, those that a CTA has taken up
+  uint32_t ties;       // unit cells that share a target with tie_least or more
+  uint32_t tied;       // too many do: the unit cells are placed in windows
+  uint32_t wbase;      // unit cells [0, wbase) have been placed in windows
   int32_t status;      // 0 ok, 1 no free site for some cell, 2 round cap, 4 cancelled
 };
 
@@ -52,6 +63,14 @@ struct LpArgs {
   int32_t *near;           // [n - n_mac] site a unit cell took near its target, -1: none
   uint32_t *pend;          // [n - n_mac] order indices of the cells left to k_lp_units, ascending
   uint32_t *left;          // [lp_chunks] how many of them in each kLpChunk unit cells
+  unsigned long long *tie_key;  // [tie_mask + 1] table of the unit cells' targets
+  uint32_t *tie_count;     // [tie_mask + 1] how many have each
+  uint32_t tie_mask;       // lp_tie_entries - 1
+  float tie_scale;         // filled in by lp_build_graph, like the next two: squares per site that tell targets apart
+  uint32_t tie_least;      // cells of one target from which they count as ties
+  uint32_t tie_limit;      // ties from which all unit cells are placed in windows, 0: decided later
+  int32_t *list;           // [kUnitWindow][kLpRingMax] sites of least cost of the window's cells
+  int32_t *list_len;       // [kUnitWindow] how many
   LpState *st;
   int2 *sites;             // [N] anchor of every cell (out)
   int2 *loc;               // [N] pin location anchor + (size - 1) / 2 (out), or nullptr
@@ -62,11 +81,19 @@ struct LpArgs {
   uint32_t max_rounds;
   cudaGraphConditionalHandle handle;  // of the loop over the macro rounds
   cudaGraphConditionalHandle many;    // of the pass over all unit cells in order
+  cudaGraphConditionalHandle windows; // of the loop over the windows
 };
 
 // The hints: one entry per size class (1 .. 8 sites) and 16 x 16 sites.
 constexpr int kLpHintClasses = 8;
 inline size_t lp_hint_count(int W, int H) { return (size_t)kLpHintClasses * ((W + 15) / 16) * ((H + 15) / 16); }
+
+// Entries of the table of the unit cells' targets.
+inline size_t lp_tie_entries(size_t units) {
+  size_t n = 64;
+  while (n < 2 * units) n *= 2;
+  return n;
+}
 
 // Unit cells that a CTA looks through for ones that are left.
 constexpr uint32_t kLpChunk = 1024;
@@ -79,7 +106,8 @@ inline bool legalize_supported(int W, int H) { return W > 0 && H > 0 && W <= 409
 // A legalisation as one CUDA graph: initialisation, a device-side while
 // loop over the macro rounds (when there are macros), the unit cells (all at
 // once and the few left over, or, where too many are, all in order: an if
-// node), the displacement sum.  Built once per slot and problem load; launched per
+// node; or, where many share a target, in windows: a while node), the
+// displacement sum.  Built once per slot and problem load; launched per
 // checkpoint.
 struct LpGraph {
   cudaGraphExec_t exec = nullptr;

@@ -316,3 +316,73 @@ def test_device_legalizer_long_chains(n, piles):
         for _ in range(3):
             gx, gy, gd, _ = ctx.legalize_device(x, y)
             assert np.array_equal(gx, hx) and np.array_equal(gy, hy) and gd == hd
+
+
+@pytest.mark.parametrize("n", [40, 255, 256, 257, 700, 5000, 16383, 16384, 17000])
+@pytest.mark.parametrize("macros", [0, 9])
+def test_device_legalizer_cells_on_one_target(n, macros):
+    """Many cells on one target, alone and beside others, in corners, on edges,
+    nearly equal, off the chip, and around the counts from which cells are
+    placed in windows and all at once; blocked sites around the target."""
+    rng = np.random.default_rng(n + macros)
+    side = 32 if n < 800 else 96 if n <= 5000 else 140
+    cw = np.ones(n, np.uint8)
+    cw[rng.permutation(n)[:macros]] = 3
+    fx, fy = rng.integers(0, side // 2, (2, 20)).astype(np.int32)
+    nl = E.Netlist(num_cells=n, net_offsets=np.array([0, 2], np.uint32), pin_cell=np.array([0, 1], np.uint32),
+                   fixed_x=fx, fixed_y=fy, fixed_on_logic=np.ones(20, np.uint8), cell_w=cw, cell_h=np.ones(n, np.uint8))
+    u = rng.uniform(0, side - 1, (2, n))
+    spread = lambda share, x, y: np.where(rng.random(n) < share, np.array([[x], [y]]), u)
+    k = rng.integers(0, 3, n)
+    spots = rng.uniform(0.2 * side, 0.8 * side, (2, 3))
+    layouts = {
+        "spot": np.array([[0.37 * side], [0.61 * side]]) + np.zeros((2, n)),
+        "half": np.full((2, n), side // 2 + 0.5),  # four sites tie
+        "corner": spread(0.97, 0.0, 0.0),
+        "corner, others": spread(0.4, side - 1.0, 0.0),
+        "few": spread(0.04, 0.0, side - 1.0),
+        "spots": spots[:, k],
+        "nearly": np.array([[0.4 * side], [0.5 * side]]) + rng.normal(0, 0.004, (2, n)),
+        "in a pile": np.where(rng.random(n) < 0.5, 0.5 * side, 0.5 * side + rng.normal(0, 0.06 * side, (2, n))),
+        "off": spread(0.8, -300.0, 0.3 * side),
+    }
+    with E.PlacementContext(nl, E.Chip(side, side)) as ctx:
+        for name, (x, y) in layouts.items():
+            hx, hy, hd = ctx.legalize(x, y)
+            for _ in range(2):
+                gx, gy, gd, _ = ctx.legalize_device(x, y)
+                assert np.array_equal(gx, hx) and np.array_equal(gy, hy), name
+                assert gd == hd, name
+
+
+@pytest.mark.parametrize("side", [16, 130])
+def test_device_legalizer_full_chip_on_one_target(side):
+    """As many cells as sites, all on one target, and one more than that."""
+    for n, fits in ((side * side, True), (side * side + 1, False)):
+        nl = E.Netlist(num_cells=n, net_offsets=np.array([0, 2], np.uint32), pin_cell=np.array([0, 1], np.uint32))
+        x = np.full(n, 0.25 * side, np.float32)
+        try:
+            ctx = E.PlacementContext(nl, E.Chip(side, side))
+        except E.NoBelsAvailable:
+            assert not fits
+            continue
+        with ctx:
+            if not fits:
+                with pytest.raises(E.NoBelsAvailable):
+                    ctx.legalize_device(x, x)
+                continue
+            hx, hy, hd = ctx.legalize(x, x)
+            gx, gy, gd, _ = ctx.legalize_device(x, x)
+            assert np.array_equal(gx, hx) and np.array_equal(gy, hy) and gd == hd
+
+
+@pytest.mark.parametrize("cells,side,bins", [(1000, 64, 64), (20000, 200, 100)])
+def test_run_with_device_legalizer_and_reference_field(cells, side, bins):
+    """The reference's field leaves most cells on one corner: the same run as
+    with the host legaliser, checkpoints no longer wanted among them."""
+    nl, chip = E.synth_netlist(E.SynthSpec(seed=5, num_cells=cells, num_nets=cells, num_pads=60, width=side,
+                                           height=side, bins_x=bins, bins_y=bins, cluster_size=32))
+    cfg = E.ElectroPlaceCfg(max_iters=70)
+    a = E.place_electro(nl, chip, cfg, E.RunOptions(legal_mode=0))
+    b = E.place_electro(nl, chip, cfg, E.RunOptions(legal_mode=1))
+    assert a.hpwl == b.hpwl and np.array_equal(a.bel_tile, b.bel_tile) and a.trajectory == b.trajectory
