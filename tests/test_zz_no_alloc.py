@@ -278,3 +278,29 @@ def test_density_noalloc_after_overlapping_calls():
             st, got, o = _noalloc(torch, nl, chip, x, y, None, dens, ov)
             assert st == _abi.EPLACE_OK
             assert np.array_equal(got, want) and abs(o - ref) <= 1e-12
+
+
+@pytest.mark.parametrize("cells", [1, 33, 700])
+@pytest.mark.parametrize("share,bins_wide", [(1.0, 1.0), (1.0, 5.0), (0.05, 1.0), (0.05, 9.0), (0.5, 2.5)])
+def test_density_noalloc_shares_of_wide_footprints(cells, share, bins_wide):
+    """Warps in which all, half and few cells cover more than 2 x 2 bins, up to
+    a bin or two more than a warp has lanes."""
+    import torch
+
+    dev = torch.device("cuda:0")
+    torch.cuda.set_device(dev)
+    rng = np.random.default_rng(cells)
+    nl = E.Netlist(num_cells=cells, net_offsets=np.zeros(1, np.uint32), pin_cell=np.zeros(0, np.uint32))
+    w, h, bx, by = 240, 160, 60, 80  # 4 x 2 sites a bin
+    chip = E.Chip(w, h, bx, by)
+    x, y = rng.uniform(0, w - 1, cells).astype(np.float32), rng.uniform(0, h - 1, cells).astype(np.float32)
+    wide = rng.random(cells) < share
+    hf = np.where(wide[:, None], np.array([[2.0 * bins_wide, 1.0 * bins_wide]]), 0.5).astype(np.float32)
+    dens_d = torch.full((by, bx), -1.0, dtype=torch.float64, device=dev)
+    ov_d = torch.full((1,), -1.0, dtype=torch.float64, device=dev)
+    want = _axis(y, hf[:, 1], 2, by).T @ _axis(x, hf[:, 0], 4, bx)
+    over = np.maximum(want - 8.0, 0).sum() / want.sum()
+    st, got, ov = _noalloc(torch, nl, chip, x, y, torch.from_numpy(hf).to(dev), dens_d, ov_d)
+    assert st == _abi.EPLACE_OK
+    assert np.abs(got - want).max() <= 1e-6 * want.max()
+    assert abs(ov - over) <= 1e-6
