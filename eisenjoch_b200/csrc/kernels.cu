@@ -937,7 +937,8 @@ bool sgemm_small_tile(int M, int N, int nb) {
 //    crosses blocks, and the state that the second half needs is loaded while
 //    the block waits for the others;
 //  * a macro (25 bins and more) is gathered by eight lanes, a column of bins
-//    each, four macros a warp, spread over all blocks.  The bins are summed in
+//    each, four macros a warp, spread over all blocks (MANY: a thread each, see
+//    step_kernel).  The bins are summed in
 //    the row-major order of one thread, so the bits are the same; one thread
 //    per macro walked its rows one memory latency at a time, and held the
 //    barrier up for 8 us at 200k cells (10k macros);
@@ -953,8 +954,8 @@ bool sgemm_small_tile(int M, int N, int nb) {
 // Inside one launch (5k / 200k / 800k cells), first half done 3 / 9 / 33 us,
 // sums known 5 / 12 / 36, end 8 / 20 / 67 (with the scatter; before, without
 // it: 200k 14, 20, 25).  Whole iterations with the FFT transform, reference
-// field: 5k cells 30.9 -> 21.5 us, 30k 52.7 -> 44.9, 200k 111.6 -> 98.2, 800k
-// 229 -> 213.
+// field, mean of 100: 5k cells 30.9 -> 20.6 us, 30k 52.7 -> 35.5, 200k 111.6 ->
+// 58.5, 800k 229 -> 200 (the last three with the cells of a bin added once).
 // ---------------------------------------------------------------------------
 
 // The four sums v over the block; lane k < 4 of warp 0 gets sum k in v[0].
@@ -1153,6 +1154,42 @@ __device__ __forceinline__ float2 gather_macro(const StepArgs &a, const Macro &m
   return g;
 }
 
+// The same by one thread, four bins of a row in flight, summed in the same
+// order: for designs with so many macros that eight lanes each would be work for
+// more warps than there are.
+__device__ __forceinline__ float2 gather_wide(const StepArgs &a, float2 p, float2 hf, float area) {
+  const Foot f = make_foot(p, hf.x, hf.y, a.BX, a.BY, a.isx, a.isy);
+  float fx = 0.f, fy = 0.f, wt = 0.f;
+#pragma unroll 1
+  for (int by = f.by0; by < f.by1; ++by) {
+    const float oy = overlap_y(f, by, a.isy);
+#pragma unroll 1
+    for (int b0 = f.bx0; b0 < f.bx1; b0 += 4) {
+      float w[4], e[4], h[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        w[k] = b0 + k < f.bx1 ? overlap_x(f, b0 + k, a.isx) * oy : 0.0f;
+        const int at = by * a.BX + b0 + k;
+        e[k] = w[k] > 0.0f ? a.Ex[at] : 0.0f;
+        h[k] = w[k] > 0.0f ? a.Ey[at] : 0.0f;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (w[k] > 0.0f) {
+          fx = fmaf(w[k], e[k], fx);
+          fy = fmaf(w[k], h[k], fy);
+          wt += w[k];
+        }
+    }
+  }
+  float2 g = make_float2(0.f, 0.f);
+  if (wt > 1e-10f) {
+    g.x = area * (fx / wt);
+    g.y = area * (fy / wt);
+  }
+  return g;
+}
+
 // g = (g_wl + lam g_den) / max(1, pw + lam area)   (mod.rs:145-156)
 __device__ __forceinline__ float2 combine(float2 gw, float2 gd, double lam, float pw, float area) {
   const double ipc = 1.0 / fmax((double)pw + lam * (double)area, 1.0);
@@ -1290,7 +1327,9 @@ __device__ __forceinline__ void scatter_macro(const StepArgs &a, const Macro &m,
 struct Shares {
   int unit, macro;
 };
+template <bool MANY>
 __device__ __forceinline__ Shares shares(const StepArgs &a) {
+  if (MANY) return Shares{(int)(blockDim.x >> 5), 0};
   const int nwb = blockDim.x >> 5;
   const uint32_t per = ((a.n_mac + 3) / 4 + gridDim.x - 1) / gridDim.x;  // tasks of a block, at most
   if (per == 0 || per > (uint32_t)(3 * nwb / 4)) return Shares{nwb, nwb};
@@ -1316,11 +1355,21 @@ __device__ __forceinline__ void each_macro(const StepArgs &a, const Shares &sh, 
   }
 }
 
+// With MANY, a thread per macro instead: fn(cell), from the grid's last thread
+// on, where the unit cells' passes are shortest.
+template <typename F>
+__device__ __forceinline__ void each_macro_alone(const StepArgs &a, F fn) {
+  const uint32_t threads = gridDim.x * blockDim.x;
+#pragma unroll 1
+  for (uint32_t k = threads - 1 - (blockIdx.x * blockDim.x + threadIdx.x); k < a.n_mac; k += threads) fn(a.mac_idx[k]);
+}
+
 // Modes: 0: the whole step in one cooperative launch (grid barriers between
 // its halves); 1: gather only (tmp_den <- density gradient); 2, 3, 4: first
 // half, penalty-initialisation pass and second half as three ordinary launches
 // of the same grid (launch order replaces the barriers, so no block ever waits
 // for another).
+template <bool MANY>
 __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
   __shared__ __align__(16) double sm[64], sm2[64], tot[4];
   __shared__ int gave_up;
@@ -1328,7 +1377,7 @@ __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   // this thread's unit cells: tid0, tid0 + gstride, ...
-  const Shares sh = shares(a);
+  const Shares sh = shares<MANY>(a);
   const bool units = (int)(threadIdx.x >> 5) < sh.unit;
   const uint32_t gstride = gridDim.x * (uint32_t)sh.unit * 32;
   const uint32_t tid0 = units ? blockIdx.x * (uint32_t)sh.unit * 32 + threadIdx.x : a.N;
@@ -1344,10 +1393,14 @@ __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
   if (a.sc->err) return;
 
   if (a.mode == 1) {  // gather only: no barrier is reached
-    each_macro(a, sh, [&](const Macro &m) {
-      const float2 g = gather_macro(a, m, a.look[m.i]);
-      if (m.in && m.col == 0) a.tmp_den[m.i] = g;
-    });
+    if constexpr (MANY) {
+      each_macro_alone(a, [&](uint32_t i) { a.tmp_den[i] = gather_wide(a, a.look[i], a.half[i], a.area[i]); });
+    } else {
+      each_macro(a, sh, [&](const Macro &m) {
+        const float2 g = gather_macro(a, m, a.look[m.i]);
+        if (m.in && m.col == 0) a.tmp_den[m.i] = g;
+      });
+    }
     for (uint32_t i = tid0; i < a.N; i += gstride)
       if (!a.mflag || !a.mflag[i]) a.tmp_den[i] = gather_unit(a, a.look[i]);
     return;
@@ -1367,13 +1420,21 @@ __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
   State s0{};
   double v[4] = {0.0, 0.0, 0.0, 0.0};
   if (coop || a.mode == 2) {
-    each_macro(a, sh, [&](const Macro &m) {
-      CellIn c;
-      c.look = a.look[m.i];
-      if (m.col == 0) c = load_in(a, m.i, was_init);
-      const float2 gd = gather_macro(a, m, c.look);
-      if (m.in && m.col == 0) first_half(a, m.i, c, gd, m.area, was_init, lam, v);
-    });
+    if constexpr (MANY) {
+      each_macro_alone(a, [&](uint32_t i) {
+        const CellIn c = load_in(a, i, was_init);
+        const float area = a.area[i];
+        first_half(a, i, c, gather_wide(a, c.look, a.half[i], area), area, was_init, lam, v);
+      });
+    } else {
+      each_macro(a, sh, [&](const Macro &m) {
+        CellIn c;
+        c.look = a.look[m.i];
+        if (m.col == 0) c = load_in(a, m.i, was_init);
+        const float2 gd = gather_macro(a, m, c.look);
+        if (m.in && m.col == 0) first_half(a, m.i, c, gd, m.area, was_init, lam, v);
+      });
+    }
     // One cell at a time, the next one's state on the way (a macro's is loaded
     // for nothing: its flag arrives with it).
     CellIn c{};
@@ -1413,9 +1474,13 @@ __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
         a.g[i] = g;
         bb_terms(v, a.x[i], a.xp[i], g, a.gprev[i]);
       };
-      each_macro(a, sh, [&](const Macro &m) {
-        if (m.in && m.col == 0) pass(m.i, m.area);
-      });
+      if constexpr (MANY) {
+        each_macro_alone(a, [&](uint32_t i) { pass(i, a.area[i]); });
+      } else {
+        each_macro(a, sh, [&](const Macro &m) {
+          if (m.in && m.col == 0) pass(m.i, m.area);
+        });
+      }
       for (uint32_t i = tid0; i < a.N; i += gstride)
         if (!a.mflag || !a.mflag[i]) pass(i, 1.0f);
       const double t = block_sum4(v, sm);
@@ -1466,15 +1531,28 @@ __global__ void __launch_bounds__(kStepBlock, 2) k_step(const StepArgs a) {
   // (:95-101) clamped to the chip (common.rs:410-415), and its density.
   const double m = a.mom[it], mn = a.mom[it + 1];
   double nrm[4] = {0.0, 0.0, 0.0, 0.0};
-  each_macro(a, sh, [&](const Macro &c) {
-    float2 p = make_float2(0.f, 0.f);
-    if (c.in && c.col == 0) p = fista_cell(a, c.i, a.x[c.i], a.xp[c.i], a.g[c.i], m, mn, alpha, nrm);
-    if (a.dens) {
-      const int lead = threadIdx.x & 24;
-      p = make_float2(__shfl_sync(kFull, p.x, lead), __shfl_sync(kFull, p.y, lead));
-      scatter_macro(a, c, p);
-    }
-  });
+  if constexpr (MANY) {
+    each_macro_alone(a, [&](uint32_t i) {
+      const float2 p = fista_cell(a, i, a.x[i], a.xp[i], a.g[i], m, mn, alpha, nrm);
+      if (!a.dens) return;
+      const float2 hf = a.half[i];
+      const Foot f = make_foot(p, hf.x, hf.y, a.BX, a.BY, a.isx, a.isy);
+#pragma unroll 1
+      for (int by = f.by0; by < f.by1; ++by)
+#pragma unroll 1
+        for (int bx = f.bx0; bx < f.bx1; ++bx) add_bin(a.dens, f, bx, by, a.BX, a.isx, a.isy);
+    });
+  } else {
+    each_macro(a, sh, [&](const Macro &c) {
+      float2 p = make_float2(0.f, 0.f);
+      if (c.in && c.col == 0) p = fista_cell(a, c.i, a.x[c.i], a.xp[c.i], a.g[c.i], m, mn, alpha, nrm);
+      if (a.dens) {
+        const int lead = threadIdx.x & 24;
+        p = make_float2(__shfl_sync(kFull, p.x, lead), __shfl_sync(kFull, p.y, lead));
+        scatter_macro(a, c, p);
+      }
+    });
+  }
 #pragma unroll 1
   for (uint32_t i = tid0; units && (i & ~31u) < a.N; i += gstride) {  // a warp's 32 cells at a time
     const bool unit = unit_at(i);
@@ -1653,16 +1731,28 @@ int step_block(int device, uint32_t cells) {
   return cells <= 128u * (unsigned)sms ? 128 : cells <= 512u * (unsigned)sms ? 256 : kStepBlock;
 }
 
+// A thread per macro from three macros in ten cells on.  An iteration, eight
+// lanes per macro / a thread each (before macros had lanes), us: macros of 2 x 2
+// sites, all of 20k cells 55.5 / 29.7 (36.9), of 100k 85 / 49 (51), 40 % of 20k
+// 41.6 / 30.6 (39.3); of 2 to 8 sites, 20 % of 100k cells 56 / 65 (58), 5 % of
+// 20k 28.8 / 42.3 (42.2).
+using StepKernel = void (*)(StepArgs);
+StepKernel step_kernel(const StepArgs &a) { return 10ull * a.n_mac >= 3ull * a.N ? k_step<true> : k_step<false>; }
+
 int step_max_grid(int device, int block) {
   int sms = 0, occ = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_step, block, 0) != cudaSuccess) return 0;
-  return sms * occ;
+  int least = 1 << 30;
+  for (StepKernel k : {k_step<false>, k_step<true>}) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, block, 0) != cudaSuccess) return 0;
+    least = occ < least ? occ : least;
+  }
+  return sms * least;
 }
 
 cudaError_t launch_step(const StepArgs &a, int grid, int block, cudaStream_t s) {
   void *args[] = {const_cast<StepArgs *>(&a)};
-  return cudaLaunchCooperativeKernel((const void *)k_step, dim3(grid), dim3(block), args, 0, s);
+  return cudaLaunchCooperativeKernel((const void *)step_kernel(a), dim3(grid), dim3(block), args, 0, s);
 }
 cudaError_t launch_step_split(const StepArgs &a, int grid, int block, cudaStream_t s) {
   for (int mode = 2; mode <= 4; ++mode) {
@@ -1670,7 +1760,7 @@ cudaError_t launch_step_split(const StepArgs &a, int grid, int block, cudaStream
     b.mode = mode;
     // the second and third may start while the one before ends (k_step waits)
     Launch l(grid, block, s, mode > 2);
-    const cudaError_t e = cudaLaunchKernelEx(&l.cfg, k_step, b);
+    const cudaError_t e = cudaLaunchKernelEx(&l.cfg, step_kernel(a), b);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
