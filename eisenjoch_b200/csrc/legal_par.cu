@@ -373,35 +373,89 @@ __device__ Best search_block(const LpArgs &a, int32_t q, const Cell &c, double c
   return b;
 }
 
-// The same for any footprint (wider or higher ones): a lane per anchor.
-__device__ Best search_any(const LpArgs &a, int32_t q, const Cell &c, int lane) {
+// The same for any footprint (wider or higher ones): a warp per anchor row, the
+// rows outward from the target, a lane per site row of the block (32 at a time),
+// whose words tell 32 anchors at once: a run of w open sites is one of 32 and
+// those behind it, the last shifted.  (A lane per anchor that looked at each
+// site of its block, by one warp: 15 macros of 40 x 40 among 20k cells, all in a
+// pile, 468 ms -> 5.1 (61 as rounds of lists); 20 of 90 to 130 x 70 to 110 among
+// 100k, spread, 631 -> 3.3 ms (41).)
+__device__ Best search_large(const LpArgs &a, int32_t q, const Cell &c, double c0, int warp, int lane,
+                             unsigned *least) {
   Best b = no_best();
-  int bhi = kInfHi;
-  const int gc = c.cx >> 5;
-  for (int k = 0;; ++k) {
-    bool any = false;
-    for (int side = 0; side < (k ? 2 : 1); ++side) {
-      const int ay = c.cy + (side ? -k : k);
-      if (ay < 0 || ay >= c.AH) continue;
-      const double dy2 = row_dy2(c, ay);
-      if (__double2hiint(dy2) > bhi) continue;
-      any = true;
-      for (int dir = 0; dir < 2; ++dir)
-        for (int g = dir ? gc - 1 : gc; g >= 0 && 32 * g < c.AW; g += dir ? -1 : 1) {
-          if (g != gc && __double2hiint(__dadd_rn(col_dx2(c, dir ? 32 * g + 31 : 32 * g), dy2)) > bhi) break;
-          const int ax = 32 * g + lane;
-          if (ax < c.AW) {
-            bool open = true;
-            for (int s = 0; s < c.w * c.h && open; ++s)
-              open = ld_own(own_at(a, ax + s % c.w, ay + s / c.w)) >= q;
-            if (open) b.take(__dadd_rn(col_dx2(c, ax), dy2), ay * a.W + ax);
-          }
-          bhi = (int)__reduce_min_sync(kFull, (unsigned)__double2hiint(b.cost));
-        }
+  const float tx = (float)c.tx, ty = (float)c.ty, ox = (float)c.ox, oy = (float)c.oy;
+  const int one = min(c.w, 32), rows = max(c.cy, c.AH - 1 - c.cy);
+  auto d2 = [](float at, float off, float t) {
+    const float d = at + off - t;
+    return d * d;
+  };
+  // bit k: sites 32 g + k .. + one - 1 of row y are open
+  auto run = [&](int y, int g) -> unsigned {
+    const uint2 *seg = a.seg + (size_t)y * a.SW;
+    const uint2 s0 = g < a.SW ? ld_seg(seg + g) : make_uint2(0u, 0u);
+    const uint2 s1 = g + 1 < a.SW ? ld_seg(seg + g + 1) : make_uint2(0u, 0u);
+    uint64_t t = (uint64_t)open_word(a, q, y, g, s0) | (uint64_t)open_word(a, q, y, g + 1, s1) << 32;
+    for (int s = 1; s < one;) {
+      const int d = min(s, one - s);
+      t &= t >> d;
+      s += d;
     }
-    if (!any) break;
+    return (unsigned)t;
+  };
+  auto anchors = [&](int ay, int g) -> unsigned {
+    unsigned v = ~0u;
+    for (int y0 = 0; y0 < c.h && v; y0 += 32) {
+      unsigned r = ~0u;
+      if (y0 + lane < c.h) {
+        const int y = ay + y0 + lane;
+        r = run(y, g);
+        for (int k = 1; 32 * (k + 1) <= c.w && r; ++k) r &= run(y, g + k);
+        const int rest = c.w & 31, k = c.w >> 5;
+        if (c.w > 32 && rest && r) r &= (run(y, g + k - 1) >> rest) | (run(y, g + k) << (32 - rest));
+      }
+      v &= __reduce_and_sync(kFull, r);
+    }
+    return v;
+  };
+  float most = kInf;
+  auto found = [&](int x, int ay) {
+    b.take(__dadd_rn(col_dx2(c, x), row_dy2(c, ay)), ay * a.W + x);
+    const unsigned mine = __float_as_uint((d2((float)x, ox, tx) + d2((float)ay, oy, ty)) * kOver);
+    if (lane == 0) atomicMin(least, mine);
+  };
+  for (int k = warp; k <= 2 * rows; k += kLpWarps) {
+    most = __uint_as_float(*(volatile unsigned *)least);
+    const float away = (float)((k + 1) >> 1) - 0.5f;
+    if (k && away * away > most) break;
+    const int ay = c.cy + ((k & 1) ? -(k + 1) / 2 : k / 2);
+    if (ay < 0 || ay >= c.AH) continue;
+    const float dy2 = d2((float)ay, oy, ty);
+    if (dy2 > most) continue;
+    const double far = row_dy2(c, ay);
+    const int skip = c0 > far ? max((int)sqrtf((float)__dsub_rn(c0, far)) - 2, 0) : 0;
+    const int gr = min(max(c.fx + skip, 0), c.AW - 1) >> 5, gl = max(c.fx - skip, 0) >> 5;
+    for (int g = gr; 32 * g < c.AW; ++g) {
+      most = __uint_as_float(*(volatile unsigned *)least);
+      if (g > gr && d2((float)(32 * g), ox, tx) + dy2 > most) break;
+      const int f = c.fx - 32 * g;
+      const unsigned v = anchors(ay, g) & (f < 0 ? ~0u : f >= 31 ? 0u : ~0u << (f + 1));
+      if (v) {
+        found(32 * g + __ffs(v) - 1, ay);
+        break;
+      }
+    }
+    for (int g = gl; g >= 0; --g) {
+      most = __uint_as_float(*(volatile unsigned *)least);
+      if (g < gl && d2((float)(32 * g + 31), ox, tx) + dy2 > most) break;
+      const int f = c.fx - 32 * g;
+      const unsigned v = anchors(ay, g) & (f < 0 ? 0u : f >= 31 ? ~0u : (2u << f) - 1u);
+      if (v) {
+        found(32 * g + 31 - __clz(v), ay);
+        break;
+      }
+    }
   }
-  return b.warp_min();
+  return b;
 }
 
 // Targets in the same square of 1 / tie_scale sites have one key.
@@ -466,7 +520,7 @@ __global__ void __launch_bounds__(kLpWarps * 32) k_lp_choose(const LpArgs a) {
     Best b = no_best();
     if (placeable(c)) {
       if (c.w <= 32 && c.h <= 16) b = search_block(a, q, c, c0, warp, lane, &least);
-      else if (warp == 0) b = search_any(a, q, c, lane);
+      else b = search_large(a, q, c, c0, warp, lane, &least);
     }
     b = b.warp_min();
     if (lane == 0) sbest[warp] = b;

@@ -386,3 +386,34 @@ def test_run_with_device_legalizer_and_reference_field(cells, side, bins):
     a = E.place_electro(nl, chip, cfg, E.RunOptions(legal_mode=0))
     b = E.place_electro(nl, chip, cfg, E.RunOptions(legal_mode=1))
     assert a.hpwl == b.hpwl and np.array_equal(a.bel_tile, b.bel_tile) and a.trajectory == b.trajectory
+
+
+@pytest.mark.parametrize("w,h", [(32, 17), (33, 1), (33, 33), (40, 40), (63, 31), (64, 32), (65, 3), (96, 34), (97, 64),
+                                 (130, 65), (1, 100)])
+@pytest.mark.parametrize("blocked", [0, 25])
+def test_device_legalizer_large_macros(w, h, blocked):
+    """Footprints beyond what the word search takes, around multiples of 32 along
+    both axes, on one spot, spread, and beside blocked sites: against the
+    oracle's exhaustive scan."""
+    rng = np.random.default_rng(w * 1000 + h + blocked)
+    W, H, macros, units = 300, 170, 4, 150
+    cw, ch = np.ones(macros + units, np.uint8), np.ones(macros + units, np.uint8)
+    cw[:macros], ch[:macros] = [w, w, max(w - 1, 1), w], [h, max(h - 1, 1), h, h]
+    fx, fy = rng.integers(0, W, blocked).astype(np.int32), rng.integers(0, H, blocked).astype(np.int32)
+    nl = E.Netlist(num_cells=macros + units, net_offsets=np.array([0, 2], np.uint32),
+                   pin_cell=np.array([0, 1], np.uint32), fixed_x=fx, fixed_y=fy,
+                   fixed_on_logic=np.ones(blocked, np.uint8), cell_w=cw, cell_h=ch)
+    chip = E.Chip(W, H)
+    orc = Oracle(nl, chip)
+    n = macros + units
+    with E.PlacementContext(nl, chip) as ctx:
+        for x, y in ((np.full(n, 0.47 * W), np.full(n, 0.53 * H)), (np.zeros(n), np.full(n, H - 1.0)),
+                     (rng.uniform(0, W - 1, n), rng.uniform(0, H - 1, n))):
+            st, ox, oy, od = orc.legalize(x.astype(np.float32), y.astype(np.float32), 0)
+            if st != 0:
+                with pytest.raises(E.NoBelsAvailable):
+                    ctx.legalize_device(x, y)
+                continue
+            gx, gy, gd, _ = ctx.legalize_device(x, y)
+            assert np.array_equal(gx, ox) and np.array_equal(gy, oy)
+            assert gd == od
