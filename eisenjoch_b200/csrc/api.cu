@@ -1483,7 +1483,7 @@ void prepare_slot(eplace_ctx *c, LegalSlot &L) {
   a.status = &L.out.p->status;
   a.cancel = &L.out.p->cancel;
   a.max_rounds = 2 * n_mac + 64;
-  CK(lp_build_graph(a, L.graph, L.stream));
+  CK(lp_build_graph(a, L.graph));
   L.gen = c->load_gen;
 }
 

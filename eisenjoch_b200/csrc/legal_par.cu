@@ -814,10 +814,7 @@ __global__ void __launch_bounds__(kLpChunk) k_lp_pending(const LpArgs a) {
     const uint32_t npend = before + mine + __popc(m), ties = a.st->ties, units = a.n - a.n_mac;
     a.st->npend = npend;
     const bool tied = 64ull * ties >= units && 5ull * ties >= npend;  // (the rule: at k_lp_lists)
-    if (tied) {
-      a.st->tied = 1u;
-      cudaGraphSetConditional(a.windows, 1u);
-    }
+    if (tied) a.st->tied = 1u;
     if (tied || !few_left(a)) cudaGraphSetConditional(a.many, 1u);
   }
 }
@@ -825,6 +822,7 @@ __global__ void __launch_bounds__(kLpChunk) k_lp_pending(const LpArgs a) {
 // Undoes the claims of the unit cells when too many are left over.
 __global__ void __launch_bounds__(256) k_lp_undo(const LpArgs a) {
   const int lane = threadIdx.x & 31;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && a.st->tied) cudaGraphSetConditional(a.windows, 1u);
   const int nseg = a.SW * a.H;
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nseg; i += (gridDim.x * blockDim.x) >> 5) {
     const bool open = a.own[(size_t)32 * i + lane] >= (int32_t)a.n_mac;  // (kNone too)
@@ -1240,8 +1238,8 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
 // where both ways take about as long: 200k cells, 2 % in a corner 29 -> 18 ms,
 // 30k 2.8 -> 2.6; 16 spots of 30k cells 23 -> 3.4; but a wide pile of 30k cells
 // of which 10 % are on one spot would take 14 -> 70 (40 %: 86 -> 64): its other
-// cells use up their lists too.  A loop that is not entered costs a graph
-// without other conditional nodes 15 us (3k spread cells 135 -> 150 us).
+// cells use up their lists too.  A loop that is not entered costs some 12 us: it
+// stands inside the if node where there is one; 3k spread cells 135 -> 150 us.
 
 // A CTA per cell of the window: the open sites of least cost, in order.
 __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_lists(const LpArgs a) {
@@ -1528,7 +1526,7 @@ LpGraph::~LpGraph() {
   if (graph) cudaGraphDestroy(graph);
 }
 
-cudaError_t lp_build_graph(LpArgs a, LpGraph &g, cudaStream_t cs) {
+cudaError_t lp_build_graph(LpArgs a, LpGraph &g) {
   if (g.exec) cudaGraphExecDestroy(g.exec);
   if (g.graph) cudaGraphDestroy(g.graph);
   g.exec = nullptr;
@@ -1537,45 +1535,45 @@ cudaError_t lp_build_graph(LpArgs a, LpGraph &g, cudaStream_t cs) {
   cudaGraph_t graph = nullptr;
   if ((e = cudaGraphCreate(&graph, 0)) != cudaSuccess) return e;
   g.graph = graph;
-  cudaGraphNode_t tail = nullptr;
-  auto add = [&](const void *func, unsigned grid, unsigned block) -> cudaError_t {
+  // Nodes of a graph, one after the other.
+  struct Chain {
+    cudaGraph_t graph;
+    cudaGraphNode_t tail = nullptr;
+  };
+  auto add = [&](Chain &c, void (*func)(LpArgs), unsigned grid, unsigned block, unsigned shared = 0) -> cudaError_t {
     void *args[] = {&a};
     cudaKernelNodeParams kp = {};
-    kp.func = const_cast<void *>(func);
+    kp.func = reinterpret_cast<void *>(func);
     kp.gridDim = dim3(grid);
     kp.blockDim = dim3(block);
+    kp.sharedMemBytes = shared;
     kp.kernelParams = args;
     cudaGraphNode_t node;
-    const cudaError_t r = cudaGraphAddKernelNode(&node, graph, tail ? &tail : nullptr, tail ? 1 : 0, &kp);
-    tail = node;
+    const cudaError_t r = cudaGraphAddKernelNode(&node, c.graph, c.tail ? &c.tail : nullptr, c.tail ? 1 : 0, &kp);
+    c.tail = node;
     return r;
   };
-  auto add_cond = [&](cudaGraphConditionalHandle handle, cudaGraphConditionalNodeType type, cudaGraph_t *body) {
+  auto add_cond = [&](Chain &c, cudaGraphConditionalHandle handle, cudaGraphConditionalNodeType type, Chain *body) {
     cudaGraphNodeParams cp = {};
     cp.type = cudaGraphNodeTypeConditional;
     cp.conditional.handle = handle;
     cp.conditional.type = type;
     cp.conditional.size = 1;
     cudaGraphNode_t node;
-    const cudaError_t r = cudaGraphAddNode(&node, graph, tail ? &tail : nullptr, tail ? 1 : 0, &cp);
-    tail = node;
-    if (r == cudaSuccess) *body = cp.conditional.phGraph_out[0];
+    const cudaError_t r = cudaGraphAddNode(&node, c.graph, c.tail ? &c.tail : nullptr, c.tail ? 1 : 0, &cp);
+    c.tail = node;
+    if (r == cudaSuccess) body->graph = cp.conditional.phGraph_out[0];
     return r;
   };
-  auto end_body = [&] {  // of a body captured from cs
-    const cudaError_t launched = cudaGetLastError();
-    cudaGraph_t captured = nullptr;
-    const cudaError_t r = cudaStreamEndCapture(cs, &captured);
-    return launched != cudaSuccess ? launched : r;
+  auto handle = [](cudaGraphConditionalHandle *h, const Chain &c, unsigned value) {
+    return cudaGraphConditionalHandleCreate(h, c.graph, value, cudaGraphCondAssignDefault);
   };
   const size_t sites = (size_t)a.W * a.H;
   const unsigned site_grid = (unsigned)((sites + 255) / 256 < 1184 ? (sites + 255) / 256 : 1184);
-  if (a.n_mac &&
-      (e = cudaGraphConditionalHandleCreate(&a.handle, graph, 1, cudaGraphCondAssignDefault)) != cudaSuccess)
-    return e;
   const uint32_t units = a.n - a.n_mac;
-  constexpr int kTakeShared = (int)(sizeof(int32_t) * kUnitWindow * (kLpRingMax + 1));
-  if ((e = cudaFuncSetAttribute(k_lp_take, cudaFuncAttributeMaxDynamicSharedMemorySize, kTakeShared)) != cudaSuccess)
+  constexpr unsigned kTakeShared = (unsigned)(sizeof(int32_t) * kUnitWindow * (kLpRingMax + 1));
+  if ((e = cudaFuncSetAttribute(k_lp_take, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTakeShared)) !=
+      cudaSuccess)
     return e;
   const bool at_once = units >= kNearFrom;
   // Few cells: targets that differ by less than a tenth of a site crowd like equal
@@ -1583,60 +1581,47 @@ cudaError_t lp_build_graph(LpArgs a, LpGraph &g, cudaStream_t cs) {
   a.tie_scale = at_once ? 64.0f : 16.0f;
   a.tie_least = units / (at_once ? 64 : 32) > 32 ? units / (at_once ? 64 : 32) : 32;
   a.tie_limit = at_once ? 0 : units / 10 > 32 ? units / 10 : 32;
-  if (at_once &&
-      (e = cudaGraphConditionalHandleCreate(&a.many, graph, 0, cudaGraphCondAssignDefault)) != cudaSuccess)
-    return e;
-  if (units && (e = cudaGraphConditionalHandleCreate(&a.windows, graph, 0, cudaGraphCondAssignDefault)) != cudaSuccess)
-    return e;
-  if ((e = add((const void *)k_lp_init, site_grid, 256)) != cudaSuccess) return e;
-  if (a.n_mac) {
-    cudaGraph_t body;
-    if ((e = add_cond(a.handle, cudaGraphCondTypeWhile, &body)) != cudaSuccess) return e;
-    // The round, captured into the loop body.
-    if ((e = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
-        cudaSuccess)
-      return e;
-    const uint32_t most = a.n_mac < kLpWindow ? a.n_mac : kLpWindow;
-    const unsigned grid = (most + kLpWarps - 1) / kLpWarps;
-    k_lp_choose<<<most < 592 ? most : 592, kLpWarps * 32, 0, cs>>>(a);
-    k_lp_claim<<<grid, kLpWarps * 32, 0, cs>>>(a);
-    if ((e = end_body()) != cudaSuccess) return e;
-  }
-  if ((e = add((const void *)k_lp_segments, site_grid, 256)) != cudaSuccess) return e;
-  // the loop over the windows
-  auto add_windows = [&]() -> cudaError_t {
-    cudaGraph_t body;
+  Chain top{graph};
+  // The loop over the windows of unit cells, entered when some kernel of the
+  // chain before it has set its handle.
+  auto add_windows = [&](Chain &c) -> cudaError_t {
+    Chain body{};
     cudaError_t r;
-    if ((r = add_cond(a.windows, cudaGraphCondTypeWhile, &body)) != cudaSuccess) return r;
-    if ((r = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
-        cudaSuccess)
-      return r;
-    k_lp_lists<<<units < kUnitWindow ? units : kUnitWindow, kUnitWarps * 32, 0, cs>>>(a);
-    k_lp_take<<<1, kUnitWindow, kTakeShared, cs>>>(a);
-    return end_body();
+    if ((r = add_cond(c, a.windows, cudaGraphCondTypeWhile, &body)) != cudaSuccess) return r;
+    if ((r = add(body, k_lp_lists, units < kUnitWindow ? units : kUnitWindow, kUnitWarps * 32)) != cudaSuccess) return r;
+    return add(body, k_lp_take, 1, kUnitWindow, kTakeShared);
   };
+  if (a.n_mac && (e = handle(&a.handle, top, 1)) != cudaSuccess) return e;
+  if (at_once && (e = handle(&a.many, top, 0)) != cudaSuccess) return e;
+  if (units && !at_once && (e = handle(&a.windows, top, 0)) != cudaSuccess) return e;
+  if ((e = add(top, k_lp_init, site_grid, 256)) != cudaSuccess) return e;
+  if (a.n_mac) {
+    Chain body{};
+    if ((e = add_cond(top, a.handle, cudaGraphCondTypeWhile, &body)) != cudaSuccess) return e;
+    const uint32_t most = a.n_mac < kLpWindow ? a.n_mac : kLpWindow;
+    if ((e = add(body, k_lp_choose, most < 592 ? most : 592, kLpWarps * 32)) != cudaSuccess) return e;
+    if ((e = add(body, k_lp_claim, (most + kLpWarps - 1) / kLpWarps, kLpWarps * 32)) != cudaSuccess) return e;
+  }
+  if ((e = add(top, k_lp_segments, site_grid, 256)) != cudaSuccess) return e;
   if (units && !at_once) {
-    if ((e = add((const void *)k_lp_units<true>, units, kUnitWarps * 32)) != cudaSuccess) return e;
-    if ((e = add_windows()) != cudaSuccess) return e;
+    if ((e = add(top, k_lp_units<true>, units, kUnitWarps * 32)) != cudaSuccess) return e;
+    if ((e = add_windows(top)) != cudaSuccess) return e;
   } else if (units) {
     const uint32_t chunks = (uint32_t)lp_chunks(units);
-    if ((e = add((const void *)k_lp_near, (units + 7) / 8, 256)) != cudaSuccess) return e;
-    if ((e = add((const void *)k_lp_count, chunks, kLpChunk)) != cudaSuccess) return e;
-    if ((e = add((const void *)k_lp_pending, chunks, kLpChunk)) != cudaSuccess) return e;
-    cudaGraph_t body;
-    if ((e = add_cond(a.many, cudaGraphCondTypeIf, &body)) != cudaSuccess) return e;
-    if ((e = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
-        cudaSuccess)
-      return e;
-    k_lp_undo<<<site_grid, 256, 0, cs>>>(a);
-    k_lp_units<true><<<units, kUnitWarps * 32, 0, cs>>>(a);
-    if ((e = end_body()) != cudaSuccess) return e;
-    if ((e = add_windows()) != cudaSuccess) return e;
-    if ((e = add((const void *)k_lp_units<false>, 296, kUnitWarps * 32)) != cudaSuccess)
-      return e;
+    if ((e = add(top, k_lp_near, (units + 7) / 8, 256)) != cudaSuccess) return e;
+    if ((e = add(top, k_lp_count, chunks, kLpChunk)) != cudaSuccess) return e;
+    if ((e = add(top, k_lp_pending, chunks, kLpChunk)) != cudaSuccess) return e;
+    // too many left over, or ties: all of them again, in order or in windows
+    Chain body{};
+    if ((e = add_cond(top, a.many, cudaGraphCondTypeIf, &body)) != cudaSuccess) return e;
+    if ((e = handle(&a.windows, body, 0)) != cudaSuccess) return e;
+    if ((e = add(body, k_lp_undo, site_grid, 256)) != cudaSuccess) return e;
+    if ((e = add(body, k_lp_units<true>, units, kUnitWarps * 32)) != cudaSuccess) return e;
+    if ((e = add_windows(body)) != cudaSuccess) return e;
+    if ((e = add(top, k_lp_units<false>, 296, kUnitWarps * 32)) != cudaSuccess) return e;
   }
-  if ((e = add((const void *)k_lp_result, site_grid, 256)) != cudaSuccess) return e;
-  if ((e = add((const void *)k_lp_finish, 1, kSumThreads)) != cudaSuccess) return e;
+  if ((e = add(top, k_lp_result, site_grid, 256)) != cudaSuccess) return e;
+  if ((e = add(top, k_lp_finish, 1, kSumThreads)) != cudaSuccess) return e;
   return cudaGraphInstantiate(&g.exec, graph, 0);
 }
 

@@ -116,6 +116,6 @@ struct LpGraph {
 };
 
 // Builds the graph for args `a` (the handles are filled in).
-cudaError_t lp_build_graph(LpArgs a, LpGraph &g, cudaStream_t capture_stream);
+cudaError_t lp_build_graph(LpArgs a, LpGraph &g);
 
 }  // namespace eplace
