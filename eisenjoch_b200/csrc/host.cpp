@@ -820,7 +820,9 @@ eplace_status Legalizer::run(const float *x, const float *y, size_t stride, int3
         const int32_t cy = std::min(std::max((int32_t)floor_exact(uy + 0.5), 0), AH - 1);
         const int32_t fa = std::min(std::max((int32_t)floor_exact(ux), -1), AW - 1);
         const int32_t lastw = (AW - 1) >> 6;
-        auto valid_word = [&](int32_t ay, int32_t j) -> uint64_t {
+        // bit k: sites 64 j + k .. + n - 1 (n <= 64) are free in rows ay .. ay + h - 1
+        auto runs = [&](int32_t ay, int32_t j, int n) -> uint64_t {
+          if (j >= WR) return 0;
           uint64_t m = ~0ull, mn = ~0ull;
           for (int dy = 0; dy < h; ++dy) {
             const uint64_t *r = fm + (size_t)(ay + dy) * WR;
@@ -828,7 +830,16 @@ eplace_status Legalizer::run(const float *x, const float *y, size_t stride, int3
             mn &= (j + 1 < WR) ? r[j + 1] : 0ull;
           }
           uint64_t v = m;
-          for (int k = 1; k < w; ++k) v &= (m >> k) | (mn << (64 - k));
+          for (int k = 1; k < n; ++k) v &= (m >> k) | (mn << (64 - k));
+          return v;
+        };
+        auto valid_word = [&](int32_t ay, int32_t j) -> uint64_t {
+          uint64_t v = runs(ay, j, std::min(w, 64));
+          if (w > 64) {  // the runs of 64 behind it, the last one shifted
+            const int full = w >> 6, rest = w & 63;
+            for (int k = 1; k < full; ++k) v &= runs(ay, j + k, 64);
+            if (rest) v &= (runs(ay, j + full - 1, 64) >> rest) | (runs(ay, j + full, 64) << (64 - rest));
+          }
           if (j == lastw && ((AW - 1) & 63) != 63) v &= (2ull << ((AW - 1) & 63)) - 1;
           return v;
         };

@@ -120,6 +120,32 @@ def test_host_legaliser_equals_reference_scan(macro, fixed):
         assert E.placer.hpwl_host(nl, chip, sx, sy) == o.hpwl(sx, sy)
 
 
+@pytest.mark.parametrize("w,h", [(63, 3), (64, 2), (65, 3), (96, 7), (127, 2), (128, 4), (129, 2), (200, 3)])
+@pytest.mark.parametrize("blocked", [0, 20])
+def test_host_legaliser_wide_macros(w, h, blocked):
+    """Macros around multiples of 64 sites wide: every site of a block is free."""
+    rng = np.random.default_rng(w + h + blocked)
+    W, H, macros, units = 450, 40, 4, 120
+    cw, ch = np.ones(macros + units, np.uint8), np.ones(macros + units, np.uint8)
+    cw[:macros], ch[:macros] = [w, w, w - 1, w], [h, 1, h, h]
+    fx, fy = rng.integers(0, W, blocked).astype(np.int32), rng.integers(0, H, blocked).astype(np.int32)
+    n = macros + units
+    nl = E.Netlist(num_cells=n, net_offsets=np.array([0, 2], np.uint32), pin_cell=np.array([0, 1], np.uint32),
+                   fixed_x=fx, fixed_y=fy, fixed_on_logic=np.ones(blocked, np.uint8), cell_w=cw, cell_h=ch)
+    chip = E.Chip(W, H)
+    o = O.Oracle(nl, chip)
+    for x, y in ((np.full(n, 0.47 * W), np.full(n, 0.53 * H)), (np.zeros(n), np.full(n, H - 1.0)),
+                 (rng.uniform(0, W - 1, n), rng.uniform(0, H - 1, n))):
+        x, y = x.astype(np.float32), y.astype(np.float32)
+        st, ox, oy, od = o.legalize(x, y, 0)
+        if st != 0:
+            with pytest.raises(E.NoBelsAvailable):
+                E.placer.legalize_host(nl, chip, x, y)
+            continue
+        sx, sy, d = E.placer.legalize_host(nl, chip, x, y)
+        assert np.array_equal(sx, ox) and np.array_equal(sy, oy) and d == od
+
+
 @pytest.mark.parametrize("seed", [1, 7, 99])
 def test_host_initial_placement_equals_oracle(seed):
     nl, chip = _case(22, 400, 32, 0.05, 30)
