@@ -184,8 +184,8 @@ __global__ void __launch_bounds__(128, 1)
     // no kernel writes: its loads of the first ring are under way while the
     // kernel before this one ends.  (These products are bound by latency up to
     // 512^2 bins: start of the CTA, first loads, epilogue.  With this and the
-    // overlapped launches an iteration takes 34.4 -> 33.9 us at 128^2 bins, 45.6
-    // -> 41.9 at 256^2, 73.5 -> 65.7 at 512^2, 198 -> 195 at 1024^2.)
+    // overlapped launches an iteration takes 34.4 -> 34.5 us at 128^2 bins, 45.6
+    // -> 41.8 at 256^2, 73.5 -> 64.2 at 512^2, 198 -> 193 at 1024^2.)
     auto load_a = [&](int kb) {
       uint8_t *st = smem + (kb % STAGES) * S::STAGE_BYTES;
       tma_load_2d(st, &om.a_hi, kb * BK, m0, &full[kb % STAGES]);

@@ -1767,7 +1767,7 @@ cudaError_t launch_step_split(const StepArgs &a, int grid, int block, cudaStream
 }
 
 cudaError_t launch_snapshot(const SnapArgs &a, cudaStream_t s) {
-  const unsigned g = (a.n + 255) / 256;
+  const unsigned g = (a.n + 255) / 256;  // up to 4 CTAs for each of the 148 SMs; the kernel loops
   k_snapshot<<<g < 1 ? 1 : g < 592 ? g : 592, 256, 0, s>>>(a);
   return cudaGetLastError();
 }

@@ -40,7 +40,7 @@
 // A 200k-cell checkpoint (5 % macros, half of the cells in six piles): 150 to
 // 200 ms as rounds of candidate lists, disturbance passes and one CTA's serial
 // pass over the cells whose lists interact (a hundred rounds and more of 20
-// launches), 7.3 ms in this form (macros 2.2 ms in 54 rounds, units 4.7, the
+// launches), 7.4 ms in this form (macros 2.3 ms in 54 rounds, units 4.7, the
 // displacement's sum 0.33).  The checkpoint at the end of such a run, cells
 // spread: 1.3 to 3 ms (macros 0.6, units 0.2 to 2.1 by the design, sum 0.26).
 #include <cuda_runtime.h>
@@ -1225,12 +1225,12 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
 // not change: first each cell's list, then each takes of its list what the
 // cells before it leave.  A window ends early at the first cell whose list is
 // used up: after some 50 cells of one target.
-// ms, in the order without windows -> with (before deferred acceptance, as
-// rounds of lists and a serial pass), unit cells alone: all on one spot 1k 11.0
+// ms, in order without windows -> with (in brackets as rounds of lists and a
+// serial pass, before deferred acceptance), unit cells alone: all on one spot 1k 11.0
 // -> 0.9 (2.2), 30k 419 -> 27 (87), 200k 3697 -> 192 (1173); 40 % in a corner,
 // the others spread: 5k 17 -> 2.1 (6.5), 60k 308 -> 24 (84).  Runs with the
-// reference's field, 5k cells, 300 iterations 1297 -> 32 (48), 30k, 100
-// iterations, 4568 -> 290 (285).  Bound by the list kernel: two dependent
+// reference's field, 5k cells, 300 iterations 1297 -> 31 (48), 30k with macros,
+// 100 iterations, 4568 -> 290 (285).  Bound by the list kernel: two dependent
 // passes over the rows, 20 us a window, and two launches.
 // The rule (lp_build_graph, k_lp_pending): ties (cells of a target that has
 // tie_least or more) are at least 1/64 of the unit cells and 1/5 of those left
@@ -1568,6 +1568,8 @@ cudaError_t lp_build_graph(LpArgs a, LpGraph &g) {
   auto handle = [](cudaGraphConditionalHandle *h, const Chain &c, unsigned value) {
     return cudaGraphConditionalHandleCreate(h, c.graph, value, cudaGraphCondAssignDefault);
   };
+  // (grids of 8, 4 and 2 CTAs for each of this chip's 148 SMs: what is resident;
+  // the kernels loop, so any other number gives the same)
   const size_t sites = (size_t)a.W * a.H;
   const unsigned site_grid = (unsigned)((sites + 255) / 256 < 1184 ? (sites + 255) / 256 : 1184);
   const uint32_t units = a.n - a.n_mac;
