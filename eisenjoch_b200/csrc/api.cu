@@ -268,7 +268,9 @@ struct LegalSlot {
   DBuf<uint32_t> tie_count;
   DBuf<int32_t> list;
   DBuf<LpState> lst;
+  LpArgs args;          // what its graphs are built from
   LpGraph graph;        // the whole legalisation: rounds in a device-side loop
+  LpGraph tied;         // the same with windows, built when a first legalisation asks for it (kLpTied)
   uint64_t gen = ~0ull;  // problem load this slot is prepared for
   cudaStream_t stream = nullptr;
   cudaEvent_t snap = nullptr, start = nullptr, done = nullptr;
@@ -1483,7 +1485,9 @@ void prepare_slot(eplace_ctx *c, LegalSlot &L) {
   a.status = &L.out.p->status;
   a.cancel = &L.out.p->cancel;
   a.max_rounds = 2 * n_mac + 64;
-  CK(lp_build_graph(a, L.graph));
+  CK(lp_build_graph(a, L.graph, false));
+  L.args = a;
+  L.tied.clear();
   L.gen = c->load_gen;
 }
 
@@ -1507,11 +1511,14 @@ LegalSlot *new_legal_slot(eplace_ctx *c) {
 // Legalises slot L's positions and takes the HPWL of the binding, all on
 // L's stream, then copies the 24-byte outcome to pinned memory and records
 // L.done.  The caller has already ordered the positions before this work.
-void launch_gpu_legal(eplace_ctx *c, LegalSlot &L) {
+// tied: with the graph that has windows; one without them may end with status
+// kLpTied, and the same positions are to be launched again with it.
+void launch_gpu_legal(eplace_ctx *c, LegalSlot &L, bool tied) {
   const HostProblem &hp = c->hp;
+  if (tied && !L.tied.exec) CK(lp_build_graph(L.args, L.tied, true));
   CK(cudaMemsetAsync(L.out.p, 0, sizeof(LegalOut), L.stream));
   CK(cudaEventRecord(L.start, L.stream));
-  CK(cudaGraphLaunch(L.graph.exec, L.stream));
+  CK(cudaGraphLaunch(tied ? L.tied.exec : L.graph.exec, L.stream));
   HpwlArgs h{c->net_off.p, c->pin_cell.p, c->has_driver.p, L.loc.p, hp.NN, &L.out.p->hpwl};
   if (hp.NN) CK(launch_hpwl(h, grid_for((int)hp.NN, kHpwlBlock, c->num_sms * 2), L.stream));
   CK(cudaMemcpyAsync(L.hout.p, L.out.p, sizeof(LegalOut), cudaMemcpyDeviceToHost, L.stream));
@@ -2231,6 +2238,15 @@ struct JobState {
             CK(q);
           }
           const LegalOut &o = *L.hout.p;
+          if (o.status == kLpTied) {  // the run's later checkpoints will be too: those that have ended so go on with it
+            legal_tied = true;
+            for (size_t k = fold_next; k < cps.size(); ++k) {
+              if (cps[k]->discard || cps[k]->slot < 0) continue;
+              LegalSlot &M = *c->lslots[cps[k]->slot];
+              if (cudaEventQuery(M.done) == cudaSuccess && M.hout.p->status == kLpTied) launch_gpu_legal(c, M, true);
+            }
+            continue;
+          }
           float lms = 0.f;
           if (cudaEventElapsedTime(&lms, L.start, L.done) == cudaSuccess) cp->secs = 1e-3 * lms;
           cp->st = o.status == 0 ? EPLACE_OK : (o.status == 1 ? EPLACE_ERR_NO_BELS : EPLACE_ERR_PLACEMENT_FAILED);
@@ -2341,7 +2357,7 @@ struct JobState {
         launch_snapshot_stage(c, L.pos.p, c->snap_sc[slot]->p);
         CK(cudaEventRecord(L.snap, s));
         CK(cudaStreamWaitEvent(L.stream, L.snap, 0));
-        launch_gpu_legal(c, L);
+        launch_gpu_legal(c, L, legal_tied);
         cps.push_back(std::move(cp));
       } else {
         hs = take_snap();
@@ -2564,7 +2580,8 @@ struct JobState {
   std::vector<Chunk> chunks;
   int inflight = 1;
   std::vector<int> free_slots;
-  bool discarded = false;  // a legalisation has been cancelled
+  bool discarded = false;   // a legalisation has been cancelled
+  bool legal_tied = false;  // one has found too many cells on one target for the graph without windows
   uint64_t launched_iters = 0;
   struct Pending {
     size_t chunk;
@@ -3294,10 +3311,15 @@ eplace_status eplace_stage_legalize(eplace_ctx *c, const float *x, const float *
     prepare_slot(c, *L);
     c->io_in.reserve(2 * sizeof(float) * io_pitch(hp.N));
     io_in(c, L->stream, static_cast<float *>(c->io_in.p), {{x, y}}, {L->pos.p});
-    launch_gpu_legal(c, *L);
-    const IoArgs io = io_out(c, L->stream, {reinterpret_cast<float2 *>(L->sites.p)});  // moved as they are
+    launch_gpu_legal(c, *L, false);
+    IoArgs io = io_out(c, L->stream, {reinterpret_cast<float2 *>(L->sites.p)});  // moved as they are
     CK(cudaStreamSynchronize(L->stream));
     const LegalOut &o = *L->hout.p;
+    if (o.status == kLpTied) {
+      launch_gpu_legal(c, *L, true);
+      io = io_out(c, L->stream, {reinterpret_cast<float2 *>(L->sites.p)});
+      CK(cudaStreamSynchronize(L->stream));
+    }
     if (o.status != 0) {
       set_err(c, o.status == 1 ? "logic" : "device legaliser stopped at an internal limit");
       return o.status == 1 ? EPLACE_ERR_NO_BELS : EPLACE_ERR_PLACEMENT_FAILED;

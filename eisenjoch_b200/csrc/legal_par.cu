@@ -467,6 +467,44 @@ __device__ __forceinline__ unsigned long long tie_key(const LpArgs &a, float2 p)
          (unsigned)(int)floorf(p.y * a.tie_scale);
 }
 
+// Few unit cells: whether enough of them share targets, by a CTA, from 512 of them
+// at even distances (all of fewer).  Ties are cells whose target a 32nd of these
+// have (or what 32 of all are, of few); enough is a tenth.
+constexpr uint32_t kTieSample = 512;
+__device__ void sample_ties(const LpArgs &a) {
+  constexpr uint32_t kMask = 2 * kTieSample - 1;
+  __shared__ unsigned long long key[kMask + 1];
+  __shared__ uint32_t count[kMask + 1], ties;
+  const uint32_t tid = threadIdx.x, units = a.n - a.n_mac, m = units < kTieSample ? units : kTieSample;
+  for (uint32_t h = tid; h <= kMask; h += blockDim.x) {
+    key[h] = kNoTie;
+    count[h] = 0u;
+  }
+  if (tid == 0) ties = 0u;
+  __syncthreads();
+  for (uint32_t k = tid; k < m; k += blockDim.x) {
+    const uint32_t i = (uint32_t)((uint64_t)k * units / m);
+    const unsigned long long t = tie_key(a, a.pos[a.order[a.n_mac + i]]);
+    if (t == kNoTie) continue;
+    uint32_t h = (uint32_t)((t * 0x9e3779b97f4a7c15ull) >> 32) & kMask;
+    while (true) {  // (half of the table stays empty)
+      const unsigned long long was = atomicCAS(&key[h], kNoTie, t);
+      if (was == kNoTie || was == t) break;
+      h = (h + 1) & kMask;
+    }
+    atomicAdd(&count[h], 1u);
+  }
+  __syncthreads();
+  const uint32_t few = 32u * m / units, least = few > m / 32 ? few : m / 32;
+  for (uint32_t h = tid; h <= kMask; h += blockDim.x)
+    if (count[h] >= least) atomicAdd(&ties, count[h]);
+  __syncthreads();
+  if (tid != 0 || ties < least || 10u * ties < m) return;
+  a.st->tied = 1u;
+  if (a.tie_loop) cudaGraphSetConditional(a.windows, 1u);
+  else atomicMax(&a.st->status, kLpTied);
+}
+
 __global__ void __launch_bounds__(256) k_lp_init(const LpArgs a) {
   const int lane = threadIdx.x & 31;
   const int nseg = a.SW * a.H;
@@ -487,12 +525,16 @@ __global__ void __launch_bounds__(256) k_lp_init(const LpArgs a) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < hints; i += gridDim.x * blockDim.x) a.hint[i] = 0ull;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n - a.n_mac; i += gridDim.x * blockDim.x)
     a.cand[(size_t)kLpCand * i] = -1;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= a.tie_mask; i += gridDim.x * blockDim.x) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; !a.tie_few && i <= a.tie_mask; i += gridDim.x * blockDim.x) {
     a.tie_key[i] = kNoTie;
     a.tie_count[i] = 0u;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0)
     *a.st = LpState{0u, 0u, (uint32_t)kNone, 0u, 0u, {min(a.n_mac, kLpWindow), 0u}, 0u, 0u, 0u, 0u, 0u, 0};
+  if (a.tie_few && blockIdx.x == 0) {
+    __syncthreads();  // the state is written
+    sample_ties(a);
+  }
 }
 
 // A round, first half: each macro of the work list (whose choice may have
@@ -645,9 +687,9 @@ __global__ void __launch_bounds__(kLpWarps * 32) k_lp_claim(const LpArgs a) {
 // the largest order index that cleared one of them.  A segment with x == 0 and y < q has
 // no site open to q; with y < q the bits of x are the open sites.
 //
-// Counts the unit cells of each key (the table has twice as many entries or
-// more; a warp adds those of one key together), and those of the keys that have
-// tie_least or more; of the cells that k_lp_near left over, where it is tried.
+// Counts a unit cell that k_lp_near left over under its key (the table has twice
+// as many entries as cells or more; a warp adds those of one key together), and
+// the cells of the keys that have tie_least or more.
 __device__ void count_tie(const LpArgs &a, uint32_t i, bool in) {  // a warp; in: unit cell i counts
   const unsigned long long key = in ? tie_key(a, a.pos[a.order[a.n_mac + i]]) : kNoTie;
   const unsigned same = __match_any_sync(kFull, key);
@@ -657,22 +699,13 @@ __device__ void count_tie(const LpArgs &a, uint32_t i, bool in) {  // a warp; in
     const unsigned long long was = atomicCAS(a.tie_key + h, kNoTie, key);
     if (was != kNoTie && was != key) continue;
     const uint32_t n = (uint32_t)__popc(same), had = atomicAdd(a.tie_count + h, n);
-    if (had + n < a.tie_least) return;
-    const uint32_t add = had >= a.tie_least ? n : had + n, ties = atomicAdd(&a.st->ties, add);
-    if (ties < a.tie_limit && ties + add >= a.tie_limit) {
-      a.st->tied = 1u;
-      cudaGraphSetConditional(a.windows, 1u);
-    }
+    if (had + n >= a.tie_least) atomicAdd(&a.st->ties, had >= a.tie_least ? n : had + n);
     return;
   }
 }
 
 __global__ void __launch_bounds__(256) k_lp_segments(const LpArgs a) {
   const int lane = threadIdx.x & 31;
-  const uint32_t units = a.n - a.n_mac;
-  if (a.tie_limit)
-    for (uint32_t i0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; i0 < units; i0 += gridDim.x * blockDim.x)
-      count_tie(a, i0 + lane, i0 + lane < units);
   const int nseg = a.SW * a.H;
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nseg; i += (gridDim.x * blockDim.x) >> 5) {
     const unsigned m = __ballot_sync(kFull, a.own[(size_t)32 * i + lane] == kNone);
@@ -1232,14 +1265,15 @@ __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_units(c
 // reference's field, 5k cells, 300 iterations 1297 -> 31 (48), 30k with macros,
 // 100 iterations, 4568 -> 290 (285).  Bound by the list kernel: two dependent
 // passes over the rows, 20 us a window, and two launches.
-// The rule (lp_build_graph, k_lp_pending): ties (cells of a target that has
-// tie_least or more) are at least 1/64 of the unit cells and 1/5 of those left
-// over by k_lp_near, or, where that isn't tried, 1/10 of all.  The line lies
+// The rule (k_lp_pending): ties (cells of a target that has 1/64 of all or more)
+// are at least 1/64 of the unit cells and 1/5 of those left over by k_lp_near; or,
+// where that isn't tried, 1/10 of a sample (sample_ties).  The line lies
 // where both ways take about as long: 200k cells, 2 % in a corner 29 -> 18 ms,
 // 30k 2.8 -> 2.6; 16 spots of 30k cells 23 -> 3.4; but a wide pile of 30k cells
 // of which 10 % are on one spot would take 14 -> 70 (40 %: 86 -> 64): its other
-// cells use up their lists too.  A loop that is not entered costs some 12 us: it
-// stands inside the if node where there is one; 3k spread cells 135 -> 150 us.
+// cells use up their lists too.  A loop that is not entered costs some 12 us, so
+// it stands inside the if node where there is one, and few cells have a second
+// graph for it (a run's first such checkpoint, and each call, is launched twice).
 
 // A CTA per cell of the window: the open sites of least cost, in order.
 __global__ void __launch_bounds__(kUnitWarps * 32, 32 / kUnitWarps) k_lp_lists(const LpArgs a) {
@@ -1521,16 +1555,15 @@ __global__ void __launch_bounds__(kSumThreads) k_lp_finish(const LpArgs a) {
 
 }  // namespace
 
-LpGraph::~LpGraph() {
+void LpGraph::clear() {
   if (exec) cudaGraphExecDestroy(exec);
   if (graph) cudaGraphDestroy(graph);
+  exec = nullptr;
+  graph = nullptr;
 }
 
-cudaError_t lp_build_graph(LpArgs a, LpGraph &g) {
-  if (g.exec) cudaGraphExecDestroy(g.exec);
-  if (g.graph) cudaGraphDestroy(g.graph);
-  g.exec = nullptr;
-  g.graph = nullptr;
+cudaError_t lp_build_graph(LpArgs a, LpGraph &g, bool windows) {
+  g.clear();
   cudaError_t e;
   cudaGraph_t graph = nullptr;
   if ((e = cudaGraphCreate(&graph, 0)) != cudaSuccess) return e;
@@ -1581,8 +1614,9 @@ cudaError_t lp_build_graph(LpArgs a, LpGraph &g) {
   // Few cells: targets that differ by less than a tenth of a site crowd like equal
   // ones (5k in a pile of sigma 0.1: 13.7 -> 7.0 ms, but 60k 135 -> 230).
   a.tie_scale = at_once ? 64.0f : 16.0f;
-  a.tie_least = units / (at_once ? 64 : 32) > 32 ? units / (at_once ? 64 : 32) : 32;
-  a.tie_limit = at_once ? 0 : units / 10 > 32 ? units / 10 : 32;
+  a.tie_least = units / 64;
+  a.tie_few = units && !at_once;
+  a.tie_loop = at_once || windows;
   Chain top{graph};
   // The loop over the windows of unit cells, entered when some kernel of the
   // chain before it has set its handle.
@@ -1595,7 +1629,7 @@ cudaError_t lp_build_graph(LpArgs a, LpGraph &g) {
   };
   if (a.n_mac && (e = handle(&a.handle, top, 1)) != cudaSuccess) return e;
   if (at_once && (e = handle(&a.many, top, 0)) != cudaSuccess) return e;
-  if (units && !at_once && (e = handle(&a.windows, top, 0)) != cudaSuccess) return e;
+  if (units && !at_once && windows && (e = handle(&a.windows, top, 0)) != cudaSuccess) return e;
   if ((e = add(top, k_lp_init, site_grid, 256)) != cudaSuccess) return e;
   if (a.n_mac) {
     Chain body{};
@@ -1607,7 +1641,7 @@ cudaError_t lp_build_graph(LpArgs a, LpGraph &g) {
   if ((e = add(top, k_lp_segments, site_grid, 256)) != cudaSuccess) return e;
   if (units && !at_once) {
     if ((e = add(top, k_lp_units<true>, units, kUnitWarps * 32)) != cudaSuccess) return e;
-    if ((e = add_windows(top)) != cudaSuccess) return e;
+    if (windows && (e = add_windows(top)) != cudaSuccess) return e;
   } else if (units) {
     const uint32_t chunks = (uint32_t)lp_chunks(units);
     if ((e = add(top, k_lp_near, (units + 7) / 8, 256)) != cudaSuccess) return e;

@@ -21,6 +21,9 @@ constexpr int kLpRingMax = 64;
 // Sites kept of a unit cell's search.
 constexpr int kLpCand = 16;
 
+// Status of a graph without windows whose unit cells need them.
+constexpr int32_t kLpTied = 3;
+
 // State of one legalisation in flight, in device memory.
 struct LpState {
   uint32_t base;       // macros [0, base) have their final anchors
@@ -34,7 +37,7 @@ struct LpState {
   uint32_t ties;       // unit cells that share a target with tie_least or more
   uint32_t tied;       // too many do: the unit cells are placed in windows
   uint32_t wbase;      // unit cells [0, wbase) have been placed in windows
-  int32_t status;      // 0 ok, 1 no free site for some cell, 2 round cap, 4 cancelled
+  int32_t status;      // 0 ok, 1 no free site for some cell, 2 round cap, kLpTied, 4 cancelled
 };
 
 // A block that a macro gave up in a round.
@@ -68,7 +71,8 @@ struct LpArgs {
   uint32_t tie_mask;       // lp_tie_entries - 1
   float tie_scale;         // filled in by lp_build_graph, like the next two: squares per site that tell targets apart
   uint32_t tie_least;      // cells of one target from which they count as ties
-  uint32_t tie_limit;      // ties from which all unit cells are placed in windows, 0: decided later
+  bool tie_few;            // decided before the first pass, from a sample, without the table
+  bool tie_loop;           // the graph has the loop over them (else the status says that they are needed)
   int32_t *list;           // [kUnitWindow][kLpRingMax] sites of least cost of the window's cells
   int32_t *list_len;       // [kUnitWindow] how many
   LpState *st;
@@ -105,17 +109,19 @@ inline bool legalize_supported(int W, int H) { return W > 0 && H > 0 && W <= 409
 
 // A legalisation as one CUDA graph: initialisation, a device-side while
 // loop over the macro rounds (when there are macros), the unit cells (all at
-// once and the few left over, or, where too many are, all in order: an if
-// node; or, where many share a target, in windows: a while node), the
-// displacement sum.  Built once per slot and problem load; launched per
+// once and the few left over, or, where too many are, all in order or, where
+// many share a target, in windows: an if node with a while node in it; few
+// cells all in order, or in windows), the displacement sum.  Built once per slot and problem load; launched per
 // checkpoint.
 struct LpGraph {
   cudaGraphExec_t exec = nullptr;
   cudaGraph_t graph = nullptr;
-  ~LpGraph();
+  void clear();
+  ~LpGraph() { clear(); }
 };
 
 // Builds the graph for args `a` (the handles are filled in).
-cudaError_t lp_build_graph(LpArgs a, LpGraph &g);
+// windows: also where that costs a conditional node of its own (few cells).
+cudaError_t lp_build_graph(LpArgs a, LpGraph &g, bool windows);
 
 }  // namespace eplace
